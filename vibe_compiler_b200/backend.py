@@ -10,6 +10,7 @@ computes as a whole. Every method calls the device library; nothing is computed 
 from __future__ import annotations
 
 import ctypes as C
+import struct
 import weakref
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
@@ -29,6 +30,18 @@ class WB200Error(RuntimeError):
 
 _TORCH_FORMATS = {torch.bfloat16: abi.BF16, torch.float16: abi.F16, torch.float32: abi.F32}
 FORMAT_BYTES = {abi.F16: 2, abi.BF16: 2, abi.F32: 4}
+
+# The request structures of the region calls, filled by one struct.pack each: a decode step or a short prompt takes less
+# time on the device than one assignment per ctypes field takes here (attention_fd 13 us of Python per call, now 3).
+_ATTENTION_PACK = struct.Struct("=6I4Bf3q8Q2I").pack
+_GEMM_PACK = struct.Struct("=3I6B6x5Q").pack
+assert len(_ATTENTION_PACK(*[0] * 24)) == C.sizeof(abi.AttentionParams) and len(_GEMM_PACK(*[0] * 14)) == C.sizeof(abi.GemmEpilogueParams)
+
+
+def _current_stream() -> int:
+    """The handle of the current device's current stream, without the stream object torch.cuda.current_stream() builds
+    (about 5 us per call)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 @dataclass
@@ -280,30 +293,24 @@ class B200TargetModelBackend:
 
     # ------------------------------------------------------------------ region level
     def _attention_params(self, q, k, v, out, scale, causal, zero_fully_masked, query_start, key_start, key_end,
-                          lse, row_max, row_sum, stream) -> abi.AttentionParams:
-        for name, tensor in (("q", q), ("k", k), ("v", v)):
-            if tensor.dim() != 4 or not tensor.is_contiguous():
-                raise ValueError(f"{name} must be a contiguous [batch, heads, length, head_dim] tensor")
-        if q.dtype not in _TORCH_FORMATS or k.dtype != q.dtype or v.dtype != q.dtype or out.dtype != q.dtype:
+                          lse, row_max, row_sum, stream, token_major_out=False) -> abi.AttentionParams:
+        dtype, on_device = q.dtype, q.is_cuda
+        if not (q.dim() == 4 == k.dim() == v.dim() and q.is_contiguous() and k.is_contiguous() and v.is_contiguous()):
+            name = next(n for n, t in (("q", q), ("k", k), ("v", v)) if t.dim() != 4 or not t.is_contiguous())
+            raise ValueError(f"{name} must be a contiguous [batch, heads, length, head_dim] tensor")
+        if dtype not in _TORCH_FORMATS or k.dtype != dtype or v.dtype != dtype or out.dtype != dtype:
             raise ValueError("q, k, v and out must share one of bfloat16 / float16 / float32")
-        on_device = q.is_cuda
-        for tensor in (k, v, out, lse, row_max, row_sum):
-            if tensor is not None and tensor.is_cuda != on_device:
-                raise ValueError("all attention buffers must live in the same memory space")
-        p = abi.AttentionParams()
-        p.batch, p.q_heads, p.q_len, p.head_dim = q.shape
-        p.kv_heads, p.kv_len = k.shape[1], k.shape[2]
-        p.format = _TORCH_FORMATS[q.dtype]
-        p.causal, p.zero_fully_masked = int(causal), int(zero_fully_masked)
-        p.memory = abi.MEM_DEVICE if on_device else abi.MEM_HOST
-        p.scale = float(scale)
-        p.query_start, p.key_start, p.key_end = int(query_start), int(key_start), int(key_end)
-        p.q, p.k, p.v, p.out = q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr()
-        p.lse = lse.data_ptr() if lse is not None else None
-        p.row_max = row_max.data_ptr() if row_max is not None else None
-        p.row_sum = row_sum.data_ptr() if row_sum is not None else None
-        p.stream = stream
-        return p
+        if k.is_cuda != on_device or v.is_cuda != on_device or out.is_cuda != on_device or \
+                any(t is not None and t.is_cuda != on_device for t in (lse, row_max, row_sum)):
+            raise ValueError("all attention buffers must live in the same memory space")
+        batch, q_heads, q_len, head_dim = q.shape
+        _, kv_heads, kv_len, _ = k.shape
+        return abi.AttentionParams.from_buffer_copy(_ATTENTION_PACK(
+            batch, q_heads, kv_heads, q_len, kv_len, head_dim, _TORCH_FORMATS[dtype], bool(causal), bool(zero_fully_masked),
+            abi.MEM_DEVICE if on_device else abi.MEM_HOST, scale, int(query_start), int(key_start), int(key_end),
+            q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if lse is not None else 0,
+            row_max.data_ptr() if row_max is not None else 0, row_sum.data_ptr() if row_sum is not None else 0, stream or 0,
+            abi.OUT_TOKEN_MAJOR if token_major_out else abi.OUT_HEAD_MAJOR, 0))
 
     def attention_fa(self, q, k, v, scale: float, causal: bool = False, *, out=None, lse=None, row_max=None,
                      row_sum=None, zero_fully_masked: bool = False, query_start: int = 0, key_start: int = 0,
@@ -314,10 +321,9 @@ class B200TargetModelBackend:
             out = torch.empty(q.shape[0], q.shape[2], q.shape[1], q.shape[3], dtype=q.dtype, device=q.device) if token_major_out \
                 else torch.empty_like(q)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream if q.is_cuda else 0
+            stream = _current_stream() if q.is_cuda else 0
         p = self._attention_params(q, k, v, out, scale, causal, zero_fully_masked, query_start, key_start, key_end,
-                                   lse, row_max, row_sum, stream)
-        p.out_layout = abi.OUT_TOKEN_MAJOR if token_major_out else abi.OUT_HEAD_MAJOR
+                                   lse, row_max, row_sum, stream, token_major_out)
         self._check(self._lib.wb200_attention_fa(self._handle, C.byref(p)))
         return out
 
@@ -327,7 +333,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(q)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream if q.is_cuda else 0
+            stream = _current_stream() if q.is_cuda else 0
         p = self._attention_params(q, k, v, out, scale, causal, zero_fully_masked, query_start, key_start, key_end,
                                    lse, row_max, row_sum, stream)
         self._check(self._lib.wb200_attention_fd(self._handle, C.byref(p), kv_splits))
@@ -344,7 +350,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(q)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         p = self._attention_params(q, k, v, out, scale, False, zero_fully_masked, 0, 0, 0, lse, None, None, stream)
         self._check(self._lib.wb200_attention_fd_static(self._handle, C.byref(p), kv_splits))
         return out
@@ -355,7 +361,7 @@ class B200TargetModelBackend:
         if state is None:
             state = torch.empty(q.shape[0], q.shape[1], q.shape[3] + 2, dtype=torch.float32, device=q.device)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream if q.is_cuda else 0
+            stream = _current_stream() if q.is_cuda else 0
         dummy_out = q  # not written
         p = self._attention_params(q, k, v, dummy_out, scale, False, False, 0, key_start, key_end, None, None, None, stream)
         self._check(self._lib.wb200_attention_fd_partial(self._handle, C.byref(p), kv_splits, state.data_ptr()))
@@ -371,7 +377,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(q)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         p = self._attention_params(q, k, v, out, scale, False, False, 0, 0, 0, lse, None, None, stream)
         x = abi.FdExchange()
         x.rank, x.world = rank, len(peer_pointers)
@@ -406,7 +412,7 @@ class B200TargetModelBackend:
         the sums there instead of in place; `residual`: this rank's copy of a tensor (identical on every rank) that is
         added to the sums before the store."""
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         x = abi.SwitchSumParams()
         x.rank, x.world = rank, len(signal_pointers)
         x.multicast, x.elements, x.format, x.blocks = multicast_pointer, elements, _TORCH_FORMATS[dtype], blocks
@@ -423,7 +429,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(like_q)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream if like_q.is_cuda else 0
+            stream = _current_stream() if like_q.is_cuda else 0
         p = abi.AttentionParams()
         p.batch, p.q_heads, p.q_len, p.head_dim = like_q.shape
         p.kv_heads, p.kv_len = 1, 1
@@ -448,16 +454,11 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty(m, n // 2 if epilogue == abi.EPI_SWIGLU else n, dtype=out_dtype, device=a.device)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream if a.is_cuda else 0
-        p = abi.GemmEpilogueParams()
-        p.m, p.n, p.k = m, n, k
-        p.in_format, p.out_format = _TORCH_FORMATS[a.dtype], _TORCH_FORMATS[out.dtype]
-        p.lhs_orientation, p.rhs_orientation = int(lhs_transposed), int(rhs_transposed)
-        p.epilogue = epilogue
-        p.memory = abi.MEM_DEVICE if a.is_cuda else abi.MEM_HOST
-        p.a, p.b, p.out = a.data_ptr(), b.data_ptr(), out.data_ptr()
-        p.bias = bias.data_ptr() if bias is not None else None
-        p.stream = stream
+            stream = _current_stream() if a.is_cuda else 0
+        p = abi.GemmEpilogueParams.from_buffer_copy(_GEMM_PACK(
+            m, n, k, _TORCH_FORMATS[a.dtype], _TORCH_FORMATS[out.dtype], bool(lhs_transposed), bool(rhs_transposed), epilogue,
+            abi.MEM_DEVICE if a.is_cuda else abi.MEM_HOST, a.data_ptr(), b.data_ptr(), bias.data_ptr() if bias is not None else 0,
+            out.data_ptr(), stream or 0))
         self._check(self._lib.wb200_gemm_epilogue(self._handle, C.byref(p)))
         return out
 
@@ -467,7 +468,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(x)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         rows = x.numel() // x.shape[-1]
         self._check(self._lib.wb200_rmsnorm(self._handle, _TORCH_FORMATS[x.dtype], x.data_ptr(), gamma.data_ptr(), out.data_ptr(),
                                             rows, x.shape[-1], float(eps), stream))
@@ -477,7 +478,7 @@ class B200TargetModelBackend:
                    position_offset: int = 0, stream: Optional[int] = None):
         """Token-major projection rows [q heads | k heads | v heads] -> head-major Q, K (rotary applied) and V."""
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         q = torch.empty(batch, q_heads, seq, head_dim, dtype=qkv.dtype, device=qkv.device)
         k = torch.empty(batch, kv_heads, seq, head_dim, dtype=qkv.dtype, device=qkv.device)
         v = torch.empty_like(k)
@@ -489,7 +490,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(a)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         self._check(self._lib.wb200_residual_add(self._handle, _TORCH_FORMATS[a.dtype], a.data_ptr(), b.data_ptr(), out.data_ptr(),
                                                  a.numel(), stream))
         return out
@@ -523,7 +524,7 @@ class B200TargetModelBackend:
         if out is None:
             out = torch.empty_like(x)
         if stream is None:
-            stream = torch.cuda.current_stream().cuda_stream
+            stream = _current_stream()
         p.x, p.out = x.data_ptr(), out.data_ptr()
         p.norm1, p.wqkv, p.wo, p.norm2, p.wgu, p.wdown = (t.data_ptr() for t in (norm1, wqkv, wo, norm2, wgu, wdown))
         p.workspace, p.workspace_bytes, p.stream = workspace.data_ptr(), workspace.numel(), stream

@@ -154,6 +154,20 @@ wb200_status run_fa_host_pipelined(wb200_backend *backend, const wb200_attention
   return read_device_status(backend, compute, nullptr);
 }
 
+// The scratch of a decode launch: the split records (slot 7) and the arrival counters of its (batch, kv head) units
+// (slot 11, at least 16 Ki of them so that batches rarely outgrow it).
+wb200_status decode_scratch(wb200_backend *backend, const AttentionArgs &a, FdPlan plan, float **partials, unsigned int **arrivals) {
+  void *records, *counters;
+  wb200_status st = backend->buffer(7, fd_partial_floats(a, plan.records) * sizeof(float), &records);
+  if (st != WB200_OK) return st;
+  size_t units = static_cast<size_t>(a.batch) * a.kv_heads;
+  if (units < 16384) units = 16384;
+  if ((st = backend->zeroed_buffer(11, units * sizeof(unsigned int), &counters)) != WB200_OK) return st;
+  *partials = static_cast<float *>(records);
+  *arrivals = static_cast<unsigned int *>(counters);
+  return WB200_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -184,12 +198,13 @@ wb200_status wb200_attention_fd(wb200_backend *backend, const wb200_attention_pa
   if (!attention_fd_supports(a) && p->memory == WB200_MEM_DEVICE)
     return fail(WB200_ERR_UNSUPPORTED, "flash-decoding kernel takes f16/bf16 storage, head_dim 128, group size <= 16");
   DeviceGuard guard(backend->device);
-  const uint32_t splits = kv_splits ? kv_splits : fd_choose_splits(a, backend->sm_count);
-  void *partials;
-  if ((st = backend->buffer(7, fd_partial_floats(a, splits) * sizeof(float), &partials)) != WB200_OK) return st;
+  const FdPlan plan = kv_splits ? FdPlan{1u, kv_splits} : fd_choose_plan(a, backend->sm_count);
+  float *partials;
+  unsigned int *arrivals;
+  if ((st = decode_scratch(backend, a, plan, &partials, &arrivals)) != WB200_OK) return st;
   if (p->memory == WB200_MEM_DEVICE) {
-    st = launch_attention_fd(a, splits, static_cast<float *>(partials), 1, nullptr, static_cast<cudaStream_t>(p->stream));
-    if (st == WB200_OK) backend->launches += 2;
+    st = launch_attention_fd(a, plan, partials, arrivals, nullptr, static_cast<cudaStream_t>(p->stream));
+    if (st == WB200_OK) backend->launches += 1;
     return st;
   }
   StagedAttention s;
@@ -197,8 +212,8 @@ wb200_status wb200_attention_fd(wb200_backend *backend, const wb200_attention_pa
   if ((st = stage_attention_inputs(backend, p, &s, true)) != WB200_OK) return st;
   if (!attention_fd_supports(s.args))
     return fail(WB200_ERR_UNSUPPORTED, "flash-decoding kernel takes f16/bf16 storage, head_dim 128, group size <= 16");
-  if ((st = launch_attention_fd(s.args, splits, static_cast<float *>(partials), 1, nullptr, backend->stream)) != WB200_OK) return st;
-  backend->launches += 2;
+  if ((st = launch_attention_fd(s.args, plan, partials, arrivals, nullptr, backend->stream)) != WB200_OK) return st;
+  backend->launches += 1;
   return return_attention_outputs(backend, p, s);
 }
 
@@ -209,13 +224,14 @@ wb200_status wb200_attention_fd_partial(wb200_backend *backend, const wb200_atte
   wb200_status st = make_attention_args(p, &a);
   if (st != WB200_OK) return st;
   DeviceGuard guard(backend->device);
-  const uint32_t splits = kv_splits ? kv_splits : fd_choose_splits(a, backend->sm_count);
-  void *partials;
-  if ((st = backend->buffer(7, fd_partial_floats(a, splits) * sizeof(float), &partials)) != WB200_OK) return st;
+  const FdPlan plan = kv_splits ? FdPlan{1u, kv_splits} : fd_choose_plan(a, backend->sm_count);
+  float *partials;
+  unsigned int *arrivals;
+  if ((st = decode_scratch(backend, a, plan, &partials, &arrivals)) != WB200_OK) return st;
   const size_t state_bytes = static_cast<size_t>(p->batch) * p->q_heads * (p->head_dim + 2) * sizeof(float);
   if (p->memory == WB200_MEM_DEVICE) {
-    st = launch_attention_fd(a, splits, static_cast<float *>(partials), 0, state_out, static_cast<cudaStream_t>(p->stream));
-    if (st == WB200_OK) backend->launches += 2;
+    st = launch_attention_fd(a, plan, partials, arrivals, state_out, static_cast<cudaStream_t>(p->stream));
+    if (st == WB200_OK) backend->launches += 1;
     return st;
   }
   StagedAttention s;
@@ -225,8 +241,8 @@ wb200_status wb200_attention_fd_partial(wb200_backend *backend, const wb200_atte
   if ((st = stage_attention_inputs(backend, &inputs_only, &s, false)) != WB200_OK) return st;
   void *d_state;
   if ((st = backend->buffer(8, state_bytes, &d_state)) != WB200_OK) return st;
-  if ((st = launch_attention_fd(s.args, splits, static_cast<float *>(partials), 0, static_cast<float *>(d_state), backend->stream)) != WB200_OK) return st;
-  backend->launches += 2;
+  if ((st = launch_attention_fd(s.args, plan, partials, arrivals, static_cast<float *>(d_state), backend->stream)) != WB200_OK) return st;
+  backend->launches += 1;
   WB200_CUDA_CHECK(cudaMemcpyAsync(state_out, d_state, state_bytes, cudaMemcpyDeviceToHost, backend->stream));
   return read_device_status(backend, backend->stream, nullptr);
 }
@@ -249,17 +265,15 @@ wb200_status wb200_attention_fd_exchange(wb200_backend *backend, const wb200_att
   wb200_status st = make_attention_args(p, &a);
   if (st != WB200_OK) return st;
   DeviceGuard guard(backend->device);
-  const uint32_t splits = kv_splits ? kv_splits : fd_choose_splits(a, backend->sm_count);
-  void *partials;
-  if ((st = backend->buffer(7, fd_partial_floats(a, splits) * sizeof(float), &partials)) != WB200_OK) return st;
+  const FdPlan plan = kv_splits ? FdPlan{1u, kv_splits} : fd_choose_plan(a, backend->sm_count);
+  float *partials;
+  unsigned int *arrivals;
+  if ((st = decode_scratch(backend, a, plan, &partials, &arrivals)) != WB200_OK) return st;
   // One launch: the last stage-1 CTA of every (batch, kv head) folds, exchanges and merges. WB200_FD_EXCHANGE_FUSED=0 in
   // the environment keeps the tail as a second launch.
   static const bool fused = []() { const char *env = getenv("WB200_FD_EXCHANGE_FUSED"); return !(env && env[0] == '0'); }();
-  void *arrivals = nullptr;
-  if (fused && (st = backend->zeroed_buffer(11, static_cast<size_t>(a.batch) * a.kv_heads * sizeof(unsigned int), &arrivals)) != WB200_OK) return st;
-  st = launch_attention_fd_exchange(a, splits, static_cast<float *>(partials), static_cast<int>(x->rank), static_cast<int>(x->world),
-                                    x->peer_buffers, x->epoch, static_cast<unsigned int *>(arrivals), backend->d_status,
-                                    static_cast<cudaStream_t>(p->stream));
+  st = launch_attention_fd_exchange(a, plan, partials, static_cast<int>(x->rank), static_cast<int>(x->world), x->peer_buffers, x->epoch,
+                                    fused ? arrivals : nullptr, backend->d_status, static_cast<cudaStream_t>(p->stream));
   if (st == WB200_OK) backend->launches += fused ? 1 : 2;
   return st;
 }

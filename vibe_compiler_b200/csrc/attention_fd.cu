@@ -8,15 +8,22 @@
 // exp is the target's ExpLp, exp2(x * log2e) in f32
 // (lib/Wafer/Simulator/Reference/ManagedReferenceTargetModel.cpp:265-270).
 //
-// Stage 1 (fd_partial_kernel): one CTA per (split, kv head, batch). Each of the 4 warps streams its
-// own contiguous quarter of the CTA's KV interval through a private 3-deep cp.async ring of 16-row
+// fd_partial_kernel: the keys of a (batch, kv head) are cut over `cluster * splits` CTAs. Each of a CTA's 4 warps streams
+// its own contiguous quarter of the CTA's KV interval through a private 3-deep cp.async ring of 16-row
 // tiles (128-bit coalesced copies, XOR-swizzled rows), computes S = Q K^T and acc += P V with
 // mma.sync m16n8k16 on the group's query heads (rows padded to 16) and carries (m, l, acc) in
-// registers. Warps then left-fold their states in ascending KV order through shared memory and the
-// CTA writes one (acc[D], m, l) record. Stage 2 (fd_combine_kernel) left-folds the records of all
-// splits in ascending order and finalizes. The kernel is HBM-bound: algorithmic bytes per launch
-// are the K and V bytes of the visible keys, read exactly once.
+// registers. Warps then fold their states in ascending KV order through shared memory; the CTAs of a cluster hand
+// theirs to the cluster's first CTA through distributed shared memory. With one cluster per (batch, kv head) that CTA
+// finalizes; otherwise it writes one (acc[D], m, l) record, and the cluster that finishes last folds the records of the
+// group's query heads and finalizes. A decode step is one launch either way.
+// The kernel is HBM-bound for long caches: algorithmic bytes per launch are the K and V bytes of the visible keys, read
+// exactly once. Short ones are a latency chain (launch, first tile, merge), which the cluster merge shortens: no record
+// goes through global memory and nothing is fenced or counted.
+// Measured per launch (bf16, launches replayed back to back as a graph, caches rotated through 400 MB), two launches with a
+// combine kernel -> this form: 28/4 heads, 1 x 1537 keys 8.3 -> 6.7 us; 32/8 heads, 8 x 4000 keys 28.7 -> 25.1 us (20.0 at the
+// copy rate), 33 x 900 keys 29.1 -> 20.8 us (18.6), 64 x 333 keys 30.0 -> 17.0 us (13.3), 1 x 1 Mi keys 629 -> 600 us.
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -27,8 +34,12 @@ constexpr int kWarps = 4;
 constexpr int kStagesFd = 3;
 constexpr int kTileBytes = kTileRows * kD * 2;  // 4 KiB for K, same for V
 constexpr int kRecord = kD + 2;    // acc[D], m, l
-constexpr int kQBytes = 16 * kD * 2;
-constexpr int kFdSmemBytes = kWarps * kStagesFd * 2 * kTileBytes + kQBytes;
+constexpr int kSmemRecord = kD + 4;   // the same in shared memory, rows 16-byte aligned
+constexpr int kMaxGroup = 16;      // query heads per KV head
+constexpr int kFdSmemBytes = kWarps * kStagesFd * 2 * kTileBytes;
+// The rings are reused for the warps' records and, behind them, the CTA's merged record.
+constexpr int kMergedOffset = kWarps * kMaxGroup * kSmemRecord;   // floats
+static_assert((kMergedOffset + kMaxGroup * kSmemRecord) * 4 <= kFdSmemBytes, "merge records must fit the rings");
 
 __device__ __forceinline__ float exp_lp(float x) { return exp2f(x * 0x1.715476p+0f); }
 
@@ -82,14 +93,18 @@ struct FdParams {
   int batch, q_heads, kv_heads, group;
   int kv_len;         // rows physically present per (batch, kv head)
   int kv_visible;     // keys [0, kv_visible) are visible
-  int splits, rows_per_split, rows_per_warp;
+  int splits;         // records per query head = clusters per (batch, kv head)
+  int cluster;        // CTAs per cluster
+  int rows_per_cta, rows_per_warp;
   float scale;
   const uint16_t *q, *k, *v;
   float *partials;    // [batch, q_heads, splits, kRecord]
 };
 
-// Tail of the sequence-sharded decode step, run by the last CTA of a (batch, kv head) to finish stage 1 (see
-// fd_exchange_rows): the exchange buffers of all ranks and this rank's epoch words.
+// What the last CTA of a (batch, kv head) to finish stage 1 does with the records: fold, then write the outputs or the
+// un-finalized state (kTailLocal), or exchange the state with the other ranks first (kTailExchange, fd_exchange_rows: the
+// exchange buffers of all ranks and this rank's epoch words).
+enum { kTailNone = 0, kTailLocal = 1, kTailExchange = 2 };
 constexpr int kMaxExchangeRanks = 16;
 struct FdTailParams {
   int rank, world;
@@ -99,49 +114,130 @@ struct FdTailParams {
   int out_format, zero_fully_masked;
   void *out;
   float *lse, *row_max, *row_sum;
+  float *state_out;                  // kTailLocal: non-null = write the merged state here instead of out / lse
   int *status;
 };
 template <int kRowsAtOnce>
 __device__ void fd_exchange_rows(const FdTailParams &x, const float *records, int splits, int first_row, int row_count, int rows_total);
 
+__device__ __forceinline__ void fd_merge_right(float &m, float &l, float4 &a, float m_right, float l_right, const float4 &a_right) {
+  const float m_new = fmaxf(m, m_right);
+  const float m_exp = (m_new == -INFINITY) ? 0.f : m_new;
+  const float scale_left = exp_lp(m - m_exp), scale_right = exp_lp(m_right - m_exp);
+  l = l * scale_left + l_right * scale_right;
+  a.x = a.x * scale_left + a_right.x * scale_right;
+  a.y = a.y * scale_left + a_right.y * scale_right;
+  a.z = a.z * scale_left + a_right.z * scale_right;
+  a.w = a.w * scale_left + a_right.w * scale_right;
+  m = m_new;
+}
+// Four consecutive floats of a record (records are 130 floats long: 8-byte, not 16-byte, aligned), read past L1.
+__device__ __forceinline__ float4 ldcg_quad(const float *address) {
+  const float2 lo = __ldcg(reinterpret_cast<const float2 *>(address)), hi = __ldcg(reinterpret_cast<const float2 *>(address + 2));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+// Fold of a row's split records by one warp (lane: four head dimensions). The common exponent reference of all records is
+// their maximum, so the weights come from one pass over the (m, l) pairs with a lane per record, and the accumulators are
+// summed in ascending record order with independent loads (eight records in flight). Against the pairwise left fold this
+// takes the chain of exponentials out of the loop; a one-sequence decode has the fold on its critical path.
+__device__ __forceinline__ void fd_fold_records(const float *rec, int records, int lane, float &m, float &l, float4 &a) {
+  float top = -INFINITY;
+  for (int i = lane; i < records; i += 32) top = fmaxf(top, __ldcg(rec + static_cast<size_t>(i) * kRecord + kD));
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+  const float m_exp = (top == -INFINITY) ? 0.f : top;
+  float sum = 0.f;
+  a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int base = 0; base < records; base += 32) {
+    float weight = 0.f;
+    if (base + lane < records) {
+      const float2 ml = __ldcg(reinterpret_cast<const float2 *>(rec + static_cast<size_t>(base + lane) * kRecord + kD));
+      weight = exp_lp(ml.x - m_exp);
+      sum = fmaf(ml.y, weight, sum);
+    }
+    const int count = min(32, records - base);
+    const float *src = rec + static_cast<size_t>(base) * kRecord + 4 * lane;
+    auto add = [&](int i, const float4 &right) {
+      const float w = __shfl_sync(0xffffffffu, weight, i);
+      a.x = fmaf(right.x, w, a.x); a.y = fmaf(right.y, w, a.y);
+      a.z = fmaf(right.z, w, a.z); a.w = fmaf(right.w, w, a.w);
+    };
+    int i = 0;
+    for (; i + 8 <= count; i += 8) {
+      float4 right[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) right[u] = ldcg_quad(src + static_cast<size_t>(i + u) * kRecord);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) add(i + u, right[u]);
+    }
+    for (; i < count; ++i) add(i, ldcg_quad(src + static_cast<size_t>(i) * kRecord));
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  m = top;
+  l = sum;
+}
+// Finalizes a row: out = acc / l with one narrowing, log-sum-exp and the carried state; lane = four head dimensions.
+__device__ __forceinline__ void fd_write_row(const FdTailParams &x, int row, int lane, float m, float l, const float4 &a) {
+  float coefficient = 1.0f / l;
+  if (x.zero_fully_masked && l == 0.f) coefficient = 0.f;
+  const float value[4] = {a.x * coefficient, a.y * coefficient, a.z * coefficient, a.w * coefficient};
+  if (x.out_format == WB200_F32) {
+    *(reinterpret_cast<float4 *>(x.out) + static_cast<size_t>(row) * (kD / 4) + lane) = make_float4(value[0], value[1], value[2], value[3]);
+  } else {
+    uint32_t bits[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bits[i] = narrow_bits(value[i], x.out_format);
+    if ((reinterpret_cast<uintptr_t>(x.out) & 7u) == 0) {
+      *(reinterpret_cast<uint2 *>(x.out) + static_cast<size_t>(row) * (kD / 4) + lane) = make_uint2(bits[0] | (bits[1] << 16), bits[2] | (bits[3] << 16));
+    } else {
+      uint16_t *dst = reinterpret_cast<uint16_t *>(x.out) + static_cast<size_t>(row) * kD + 4 * lane;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dst[i] = static_cast<uint16_t>(bits[i]);
+    }
+  }
+  if (lane == 0) {
+    if (x.lse) x.lse[row] = (l == 0.f) ? -INFINITY : m + logf(l);
+    if (x.row_max) x.row_max[row] = m;
+    if (x.row_sum) x.row_sum[row] = l;
+  }
+}
+// The complete state of a row: un-finalized to `state_out`, or finalized.
+__device__ __forceinline__ void fd_deliver_row(const FdTailParams &x, int row, int lane, float m, float l, const float4 &a) {
+  if (!x.state_out) { fd_write_row(x, row, lane, m, l, a); return; }
+  float *state = x.state_out + static_cast<size_t>(row) * kRecord;
+  state[4 * lane] = a.x; state[4 * lane + 1] = a.y; state[4 * lane + 2] = a.z; state[4 * lane + 3] = a.w;
+  if (lane == 0) { state[kD] = m; state[kD + 1] = l; }
+}
+// Rows [first_row, first_row + row_count) by one CTA, a warp per row.
+__device__ void fd_local_rows(const FdTailParams &x, const float *records, int splits, int first_row, int row_count) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = warp; r < row_count; r += kWarps) {
+    const int row = first_row + r;
+    float m, l;
+    float4 a;
+    fd_fold_records(records + static_cast<size_t>(row) * splits * kRecord, splits, lane, m, l, a);
+    fd_deliver_row(x, row, lane, m, l, a);
+  }
+}
 // Swizzled byte offset of 16-byte chunk `c` of row `r` inside a 16 x 256-byte tile.
 __device__ __forceinline__ uint32_t tile_offset(int r, int c) {
   return static_cast<uint32_t>(r * 256 + ((c ^ (r & 7)) << 4));
 }
 
-template <bool kBf16, bool kTail>
+// kNarrow: groups of at most 8 query heads. Scores are computed with the heads as the MMA rows either way (C fragment: head
+// g, keys 2t, 2t + 1), which is the B fragment of the transposed PV product out^T [d, heads] += V^T P^T: 8 products per
+// 16 keys instead of 16, half the accumulators, and one softmax row per lane instead of two. A CTA's rate is set by the
+// chain of a tile (scores, maximum, exponentials, products), so this is what a cache that does not fill the chip gains from.
+template <bool kBf16, int kTail, bool kNarrow>
 __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdParams p, const FdTailParams tail) {
   extern __shared__ __align__(128) uint8_t smem[];
-  const int split = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  const int hk = blockIdx.y, b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
 
-  uint8_t *q_smem = smem + kWarps * kStagesFd * 2 * kTileBytes;
-  // Stage the group's query rows, zero-padded to 16 rows.
-  {
-    const uint16_t *q_src = p.q + (static_cast<size_t>(b) * p.q_heads + static_cast<size_t>(hk) * p.group) * kD;
-    for (int i = threadIdx.x; i < 16 * kD / 8; i += blockDim.x) {
-      const int row = i / (kD / 8), chunk = i % (kD / 8);
-      uint4 value = make_uint4(0, 0, 0, 0);
-      if (row < p.group) value = *reinterpret_cast<const uint4 *>(q_src + row * kD + chunk * 8);
-      *reinterpret_cast<uint4 *>(q_smem + row * (kD * 2) + chunk * 16) = value;
-    }
-  }
-  __syncthreads();
-  uint32_t q_frag[kD / 16][4];
-#pragma unroll
-  for (int ks = 0; ks < kD / 16; ++ks) {
-    const uint32_t *row_lo = reinterpret_cast<const uint32_t *>(q_smem + g * (kD * 2));
-    const uint32_t *row_hi = reinterpret_cast<const uint32_t *>(q_smem + (g + 8) * (kD * 2));
-    q_frag[ks][0] = row_lo[ks * 8 + t];
-    q_frag[ks][1] = row_hi[ks * 8 + t];
-    q_frag[ks][2] = row_lo[ks * 8 + 4 + t];
-    q_frag[ks][3] = row_hi[ks * 8 + 4 + t];
-  }
-
   // This warp's KV interval.
-  const int split_begin = split * p.rows_per_split;
-  const int warp_begin = split_begin + warp * p.rows_per_warp;
+  const int warp_begin = static_cast<int>(blockIdx.x) * p.rows_per_cta + warp * p.rows_per_warp;
   int warp_end = warp_begin + p.rows_per_warp;
   if (warp_end > p.kv_visible) warp_end = p.kv_visible;
   const int tiles = warp_end > warp_begin ? (warp_end - warp_begin + kTileRows - 1) / kTileRows : 0;
@@ -162,7 +258,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdPara
         const int idx = i * 32 + lane;
         const int r = idx >> 4, c = idx & 15;
         const int row = row0 + r;
-        const bool in_range = row < p.kv_len;
+        const bool in_range = row < warp_end;   // rows behind the visible keys are zero-filled, not read
         const size_t src = static_cast<size_t>(in_range ? row : 0) * kD + c * 8;
         cp_async16(k_dst + tile_offset(r, c), k_base + src, in_range ? 16u : 0u);
         cp_async16(v_dst + tile_offset(r, c), v_base + src, in_range ? 16u : 0u);
@@ -171,26 +267,44 @@ __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdPara
     cp_async_commit();
   };
 
-  float m_run[2] = {-INFINITY, -INFINITY};  // rows g and g + 8
-  float l_run[2] = {0.f, 0.f};              // this lane's share of the row sum
-  float acc[kD / 8][4];
+  constexpr int kHalves = kNarrow ? 1 : 2;        // softmax rows per lane: heads g (and g + 8)
+  constexpr int kAccs = kNarrow ? kD / 16 : kD / 8;   // accumulator fragments: d blocks of 16 x 8 heads, or 16 heads x d blocks of 8
+  float m_run[kHalves], l_run[kHalves];               // l_run: this lane's share of the row sum
 #pragma unroll
-  for (int j = 0; j < kD / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  for (int h = 0; h < kHalves; ++h) { m_run[h] = -INFINITY; l_run[h] = 0.f; }
+  float acc[kAccs][4];
+#pragma unroll
+  for (int j = 0; j < kAccs; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
 
+  pdl_wait();   // everything this kernel reads may come from the kernel before it
 #pragma unroll
-  for (int s = 0; s < kStagesFd - 1; ++s) issue_tile(s, s);
+  for (int s = 0; s < kStagesFd; ++s) issue_tile(s, s);
+  pdl_launch_dependents();
+  // The group's query rows as A fragments, straight from global memory behind the first tiles' copies (rows of the 16 that
+  // the group does not fill are zero).
+  uint32_t q_frag[kD / 16][4];
+  {
+    const uint32_t *q_src = reinterpret_cast<const uint32_t *>(p.q + (static_cast<size_t>(b) * p.q_heads + static_cast<size_t>(hk) * p.group) * kD);
+    const bool lo = g < p.group, hi = g + 8 < p.group;
+    const uint32_t *row_lo = q_src + g * (kD / 2) + t, *row_hi = row_lo + 8 * (kD / 2);
+#pragma unroll
+    for (int ks = 0; ks < kD / 16; ++ks) {
+      q_frag[ks][0] = lo ? row_lo[ks * 8] : 0u;
+      q_frag[ks][1] = hi ? row_hi[ks * 8] : 0u;
+      q_frag[ks][2] = lo ? row_lo[ks * 8 + 4] : 0u;
+      q_frag[ks][3] = hi ? row_hi[ks * 8 + 4] : 0u;
+    }
+  }
 
   for (int tile = 0; tile < tiles; ++tile) {
-    cp_async_wait<kStagesFd - 2>();
+    cp_async_wait<kStagesFd - 1>();
     __syncwarp();
-    issue_tile(tile + kStagesFd - 1, (tile + kStagesFd - 1) % kStagesFd);
-
     const uint32_t k_src = ring_addr + (tile % kStagesFd) * (2 * kTileBytes);
     const uint32_t v_src = k_src + kTileBytes;
     const int row0 = warp_begin + tile * kTileRows;
 
-    // S = Q K^T for 16 keys: two n-tiles of 8 keys.
-    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    // S = Q K^T for 16 keys: two n-tiles of 8 keys, even and odd k-steps accumulated apart (four short chains).
+    float part[2][2][4] = {};
 #pragma unroll
     for (int ks = 0; ks < kD / 16; ++ks) {
       const int mi = lane >> 3;
@@ -198,27 +312,22 @@ __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdPara
       const int c = 2 * ks + (mi & 1);
       uint32_t bfrag[4];
       ldmatrix_x4(k_src + tile_offset(r, c), bfrag);
-      mma_16816<kBf16>(s0, q_frag[ks], bfrag[0], bfrag[1]);
-      mma_16816<kBf16>(s1, q_frag[ks], bfrag[2], bfrag[3]);
+      mma_16816<kBf16>(part[ks & 1][0], q_frag[ks], bfrag[0], bfrag[1]);
+      mma_16816<kBf16>(part[ks & 1][1], q_frag[ks], bfrag[2], bfrag[3]);
     }
     // score region: scale, then mask keys outside the visible interval.
     const int key0 = row0 + 2 * t;
-    float sc[2][4];  // [row half][key 2t, 2t+1, 8+2t, 8+2t+1]
-    sc[0][0] = s0[0] * p.scale; sc[0][1] = s0[1] * p.scale; sc[0][2] = s1[0] * p.scale; sc[0][3] = s1[1] * p.scale;
-    sc[1][0] = s0[2] * p.scale; sc[1][1] = s0[3] * p.scale; sc[1][2] = s1[2] * p.scale; sc[1][3] = s1[3] * p.scale;
+    float alpha[kHalves];
+    float pr[kHalves][4];   // [row half][key 2t, 2t+1, 8+2t, 8+2t+1]
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      if (key0 >= warp_end) sc[h][0] = -INFINITY;
-      if (key0 + 1 >= warp_end) sc[h][1] = -INFINITY;
-      if (key0 + 8 >= warp_end) sc[h][2] = -INFINITY;
-      if (key0 + 9 >= warp_end) sc[h][3] = -INFINITY;
-    }
-    uint32_t p_frag[4];
-    float alpha[2];
-    float pr[2][4];
+    for (int h = 0; h < kHalves; ++h) {
+      float sc[4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      float tile_max = fmaxf(fmaxf(sc[h][0], sc[h][1]), fmaxf(sc[h][2], sc[h][3]));
+      for (int i = 0; i < 4; ++i) {
+        sc[i] = (part[0][i >> 1][2 * h + (i & 1)] + part[1][i >> 1][2 * h + (i & 1)]) * p.scale;
+        if (key0 + (i >> 1) * 8 + (i & 1) >= warp_end) sc[i] = -INFINITY;
+      }
+      float tile_max = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
       tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 1));
       tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, 2));
       const float m_new = fmaxf(tile_max, m_run[h]);
@@ -227,98 +336,162 @@ __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdPara
       float row_sum = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        pr[h][i] = exp_lp(sc[h][i] - m_exp);
+        pr[h][i] = exp_lp(sc[i] - m_exp);
         row_sum += pr[h][i];
       }
       l_run[h] = l_run[h] * alpha[h] + row_sum;
       m_run[h] = m_new;
     }
     // Probabilities are rounded to the storage type of V at the PV input.
-    p_frag[0] = pack2<kBf16>(pr[0][0], pr[0][1]);
-    p_frag[1] = pack2<kBf16>(pr[1][0], pr[1][1]);
-    p_frag[2] = pack2<kBf16>(pr[0][2], pr[0][3]);
-    p_frag[3] = pack2<kBf16>(pr[1][2], pr[1][3]);
+    if constexpr (kNarrow) {
+      const uint32_t p_lo = pack2<kBf16>(pr[0][0], pr[0][1]), p_hi = pack2<kBf16>(pr[0][2], pr[0][3]);
+      const float alpha0 = __shfl_sync(0xffffffffu, alpha[0], 8 * t), alpha1 = __shfl_sync(0xffffffffu, alpha[0], 8 * t + 4);   // heads 2t, 2t + 1
 #pragma unroll
-    for (int j = 0; j < kD / 8; ++j) {
-      acc[j][0] *= alpha[0]; acc[j][1] *= alpha[0];
-      acc[j][2] *= alpha[1]; acc[j][3] *= alpha[1];
-    }
+      for (int j = 0; j < kAccs; ++j) {
+        const int mi = lane >> 3;
+        const int r = (mi >> 1) * 8 + (lane & 7);
+        const int c = 2 * j + (mi & 1);
+        uint32_t vfrag[4];
+        ldmatrix_x4_trans(v_src + tile_offset(r, c), vfrag);
+        acc[j][0] *= alpha0; acc[j][1] *= alpha1; acc[j][2] *= alpha0; acc[j][3] *= alpha1;
+        mma_16816<kBf16>(acc[j], vfrag, p_lo, p_hi);
+      }
+    } else {
+      const uint32_t p_frag[4] = {pack2<kBf16>(pr[0][0], pr[0][1]), pack2<kBf16>(pr[kHalves - 1][0], pr[kHalves - 1][1]),
+                                  pack2<kBf16>(pr[0][2], pr[0][3]), pack2<kBf16>(pr[kHalves - 1][2], pr[kHalves - 1][3])};
 #pragma unroll
-    for (int j = 0; j < kD / 8; j += 2) {
-      const int mi = lane >> 3;
-      const int r = (mi & 1) * 8 + (lane & 7);
-      const int c = j + (mi >> 1);
-      uint32_t vfrag[4];
-      ldmatrix_x4_trans(v_src + tile_offset(r, c), vfrag);
-      mma_16816<kBf16>(acc[j], p_frag, vfrag[0], vfrag[1]);
-      mma_16816<kBf16>(acc[j + 1], p_frag, vfrag[2], vfrag[3]);
+      for (int j = 0; j < kAccs; ++j) {
+        acc[j][0] *= alpha[0]; acc[j][1] *= alpha[0];
+        acc[j][2] *= alpha[kHalves - 1]; acc[j][3] *= alpha[kHalves - 1];
+      }
+#pragma unroll
+      for (int j = 0; j < kAccs; j += 2) {
+        const int mi = lane >> 3;
+        const int r = (mi & 1) * 8 + (lane & 7);
+        const int c = j + (mi >> 1);
+        uint32_t vfrag[4];
+        ldmatrix_x4_trans(v_src + tile_offset(r, c), vfrag);
+        mma_16816<kBf16>(acc[j], p_frag, vfrag[0], vfrag[1]);
+        mma_16816<kBf16>(acc[j + 1], p_frag, vfrag[2], vfrag[3]);
+      }
     }
+    __syncwarp();   // every lane has read the slot
+    issue_tile(tile + kStagesFd, tile % kStagesFd);
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < kHalves; ++h) {
     l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
     l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
   }
   __syncthreads();  // every warp is done with its ring; reuse it for the merge records
 
-  float *records = reinterpret_cast<float *>(smem);  // [warp][16][kRecord]
+  float *records = reinterpret_cast<float *>(smem);  // [warp][kMaxGroup][kSmemRecord]
   {
-    float *mine = records + static_cast<size_t>(warp) * 16 * kRecord;
+    float *mine = records + warp * (kMaxGroup * kSmemRecord);
+    if constexpr (kNarrow) {
 #pragma unroll
-    for (int j = 0; j < kD / 8; ++j) {
-      mine[g * kRecord + j * 8 + 2 * t] = acc[j][0];
-      mine[g * kRecord + j * 8 + 2 * t + 1] = acc[j][1];
-      mine[(g + 8) * kRecord + j * 8 + 2 * t] = acc[j][2];
-      mine[(g + 8) * kRecord + j * 8 + 2 * t + 1] = acc[j][3];
+      for (int j = 0; j < kAccs; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (2 * t + (i & 1) < p.group) mine[(2 * t + (i & 1)) * kSmemRecord + j * 16 + g + 8 * (i >> 1)] = acc[j][i];
     }
-    if (t == 0) {
-      mine[g * kRecord + kD] = m_run[0];
-      mine[g * kRecord + kD + 1] = l_run[0];
-      mine[(g + 8) * kRecord + kD] = m_run[1];
-      mine[(g + 8) * kRecord + kD + 1] = l_run[1];
+#pragma unroll
+    for (int h = 0; h < kHalves; ++h) {
+      const int head = g + 8 * h;
+      if (head < p.group) {
+        if constexpr (!kNarrow) {
+#pragma unroll
+          for (int j = 0; j < kAccs; ++j)
+            *reinterpret_cast<float2 *>(mine + head * kSmemRecord + j * 8 + 2 * t) = make_float2(acc[j][2 * h], acc[j][2 * h + 1]);
+        }
+        if (t == 0) *reinterpret_cast<float2 *>(mine + head * kSmemRecord + kD) = make_float2(m_run[h], l_run[h]);
+      }
     }
   }
   __syncthreads();
-  // Left fold over the warps (ascending KV order), one thread per (head, d).
-  for (int idx = threadIdx.x; idx < p.group * kD; idx += blockDim.x) {
-    const int head = idx / kD, d = idx % kD;
-    const float *rec = records + head * kRecord;
-    float m = rec[kD], l = rec[kD + 1], a = rec[d];
-    for (int w = 1; w < kWarps; ++w) {
-      const float *right = records + static_cast<size_t>(w) * 16 * kRecord + head * kRecord;
-      const float m_right = right[kD], l_right = right[kD + 1], a_right = right[d];
-      const float m_new = fmaxf(m, m_right);
-      const float m_exp = (m_new == -INFINITY) ? 0.f : m_new;
-      const float scale_left = exp_lp(m - m_exp), scale_right = exp_lp(m_right - m_exp);
-      l = l * scale_left + l_right * scale_right;
-      a = a * scale_left + a_right * scale_right;
-      m = m_new;
+  // Left fold over the warps (ascending KV order): a warp per query head, a lane per four head dimensions.
+  float *merged = records + kMergedOffset;           // [kMaxGroup][kSmemRecord]
+  const bool first_cta = p.cluster == 1 || cluster_cta_rank() == 0;
+  const int cluster_index = p.cluster == 1 ? static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) / p.cluster;
+  // What becomes of the state of query head `head` once it is complete for the cluster's keys.
+  auto deliver = [&](int head, float m, float l, const float4 &a) {
+    const int row = b * p.q_heads + hk * p.group + head;
+    if (kTail == kTailLocal && p.splits == 1) {
+      fd_deliver_row(tail, row, lane, m, l, a);
+    } else {
+      float *out = p.partials + (static_cast<size_t>(row) * p.splits + cluster_index) * kRecord;
+      *reinterpret_cast<float2 *>(out + 4 * lane) = make_float2(a.x, a.y);
+      *reinterpret_cast<float2 *>(out + 4 * lane + 2) = make_float2(a.z, a.w);
+      if (lane == 0) *reinterpret_cast<float2 *>(out + kD) = make_float2(m, l);
     }
-    float *out = p.partials +
-                 ((static_cast<size_t>(b) * p.q_heads + hk * p.group + head) * p.splits + split) * kRecord;
-    out[d] = a;
-    if (d == 0) {
-      out[kD] = m;
-      out[kD + 1] = l;
+  };
+  for (int head = warp; head < p.group; head += kWarps) {
+    const float *rec = records + head * kSmemRecord;
+    float m = rec[kD], l = rec[kD + 1];
+    float4 a = *reinterpret_cast<const float4 *>(rec + 4 * lane);
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) {
+      const float *right = rec + w * (kMaxGroup * kSmemRecord);
+      fd_merge_right(m, l, a, right[kD], right[kD + 1], *reinterpret_cast<const float4 *>(right + 4 * lane));
+    }
+    if (p.cluster == 1) {
+      deliver(head, m, l, a);
+    } else {
+      *reinterpret_cast<float4 *>(merged + head * kSmemRecord + 4 * lane) = a;
+      if (lane == 0) *reinterpret_cast<float2 *>(merged + head * kSmemRecord + kD) = make_float2(m, l);
     }
   }
-  if constexpr (kTail) {
-    // The CTA that finishes last among the splits of this (batch, kv head) folds the splits of the group's query heads,
-    // exchanges the states with the other ranks and writes the outputs: the decode step is this one launch.
+  if (p.cluster > 1) {
+    cluster_sync_all();   // the merged records of the cluster's CTAs are in their shared memory
+    if (first_cta) {
+      // Fold over the cluster's CTAs with their common maximum as the exponent reference (see fd_fold_records); lane r
+      // holds CTA r's (m, l) of the head.
+      for (int head = warp; head < p.group; head += kWarps) {
+        const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(merged + head * kSmemRecord));
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (lane < p.cluster) ml = ld_cluster_f32x2(cluster_map_shared(local + kD * 4, lane));
+        float top = ml.x;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        const float weight = exp_lp(ml.x - (top == -INFINITY ? 0.f : top));
+        float sum = ml.y * weight;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int r = 0; r < p.cluster; ++r) {
+          const float4 right = ld_cluster_f32x4(cluster_map_shared(local + 16 * lane, r));
+          const float w = __shfl_sync(0xffffffffu, weight, r);
+          a.x = fmaf(right.x, w, a.x); a.y = fmaf(right.y, w, a.y);
+          a.z = fmaf(right.z, w, a.z); a.w = fmaf(right.w, w, a.w);
+        }
+        deliver(head, top, sum, a);
+      }
+    }
+    cluster_sync_all();   // no CTA leaves while the first one may read its shared memory
+    if (!first_cta) return;
+  }
+  if (kTail == kTailLocal && p.splits == 1) return;
+  if constexpr (kTail != kTailNone) {
+    // The cluster that finishes last among those of this (batch, kv head) folds the records of the group's query heads and
+    // writes the outputs (with the exchange between the ranks in front of them): the decode step is this one launch.
     __shared__ bool last_of_head;
-    __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
+      __threadfence();      // cumulative over the CTA's record stores, which the barrier ordered before it
       unsigned int *arrivals = tail.arrivals + b * p.kv_heads + hk;
-      last_of_head = atomicAdd(arrivals, 1u) == static_cast<unsigned int>(p.splits) - 1u;
-      if (last_of_head) *arrivals = 0u;     // ready for the next launch
+      const unsigned int last = static_cast<unsigned int>(p.splits) - 1u;
+      last_of_head = atomicInc(arrivals, last) == last;   // wraps to zero, ready for the next launch
+      __threadfence();
     }
     __syncthreads();
     if (last_of_head) {
-      __threadfence();
       const int first_row = b * p.q_heads + hk * p.group;
-      fd_exchange_rows<kD / 32>(tail, p.partials, p.splits, first_row, p.group, p.batch * p.q_heads);
+      if constexpr (kTail == kTailExchange)
+        fd_exchange_rows<kD / 32>(tail, p.partials, p.splits, first_row, p.group, p.batch * p.q_heads);
+      else
+        fd_local_rows(tail, p.partials, p.splits, first_row, p.group);
     }
   }
 }
@@ -331,11 +504,12 @@ struct FdCombineParams {
   const float *records_ptr;
   int out_format;
   int zero_fully_masked;
-  int finalize;
   void *out;
-  float *lse, *row_max, *row_sum, *state_out;
+  float *lse, *row_max, *row_sum;
 };
 
+// Merge of the states of sequence shards (wb200_attention_fd_merge): left fold in ascending shard order, one thread per
+// head dimension of a row.
 __global__ void __launch_bounds__(kD) fd_combine_kernel(const FdCombineParams p) {
   const int row = blockIdx.x, d = threadIdx.x;
   const float *rec = p.records_ptr + row * p.row_stride;
@@ -349,15 +523,6 @@ __global__ void __launch_bounds__(kD) fd_combine_kernel(const FdCombineParams p)
     l = l * scale_left + l_right * scale_right;
     a = a * scale_left + a_right * scale_right;
     m = m_new;
-  }
-  if (!p.finalize) {
-    float *state = p.state_out + static_cast<size_t>(row) * kRecord;
-    state[d] = a;
-    if (d == 0) {
-      state[kD] = m;
-      state[kD + 1] = l;
-    }
-    return;
   }
   float coefficient = 1.0f / l;
   if (p.zero_fully_masked && l == 0.f) coefficient = 0.f;
@@ -397,22 +562,6 @@ __device__ __forceinline__ unsigned int ld_acquire_sys(const unsigned int *addre
 // takes a row, a lane four consecutive head dimensions. Per batch of four rows: fold of the rows' split records in
 // ascending order, stores of the states into every rank's buffer, flags, bounded wait for the world's flags, merge in
 // ascending rank order, outputs. The rows of a batch travel together, so the NVLink round trip is paid once per batch.
-__device__ __forceinline__ void fd_merge_right(float &m, float &l, float4 &a, float m_right, float l_right, const float4 &a_right) {
-  const float m_new = fmaxf(m, m_right);
-  const float m_exp = (m_new == -INFINITY) ? 0.f : m_new;
-  const float scale_left = exp_lp(m - m_exp), scale_right = exp_lp(m_right - m_exp);
-  l = l * scale_left + l_right * scale_right;
-  a.x = a.x * scale_left + a_right.x * scale_right;
-  a.y = a.y * scale_left + a_right.y * scale_right;
-  a.z = a.z * scale_left + a_right.z * scale_right;
-  a.w = a.w * scale_left + a_right.w * scale_right;
-  m = m_new;
-}
-// Four consecutive floats of a record (records are 130 floats long: 8-byte, not 16-byte, aligned), read past L1.
-__device__ __forceinline__ float4 ldcg_quad(const float *address) {
-  const float2 lo = __ldcg(reinterpret_cast<const float2 *>(address)), hi = __ldcg(reinterpret_cast<const float2 *>(address + 2));
-  return make_float4(lo.x, lo.y, hi.x, hi.y);
-}
 template <int kRowsAtOnce>
 __device__ void fd_exchange_rows(const FdTailParams &x, const float *records, int splits, int first_row, int row_count, int rows_total) {
   static_assert(kRowsAtOnce == kD / 32, "one warp per row");
@@ -426,43 +575,10 @@ __device__ void fd_exchange_rows(const FdTailParams &x, const float *records, in
     const int row = first_row + base + warp;
     const bool active = warp < count;
     if (active) {
-      // fold this rank's splits (records of other CTAs: read past L1), twelve records in flight: the fold is a chain
-      // of L2 round trips otherwise (a single resident wave of a long sequence has 37 splits per head)
-      const float *rec = records + static_cast<size_t>(row) * splits * kRecord;
-      float m = __ldcg(rec + kD), l = __ldcg(rec + kD + 1);
-      float4 a = ldcg_quad(rec + 4 * lane);
-      int s = 1;
-      constexpr int kBatch = 12;
-      for (; s + kBatch <= splits; s += kBatch) {
-        float mr[kBatch], lr[kBatch];
-        float4 ar[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-          const float *right = rec + static_cast<size_t>(s + u) * kRecord;
-          const float2 ml = __ldcg(reinterpret_cast<const float2 *>(right + kD));
-          mr[u] = ml.x; lr[u] = ml.y;
-          ar[u] = ldcg_quad(right + 4 * lane);
-        }
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) fd_merge_right(m, l, a, mr[u], lr[u], ar[u]);
-      }
-      for (; s + 4 <= splits; s += 4) {
-        float mr[4], lr[4];
-        float4 ar[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float *right = rec + static_cast<size_t>(s + u) * kRecord;
-          mr[u] = __ldcg(right + kD); lr[u] = __ldcg(right + kD + 1);
-          ar[u] = ldcg_quad(right + 4 * lane);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) fd_merge_right(m, l, a, mr[u], lr[u], ar[u]);
-      }
-      for (; s < splits; ++s) {
-        const float *right = rec + static_cast<size_t>(s) * kRecord;
-        const float4 ar = ldcg_quad(right + 4 * lane);
-        fd_merge_right(m, l, a, __ldcg(right + kD), __ldcg(right + kD + 1), ar);
-      }
+      // fold this rank's splits (records of other CTAs: read past L1)
+      float m, l;
+      float4 a;
+      fd_fold_records(records + static_cast<size_t>(row) * splits * kRecord, splits, lane, m, l, a);
       // the state into slot [parity][rank][row] of every rank's buffer (records are 130 floats: 8-byte aligned rows)
       const size_t my_slot = (static_cast<size_t>(parity) * x.world + x.rank) * rows_total + row;
       for (int r = 0; r < x.world; ++r) {
@@ -521,21 +637,7 @@ __device__ void fd_exchange_rows(const FdTailParams &x, const float *records, in
         load_state(r, m_right, l_right, a_right);
         fd_merge_right(m, l, a, m_right, l_right, a_right);
       }
-      float coefficient = 1.0f / l;
-      if (x.zero_fully_masked && l == 0.f) coefficient = 0.f;
-      const float value[4] = {a.x * coefficient, a.y * coefficient, a.z * coefficient, a.w * coefficient};
-      if (x.out_format == WB200_F32) {
-        *(reinterpret_cast<float4 *>(x.out) + static_cast<size_t>(row) * (kD / 4) + lane) = make_float4(value[0], value[1], value[2], value[3]);
-      } else {
-        const uint32_t lo = narrow_bits(value[0], x.out_format) | (static_cast<uint32_t>(narrow_bits(value[1], x.out_format)) << 16);
-        const uint32_t hi = narrow_bits(value[2], x.out_format) | (static_cast<uint32_t>(narrow_bits(value[3], x.out_format)) << 16);
-        *(reinterpret_cast<uint2 *>(x.out) + static_cast<size_t>(row) * (kD / 4) + lane) = make_uint2(lo, hi);
-      }
-      if (lane == 0) {
-        if (x.lse) x.lse[row] = (l == 0.f) ? -INFINITY : m + logf(l);
-        if (x.row_max) x.row_max[row] = m;
-        if (x.row_sum) x.row_sum[row] = l;
-      }
+      fd_write_row(x, row, lane, m, l, a);
     }
   }
   // the CTA that completes the last rows of the launch advances the epoch for the next call
@@ -573,36 +675,49 @@ bool attention_fd_supports(const AttentionArgs &a) {
   return a.kv_len > 0 && a.batch > 0;
 }
 
-uint32_t fd_choose_splits(const AttentionArgs &a, int sm_count) {
+FdPlan fd_choose_plan(const AttentionArgs &a, int sm_count) {
   const int64_t visible = visible_keys(a);
   const int64_t units = static_cast<int64_t>(a.batch) * a.kv_heads;
-  const int64_t slots = 2LL * sm_count;                 // two CTAs are resident per SM
-  const int64_t base = (visible + 2047) / 2048;         // 2048-key splits
+  const int64_t all_slots = 2LL * sm_count;             // two CTAs are resident per SM
   // More (batch, kv head) units than resident slots: 2048-key splits give many short CTAs, which the hardware deals out
-  // as slots free up (the tail is one short CTA), and the fold over a unit's few splits is short.
-  if (units >= slots) return static_cast<uint32_t>(base < 2 ? 2 : (base > 4096 ? 4096 : base));
-  // Otherwise pick the split count with the least estimated time, in units of one key streamed by one CTA:
-  // waves x (keys per split + the CTA's fixed cost) + the serial fold over the splits (one record costs about as much
-  // as six keys). A long sequence with few (batch, kv head) units ends up with exactly one resident wave.
-  int64_t limit = visible / 256;                        // at least 256 keys per split
-  if (limit > 4096) limit = 4096;
-  int64_t best_splits = 2, best_cost = -1;
-  for (int64_t splits = 2; splits <= (limit < 2 ? 2 : limit); ++splits) {
-    const int64_t rows = ((visible + splits - 1) / splits + 63) / 64 * 64;
-    const int64_t waves = (units * splits + slots - 1) / slots;
-    const int64_t cost = waves * (rows + 130) + 6 * splits;
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_splits = splits; }
+  // as slots free up (the tail is one short CTA), and the fold over a unit's few records is short.
+  if (units >= all_slots) {
+    const int64_t base = (visible + 2047) / 2048;
+    return {1u, static_cast<uint32_t>(base < 1 ? 1 : (base > 4096 ? 4096 : base))};
   }
-  return static_cast<uint32_t>(best_splits);            // flash-decoding splits K2 into at least two intervals
+  // Otherwise the candidate with the least estimated time, in nanoseconds. A CTA keeps 64 to 96 KiB of copies in flight, about
+  // 70 bytes / ns, and the HBM gives 6500 to all of them. Clusters of eight leave a part of every GPC unused. Merging inside a cluster costs about 1 us; a fold through global
+  // records (fence, counter, second read) about 3 us more, plus the fold's own reads.
+  FdPlan best{1u, 1u};
+  double best_cost = -1;
+  auto consider = [&](int64_t cluster, int64_t records) {
+    const int64_t ctas = cluster * records;
+    if (ctas > 1 && ctas * 64 > visible + 63) return;   // less than one tile per warp
+    const double rows = static_cast<double>(((visible + ctas - 1) / ctas + 63) / 64 * 64);
+    const double bytes = rows * (4.0 * kD);
+    const int64_t slots = cluster == kMaxFdCluster ? all_slots * 7 / 8 : all_slots;
+    double streaming = 0;
+    for (int64_t left = units * ctas; left > 0; left -= slots) {
+      const double active = static_cast<double>(left < slots ? left : slots);
+      const double shared = active * bytes / 6500.0, alone = bytes / 70.0;
+      streaming += (shared > alone ? shared : alone) + 500.0;
+    }
+    const double cost = streaming + (cluster > 1 ? 1000.0 : 0.0) + (records > 1 ? 3000.0 + 40.0 * static_cast<double>(records) : 0.0);
+    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = {static_cast<uint32_t>(cluster), static_cast<uint32_t>(records)}; }
+  };
+  for (int64_t cluster = 1; cluster <= kMaxFdCluster; cluster *= 2) consider(cluster, 1);
+  for (int64_t cluster = 1; cluster <= kMaxFdCluster; cluster *= 8)
+    for (int64_t records = 2; records <= 256 && units * cluster * records <= 2 * all_slots; ++records) consider(cluster, records);
+  return best;
 }
 
-size_t fd_partial_floats(const AttentionArgs &a, uint32_t splits) {
-  return static_cast<size_t>(a.batch) * a.q_heads * splits * kRecord;
+size_t fd_partial_floats(const AttentionArgs &a, uint32_t records) {
+  return static_cast<size_t>(a.batch) * a.q_heads * records * kRecord;
 }
 
 namespace {
-wb200_status launch_fd_stage1(const AttentionArgs &a, uint32_t splits, float *partials, cudaStream_t stream,
-                              const FdTailParams *tail = nullptr);
+wb200_status launch_fd_stage1(const AttentionArgs &a, FdPlan plan, float *partials, cudaStream_t stream, int tail_kind,
+                              const FdTailParams &tail);
 }
 
 size_t fd_exchange_floats(int rows, int world) {
@@ -610,7 +725,7 @@ size_t fd_exchange_floats(int rows, int world) {
   return static_cast<size_t>(2) * world * rows * (kRecord + 1);
 }
 
-wb200_status launch_attention_fd_exchange(const AttentionArgs &a, uint32_t splits, float *partials, int rank, int world,
+wb200_status launch_attention_fd_exchange(const AttentionArgs &a, FdPlan plan, float *partials, int rank, int world,
                                           void *const *peer_buffers, unsigned int *epoch, unsigned int *arrivals,
                                           int *device_status, cudaStream_t stream) {
   if (world < 1 || world > kMaxExchangeRanks || rank < 0 || rank >= world)
@@ -626,49 +741,51 @@ wb200_status launch_attention_fd_exchange(const AttentionArgs &a, uint32_t split
   x.status = device_status;
   // With arrival counters the tail runs inside stage 1 (its last CTA per (batch, kv head)): one launch per step.
   // Without them it is a launch of its own behind stage 1.
-  wb200_status st = launch_fd_stage1(a, splits, partials, stream, arrivals ? &x : nullptr);
+  wb200_status st = launch_fd_stage1(a, plan, partials, stream, arrivals ? kTailExchange : kTailNone, x);
   if (st != WB200_OK) return st;
   if (!arrivals) {
     const int rows = a.batch * a.q_heads;
-    fd_exchange_kernel<<<(rows + kD / 32 - 1) / (kD / 32), kD, 0, stream>>>(x, partials, static_cast<int>(splits), rows);
+    fd_exchange_kernel<<<(rows + kD / 32 - 1) / (kD / 32), kD, 0, stream>>>(x, partials, static_cast<int>(plan.records), rows);
     WB200_CUDA_CHECK(cudaGetLastError());
   }
   return WB200_OK;
 }
 
-wb200_status launch_attention_fd(const AttentionArgs &a, uint32_t splits, float *partials, int finalize,
+wb200_status launch_attention_fd(const AttentionArgs &a, FdPlan plan, float *partials, unsigned int *arrivals,
                                  float *state_out, cudaStream_t stream) {
-  wb200_status st = launch_fd_stage1(a, splits, partials, stream);
-  if (st != WB200_OK) return st;
-  FdCombineParams c;
-  c.rows = a.batch * a.q_heads;
-  c.records = static_cast<int>(splits);
-  c.row_stride = static_cast<size_t>(splits) * kRecord;
-  c.record_stride = kRecord;
-  c.records_ptr = partials;
-  c.out_format = a.format;
-  c.zero_fully_masked = a.zero_fully_masked;
-  c.finalize = finalize;
-  c.out = a.out; c.lse = a.lse; c.row_max = a.row_max; c.row_sum = a.row_sum; c.state_out = state_out;
-  fd_combine_kernel<<<c.rows, kD, 0, stream>>>(c);
-  WB200_CUDA_CHECK(cudaGetLastError());
-  return WB200_OK;
+  FdTailParams x{};
+  x.arrivals = arrivals;
+  x.out_format = a.format;
+  x.zero_fully_masked = a.zero_fully_masked;
+  x.out = a.out; x.lse = a.lse; x.row_max = a.row_max; x.row_sum = a.row_sum; x.state_out = state_out;
+  return launch_fd_stage1(a, plan, partials, stream, kTailLocal, x);
 }
 
 namespace {
-wb200_status launch_fd_stage1(const AttentionArgs &a, uint32_t splits, float *partials, cudaStream_t stream, const FdTailParams *tail) {
+using FdKernel = void (*)(const FdParams, const FdTailParams);
+template <int kTail, bool kNarrow>
+constexpr FdKernel fd_kernel(bool bf16) { return bf16 ? fd_partial_kernel<true, kTail, kNarrow> : fd_partial_kernel<false, kTail, kNarrow>; }
+const FdKernel kFdKernels[12] = {   // [tail][narrow][bf16]
+    fd_kernel<kTailNone, false>(false),     fd_kernel<kTailNone, false>(true),     fd_kernel<kTailNone, true>(false),     fd_kernel<kTailNone, true>(true),
+    fd_kernel<kTailLocal, false>(false),    fd_kernel<kTailLocal, false>(true),    fd_kernel<kTailLocal, true>(false),    fd_kernel<kTailLocal, true>(true),
+    fd_kernel<kTailExchange, false>(false), fd_kernel<kTailExchange, false>(true), fd_kernel<kTailExchange, true>(false), fd_kernel<kTailExchange, true>(true)};
+
+wb200_status launch_fd_stage1(const AttentionArgs &a, FdPlan plan, float *partials, cudaStream_t stream, int tail_kind,
+                              const FdTailParams &tail) {
   if (!attention_fd_supports(a)) return fail(WB200_ERR_UNSUPPORTED, "flash-decoding request outside the kernel's domain");
-  if (splits < 1) return fail(WB200_ERR_INVALID_ARGUMENT, "kv_splits must be positive");
+  if (plan.records < 1 || plan.cluster < 1) return fail(WB200_ERR_INVALID_ARGUMENT, "kv_splits must be positive");
   FdParams p;
   p.batch = a.batch; p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.group = a.q_heads / a.kv_heads;
   p.kv_len = a.kv_len;
   p.kv_visible = visible_keys(a);
-  p.splits = static_cast<int>(splits);
-  const int64_t per_split = (static_cast<int64_t>(p.kv_visible) + splits - 1) / splits;
+  p.splits = static_cast<int>(plan.records);
+  p.cluster = static_cast<int>(plan.cluster);
+  const int64_t ctas = static_cast<int64_t>(plan.records) * plan.cluster;
+  const int64_t per_cta = (static_cast<int64_t>(p.kv_visible) + ctas - 1) / ctas;
   const int64_t granule = kWarps * kTileRows;
-  p.rows_per_split = static_cast<int>(((per_split + granule - 1) / granule) * granule);
-  if (p.rows_per_split == 0) p.rows_per_split = static_cast<int>(granule);
-  p.rows_per_warp = p.rows_per_split / kWarps;
+  p.rows_per_cta = static_cast<int>(((per_cta + granule - 1) / granule) * granule);
+  if (p.rows_per_cta == 0) p.rows_per_cta = static_cast<int>(granule);
+  p.rows_per_warp = p.rows_per_cta / kWarps;
   p.scale = a.scale;
   p.q = static_cast<const uint16_t *>(a.q);
   p.k = static_cast<const uint16_t *>(a.k);
@@ -677,24 +794,25 @@ wb200_status launch_fd_stage1(const AttentionArgs &a, uint32_t splits, float *pa
 
   static PerDeviceOnce attributes;
   const wb200_status attribute_status = attributes.run([]() -> wb200_status {
-    WB200_CUDA_CHECK(cudaFuncSetAttribute(fd_partial_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFdSmemBytes));
-    WB200_CUDA_CHECK(cudaFuncSetAttribute(fd_partial_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFdSmemBytes));
-    WB200_CUDA_CHECK(cudaFuncSetAttribute(fd_partial_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFdSmemBytes));
-    WB200_CUDA_CHECK(cudaFuncSetAttribute(fd_partial_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFdSmemBytes));
+    for (const auto kernel : kFdKernels)
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFdSmemBytes));
     return WB200_OK;
   });
   if (attribute_status != WB200_OK) return attribute_status;
-  dim3 grid(splits, a.kv_heads, a.batch);
   static_assert(kWarps * 32 == kD, "the tail of the sharded decode runs with one thread per head dimension");
-  const FdTailParams none{};
-  if (tail) {
-    if (a.format == WB200_BF16) fd_partial_kernel<true, true><<<grid, kWarps * 32, kFdSmemBytes, stream>>>(p, *tail);
-    else fd_partial_kernel<false, true><<<grid, kWarps * 32, kFdSmemBytes, stream>>>(p, *tail);
-  } else {
-    if (a.format == WB200_BF16) fd_partial_kernel<true, false><<<grid, kWarps * 32, kFdSmemBytes, stream>>>(p, none);
-    else fd_partial_kernel<false, false><<<grid, kWarps * 32, kFdSmemBytes, stream>>>(p, none);
-  }
-  WB200_CUDA_CHECK(cudaGetLastError());
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(ctas), a.kv_heads, a.batch);
+  config.blockDim = dim3(kWarps * 32);
+  config.dynamicSmemBytes = kFdSmemBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[2];
+  attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute[0].val.programmaticStreamSerializationAllowed = 1;
+  attribute[1].id = cudaLaunchAttributeClusterDimension;
+  attribute[1].val.clusterDim.x = plan.cluster; attribute[1].val.clusterDim.y = 1; attribute[1].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = plan.cluster > 1 ? 2 : 1;
+  WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, kFdKernels[4 * tail_kind + (p.group <= 8 ? 2 : 0) + (a.format == WB200_BF16 ? 1 : 0)], p, tail));
   return WB200_OK;
 }
 }  // namespace
@@ -711,8 +829,7 @@ wb200_status launch_attention_fd_merge(const AttentionArgs &a, const float *stat
   c.records_ptr = states;
   c.out_format = a.format;
   c.zero_fully_masked = a.zero_fully_masked;
-  c.finalize = 1;
-  c.out = a.out; c.lse = a.lse; c.row_max = a.row_max; c.row_sum = a.row_sum; c.state_out = nullptr;
+  c.out = a.out; c.lse = a.lse; c.row_max = a.row_max; c.row_sum = a.row_sum;
   fd_combine_kernel<<<c.rows, kD, 0, stream>>>(c);
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
@@ -735,22 +852,29 @@ namespace {
 
 constexpr size_t kStaticScratchFloats = size_t(4) << 20;   // 16 MiB, held by every GPU that loads the library
 static __device__ __align__(256) float g_fd_static_scratch[kStaticScratchFloats];
+// Arrival counters of the (batch, kv head) units, left at zero by every launch; a unit has at least one row of at least one record.
+constexpr size_t kStaticArrivals = kStaticScratchFloats / kRecord;
+static __device__ unsigned int g_fd_static_arrivals[kStaticArrivals];
 
 constexpr int kMaxDevices = 64;
 float *g_fd_static_scratch_address[kMaxDevices] = {nullptr};
+unsigned int *g_fd_static_arrivals_address[kMaxDevices] = {nullptr};
 std::mutex g_fd_static_scratch_mutex;
 
 // In host code `g_fd_static_scratch` names a host-side handle, not device memory; the address a kernel
 // can use has to be asked for, once per device, with that device current.
-wb200_status static_scratch_for_device(int device, float **out) {
+wb200_status static_scratch_for_device(int device, float **out, unsigned int **arrivals) {
   if (device < 0 || device >= kMaxDevices) return fail(WB200_ERR_LIMIT, "device index beyond the static scratch table");
   std::lock_guard<std::mutex> lock(g_fd_static_scratch_mutex);
   if (!g_fd_static_scratch_address[device]) {
     void *address = nullptr;
+    WB200_CUDA_CHECK(cudaGetSymbolAddress(&address, g_fd_static_arrivals));
+    g_fd_static_arrivals_address[device] = static_cast<unsigned int *>(address);
     WB200_CUDA_CHECK(cudaGetSymbolAddress(&address, g_fd_static_scratch));
     g_fd_static_scratch_address[device] = static_cast<float *>(address);
   }
   *out = g_fd_static_scratch_address[device];
+  *arrivals = g_fd_static_arrivals_address[device];
   return WB200_OK;
 }
 
@@ -782,20 +906,21 @@ extern "C" wb200_status wb200_attention_fd_static(wb200_backend *backend, const 
   if (!attention_fd_supports(a))
     return fail(WB200_ERR_UNSUPPORTED, "flash-decoding kernel takes f16/bf16 storage, head_dim 128, group size <= 16");
   DeviceGuard guard(backend->device);
-  uint32_t splits = kv_splits;
-  if (splits == 0) {
-    splits = fd_choose_splits(a, backend->sm_count);
-    while (splits > 2 && fd_partial_floats(a, splits) > kStaticScratchFloats) splits = (splits + 1) / 2;
+  FdPlan plan{1u, kv_splits};
+  if (kv_splits == 0) {
+    plan = fd_choose_plan(a, backend->sm_count);
+    while (plan.records > 2 && fd_partial_floats(a, plan.records) > kStaticScratchFloats) plan.records = (plan.records + 1) / 2;
   }
-  const size_t needed = fd_partial_floats(a, splits);
+  const size_t needed = fd_partial_floats(a, plan.records);
   if (needed > kStaticScratchFloats)
     return fail(WB200_ERR_LIMIT, "allocation-free decode: batch * q_heads * kv_splits * (head_dim + 2) = " + std::to_string(needed) +
                                      " floats exceeds the fixed scratch of " + std::to_string(kStaticScratchFloats) + " floats (16 MiB)");
   float *scratch = nullptr;
-  wb200_status st = static_scratch_for_device(backend->device, &scratch);
+  unsigned int *arrivals = nullptr;
+  wb200_status st = static_scratch_for_device(backend->device, &scratch, &arrivals);
   if (st != WB200_OK) return st;
   // Stage 1 writes every record stage 2 reads, so nothing left by an earlier call needs clearing.
-  st = launch_attention_fd(a, splits, scratch, 1, nullptr, static_cast<cudaStream_t>(p->stream));
-  if (st == WB200_OK) backend->launches += 2;
+  st = launch_attention_fd(a, plan, scratch, arrivals, nullptr, static_cast<cudaStream_t>(p->stream));
+  if (st == WB200_OK) backend->launches += 1;
   return st;
 }

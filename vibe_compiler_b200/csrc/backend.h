@@ -84,7 +84,10 @@ struct wb200_backend {
     const size_t before = slots.size() > index ? slots[index].bytes : 0;
     wb200_status st = buffer(index, bytes, out);
     if (st != WB200_OK) return st;
-    if (slots[index].bytes != before) WB200_CUDA_CHECK(cudaMemset(*out, 0, slots[index].bytes));
+    if (slots[index].bytes != before) {
+      WB200_CUDA_CHECK(cudaMemset(*out, 0, slots[index].bytes));
+      WB200_CUDA_CHECK(cudaStreamSynchronize(cudaStreamLegacy));   // callers' streams are not ordered after the fill
+    }
     return WB200_OK;
   }
 };

@@ -194,15 +194,17 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &args, int sm_count, i
                                       cudaStream_t stream);
 wb200_status launch_attention_fa_simt(const AttentionArgs &args, cudaStream_t stream);
 
-// Flash-decoding. `partials` is scratch of fd_partial_floats(args, splits) floats.
-// Stage 1 writes one (acc[D], m, l) record per (batch, q_head, split); stage 2 left-folds records in
-// ascending split order. With `finalize` == 0 stage 2 writes the merged state to `state_out`
-// instead of out / lse.
+// Flash-decoding. `partials` is scratch of fd_partial_floats(args, plan.records) floats.
+// The keys of a (batch, kv head) are cut over `records` clusters of `cluster` CTAs. Every cluster writes one (acc[D], m, l)
+// record per query head; the last cluster of a (batch, kv head) folds them (with one record it finalizes directly). `arrivals` is batch * kv_heads zero-initialised words, which the kernel leaves zeroed.
+// With `state_out` the merged state goes there instead of out / lse.
 bool attention_fd_supports(const AttentionArgs &args);
-uint32_t fd_choose_splits(const AttentionArgs &args, int sm_count);
-size_t fd_partial_floats(const AttentionArgs &args, uint32_t splits);
-wb200_status launch_attention_fd(const AttentionArgs &args, uint32_t splits, float *partials,
-                                 int finalize, float *state_out, cudaStream_t stream);
+struct FdPlan { uint32_t cluster, records; };
+constexpr int kMaxFdCluster = 8;   // the portable cluster size
+FdPlan fd_choose_plan(const AttentionArgs &args, int sm_count);
+size_t fd_partial_floats(const AttentionArgs &args, uint32_t records);
+wb200_status launch_attention_fd(const AttentionArgs &args, FdPlan plan, float *partials, unsigned int *arrivals,
+                                 float *state_out, cudaStream_t stream);
 wb200_status launch_attention_fd_merge(const AttentionArgs &args, const float *states,
                                        uint32_t shard_count, cudaStream_t stream);
 // Sequence-sharded decode with the exchange inside the kernel: stage 1, then one kernel that folds this rank's splits,
@@ -211,7 +213,7 @@ wb200_status launch_attention_fd_merge(const AttentionArgs &args, const float *s
 // `epoch` is this rank's pair of zero-initialised words. With `arrivals` (batch * kv_heads zero-initialised words that the
 // kernel leaves zeroed) the fold, exchange and merge run in the last stage-1 CTA of every (batch, kv head): one launch.
 size_t fd_exchange_floats(int rows, int world);
-wb200_status launch_attention_fd_exchange(const AttentionArgs &args, uint32_t splits, float *partials, int rank, int world,
+wb200_status launch_attention_fd_exchange(const AttentionArgs &args, FdPlan plan, float *partials, int rank, int world,
                                           void *const *peer_buffers, unsigned int *epoch, unsigned int *arrivals,
                                           int *device_status, cudaStream_t stream);
 

@@ -1,0 +1,94 @@
+"""Command calls on host storage around the sizes where their paths change: element groups against padded channel tails and
+bank-line padding, folds of a few long chains, storage read in place (up to 1 MiB) against storage copied in pieces."""
+import numpy as np
+import pytest
+import torch
+
+from vibe_compiler_b200 import _abi as abi
+from vibe_compiler_b200.backend import B200TargetModelBackend, NumericTensor, PhysicalTensorDescriptor, WB200Error
+
+pytestmark = pytest.mark.gpu
+LAYOUTS = {"tensor": abi.LAYOUT_TENSOR, "cx": abi.LAYOUT_CX, "ncx": abi.LAYOUT_NCX}
+
+
+def physical(backend, key, values):
+    """Storage holding `values` (uint bit patterns, row-major), 0x5a in every padding byte."""
+    blank = np.full(B200TargetModelBackend.physical_bytes(key), 0x5a, dtype=np.uint8)
+    return backend.pack(key, values, blank)
+
+
+def logical(backend, key, storage, dtype):
+    return backend.unpack(NumericTensor(key, storage)).view(dtype)
+
+
+@pytest.mark.parametrize("layout,shape", [("tensor", [7]), ("tensor", [1003]), ("cx", [3, 5]), ("cx", [5, 66]), ("cx", [7, 97]), ("cx", [33, 64]),
+                                          ("ncx", [2, 3, 65]), ("ncx", [3, 2, 5, 129]), ("cx", [1031, 263]), ("tensor", [700001])])
+def test_elementwise_and_convert_keep_padding_and_match_numpy(backend, layout, shape):
+    rng = np.random.default_rng(sum(shape))
+    count = int(np.prod(shape))
+    x, y = (rng.standard_normal(count).astype(np.float32) for _ in range(2))
+    f32, bf16 = (PhysicalTensorDescriptor(f, LAYOUTS[layout], shape) for f in (abi.F32, abi.BF16))
+    blank = np.full(B200TargetModelBackend.physical_bytes(f32), 0x11, dtype=np.uint8)
+    got = backend.execute_elementwise("sub", [NumericTensor(f32, physical(backend, f32, v)) for v in (x, y)], NumericTensor(f32, blank))
+    assert np.array_equal(logical(backend, f32, got.destination.storage, np.float32), x - y)
+    # every byte that is no element keeps the template's value
+    marked = backend.pack(f32, np.full(count, 0x22222222, np.uint32), np.full_like(blank, 0x11))
+    assert np.array_equal(got.destination.storage[marked == 0x11], blank[marked == 0x11])
+    half = backend.execute_convert(167, got.destination, NumericTensor(bf16, np.zeros(B200TargetModelBackend.physical_bytes(bf16), np.uint8)))
+    want = torch.from_numpy(x - y).bfloat16().view(torch.int16).numpy().view(np.uint16)
+    assert np.array_equal(logical(backend, bf16, half.destination.storage, np.uint16), want)
+
+
+@pytest.mark.parametrize("shape,dimension,axes", [([5], "trailing0", (0,)), ([65, 7], "trailing1", (0,)), ([300, 70], "trailing1", (0,)), ([3, 130], "trailing0", (1,)),
+                                                  ([2, 4, 66, 65], "trailing1", (2,)), ([2, 3, 5, 97], "trailing2and1", (1, 2)),
+                                                  ([2, 3, 5, 97], "trailing2and1and0", (1, 2, 3)), ([3, 2, 2, 64], "trailing3", (0,)), ([1, 1, 64, 64], "trailing1", (2,))])
+@pytest.mark.parametrize("formal", [False, True])
+def test_folds_follow_the_input_order(backend, shape, dimension, axes, formal):
+    rng = np.random.default_rng(3)
+    x = (rng.standard_normal(shape) * 10.0 ** rng.integers(-3, 4, shape)).astype(np.float32)
+    x.reshape(-1)[::7] = 0.0
+    x.reshape(-1)[3::11] = -0.0
+    out_shape = [1 if d in axes else n for d, n in enumerate(shape)]
+    chains = np.moveaxis(x, axes, tuple(range(len(axes)))).reshape(-1, int(np.prod(out_shape)))   # row-major input order per output
+    for layout in (abi.LAYOUT_NCX, abi.LAYOUT_TENSOR):
+        key, out_key = PhysicalTensorDescriptor(abi.F32, layout, shape), PhysicalTensorDescriptor(abi.F32, layout, out_shape)
+        source = NumericTensor(key, physical(backend, key, x.reshape(-1)))
+        blank = NumericTensor(out_key, np.zeros(B200TargetModelBackend.physical_bytes(out_key), np.uint8))
+        total = np.zeros(chains.shape[1], np.float32)
+        for row in chains:
+            total = (total + row).astype(np.float32)
+        got = backend.execute_reduce("sum", dimension, source, blank, formal=formal)
+        assert np.array_equal(logical(backend, out_key, got.destination.storage, np.uint32), total.view(np.uint32))
+        if formal:
+            assert got.evidence.flags == (16 if chains.shape[0] > 1 else got.evidence.flags)
+        for name, pick in (("max", chains.max(0)), ("min", chains.min(0))):
+            got = backend.execute_reduce(name, dimension, source, blank, formal=formal)
+            assert np.array_equal(logical(backend, out_key, got.destination.storage, np.float32), pick)
+
+
+def test_folds_meet_exceptional_values_inside_a_chunk(backend):
+    key, out_key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [130, 3]), PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [1, 3])
+    blank = NumericTensor(out_key, np.zeros(12, np.uint8))
+    x = np.ones((130, 3), np.float32)
+    x[70, 1], x[100, 2] = np.inf, np.float32(3.4e38)
+    x[101, 2] = np.float32(3.4e38)                       # overflows in the middle of a chunk
+    got = backend.execute_reduce("sum", "trailing1", NumericTensor(key, x), blank, formal=True)
+    assert np.array_equal(got.destination.storage.view(np.float32), np.array([130, np.inf, np.inf], np.float32)) and got.evidence.flags & 4
+    x[:, 0] = -0.0
+    for name, want in (("max", 0x80000000), ("min", 0x80000000)):
+        got = backend.execute_reduce(name, "trailing1", NumericTensor(key, x), blank, formal=True)
+        assert got.destination.storage.view(np.uint32)[0] == want
+    x[66, 0] = np.nan
+    got = backend.execute_reduce("max", "trailing1", NumericTensor(key, x), blank, formal=True)
+    assert got.destination.storage.view(np.uint32)[0] == 0x7fc00000
+    with pytest.raises(WB200Error):
+        backend.execute_reduce("max", "trailing1", NumericTensor(key, x), blank)
+
+
+@pytest.mark.parametrize("elements", [(1 << 18) - 1, 1 << 18, (1 << 18) + 1, (9 << 20) + 5])
+def test_storage_in_place_and_in_pieces(backend, elements):
+    rng = np.random.default_rng(elements)
+    x, y = (rng.standard_normal(elements).astype(np.float32) for _ in range(2))
+    key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [elements])
+    got = backend.execute_elementwise("add", [NumericTensor(key, x), NumericTensor(key, y)], NumericTensor(key, np.zeros(4 * elements, np.uint8)))
+    assert np.array_equal(got.destination.storage.view(np.float32), x + y)

@@ -250,7 +250,7 @@ class B200TargetModelBackend:
             req.input_storage[i] = storage.ctypes.data
             req.input_bytes[i] = storage.size
         tmpl = _u8(destination_template.storage)
-        out = tmpl.copy()
+        out = np.empty_like(tmpl)
         req.destination = destination_template.key.c()
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size
         req.max_scalar_evaluations = max_scalar_evaluations
@@ -266,7 +266,7 @@ class B200TargetModelBackend:
         req = abi.ConvertRequest()
         req.opcode, req.rounding_mode = opcode, rounding_mode
         src, tmpl = _u8(source.storage), _u8(destination_template.storage)
-        out = tmpl.copy()
+        out = np.empty_like(tmpl)
         req.source, req.destination = source.key.c(), destination_template.key.c()
         req.source_storage, req.source_bytes = src.ctypes.data, src.size
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size
@@ -281,7 +281,7 @@ class B200TargetModelBackend:
         req = abi.ReduceRequest()
         req.operation, req.dimension = abi.REDUCE_OPS[operation], abi.REDUCE_DIMS[dimension]
         src, tmpl = _u8(source.storage), _u8(destination_template.storage)
-        out = tmpl.copy()
+        out = np.empty_like(tmpl)
         req.input, req.destination = source.key.c(), destination_template.key.c()
         req.input_storage, req.input_bytes = src.ctypes.data, src.size
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size

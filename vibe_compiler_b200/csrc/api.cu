@@ -30,8 +30,9 @@ wb200_status wb200_backend_create(int device, wb200_backend **out) {
   backend->sm_count = prop.multiProcessorCount;
   snprintf(backend->digest, sizeof(backend->digest), "b200:%s:sm_%d%d:abi%d", prop.name, prop.major, prop.minor, WB200_ABI_VERSION);
   cudaError_t err = cudaStreamCreateWithFlags(&backend->stream, cudaStreamNonBlocking);
-  if (err == cudaSuccess) err = cudaMalloc(&backend->d_status, 2 * sizeof(int));
-  if (err == cudaSuccess) err = cudaMemset(backend->d_status, 0, 2 * sizeof(int));
+  if (err == cudaSuccess) err = cudaHostAlloc(reinterpret_cast<void **>(&backend->h_status), 2 * sizeof(int), cudaHostAllocMapped);
+  if (err == cudaSuccess) err = cudaHostGetDevicePointer(reinterpret_cast<void **>(&backend->d_status), backend->h_status, 0);
+  if (err == cudaSuccess) backend->h_status[0] = backend->h_status[1] = 0;
   if (err != cudaSuccess) {
     delete backend;
     return fail(WB200_ERR_CUDA, std::string("backend setup: ") + cudaGetErrorString(err));
@@ -46,7 +47,8 @@ void wb200_backend_destroy(wb200_backend *backend) {
   cudaStreamSynchronize(backend->stream);
   for (auto &slot : backend->slots)
     if (slot.ptr) cudaFree(slot.ptr);
-  if (backend->d_status) cudaFree(backend->d_status);
+  if (backend->h_status) cudaFreeHost(backend->h_status);
+  if (backend->stage) cudaFreeHost(backend->stage);
   for (cudaStream_t aux : backend->aux_stream)
     if (aux) { cudaStreamSynchronize(aux); cudaStreamDestroy(aux); }
   for (cudaEvent_t event : backend->aux_event)

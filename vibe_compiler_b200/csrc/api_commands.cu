@@ -2,7 +2,7 @@
 // its numeric backends, executed on physical storage bytes. Validation mirrors
 // lib/Wafer/Simulator/Reference/ManagedReferenceTargetModel.cpp:301-319, 344-364, 381-400 and
 // lib/Wafer/Simulator/OneDNN/OneDNNGemmAdapter.cpp:176-210.
-#include "backend.h"
+#include "command_io.h"
 
 using namespace wb200;
 
@@ -129,25 +129,26 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   }
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_lhs, *d_rhs, *d_dst, *d_psum = nullptr;
-  if ((st = backend->buffer(0, r->lhs_bytes, &d_lhs)) != WB200_OK) return st;
-  if ((st = backend->buffer(1, r->rhs_bytes, &d_rhs)) != WB200_OK) return st;
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
-  if (r->has_psum && (st = backend->buffer(3, r->psum_bytes, &d_psum)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_lhs, r->lhs_storage, r->lhs_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_rhs, r->rhs_storage, r->rhs_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
-  if (r->has_psum) WB200_CUDA_CHECK(cudaMemcpyAsync(d_psum, r->psum_storage, r->psum_bytes, cudaMemcpyHostToDevice, stream));
+  // The tensor policy unpacks each operand once; the bit-exact kernel reads operands (and nothing else) again per output tile.
+  const bool reread = r->policy == WB200_GEMM_FORMAL;
+  CommandIO io(backend, r->lhs_bytes + r->rhs_bytes + r->destination_bytes + (r->has_psum ? r->psum_bytes : 0));
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_lhs, *d_rhs, *d_psum = nullptr;
+  uint8_t *d_dst;
+  if ((st = io.input(0, r->lhs_storage, r->lhs_bytes, &d_lhs, reread)) != WB200_OK) return st;
+  if ((st = io.input(1, r->rhs_storage, r->rhs_bytes, &d_rhs, reread)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(g.dst_map), &d_dst)) != WB200_OK) return st;
+  if (r->has_psum && (st = io.input(3, r->psum_storage, r->psum_bytes, &d_psum)) != WB200_OK) return st;
   g.m = r->m; g.k = r->k; g.n = r->n; g.batch = r->batch_count;
   g.in_format = r->lhs.format; g.out_format = r->destination.format;
   g.lhs_transposed = lt; g.rhs_transposed = rt; g.has_psum = r->has_psum ? 1 : 0;
-  g.lhs = static_cast<const uint8_t *>(d_lhs); g.rhs = static_cast<const uint8_t *>(d_rhs);
-  g.psum = static_cast<const uint8_t *>(d_psum); g.dst = static_cast<uint8_t *>(d_dst);
+  g.lhs = d_lhs; g.rhs = d_rhs;
+  g.psum = d_psum; g.dst = d_dst;
   const uint64_t launches_before = backend->launches;
   const char *implementation = "";
   if ((st = run_device_gemm(backend, g, r->policy, 4, stream, &implementation)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  if ((st = read_device_status(backend, stream, nullptr)) != WB200_OK) return st;
+  if ((st = io.finish(nullptr)) != WB200_OK) return st;
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   *handled = 1;
   fill_evidence(backend, evidence, implementation);
   if (evidence) {
@@ -189,24 +190,21 @@ wb200_status wb200_elementwise(wb200_backend *backend, const wb200_elementwise_r
   if ((st = check_budget(backend, map.element_count, r->max_scalar_evaluations, total_bytes, logical)) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_in[2] = {nullptr, nullptr}, *d_dst;
-  for (int i = 0; i < arity; ++i) {
-    if ((st = backend->buffer(i, r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
-    WB200_CUDA_CHECK(cudaMemcpyAsync(d_in[i], r->input_storage[i], r->input_bytes[i], cudaMemcpyHostToDevice, stream));
-  }
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
+  CommandIO io(backend, total_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_in[2] = {nullptr, nullptr};
+  uint8_t *d_dst;
+  for (int i = 0; i < arity; ++i)
+    if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  st = launch_elementwise(r->operation, dst.format, arity, static_cast<const uint8_t *>(d_in[0]), static_cast<const uint8_t *>(d_in[1]),
-                          static_cast<uint8_t *>(d_dst), map, backend->d_status + 1, stream);
-  if (st != WB200_OK) return st;
+  if ((st = launch_elementwise(r->operation, dst.format, arity, d_in[0], d_in[1], d_dst, map, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
   int nan_flag = 0;
-  if ((st = read_device_status(backend, stream, &nan_flag)) != WB200_OK) return st;
+  if ((st = io.finish(&nan_flag)) != WB200_OK) return st;
   if (nan_flag) return fail(WB200_ERR_NAN_DOMAIN, "managed-reference tensor: value is outside the non-NaN domain");
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-non-nan-f16-bf16-f32-tensor");
   if (evidence) evidence->device_us = backend->timing_microseconds();
   if (evidence) { evidence->scalar_evaluations = map.element_count; evidence->gpu_launches = 1; }
@@ -257,26 +255,27 @@ wb200_status wb200_elementwise_formal(wb200_backend *backend, const wb200_elemen
   if ((st = check_budget(backend, out_map.element_count, r->max_scalar_evaluations, total_bytes, logical)) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_in[2] = {nullptr, nullptr}, *d_dst, *d_flags;
-  for (int i = 0; i < arity; ++i) {
-    if ((st = backend->buffer(i, r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
-    WB200_CUDA_CHECK(cudaMemcpyAsync(d_in[i], r->input_storage[i], r->input_bytes[i], cudaMemcpyHostToDevice, stream));
-  }
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
+  CommandIO io(backend, total_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_in[2] = {nullptr, nullptr}, *h_flags;
+  uint8_t *d_dst;
+  void *d_flags;
+  for (int i = 0; i < arity; ++i)
+    if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
+  // bit-packed results keep the template's bits behind the last element
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, bool_out || has_padding(out_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->buffer(3, sizeof(uint32_t), &d_flags)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
   WB200_CUDA_CHECK(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), stream));
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  st = launch_elementwise_formal(r->operation, first.format, dst.format, arity, static_cast<const uint8_t *>(d_in[0]),
-                                 static_cast<const uint8_t *>(d_in[1]), static_cast<uint8_t *>(d_dst), in_map, out_map,
+  st = launch_elementwise_formal(r->operation, first.format, dst.format, arity, d_in[0], d_in[1], d_dst, in_map, out_map,
                                  static_cast<uint32_t *>(d_flags), stream);
   if (st != WB200_OK) return st;
   backend->launches += 1;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
-  uint32_t flags = 0;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.read_back(d_flags, sizeof(uint32_t), &h_flags)) != WB200_OK) return st;
+  if ((st = io.finish(nullptr)) != WB200_OK) return st;
+  const uint32_t flags = *reinterpret_cast<const uint32_t *>(h_flags);
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-formal-elementwise");
   if (evidence) evidence->device_us = backend->timing_microseconds();
   if (evidence) { evidence->scalar_evaluations = out_map.element_count; evidence->gpu_launches = 1; evidence->flags = flags; }
@@ -306,22 +305,20 @@ wb200_status wb200_convert(wb200_backend *backend, const wb200_convert_request *
                          2 * static_cast<uint64_t>(dst_map.element_count))) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_src, *d_dst;
-  if ((st = backend->buffer(0, r->source_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_src, r->source_storage, r->source_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
+  CommandIO io(backend, r->source_bytes + r->destination_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_src;
+  uint8_t *d_dst;
+  if ((st = io.input(0, r->source_storage, r->source_bytes, &d_src)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  st = launch_convert(src.format, dst.format, static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), src_map, dst_map,
-                      backend->d_status + 1, stream);
-  if (st != WB200_OK) return st;
+  if ((st = launch_convert(src.format, dst.format, d_src, d_dst, src_map, dst_map, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
   int nan_flag = 0;
-  if ((st = read_device_status(backend, stream, &nan_flag)) != WB200_OK) return st;
+  if ((st = io.finish(&nan_flag)) != WB200_OK) return st;
   if (nan_flag) return fail(WB200_ERR_NAN_DOMAIN, "managed-reference tensor: input value is outside the non-NaN domain");
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-non-nan-f16-bf16-f32-tensor");
   if (evidence) evidence->device_us = backend->timing_microseconds();
   if (evidence) { evidence->scalar_evaluations = dst_map.element_count; evidence->gpu_launches = 1; }
@@ -371,22 +368,20 @@ wb200_status wb200_reduce(wb200_backend *backend, const wb200_reduce_request *r,
                          static_cast<uint64_t>(in_map.element_count) + dst_map.element_count)) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_src, *d_dst;
-  if ((st = backend->buffer(0, r->input_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_src, r->input_storage, r->input_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
+  CommandIO io(backend, r->input_bytes + r->destination_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_src;
+  uint8_t *d_dst;
+  if ((st = io.input(0, r->input_storage, r->input_bytes, &d_src)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  st = launch_reduce(r->operation, in.format, static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), in_map, dst_map, mask,
-                     backend->d_status + 1, stream);
-  if (st != WB200_OK) return st;
+  if ((st = launch_reduce(r->operation, in.format, d_src, d_dst, in_map, dst_map, mask, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
   int nan_flag = 0;
-  if ((st = read_device_status(backend, stream, &nan_flag)) != WB200_OK) return st;
+  if ((st = io.finish(&nan_flag)) != WB200_OK) return st;
   if (nan_flag) return fail(WB200_ERR_NAN_DOMAIN, "managed-reference tensor: reduce left the non-NaN domain");
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-non-nan-f16-bf16-f32-tensor");
   if (evidence) evidence->device_us = backend->timing_microseconds();
   if (evidence) { evidence->scalar_evaluations = in_map.element_count; evidence->gpu_launches = 1; }
@@ -407,22 +402,23 @@ wb200_status wb200_reduce_formal(wb200_backend *backend, const wb200_reduce_requ
                          static_cast<uint64_t>(in_map.element_count) + dst_map.element_count)) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_src, *d_dst, *d_flags;
-  if ((st = backend->buffer(0, r->input_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
+  CommandIO io(backend, r->input_bytes + r->destination_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_src, *h_flags;
+  uint8_t *d_dst;
+  void *d_flags;
+  if ((st = io.input(0, r->input_storage, r->input_bytes, &d_src)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->buffer(3, sizeof(uint32_t), &d_flags)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_src, r->input_storage, r->input_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
   WB200_CUDA_CHECK(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), stream));
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  if ((st = launch_reduce_formal(r->operation, in.format, static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), in_map, dst_map, mask,
-                                 static_cast<uint32_t *>(d_flags), stream)) != WB200_OK) return st;
+  if ((st = launch_reduce_formal(r->operation, in.format, d_src, d_dst, in_map, dst_map, mask, static_cast<uint32_t *>(d_flags), stream)) != WB200_OK) return st;
   backend->launches += 1;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
-  uint32_t flags = 0;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(&flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.read_back(d_flags, sizeof(uint32_t), &h_flags)) != WB200_OK) return st;
+  if ((st = io.finish(nullptr)) != WB200_OK) return st;
+  const uint32_t flags = *reinterpret_cast<const uint32_t *>(h_flags);
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-formal-reduce");
   if (evidence) evidence->device_us = backend->timing_microseconds();
   if (evidence) { evidence->scalar_evaluations = in_map.element_count; evidence->gpu_launches = 1; evidence->flags = flags; }

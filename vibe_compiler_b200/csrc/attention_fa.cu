@@ -602,7 +602,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   __syncthreads();
   if (*abort_word != 0) {
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
-    if (threadIdx.x == 0) atomicExch(p.status, *abort_word);
+    if (threadIdx.x == 0) raise_status(p.status, *abort_word);
     __syncthreads();
   }
   if (warp == 1) {

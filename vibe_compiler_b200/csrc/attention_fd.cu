@@ -605,7 +605,7 @@ __device__ void fd_exchange_rows(const FdTailParams &x, const float *records, in
       unsigned int polls = 0;
       while (ld_acquire_sys(flag) != tag) {
         if ((++polls & 63u) == 0u && clock64() - start > 2000000000LL) {   // about a second: give up, report, carry on
-          atomicExch(x.status, 2);
+          raise_status(x.status, 2);
           break;
         }
       }

@@ -17,7 +17,30 @@ struct wb200_backend {
   int device = 0;
   int sm_count = 0;
   cudaStream_t stream = nullptr;  // used by WB200_MEM_HOST calls
-  int *d_status = nullptr;        // [0] bounded-wait status, [1] NaN flag
+  // [0] bounded-wait status, [1] NaN flag: pinned host memory the kernels store to when something is wrong, so that reading
+  // it takes no copy (d_status: its device address).
+  int *h_status = nullptr, *d_status = nullptr;
+  // Pinned, device-mapped staging area of the command calls (command_io.h), grown on demand up to kMaxStageBytes.
+  static constexpr size_t kMaxStageBytes = size_t(32) << 20;
+  uint8_t *stage = nullptr;
+  size_t stage_bytes = 0, stage_low = 0, stage_high = 0;
+  wb200_status stage_reserve(size_t expected) {
+    size_t wanted = size_t(1) << 20;
+    while (wanted < expected + 4096 && wanted < kMaxStageBytes) wanted *= 2;
+    if (stage_bytes < wanted) {
+      WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+      if (stage) cudaFreeHost(stage);
+      stage = nullptr;
+      stage_bytes = 0;
+      void *area;
+      WB200_CUDA_CHECK(cudaHostAlloc(&area, wanted, cudaHostAllocMapped));
+      stage = static_cast<uint8_t *>(area);
+      stage_bytes = wanted;
+    }
+    stage_low = 0;
+    stage_high = stage_bytes;
+    return WB200_OK;
+  }
   uint64_t launches = 0;
   uint64_t max_total_bytes = 0, max_scratch_bytes = 0;
   char digest[96] = {0};
@@ -149,17 +172,15 @@ inline void fill_evidence(const wb200_backend *backend, wb200_evidence *evidence
   strncpy(evidence->implementation, implementation, sizeof(evidence->implementation) - 1);
 }
 
-// Reads and clears the device status words. status[0] != 0 -> a bounded wait gave up.
+// Waits for `stream`, then reads and clears the status words. status[0] != 0 -> a bounded wait gave up.
 inline wb200_status read_device_status(wb200_backend *backend, cudaStream_t stream, int *nan_flag) {
-  int host[2] = {0, 0};
-  WB200_CUDA_CHECK(cudaMemcpyAsync(host, backend->d_status, sizeof(host), cudaMemcpyDeviceToHost, stream));
   WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
-  if (host[0] != 0 || host[1] != 0) {
-    WB200_CUDA_CHECK(cudaMemsetAsync(backend->d_status, 0, sizeof(host), stream));
-    WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
-  }
-  if (nan_flag) *nan_flag = host[1];
-  if (host[0] != 0) return fail(WB200_ERR_DEVICE_TIMEOUT, "a device-side bounded wait gave up (status " + std::to_string(host[0]) + ")");
+  volatile int *status = backend->h_status;
+  const int wait = status[0], nan = status[1];
+  if (wait != 0) status[0] = 0;
+  if (nan != 0) status[1] = 0;
+  if (nan_flag) *nan_flag = nan;
+  if (wait != 0) return fail(WB200_ERR_DEVICE_TIMEOUT, "a device-side bounded wait gave up (status " + std::to_string(wait) + ")");
   return WB200_OK;
 }
 
@@ -172,6 +193,9 @@ inline wb200_status check_storage(const wb200_tensor_desc &desc, uint64_t bytes,
     return fail(WB200_ERR_INVALID_ARGUMENT, std::string(what) + " storage size does not match its physical geometry");
   return WB200_OK;
 }
+
+// The physical storage of `map` holds bytes that belong to no element (they keep the destination template's values).
+inline bool has_padding(const LayoutMap &map) { return map.physical_elements != map.element_count; }
 
 inline bool same_shape(const wb200_tensor_desc &a, const wb200_tensor_desc &b) {
   if (a.rank != b.rank) return false;

@@ -1,0 +1,128 @@
+// Host storage in and out of one command call. The reference hands commands over as pageable host vectors; a pageable
+// cudaMemcpyAsync costs 10-40 us each (driver staging and, for results, a synchronisation of its own), more than the
+// commands themselves. Storage goes through one pinned, device-mapped area of the backend instead:
+//   up to kMappedBytes per operand (or result) the kernel reads (writes) the area directly over PCIe - every command
+//   kernel but the formal GEMM touches a byte once - so there is no copy command at all;
+//   larger storage is copied through the area in pieces, so that the CPU copy of a piece overlaps the DMA of the one before.
+// One synchronisation ends the call. A result is copied to the caller only after the call's status words are known.
+#pragma once
+
+#include "backend.h"
+
+namespace wb200 {
+
+class CommandIO {
+ public:
+  static constexpr size_t kMappedBytes = size_t(1) << 20;
+  static constexpr size_t kPieceBytes = size_t(1) << 20;
+
+  // `expected` bytes of host storage will pass through the call (sizes the pinned area, up to its limit).
+  CommandIO(wb200_backend *backend, size_t expected) : backend_(backend), stream_(backend->stream) {
+    status_ = backend->stage_reserve(expected);
+  }
+  wb200_status status() const { return status_; }
+
+  // An operand. `reread`: the kernels read it more than once, so it belongs in device memory (slot `slot`).
+  wb200_status input(size_t slot, const uint8_t *host, size_t bytes, const uint8_t **device, bool reread = false) {
+    if (!reread && bytes <= kMappedBytes) {
+      uint8_t *area = take(bytes);
+      if (area) {
+        memcpy(area, host, bytes);
+        *device = area;
+        return WB200_OK;
+      }
+    }
+    void *buffer;
+    wb200_status st = backend_->buffer(slot, bytes, &buffer);
+    if (st != WB200_OK) return st;
+    *device = static_cast<uint8_t *>(buffer);
+    return upload(buffer, host, bytes);
+  }
+
+  // The result. `padded`: its layout has bytes that are no element, which keep the template's values.
+  wb200_status output(size_t slot, const uint8_t *storage_template, size_t bytes, bool padded, uint8_t **device) {
+    bytes_ = bytes;
+    if (bytes <= kMappedBytes && (mapped_ = take(bytes)) != nullptr) {
+      if (padded) memcpy(mapped_, storage_template, bytes);
+      *device = mapped_;
+      return WB200_OK;
+    }
+    void *buffer;
+    wb200_status st = backend_->buffer(slot, bytes, &buffer);
+    if (st != WB200_OK) return st;
+    *device = device_ = static_cast<uint8_t *>(buffer);
+    return padded ? upload(buffer, storage_template, bytes) : WB200_OK;
+  }
+
+  // A small device word (flags, refusals) to be read back with the result.
+  wb200_status read_back(const void *device_word, size_t bytes, const uint8_t **host) {
+    uint8_t *area = take(bytes);
+    if (!area) return fail(WB200_ERR_LIMIT, "command staging area exhausted");
+    WB200_CUDA_CHECK(cudaMemcpyAsync(area, device_word, bytes, cudaMemcpyDeviceToHost, stream_));
+    *host = area;
+    return WB200_OK;
+  }
+
+  // Ends the device part: everything enqueued has run, the status words are read (and cleared), words of read_back() are
+  // there. *nan_flag as in read_device_status().
+  wb200_status finish(int *nan_flag) { return read_device_status(backend_, stream_, nan_flag); }
+
+  // Copies the result to the caller (after finish(), and after the caller has accepted the status).
+  wb200_status deliver(uint8_t *host) {
+    if (!device_) {
+      memcpy(host, mapped_, bytes_);
+      return WB200_OK;
+    }
+    // two halves of the area alternate: the DMA of a piece overlaps the CPU copy of the one before
+    const size_t piece = kPieceBytes < backend_->stage_bytes / 2 ? kPieceBytes : backend_->stage_bytes / 2;
+    wb200_status st = backend_->auxiliary_streams();   // for the events
+    if (st != WB200_OK) return st;
+    const size_t pieces = (bytes_ + piece - 1) / piece;
+    auto size_of = [&](size_t i) { return i + 1 < pieces ? piece : bytes_ - (pieces - 1) * piece; };
+    auto issue = [&](size_t i) -> wb200_status {
+      WB200_CUDA_CHECK(cudaMemcpyAsync(backend_->stage + (i & 1) * piece, device_ + i * piece, size_of(i), cudaMemcpyDeviceToHost, stream_));
+      WB200_CUDA_CHECK(cudaEventRecord(backend_->aux_event[i & 1], stream_));
+      return WB200_OK;
+    };
+    for (size_t i = 0; i < pieces && i < 2; ++i)
+      if ((st = issue(i)) != WB200_OK) return st;
+    for (size_t i = 0; i < pieces; ++i) {
+      WB200_CUDA_CHECK(cudaEventSynchronize(backend_->aux_event[i & 1]));
+      memcpy(host + i * piece, backend_->stage + (i & 1) * piece, size_of(i));
+      if (i + 2 < pieces && (st = issue(i + 2)) != WB200_OK) return st;
+    }
+    return WB200_OK;
+  }
+
+ private:
+  // What kernels access in place lies at the end of the area, pieces on their way to device memory at its start.
+  uint8_t *take(size_t bytes) {
+    const size_t rounded = (bytes + 255) / 256 * 256;
+    if (backend_->stage_low + rounded > backend_->stage_high) return nullptr;
+    backend_->stage_high -= rounded;
+    return backend_->stage + backend_->stage_high;
+  }
+  wb200_status upload(void *device, const uint8_t *host, size_t bytes) {
+    for (size_t at = 0; at < bytes; at += kPieceBytes) {
+      const size_t count = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
+      if (backend_->stage_low + count > backend_->stage_high) {
+        WB200_CUDA_CHECK(cudaStreamSynchronize(stream_));   // the pieces have left the area
+        backend_->stage_low = 0;
+        if (count > backend_->stage_high) return fail(WB200_ERR_LIMIT, "command staging area exhausted");
+      }
+      uint8_t *piece = backend_->stage + backend_->stage_low;
+      backend_->stage_low += count;
+      memcpy(piece, host + at, count);
+      WB200_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t *>(device) + at, piece, count, cudaMemcpyHostToDevice, stream_));
+    }
+    return WB200_OK;
+  }
+
+  wb200_backend *backend_;
+  cudaStream_t stream_;
+  wb200_status status_;
+  uint8_t *mapped_ = nullptr, *device_ = nullptr;
+  size_t bytes_ = 0;
+};
+
+}  // namespace wb200

@@ -107,6 +107,9 @@ inline bool all_aligned16(const void *a, const void *b = nullptr, const void *c 
   return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
 }
 
+// Status words lie in pinned host memory (any non-zero value tells the host): a plain store, no atomic over PCIe.
+__device__ __forceinline__ void raise_status(int *word, int code) { *reinterpret_cast<volatile int *>(word) = code; }
+
 // ORs every thread's `flags` into *word with one global atomic per block (a single hot word would otherwise serialise
 // one atomic per thread). Every thread of the block must reach the call.
 __device__ __forceinline__ void merge_block_flags(uint32_t *word, uint32_t flags) {

@@ -4,7 +4,7 @@
 // 82-158; the directed-overflow completion of TargetScalarConversion.cpp:60-76, 128-136) and its refusals. Every value
 // is handled as an exact dyadic sign * significand * 2^exponent in integer arithmetic, so no rounding depends on the
 // device's floating-point unit. HBM-bound: source bytes in, destination bytes out.
-#include "backend.h"
+#include "command_io.h"
 
 using namespace wb200;
 
@@ -453,18 +453,19 @@ wb200_status wb200_convert_formal(wb200_backend *backend, const wb200_convert_re
                          2 * static_cast<uint64_t>(dst_map.element_count))) != WB200_OK) return st;
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  void *d_src, *d_dst;
-  if ((st = backend->buffer(0, r->source_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = backend->buffer(2, r->destination_bytes, &d_dst)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_src, r->source_storage, r->source_bytes, cudaMemcpyHostToDevice, stream));
-  WB200_CUDA_CHECK(cudaMemcpyAsync(d_dst, r->destination_template, r->destination_bytes, cudaMemcpyHostToDevice, stream));
+  CommandIO io(backend, r->source_bytes + r->destination_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
+  const uint8_t *d_src;
+  uint8_t *d_dst;
+  if ((st = io.input(0, r->source_storage, r->source_bytes, &d_src, true)) != WB200_OK) return st;   // validated, then converted
+  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   uint32_t flags = 0;
   const uint64_t before = backend->launches;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
-  if ((st = run_convert(backend, route, mode, static_cast<const uint8_t *>(d_src), static_cast<uint8_t *>(d_dst), src_map, dst_map, stream, &flags)) != WB200_OK) return st;
+  if ((st = run_convert(backend, route, mode, d_src, d_dst, src_map, dst_map, stream, &flags)) != WB200_OK) return st;
   if ((st = backend->timing_end(stream)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemcpyAsync(r->destination_out, d_dst, r->destination_bytes, cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  if ((st = io.finish(nullptr)) != WB200_OK) return st;
+  if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   fill_evidence(backend, evidence, "sm100a-formal-convert");
   if (evidence) {
     evidence->device_us = backend->timing_microseconds();

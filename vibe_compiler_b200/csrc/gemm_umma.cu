@@ -262,7 +262,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (*abort_word != 0) {
     // Give copies still in flight time to land before the shared memory is released.
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
-    if (threadIdx.x == 0) atomicExch(p.status, *abort_word);
+    if (threadIdx.x == 0) raise_status(p.status, *abort_word);
     __syncthreads();
   }
   if (warp == 1) {
@@ -445,7 +445,7 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   __syncthreads();
   if (*abort_word != 0) {
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
-    if (threadIdx.x == 0) atomicExch(p.status, *abort_word);
+    if (threadIdx.x == 0) raise_status(p.status, *abort_word);
   }
   cluster_sync_all();     // neither CTA leaves while the partner may still read its shared memory or signal its barriers
   if (warp == 1) {

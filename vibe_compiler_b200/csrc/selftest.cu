@@ -21,7 +21,7 @@ __global__ void bounded_wait_kernel(long long cycle_limit, int *status, long lon
     const long long start = clock64();
     const bool arrived = mbar_wait(smem_u32(&barrier), 0, &abort_word, kDeviceWaitTimeout, cycle_limit);
     *waited_cycles = clock64() - start;
-    if (!arrived) atomicExch(status, abort_word);
+    if (!arrived) raise_status(status, abort_word);
   }
 }
 

@@ -123,7 +123,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSwitchThreads) swit
     __threadfence_system();
     signal_store(p.signals[threadIdx.x] + p.rank, tag);
   }
-  if (threadIdx.x < p.world && !signal_wait(own + threadIdx.x, tag)) atomicExch(p.status, 3);
+  if (threadIdx.x < p.world && !signal_wait(own + threadIdx.x, tag)) raise_status(p.status, 3);
   __syncthreads();
 
   // ---- this rank's slice: switch-side sum, then switch-side broadcast
@@ -161,7 +161,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSwitchThreads) swit
   if (threadIdx.x < p.world) {
     __threadfence_system();
     signal_store(p.signals[threadIdx.x] + p.world + p.rank, tag);
-    if (!signal_wait(own + p.world + threadIdx.x, tag)) atomicExch(p.status, 3);
+    if (!signal_wait(own + p.world + threadIdx.x, tag)) raise_status(p.status, 3);
   }
   __syncthreads();
   if (threadIdx.x == 0) {

@@ -157,7 +157,9 @@ wb200_status wb200_pack(wb200_backend *backend, const wb200_tensor_desc *desc,
 /* ------------------------------------------------------------------ command level (Seam 1) */
 /* All storage pointers are HOST pointers to full physical storage, as the reference's
  * TargetModelNumericTensor::storage vectors are. `destination_out` receives the full physical
- * storage of the result, padding bytes copied from `destination_template`. */
+ * storage of the result, padding bytes copied from `destination_template`. Page-locked storage is read and written where
+ * it lies, without a copy; when a call fails with WB200_ERR_NAN_DOMAIN the contents of a page-locked `destination_out` are
+ * unspecified (pageable storage is left as it was). */
 
 typedef struct wb200_gemm_request { /* FormalGemmOperation + TargetModelNumericOperands */
   wb200_tensor_desc lhs, rhs, destination, psum;

@@ -10,7 +10,9 @@ computes as a whole. Every method calls the device library; nothing is computed 
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import struct
+import threading
 import weakref
 from dataclasses import dataclass, field
 from typing import Optional, Sequence
@@ -44,6 +46,11 @@ def _current_stream() -> int:
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
+@functools.lru_cache(maxsize=4096)
+def _c_descriptor(format: int, layout: int, shape: tuple) -> abi.TensorDesc:
+    return abi.make_desc(format, layout, shape)
+
+
 @dataclass
 class PhysicalTensorDescriptor:
     """Mirror of wafer::PhysicalTensorDescriptor {format, layout, shape}."""
@@ -52,7 +59,8 @@ class PhysicalTensorDescriptor:
     shape: Sequence[int]
 
     def c(self) -> abi.TensorDesc:
-        return abi.make_desc(self.format, self.layout, self.shape)
+        """The C form (shared between equal descriptors: copy it before changing it)."""
+        return _c_descriptor(self.format, self.layout, tuple(self.shape))
 
     @property
     def element_count(self) -> int:
@@ -114,7 +122,39 @@ def _ptr(array: Optional[np.ndarray]) -> Optional[int]:
     return None if array is None else array.ctypes.data
 
 
+class ResultPool:
+    """Storage for command results: page-locked memory (torch's caching host allocator), which the device writes directly
+    and reads directly when the result is the next command's operand. At most `limit` bytes of results that are still
+    referenced are page-locked; beyond that, and for small results, storage is ordinary memory. The bytes return to the
+    allocator with the last reference to the array."""
+
+    def __init__(self, limit: int = 64 << 20, smallest: int = 16 << 10):
+        self.limit, self.smallest, self.live = limit, smallest, 0
+        self._lock = threading.RLock()   # finalizers may run inside empty()
+
+    def _returned(self, size: int):
+        with self._lock:
+            self.live -= size
+
+    def empty(self, size: int) -> np.ndarray:
+        if size < self.smallest:
+            return np.empty(size, dtype=np.uint8)
+        with self._lock:
+            if self.live + size > self.limit:
+                return np.empty(size, dtype=np.uint8)
+            self.live += size
+        try:
+            array = torch.empty(size, dtype=torch.uint8, pin_memory=True).numpy()
+        except RuntimeError:     # no page-locked memory to be had
+            self._returned(size)
+            return np.empty(size, dtype=np.uint8)
+        weakref.finalize(array, self._returned, size).atexit = False
+        return array
+
+
 class B200TargetModelBackend:
+    _results = ResultPool()   # shared by the backends of the process
+
     def __init__(self, device: int = 0):
         self._lib = abi.load()
         handle = C.c_void_p()
@@ -216,7 +256,7 @@ class B200TargetModelBackend:
         req.lhs_orientation, req.rhs_orientation = operation.lhs_orientation, operation.rhs_orientation
         req.policy = policy
         lhs_s, rhs_s, tmpl = _u8(lhs.storage), _u8(rhs.storage), _u8(destination_template.storage)
-        out = np.empty_like(tmpl)
+        out = self._results.empty(tmpl.size)
         req.lhs_storage, req.lhs_bytes = lhs_s.ctypes.data, lhs_s.size
         req.rhs_storage, req.rhs_bytes = rhs_s.ctypes.data, rhs_s.size
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size
@@ -250,7 +290,7 @@ class B200TargetModelBackend:
             req.input_storage[i] = storage.ctypes.data
             req.input_bytes[i] = storage.size
         tmpl = _u8(destination_template.storage)
-        out = np.empty_like(tmpl)
+        out = self._results.empty(tmpl.size)
         req.destination = destination_template.key.c()
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size
         req.max_scalar_evaluations = max_scalar_evaluations
@@ -266,7 +306,7 @@ class B200TargetModelBackend:
         req = abi.ConvertRequest()
         req.opcode, req.rounding_mode = opcode, rounding_mode
         src, tmpl = _u8(source.storage), _u8(destination_template.storage)
-        out = np.empty_like(tmpl)
+        out = self._results.empty(tmpl.size)
         req.source, req.destination = source.key.c(), destination_template.key.c()
         req.source_storage, req.source_bytes = src.ctypes.data, src.size
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size
@@ -281,7 +321,7 @@ class B200TargetModelBackend:
         req = abi.ReduceRequest()
         req.operation, req.dimension = abi.REDUCE_OPS[operation], abi.REDUCE_DIMS[dimension]
         src, tmpl = _u8(source.storage), _u8(destination_template.storage)
-        out = np.empty_like(tmpl)
+        out = self._results.empty(tmpl.size)
         req.input, req.destination = source.key.c(), destination_template.key.c()
         req.input_storage, req.input_bytes = src.ctypes.data, src.size
         req.destination_template, req.destination_out, req.destination_bytes = tmpl.ctypes.data, out.ctypes.data, tmpl.size

@@ -20,9 +20,10 @@ struct DeviceGemm {
 // Runs one GEMM command whose operands already sit on the device. `scratch_slot` is the first of
 // three backend staging slots the tensor path may use for compact operands.
 // `private_staging` (three areas of `private_each` bytes) replaces the backend slots when given: commands of different
-// Tiles that run side by side on streams of their own must not share the compact operands.
+// Tiles that run side by side on streams of their own must not share the compact operands. `host_operands`: the operands are
+// read over PCIe, both in one launch (a replayed command keeps one unpack per operand, as its launch accounting states).
 wb200_status run_device_gemm(wb200_backend *backend, const DeviceGemm &g, int policy, size_t scratch_slot,
-                             cudaStream_t stream, const char **implementation, uint8_t *private_staging = nullptr,
+                             cudaStream_t stream, const char **implementation, bool host_operands, uint8_t *private_staging = nullptr,
                              size_t private_each = 0) {
   const bool tensor_domain = policy == WB200_GEMM_TENSOR && !g.has_psum &&
                              (g.in_format == WB200_BF16 || g.in_format == WB200_F16);
@@ -53,9 +54,15 @@ wb200_status run_device_gemm(wb200_backend *backend, const DeviceGemm &g, int po
     }
     probe.a = c_lhs; probe.b = c_rhs; probe.out = c_dst;
     if (batch_aligned && gemm_umma_supports(probe)) {
-      if ((st = launch_unpack(g.lhs, static_cast<uint8_t *>(c_lhs), g.lhs_map, 2, stream)) != WB200_OK) return st;
-      if ((st = launch_unpack(g.rhs, static_cast<uint8_t *>(c_rhs), g.rhs_map, 2, stream)) != WB200_OK) return st;
-      backend->launches += 2;
+      int unpacks = 2;
+      if (host_operands) {
+        st = launch_unpack_pair(g.lhs, static_cast<uint8_t *>(c_lhs), g.lhs_map, g.rhs, static_cast<uint8_t *>(c_rhs), g.rhs_map, 2, &unpacks, stream);
+      } else {
+        st = launch_unpack(g.lhs, static_cast<uint8_t *>(c_lhs), g.lhs_map, 2, stream);
+        if (st == WB200_OK) st = launch_unpack(g.rhs, static_cast<uint8_t *>(c_rhs), g.rhs_map, 2, stream);
+      }
+      if (st != WB200_OK) return st;
+      backend->launches += unpacks;
       for (uint32_t b = 0; b < g.batch; ++b) {
         GemmUmmaArgs args = probe;
         args.a = static_cast<uint8_t *>(c_lhs) + static_cast<size_t>(b) * g.m * g.k * in_bytes;
@@ -137,8 +144,8 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   uint8_t *d_dst;
   if ((st = io.input(0, r->lhs_storage, r->lhs_bytes, &d_lhs, reread)) != WB200_OK) return st;
   if ((st = io.input(1, r->rhs_storage, r->rhs_bytes, &d_rhs, reread)) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(g.dst_map), &d_dst)) != WB200_OK) return st;
   if (r->has_psum && (st = io.input(3, r->psum_storage, r->psum_bytes, &d_psum)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(g.dst_map), &d_dst)) != WB200_OK) return st;
   g.m = r->m; g.k = r->k; g.n = r->n; g.batch = r->batch_count;
   g.in_format = r->lhs.format; g.out_format = r->destination.format;
   g.lhs_transposed = lt; g.rhs_transposed = rt; g.has_psum = r->has_psum ? 1 : 0;
@@ -146,7 +153,7 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   g.psum = d_psum; g.dst = d_dst;
   const uint64_t launches_before = backend->launches;
   const char *implementation = "";
-  if ((st = run_device_gemm(backend, g, r->policy, 4, stream, &implementation)) != WB200_OK) return st;
+  if ((st = run_device_gemm(backend, g, r->policy, 4, stream, &implementation, true)) != WB200_OK) return st;
   if ((st = io.finish(nullptr)) != WB200_OK) return st;
   if ((st = io.deliver(r->destination_out)) != WB200_OK) return st;
   *handled = 1;
@@ -196,7 +203,7 @@ wb200_status wb200_elementwise(wb200_backend *backend, const wb200_elementwise_r
   uint8_t *d_dst;
   for (int i = 0; i < arity; ++i)
     if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
   if ((st = launch_elementwise(r->operation, dst.format, arity, d_in[0], d_in[1], d_dst, map, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
@@ -263,7 +270,7 @@ wb200_status wb200_elementwise_formal(wb200_backend *backend, const wb200_elemen
   for (int i = 0; i < arity; ++i)
     if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
   // bit-packed results keep the template's bits behind the last element
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, bool_out || has_padding(out_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, bool_out || has_padding(out_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->buffer(3, sizeof(uint32_t), &d_flags)) != WB200_OK) return st;
   WB200_CUDA_CHECK(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), stream));
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
@@ -310,7 +317,7 @@ wb200_status wb200_convert(wb200_backend *backend, const wb200_convert_request *
   const uint8_t *d_src;
   uint8_t *d_dst;
   if ((st = io.input(0, r->source_storage, r->source_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
   if ((st = launch_convert(src.format, dst.format, d_src, d_dst, src_map, dst_map, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
@@ -373,7 +380,7 @@ wb200_status wb200_reduce(wb200_backend *backend, const wb200_reduce_request *r,
   const uint8_t *d_src;
   uint8_t *d_dst;
   if ((st = io.input(0, r->input_storage, r->input_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
   if ((st = launch_reduce(r->operation, in.format, d_src, d_dst, in_map, dst_map, mask, backend->d_status + 1, stream)) != WB200_OK) return st;
   backend->launches += 1;
@@ -408,7 +415,7 @@ wb200_status wb200_reduce_formal(wb200_backend *backend, const wb200_reduce_requ
   uint8_t *d_dst;
   void *d_flags;
   if ((st = io.input(0, r->input_storage, r->input_bytes, &d_src)) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(dst_map), &d_dst)) != WB200_OK) return st;
   if ((st = backend->buffer(3, sizeof(uint32_t), &d_flags)) != WB200_OK) return st;
   WB200_CUDA_CHECK(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), stream));
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;
@@ -435,7 +442,7 @@ wb200_status wb200_spm_create(wb200_backend *backend, uint64_t base_address, uin
   DeviceGuard guard(backend->device);
   wb200_spm_image *image = new wb200_spm_image{backend, base_address, bytes, nullptr};
   cudaError_t err = cudaMalloc(&image->device, bytes);
-  if (err == cudaSuccess) err = cudaMemset(image->device, 0, bytes);
+  if (err == cudaSuccess) err = cudaMemsetAsync(image->device, 0, bytes, backend->stream);
   if (err != cudaSuccess) { delete image; return fail(WB200_ERR_CUDA, std::string("scratch-pad image: ") + cudaGetErrorString(err)); }
   *out = image;
   return WB200_OK;
@@ -553,7 +560,7 @@ wb200_status enqueue_image_gemm(wb200_spm_image *image, uint64_t lhs, uint64_t r
     return WB200_OK;
   }
   if (defer && deferred) return WB200_OK;   // tensor-core policy: not part of a run, *deferred stays false
-  return run_device_gemm(backend, g, effective_policy, 4, image->work_stream(), &implementation, image->gemm_staging,
+  return run_device_gemm(backend, g, effective_policy, 4, image->work_stream(), &implementation, false, image->gemm_staging,
                          static_cast<size_t>(image->bytes));
 }
 

@@ -4,6 +4,8 @@
 //   up to kMappedBytes per operand (or result) the kernel reads (writes) the area directly over PCIe - every command
 //   kernel but the formal GEMM touches a byte once - so there is no copy command at all;
 //   larger storage is copied through the area in pieces, so that the CPU copy of a piece overlaps the DMA of the one before.
+// Storage that is page-locked already (the results the Python layer hands out, see ResultPool; a caller's own pinned
+// memory) is read and written where it lies, so a chain of commands copies nothing between its calls.
 // One synchronisation ends the call. A result is copied to the caller only after the call's status words are known.
 #pragma once
 
@@ -24,6 +26,13 @@ class CommandIO {
 
   // An operand. `reread`: the kernels read it more than once, so it belongs in device memory (slot `slot`).
   wb200_status input(size_t slot, const uint8_t *host, size_t bytes, const uint8_t **device, bool reread = false) {
+    const bool pinned = page_locked(host, bytes);
+    if (pinned && !reread) {
+      in_place_[in_place_count_] = host;
+      in_place_bytes_[in_place_count_++] = bytes;
+      *device = host;
+      return WB200_OK;
+    }
     if (!reread && bytes <= kMappedBytes) {
       uint8_t *area = take(bytes);
       if (area) {
@@ -36,12 +45,25 @@ class CommandIO {
     wb200_status st = backend_->buffer(slot, bytes, &buffer);
     if (st != WB200_OK) return st;
     *device = static_cast<uint8_t *>(buffer);
+    if (pinned) {
+      WB200_CUDA_CHECK(cudaMemcpyAsync(buffer, host, bytes, cudaMemcpyHostToDevice, stream_));
+      return WB200_OK;
+    }
     return upload(buffer, host, bytes);
   }
 
-  // The result. `padded`: its layout has bytes that are no element, which keep the template's values.
-  wb200_status output(size_t slot, const uint8_t *storage_template, size_t bytes, bool padded, uint8_t **device) {
+  // The result, after all operands. `padded`: its layout has bytes that are no element, which keep the template's values.
+  // `host` is where deliver() puts it.
+  wb200_status output(size_t slot, const uint8_t *storage_template, uint8_t *host, size_t bytes, bool padded, uint8_t **device) {
     bytes_ = bytes;
+    bool overlaps = false;
+    for (int i = 0; i < in_place_count_; ++i) overlaps |= host < in_place_[i] + in_place_bytes_[i] && in_place_[i] < host + bytes;
+    if (!overlaps && page_locked(host, bytes)) {
+      if (padded && host != storage_template) memmove(host, storage_template, bytes);
+      *device = host;
+      in_place_result_ = true;
+      return WB200_OK;
+    }
     if (bytes <= kMappedBytes && (mapped_ = take(bytes)) != nullptr) {
       if (padded) memcpy(mapped_, storage_template, bytes);
       *device = mapped_;
@@ -69,6 +91,7 @@ class CommandIO {
 
   // Copies the result to the caller (after finish(), and after the caller has accepted the status).
   wb200_status deliver(uint8_t *host) {
+    if (in_place_result_) return WB200_OK;
     if (!device_) {
       memcpy(host, mapped_, bytes_);
       return WB200_OK;
@@ -95,6 +118,14 @@ class CommandIO {
   }
 
  private:
+  // Page-locked by the CUDA runtime and addressable by the device at the same, 16-byte aligned address. Small operands are
+  // not worth the query.
+  static bool page_locked(const void *host, size_t bytes) {
+    if (bytes < 16384 || (reinterpret_cast<uintptr_t>(host) & 15u)) return false;
+    cudaPointerAttributes attributes;
+    if (cudaPointerGetAttributes(&attributes, host) != cudaSuccess) { cudaGetLastError(); return false; }
+    return attributes.type == cudaMemoryTypeHost && attributes.devicePointer == host;
+  }
   // What kernels access in place lies at the end of the area, pieces on their way to device memory at its start.
   uint8_t *take(size_t bytes) {
     const size_t rounded = (bytes + 255) / 256 * 256;
@@ -122,6 +153,10 @@ class CommandIO {
   cudaStream_t stream_;
   wb200_status status_;
   uint8_t *mapped_ = nullptr, *device_ = nullptr;
+  bool in_place_result_ = false;
+  const uint8_t *in_place_[4];
+  size_t in_place_bytes_[4];
+  int in_place_count_ = 0;
   size_t bytes_ = 0;
 };
 

@@ -173,6 +173,9 @@ wb200_status launch_reduce(int op, int format, const uint8_t *src, uint8_t *dst,
 // Device codec: compact <-> physical.
 wb200_status launch_unpack(const uint8_t *storage, uint8_t *compact, const LayoutMap &map,
                            int element_bytes, cudaStream_t stream);
+// The same for two tensors, in one launch where both move in 16-byte units (*launches: kernels launched).
+wb200_status launch_unpack_pair(const uint8_t *storage0, uint8_t *compact0, const LayoutMap &map0, const uint8_t *storage1, uint8_t *compact1,
+                                const LayoutMap &map1, int element_bytes, int *launches, cudaStream_t stream);
 wb200_status launch_pack(const uint8_t *compact, uint8_t *storage, const LayoutMap &map,
                          int element_bytes, cudaStream_t stream);
 

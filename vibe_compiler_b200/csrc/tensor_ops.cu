@@ -214,13 +214,18 @@ codec_kernel(const T *src, T *dst, const LayoutMap map, int pack) {
 }
 // The same in 16-byte units: with the channel count a multiple of the unit's elements, a unit never straddles a row, a
 // channel block or the tail's width, so both sides are contiguous and aligned. 256 x 520 two-byte elements: 5.6 -> 2 us.
+// `job` of a launch by blockIdx.y: the two operands of a GEMM travel together (both over PCIe when they lie in host memory).
+struct CodecJob { const uint4 *src; uint4 *dst; LayoutMap map; uint32_t units; };
+struct CodecJobs { CodecJob job[2]; };
 template <int kUnit>
 __global__ void __launch_bounds__(kThreads)
-codec_wide_kernel(const uint4 *src, uint4 *dst, const LayoutMap map, uint32_t units, int pack) {
+codec_wide_kernel(const __grid_constant__ CodecJobs jobs, int pack) {
+  const CodecJob &job = jobs.job[blockIdx.y];
+  const LayoutMap &map = job.map;
   const uint32_t row_units = static_cast<uint32_t>(map.shape[map.rank - 1]) / kUnit;
   const bool sliced = map.layout == WB200_LAYOUT_NCX && map.rank > 1;
   const uint32_t full_c = static_cast<uint32_t>(map.cx_blocks * map.c_block);
-  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < units; u += gridDim.x * blockDim.x) {
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < job.units; u += gridDim.x * blockDim.x) {
     uint32_t outer = u / row_units;
     const uint32_t c = (u - outer * row_units) * kUnit;
     int64_t at = 0;
@@ -235,8 +240,8 @@ codec_wide_kernel(const uint4 *src, uint4 *dst, const LayoutMap map, uint32_t un
     } else {
       at += map.cx_blocks * map.block_outer_elements * map.c_block + outer * map.c0 + (c - full_c);
     }
-    if (pack) dst[at / kUnit] = src[u];
-    else dst[u] = src[at / kUnit];
+    if (pack) job.dst[at / kUnit] = job.src[u];
+    else job.dst[u] = job.src[at / kUnit];
   }
 }
 
@@ -1174,16 +1179,23 @@ int grid_for(int64_t elements) {
   return static_cast<int>(blocks);
 }
 
+bool codec_takes_units(const uint8_t *src, const uint8_t *dst, const LayoutMap &map, int element_bytes) {
+  const bool blocked = map.layout == WB200_LAYOUT_CX || map.layout == WB200_LAYOUT_NCX;
+  return (element_bytes == 2 || element_bytes == 4) && blocked && map.shape[map.rank - 1] % (16 / element_bytes) == 0 && all_aligned16(src, dst) &&
+         map.physical_elements < (1ll << 31);
+}
+CodecJob codec_job(const uint8_t *src, uint8_t *dst, const LayoutMap &map, int element_bytes) {
+  return {reinterpret_cast<const uint4 *>(src), reinterpret_cast<uint4 *>(dst), map, static_cast<uint32_t>(map.element_count * element_bytes / 16)};
+}
+
 wb200_status launch_codec(const uint8_t *src, uint8_t *dst, const LayoutMap &map, int element_bytes, int pack,
                           cudaStream_t stream) {
-  const int64_t bytes = map.element_count * element_bytes, channels = map.shape[map.rank - 1];
-  const bool blocked = map.layout == WB200_LAYOUT_CX || map.layout == WB200_LAYOUT_NCX;
-  if ((element_bytes == 2 || element_bytes == 4) && blocked && channels % (16 / element_bytes) == 0 && all_aligned16(src, dst) &&
-      map.physical_elements < (1ll << 31)) {
-    const uint32_t units = static_cast<uint32_t>(bytes / 16);
-    const int grid = grid_for(units);
-    if (element_bytes == 2) codec_wide_kernel<8><<<grid, kThreads, 0, stream>>>(reinterpret_cast<const uint4 *>(src), reinterpret_cast<uint4 *>(dst), map, units, pack);
-    else codec_wide_kernel<4><<<grid, kThreads, 0, stream>>>(reinterpret_cast<const uint4 *>(src), reinterpret_cast<uint4 *>(dst), map, units, pack);
+  if (codec_takes_units(src, dst, map, element_bytes)) {
+    CodecJobs jobs{};
+    jobs.job[0] = codec_job(src, dst, map, element_bytes);
+    const int grid = grid_for(jobs.job[0].units);
+    if (element_bytes == 2) codec_wide_kernel<8><<<grid, kThreads, 0, stream>>>(jobs, pack);
+    else codec_wide_kernel<4><<<grid, kThreads, 0, stream>>>(jobs, pack);
     WB200_CUDA_CHECK(cudaGetLastError());
     return WB200_OK;
   }
@@ -1468,6 +1480,23 @@ wb200_status launch_reduce(int op, int format, const uint8_t *src, uint8_t *dst,
 
 wb200_status launch_unpack(const uint8_t *storage, uint8_t *compact, const LayoutMap &map, int element_bytes, cudaStream_t stream) {
   return launch_codec(storage, compact, map, element_bytes, 0, stream);
+}
+wb200_status launch_unpack_pair(const uint8_t *storage0, uint8_t *compact0, const LayoutMap &map0, const uint8_t *storage1, uint8_t *compact1,
+                                const LayoutMap &map1, int element_bytes, int *launches, cudaStream_t stream) {
+  if (!codec_takes_units(storage0, compact0, map0, element_bytes) || !codec_takes_units(storage1, compact1, map1, element_bytes)) {
+    *launches = 2;
+    wb200_status st = launch_unpack(storage0, compact0, map0, element_bytes, stream);
+    return st != WB200_OK ? st : launch_unpack(storage1, compact1, map1, element_bytes, stream);
+  }
+  *launches = 1;
+  CodecJobs jobs;
+  jobs.job[0] = codec_job(storage0, compact0, map0, element_bytes);
+  jobs.job[1] = codec_job(storage1, compact1, map1, element_bytes);
+  const dim3 grid(grid_for(jobs.job[0].units > jobs.job[1].units ? jobs.job[0].units : jobs.job[1].units), 2);
+  if (element_bytes == 2) codec_wide_kernel<8><<<grid, kThreads, 0, stream>>>(jobs, 0);
+  else codec_wide_kernel<4><<<grid, kThreads, 0, stream>>>(jobs, 0);
+  WB200_CUDA_CHECK(cudaGetLastError());
+  return WB200_OK;
 }
 wb200_status launch_pack(const uint8_t *compact, uint8_t *storage, const LayoutMap &map, int element_bytes, cudaStream_t stream) {
   return launch_codec(compact, storage, map, element_bytes, 1, stream);

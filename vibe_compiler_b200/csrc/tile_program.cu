@@ -1593,12 +1593,12 @@ wb200_status wb200_tile_program_load(wb200_backend *backend, const char *const *
     DeviceGuard guard(backend->device);
     program->ddr = wb200_spm_image{backend, kDdrBase, program->ddr_bytes, nullptr};
     WB200_CUDA_CHECK(cudaMalloc(&program->ddr.device, program->ddr_bytes));
-    WB200_CUDA_CHECK(cudaMemset(program->ddr.device, 0, program->ddr_bytes));
+    WB200_CUDA_CHECK(cudaMemsetAsync(program->ddr.device, 0, program->ddr_bytes, backend->stream));
     program->spm.assign(tile_count, wb200_spm_image{backend, 0, program->spm_bytes, nullptr});
     for (uint32_t t = 0; t < tile_count; ++t) {
       // the second half of each allocation is the Tile's private staging area for in-place gather / scatter
       cudaError_t err = cudaMalloc(&program->spm[t].device, 2 * program->spm_bytes);
-      if (err == cudaSuccess) err = cudaMemset(program->spm[t].device, 0, 2 * program->spm_bytes);
+      if (err == cudaSuccess) err = cudaMemsetAsync(program->spm[t].device, 0, 2 * program->spm_bytes, backend->stream);
       cudaStream_t tile_stream = nullptr;
       if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&tile_stream, cudaStreamNonBlocking);
       if (err == cudaSuccess) program->tile_streams.push_back(tile_stream);

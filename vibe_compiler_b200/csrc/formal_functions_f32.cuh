@@ -16,8 +16,10 @@
 
 #if defined(__CUDACC__)
 #define WB200_HD __host__ __device__ __forceinline__
+#define WB200_HD_COLD __host__ __device__ __noinline__
 #else
 #define WB200_HD inline
+#define WB200_HD_COLD inline
 #endif
 
 namespace wb200 {
@@ -300,8 +302,9 @@ WB200_HD bool tiny_after_rounding_dd(double value, int precision, double min_nor
 
 enum Function { kSqrt, kRsqrt, kLog2, kLn, kPow2, kExp, kSin, kCos, kTanh, kSigmoid, kSoftplus };
 
-// The accurate step: the function of a finite, non-special binary32 operand x (as binary64) in double-double.
-WB200_HD dd evaluate_dd(int function, double x) {
+// The accurate step: the function of a finite, non-special binary32 operand x (as binary64) in double-double. Out of line:
+// about one operand in four million comes here, and its thousands of instructions would sit in every caller's loop.
+WB200_HD_COLD static dd evaluate_dd(int function, double x) {
   switch (function) {
     case kSqrt: {
       const double y = sqrt(x);
@@ -415,6 +418,7 @@ WB200_HD uint32_t correctly_rounded(int function, bool tf32, uint32_t a, uint32_
   pun.u = a;
   const double x = static_cast<double>(pun.f);
   bool exact = false;
+  double exact_value = 0.0;   // the function's value where `exact`
   switch (function) {
     case kSqrt:
       if (zero) return finish(a, 0);
@@ -425,14 +429,14 @@ WB200_HD uint32_t correctly_rounded(int function, bool tf32, uint32_t a, uint32_
       if (zero) return finish(negative ? neg_inf : pos_inf, kDivByZero);
       if (negative) return finish(canonical_nan, kInvalid);
       if (inf) return finish(0u, 0);
-      { int e; exact = frexp(x, &e) == 0.5 && ((e - 1) & 1) == 0; }
+      { int e; exact = frexp(x, &e) == 0.5 && ((e - 1) & 1) == 0; if (exact) exact_value = ldexp(1.0, -((e - 1) / 2)); }
       break;
     case kLog2:
     case kLn:
       if (zero) return finish(neg_inf, kDivByZero);
       if (negative) return finish(canonical_nan, kInvalid);
       if (inf) return finish(pos_inf, 0);
-      if (function == kLog2) { int e; exact = frexp(x, &e) == 0.5; }
+      if (function == kLog2) { int e; exact = frexp(x, &e) == 0.5; exact_value = static_cast<double>(e - 1); }
       else exact = x == 1.0;
       break;
     case kPow2:
@@ -442,6 +446,7 @@ WB200_HD uint32_t correctly_rounded(int function, bool tf32, uint32_t a, uint32_
       // far outside the result range: the rounding is decided (and the evaluations below stay in their domain)
       if (x >= 200.0) return finish(pos_inf, kOverflow | kInexact);
       if (x <= -200.0) return finish(0u, kUnderflow | kInexact);
+      if (exact) exact_value = ldexp(1.0, static_cast<int>(x));   // e^0 or 2^n
       break;
     case kSin:
     case kCos:
@@ -465,15 +470,17 @@ WB200_HD uint32_t correctly_rounded(int function, bool tf32, uint32_t a, uint32_
       if (x <= -200.0) return finish(0u, kUnderflow | kInexact);
       break;
   }
-  // first step
-  const double value = evaluate_f64(function, x);
+  // first step (the exact cases - e^0 among them, which every row of a softmax meets - need no second one)
+  const double value = exact ? exact_value : evaluate_f64(function, x);
   uint32_t bits;
-  {
+  if (exact) {
+    bits = tf32 ? round_nearest_tf32(dd{exact_value, 0.0}) : round_nearest_f32(dd{exact_value, 0.0});
+  } else {
     const double slack = fabs(value) * 0x1p-47;
     const dd low = {value - slack, 0.0}, high = {value + slack, 0.0};
     const uint32_t bits_low = tf32 ? round_nearest_tf32(low) : round_nearest_f32(low);
     const uint32_t bits_high = tf32 ? round_nearest_tf32(high) : round_nearest_f32(high);
-    if (bits_low == bits_high && !exact) {
+    if (bits_low == bits_high) {
       bits = bits_low;
     } else {
       if (second_step) *second_step = true;

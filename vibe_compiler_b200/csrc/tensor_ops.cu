@@ -672,14 +672,54 @@ formal_elementwise_kernel(int runtime_op, int runtime_format, int out_format, in
   merge_block_flags(flags_word, flags);
 }
 
-// One step of a chain on a thread's eight values. The switch gives every arithmetic operation its own copy of the scalar
+// Short vectors in linear layouts: one element per thread in blocks of 128, 32-bit indexes. With eight elements per thread a
+// Tile-sized vector runs on a handful of warps that evaluate their elements one after the other (4096 f32: 3.7 -> 2 us; a
+// repeated-unit operand also lost its 64-bit remainders). Bool operands and results stay with the group kernel.
+constexpr int kShortVector = 1 << 15, kShortThreads = 128;
+__device__ __forceinline__ uint32_t rhs_bits(const uint8_t *in1, const RhsBroadcast &rhs, uint32_t i, int format) {
+  if (rhs.mode == WB200_RHS_SCALAR) return rhs.parameter;
+  if (rhs.mode == WB200_RHS_UNIT) i %= rhs.parameter;
+  else if (rhs.mode == WB200_RHS_GROUP) i = i / rhs.parameter * 64u + i % 64u;
+  return load_element_bits(in1, i, format);
+}
+template <int kOp, int kFormat>
+__global__ void __launch_bounds__(kShortThreads)
+formal_elementwise_short_kernel(int out_format, int input_count, const uint8_t *in0, const uint8_t *in1, uint8_t *dst, uint32_t count,
+                                const RhsBroadcast rhs, uint32_t *flags_word) {
+  const uint32_t i = blockIdx.x * kShortThreads + threadIdx.x;
+  uint32_t flags = 0;
+  if (i < count) {
+    const uint32_t a = load_element_bits(in0, i, kFormat), b = input_count > 1 ? rhs_bits(in1, rhs, i, kFormat) : 0u;
+    store_element_bits(dst, i, out_format, formal_scalar(kOp, kFormat, out_format, a, b, &flags));
+  }
+  merge_block_flags(flags_word, flags);
+}
+
+// The correctly rounded functions in linear layouts, one element per thread, the function fixed at compile time: one
+// evaluator instead of eleven behind a switch, so a block's code fits the instruction cache. kSingle: binary32 and TF32.
+template <int kOp, bool kSingle>
+__global__ void __launch_bounds__(kShortThreads)
+formal_function_kernel(int format, const uint8_t *in0, uint8_t *dst, int64_t count, uint32_t *flags_word) {
+  uint32_t flags = 0;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kShortThreads;
+  const int fixed = kSingle ? (format == WB200_TF32 ? WB200_TF32 : WB200_F32) : (format == WB200_BF16 ? WB200_BF16 : WB200_F16);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kShortThreads + threadIdx.x; i < count; i += stride) {
+    uint32_t element_flags = 0;
+    const uint32_t value = formal_mpfr_scalar(kOp, fixed, load_element_bits(in0, i, fixed), &element_flags);
+    flags |= element_flags;
+    store_element_bits(dst, i, fixed, value);
+  }
+  merge_block_flags(flags_word, flags);
+}
+
+// One step of a chain on a thread's kPer (8 or 1) values. The switch gives every arithmetic operation its own copy of the scalar
 // evaluator with the operation and format fixed at compile time (a few dozen instructions each); only the cases a chain
 // uses are ever fetched. The correctly rounded function family is one out-of-line call.
-template <int kFormat>
-__device__ __forceinline__ void chain_step(int op, uint32_t (&value)[8], const uint32_t (&b)[8], int count, uint32_t &flags) {
+template <int kFormat, int kPer>
+__device__ __forceinline__ void chain_step(int op, uint32_t (&value)[kPer], const uint32_t (&b)[kPer], int count, uint32_t &flags) {
 #define WB200_CHAIN_CASE(OP)                                                             \
   case OP:                                                                               \
-    _Pragma("unroll") for (int e = 0; e < 8; ++e) {                                      \
+    _Pragma("unroll") for (int e = 0; e < kPer; ++e) {                                   \
       if (e < count) {                                                                   \
         uint32_t element_flags = 0;                                                      \
         value[e] = formal_scalar(OP, kFormat, kFormat, value[e], b[e], &element_flags);  \
@@ -704,25 +744,27 @@ __device__ __forceinline__ void chain_step(int op, uint32_t (&value)[8], const u
 }
 
 // A chain of formal elementwise commands (see ElementwiseChain): the running value stays in registers, every step's
-// destination is still written, second operands are read where the step names one. A thread owns the same eight
-// elements of every vector, so a step may read what an earlier step of the chain wrote at the same address.
-template <int kFormat>
-__global__ void __launch_bounds__(kThreads)
+// destination is still written, second operands are read where the step names one. A thread owns the same kPer
+// elements of every vector, so a step may read what an earlier step of the chain wrote at the same address. One element
+// per thread where the vector is short or the chain holds a correctly rounded function (whose eight evaluations in a row
+// made a 64-element subtract - exp - multiply chain take 67 us; it takes 4).
+template <int kFormat, int kPer>
+__global__ void __launch_bounds__(kPer == 1 ? kShortThreads : kThreads)
 formal_chain_kernel(const ElementwiseChain chain, int vector, uint32_t *flags_word) {
   constexpr int format = kFormat, bytes = kFormat == WB200_F32 ? 4 : 2;
-  const int64_t total = chain.count, groups = (total + 7) / 8;
+  const int64_t total = chain.count, groups = (total + kPer - 1) / kPer;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   uint32_t flags = 0;
   for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < groups; g += stride) {
-    const int64_t first = g * 8;
-    const int count = total - first < 8 ? static_cast<int>(total - first) : 8;
-    const bool wide = vector && count == 8;
-    uint32_t value[8], b[8];
+    const int64_t first = g * kPer;
+    const int count = total - first < kPer ? static_cast<int>(total - first) : kPer;
+    const bool wide = kPer == 8 && vector && count == 8;
+    uint32_t value[kPer], b[kPer];
     if (wide) {
-      load_group8(chain.lhs, g, bytes, value);
+      if constexpr (kPer == 8) load_group8(chain.lhs, g, bytes, value);
     } else {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) value[e] = e < count ? load_element_bits(chain.lhs, first + e, format) : 0u;
+      for (int e = 0; e < kPer; ++e) value[e] = e < count ? load_element_bits(chain.lhs, first + e, format) : 0u;
     }
 #pragma unroll 1
     for (int s = 0; s < chain.steps; ++s) {
@@ -730,21 +772,21 @@ formal_chain_kernel(const ElementwiseChain chain, int vector, uint32_t *flags_wo
       uint8_t *dst = chain.step[s].dst;
       if (chain.step[s].rhs_mode == WB200_RHS_SAME) {
         if (wide) {
-          load_group8(rhs, g, bytes, b);
+          if constexpr (kPer == 8) load_group8(rhs, g, bytes, b);
         } else {
 #pragma unroll
-          for (int e = 0; e < 8; ++e) b[e] = e < count ? load_element_bits(rhs, first + e, format) : 0u;
+          for (int e = 0; e < kPer; ++e) b[e] = e < count ? load_element_bits(rhs, first + e, format) : 0u;
         }
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) b[e] = chain.step[s].scalar;
+        for (int e = 0; e < kPer; ++e) b[e] = chain.step[s].scalar;
       }
-      chain_step<kFormat>(chain.step[s].op, value, b, count, flags);
+      chain_step<kFormat, kPer>(chain.step[s].op, value, b, count, flags);
       if (wide) {
-        store_group8(dst, g, bytes, value);
+        if constexpr (kPer == 8) store_group8(dst, g, bytes, value);
       } else {
 #pragma unroll
-        for (int e = 0; e < 8; ++e)
+        for (int e = 0; e < kPer; ++e)
           if (e < count) store_element_bits(dst, first + e, format, value[e]);
       }
     }
@@ -836,72 +878,74 @@ struct FoldPlan {
   int64_t outer_step[3];
   int along_steps;            // consecutive steps are neighbours in memory (the channel is reduced)
 };
-constexpr int kFoldOutputs = 32, kFoldChunk = 64;
+constexpr int kFoldOutputs = 32, kFoldChunk = 64, kFoldPerThread = kFoldOutputs * kFoldChunk / kThreads;
 
 __device__ __forceinline__ int64_t fold_address(const LayoutMap &m, int64_t slice, int64_t outer, int64_t c) {
   if (m.layout == WB200_LAYOUT_TENSOR || m.layout == WB200_LAYOUT_NTENSOR) return outer * m.shape[m.rank - 1] + c;
   return physical_index_nhwc(m, slice, outer, c);
 }
 
-template <bool kFormal, int kCombine, int kFormat>
-__global__ void __launch_bounds__(kThreads)
-fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ FoldPlan plan, int *nan_flag, uint32_t *flags_word) {
-  static_assert(kCombine != WB200_EW_ADD || kFormat == WB200_F32, "sums are f32");
-  constexpr int kPerThread = kFoldOutputs * kFoldChunk / kThreads;
-  __shared__ uint32_t panel[2][kFoldChunk][kFoldOutputs + 1];
-  __shared__ int64_t kept_slice[kFoldOutputs], kept_outer[kFoldOutputs], kept_c[kFoldOutputs];
-  const int tid = threadIdx.x;
-  const int64_t first_output = static_cast<int64_t>(blockIdx.x) * kFoldOutputs;
-  const int outputs = static_cast<int>(min(static_cast<int64_t>(kFoldOutputs), plan.dst.element_count - first_output));
-  if (tid < outputs) {
-    // coordinates the output keeps (the reduced ones are zero)
-    int64_t remaining = first_output + tid, outer = 0, slice = 0, c = 0, scale = 1;
-    const int rank = plan.src.rank;
-    const bool sliced = plan.src.layout == WB200_LAYOUT_NCX && rank > 1;
-    for (int d = rank - 1; d >= 0; --d) {
-      int64_t coord = 0;
-      if (!(plan.reduced_mask & (1u << d))) {
-        coord = remaining % plan.src.shape[d];
-        remaining /= plan.src.shape[d];
-      }
-      if (d == rank - 1) c = coord;
-      else if (d == 0 && sliced) slice = coord;
-      else { outer += coord * scale; scale *= plan.src.shape[d]; }
+// Address arithmetic and the rare full step are out of line: these kernels run for a few microseconds between others, so the
+// instructions they fetch count as much as those they execute.
+__device__ __noinline__ void fold_kept_coordinates(const FoldPlan &plan, int64_t output, int64_t *slice_out, int64_t *outer_out, int64_t *c_out, int64_t *dst_at) {
+  // coordinates the output keeps (the reduced ones are zero), and where it is stored; 64-bit divisions only where needed
+  int64_t remaining = output, outer = 0, slice = 0, c = 0, scale = 1, dst_outer = 0, dst_scale = 1;
+  const int rank = plan.src.rank;
+  const bool sliced = plan.src.layout == WB200_LAYOUT_NCX && rank > 1, narrow = plan.dst.element_count < (1ll << 31);
+#pragma unroll 1
+  for (int d = rank - 1; d >= 0; --d) {
+    const bool reduced = (plan.reduced_mask >> d) & 1u;
+    const int64_t extent = plan.src.shape[d];
+    int64_t coord = 0;
+    if (!reduced) {
+      const int64_t quotient = narrow ? static_cast<uint32_t>(remaining) / static_cast<uint32_t>(extent) : remaining / extent;
+      coord = remaining - quotient * extent;
+      remaining = quotient;
     }
-    kept_slice[tid] = slice; kept_outer[tid] = outer; kept_c[tid] = c;
+    if (d == rank - 1) c = coord;
+    else if (d == 0 && sliced) slice = coord;
+    else {
+      outer += coord * scale;
+      scale *= extent;
+      dst_outer += coord * dst_scale;
+      if (!reduced) dst_scale *= extent;
+    }
   }
-  __syncthreads();
-  auto place = [&](int i, int &out, uint32_t &step) {
-    if (plan.along_steps) { step = (tid & 31) + 32 * (i & 1); out = (tid >> 5) + 8 * (i >> 1); }
-    else { out = tid & 31; step = (tid >> 5) + 8 * i; }
-  };
-  auto fetch = [&](uint32_t base, uint32_t (&v)[kPerThread]) {
+  *slice_out = slice; *outer_out = outer; *c_out = c;
+  *dst_at = fold_address(plan.dst, slice, dst_outer, c);
+}
+__device__ __noinline__ int64_t fold_element(const FoldPlan &plan, int64_t slice, int64_t outer, int64_t c, uint32_t step) {
+#pragma unroll 1
+  for (int d = plan.count - 1; d >= 0; --d) {
+    const uint32_t quotient = step / plan.size[d], coord = step - quotient * plan.size[d];
+    step = quotient;
+    if (plan.kind[d] == 2) c += coord;
+    else if (plan.kind[d] == 1) outer += coord * plan.outer_step[d];
+    else slice += coord;
+  }
+  return fold_address(plan.src, slice, outer, c);
+}
+template <int kCombine, int kFormat>
+__device__ __noinline__ uint32_t fold_full_steps(const uint32_t *column, int stride, int count, uint32_t acc, uint32_t *flags) {
+#pragma unroll 1
+  for (int s = 0; s < count; ++s) {
+    uint32_t step_flags = 0;
+    acc = formal_scalar(kCombine, kFormat, kFormat, acc, column[s * stride], &step_flags, kFoldCommonCase);
+    *flags |= step_flags;
+  }
+  return acc;
+}
+
+// The chains of a block: `fetch(base, v)` loads this thread's inputs of the chunk at step `base`, `place(i, out, step)` says
+// which output and step element i is. The result of output `tid` is returned in threads tid < outputs.
+template <bool kFormal, int kCombine, int kFormat, typename Fetch, typename Place>
+__device__ __forceinline__ uint32_t fold_block(uint32_t steps, int outputs, Fetch &&fetch, Place &&place, uint32_t &flags, bool &saw_nan) {
+  static_assert(kCombine != WB200_EW_ADD || kFormat == WB200_F32, "sums are f32");
+  __shared__ uint32_t panel[2][kFoldChunk][kFoldOutputs + 1];
+  const int tid = threadIdx.x;
+  auto stage = [&](int which, const uint32_t (&v)[kFoldPerThread]) {
 #pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
-      int out;
-      uint32_t step;
-      place(i, out, step);
-      step += base;
-      v[i] = 0;
-      if (out < outputs && step < plan.steps) {
-        int64_t slice = kept_slice[out], outer = kept_outer[out], c = kept_c[out];
-        uint32_t rest = step;
-#pragma unroll
-        for (int d = 2; d >= 0; --d) {
-          if (d >= plan.count) continue;
-          const uint32_t quotient = d == 0 ? 0u : rest / plan.size[d], coord = rest - quotient * plan.size[d];
-          rest = quotient;
-          if (plan.kind[d] == 2) c += coord;
-          else if (plan.kind[d] == 1) outer += coord * plan.outer_step[d];
-          else slice += coord;
-        }
-        v[i] = load_element_bits(src, fold_address(plan.src, slice, outer, c), kFormat);
-      }
-    }
-  };
-  auto stage = [&](int which, const uint32_t (&v)[kPerThread]) {
-#pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
+    for (int i = 0; i < kFoldPerThread; ++i) {
       int out;
       uint32_t step;
       place(i, out, step);
@@ -919,8 +963,6 @@ fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ Fol
     return static_cast<uint32_t>(v) & (kFormat == WB200_F32 ? 0xffffffffu : 0xffffu);
   };
   uint32_t acc = kCombine == WB200_EW_ADD ? 0u : kCombine == WB200_EW_MAX ? (infinity | sign) : infinity;
-  uint32_t flags = 0;
-  bool saw_nan = false;
   auto fold = [&](int which, int count) {
     const uint32_t (*column)[kFoldOutputs + 1] = panel[which];
     uint32_t top = 0, residual = 0, result;
@@ -955,11 +997,7 @@ fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ Fol
     const bool exceptional = kCombine == WB200_EW_ADD ? top >= infinity : top > infinity;
     if constexpr (kFormal) {
       if (exceptional) {
-        for (int s = 0; s < count; ++s) {
-          uint32_t step_flags = 0;
-          acc = formal_scalar(kCombine, kFormat, kFormat, acc, column[s][tid], &step_flags, kFoldCommonCase);
-          flags |= step_flags;
-        }
+        acc = fold_full_steps<kCombine, kFormat>(&column[0][tid], kFoldOutputs + 1, count, acc, &flags);
         return;
       }
       if (residual) flags |= kFlagInexact;
@@ -968,19 +1006,95 @@ fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ Fol
     }
     acc = result;
   };
-  uint32_t v[kPerThread];
+  uint32_t v[kFoldPerThread];
   fetch(0, v);
   stage(0, v);
   __syncthreads();
   int which = 0;
-  for (uint32_t base = 0; base < plan.steps; base += kFoldChunk, which ^= 1) {
-    const bool more = base + kFoldChunk < plan.steps;
+  for (uint32_t base = 0; base < steps; base += kFoldChunk, which ^= 1) {
+    const bool more = base + kFoldChunk < steps;
     if (more) fetch(base + kFoldChunk, v);
-    if (tid < outputs) fold(which, static_cast<int>(min(static_cast<uint32_t>(kFoldChunk), plan.steps - base)));
+    if (tid < outputs) fold(which, static_cast<int>(min(static_cast<uint32_t>(kFoldChunk), steps - base)));
     if (more) stage(which ^ 1, v);
     __syncthreads();
   }
-  if (tid < outputs) store_element_bits(dst, physical_index(plan.dst, first_output + tid), kFormat, acc);
+  return acc;
+}
+
+// Any rank, layout and set of reduced dimensions.
+template <bool kFormal, int kCombine, int kFormat>
+__global__ void __launch_bounds__(kThreads)
+fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ FoldPlan plan, int *nan_flag, uint32_t *flags_word) {
+  __shared__ int64_t kept_slice[kFoldOutputs], kept_outer[kFoldOutputs], kept_c[kFoldOutputs], kept_dst[kFoldOutputs];
+  const int tid = threadIdx.x;
+  const int64_t first_output = static_cast<int64_t>(blockIdx.x) * kFoldOutputs;
+  const int outputs = static_cast<int>(min(static_cast<int64_t>(kFoldOutputs), plan.dst.element_count - first_output));
+  if (tid < outputs) fold_kept_coordinates(plan, first_output + tid, &kept_slice[tid], &kept_outer[tid], &kept_c[tid], &kept_dst[tid]);
+  __syncthreads();
+  auto place = [&](int i, int &out, uint32_t &step) {
+    if (plan.along_steps) { step = (tid & 31) + 32 * (i & 1); out = (tid >> 5) + 8 * (i >> 1); }
+    else { out = tid & 31; step = (tid >> 5) + 8 * i; }
+  };
+  auto fetch = [&](uint32_t base, uint32_t (&v)[kFoldPerThread]) {
+#pragma unroll
+    for (int i = 0; i < kFoldPerThread; ++i) {
+      int out;
+      uint32_t step;
+      place(i, out, step);
+      step += base;
+      v[i] = 0;
+      if (out < outputs && step < plan.steps)
+        v[i] = load_element_bits(src, fold_element(plan, kept_slice[out], kept_outer[out], kept_c[out], step), kFormat);
+    }
+  };
+  uint32_t flags = 0;
+  bool saw_nan = false;
+  const uint32_t acc = fold_block<kFormal, kCombine, kFormat>(plan.steps, outputs, fetch, place, flags, saw_nan);
+  if (tid < outputs) store_element_bits(dst, kept_dst[tid], kFormat, acc);
+  if constexpr (kFormal) merge_block_flags(flags_word, flags);
+  else if (saw_nan) raise_status(nan_flag, 1);
+}
+
+// One reduced dimension that is not the channel, tensors of fewer than 2^31 elements: the address is linear in the step, and
+// the placement fits a few 32-bit words (a launch of a microsecond or two waits for every line of its parameters).
+struct LinearFold {
+  uint32_t outputs, steps;
+  uint32_t channels;          // outputs are [.., kept outer, channel]
+  uint32_t kept_per_slice;    // kept outer extents of a leading slice (all of them where there are no slices)
+  uint32_t inner;             // extents between the reduced dimension and the channel
+  uint32_t full;              // channels in 64-wide blocks; the others lie `tail` wide behind them (Tensor: 0 and `channels`)
+  uint32_t tail, src_block, src_tail, src_slice, dst_block, dst_tail, dst_slice;   // elements: block pitch, tail start, slice pitch
+  uint32_t reduced_outer;     // extent of the reduced dimension within the outer index (1 when slices are reduced)
+  uint32_t slice_step;        // slices are reduced: elements between steps, else 0
+};
+template <bool kFormal, int kCombine, int kFormat>
+__global__ void __launch_bounds__(kThreads)
+fold_linear_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ LinearFold f, int *nan_flag, uint32_t *flags_word) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  const uint32_t output = blockIdx.x * kFoldOutputs + lane;
+  const int outputs = static_cast<int>(min(static_cast<uint32_t>(kFoldOutputs), f.outputs - blockIdx.x * kFoldOutputs));
+  const uint32_t rest = output / f.channels, c = output - rest * f.channels;
+  const uint32_t slice = rest / f.kept_per_slice, kept = rest - slice * f.kept_per_slice;
+  const uint32_t hi = kept / f.inner, outer = hi * f.inner * f.reduced_outer + (kept - hi * f.inner);
+  const bool blocked = c < f.full;
+  const uint32_t width = blocked ? 64u : f.tail;
+  const uint32_t in_row = blocked ? c & 63u : c - f.full;
+  const uint32_t line = slice * f.src_slice + (blocked ? (c >> 6) * f.src_block : f.src_tail) + outer * width + in_row;
+  const uint32_t line_step = f.slice_step ? f.slice_step : f.inner * width;
+  const uint32_t dst_at = slice * f.dst_slice + (blocked ? (c >> 6) * f.dst_block : f.dst_tail) + kept * width + in_row;
+  auto place = [&](int i, int &out, uint32_t &step) { out = lane; step = (tid >> 5) + 8 * i; };
+  auto fetch = [&](uint32_t base, uint32_t (&v)[kFoldPerThread]) {
+    const uint32_t first = base + (tid >> 5);
+#pragma unroll
+    for (int i = 0; i < kFoldPerThread; ++i) {
+      v[i] = 0;
+      if (lane < outputs && first + 8 * i < f.steps) v[i] = load_element_bits(src, line + (first + 8 * i) * line_step, kFormat);
+    }
+  };
+  uint32_t flags = 0;
+  bool saw_nan = false;
+  const uint32_t acc = fold_block<kFormal, kCombine, kFormat>(f.steps, outputs, fetch, place, flags, saw_nan);
+  if (tid < outputs) store_element_bits(dst, dst_at, kFormat, acc);
   if constexpr (kFormal) merge_block_flags(flags_word, flags);
   else if (saw_nan) raise_status(nan_flag, 1);
 }
@@ -1263,7 +1377,34 @@ wb200_status launch_fold_staged(int op, int format, const uint8_t *src, uint8_t 
   const int64_t blocks = (dst_map.element_count + kFoldOutputs - 1) / kFoldOutputs;
   if (blocks >= (1ll << 31)) return fail(WB200_ERR_LIMIT, "reduction output too large");
   const int grid = static_cast<int>(blocks < 1 ? 1 : blocks);
-#define WB200_FOLD(COMBINE, FORMAT) fold_staged_kernel<kFormal, COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, plan, nan_flag, flags_word)
+  LinearFold linear{};
+  const bool is_linear = plan.count == 1 && plan.kind[0] != 2 && dst_map.element_count > 0 && steps > 0 && src_map.physical_elements < (1ll << 31);
+  if (is_linear) {
+    const bool blocked = src_map.layout == WB200_LAYOUT_CX || src_map.layout == WB200_LAYOUT_NCX;
+    linear.outputs = static_cast<uint32_t>(dst_map.element_count);
+    linear.steps = plan.steps;
+    linear.channels = static_cast<uint32_t>(src_map.shape[rank - 1]);
+    const int64_t slices = sliced ? dst_map.shape[0] : 1;
+    linear.kept_per_slice = static_cast<uint32_t>(dst_map.element_count / linear.channels / slices);
+    linear.inner = plan.kind[0] == 1 ? static_cast<uint32_t>(plan.outer_step[0]) : linear.kept_per_slice;
+    linear.reduced_outer = plan.kind[0] == 1 ? plan.size[0] : 1u;
+    linear.slice_step = plan.kind[0] == 0 ? static_cast<uint32_t>(src_map.outer_slice_stride) : 0u;
+    linear.full = blocked ? static_cast<uint32_t>(src_map.cx_blocks * src_map.c_block) : 0u;
+    linear.tail = blocked ? static_cast<uint32_t>(src_map.c0) : linear.channels;
+    if (blocked) {
+      linear.src_block = static_cast<uint32_t>(src_map.block_outer_elements * src_map.c_block);
+      linear.src_tail = static_cast<uint32_t>(src_map.cx_blocks) * linear.src_block;
+      linear.src_slice = static_cast<uint32_t>(src_map.outer_slice_stride);
+      linear.dst_block = static_cast<uint32_t>(dst_map.block_outer_elements * dst_map.c_block);
+      linear.dst_tail = static_cast<uint32_t>(dst_map.cx_blocks) * linear.dst_block;
+      linear.dst_slice = static_cast<uint32_t>(dst_map.outer_slice_stride);
+    }
+  }
+#define WB200_FOLD(COMBINE, FORMAT)                                                                                                      \
+  do {                                                                                                                                  \
+    if (is_linear) fold_linear_kernel<kFormal, COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, linear, nan_flag, flags_word); \
+    else fold_staged_kernel<kFormal, COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, plan, nan_flag, flags_word);             \
+  } while (0)
 #define WB200_FOLD_FORMATS(COMBINE)                                   \
   if (format == WB200_F32) WB200_FOLD(COMBINE, WB200_F32);            \
   else if (format == WB200_BF16) WB200_FOLD(COMBINE, WB200_BF16);     \
@@ -1309,12 +1450,59 @@ wb200_status launch_elementwise(int op, int format, int input_count, const uint8
   return WB200_OK;
 }
 
+static bool is_function(int op) {
+  return op == WB200_EW_SQRT || op == WB200_EW_RSQRT || (op >= WB200_EW_LOG2 && op <= WB200_EW_EXP) ||
+         (op >= WB200_EW_SIN && op <= WB200_EW_SIGMOID) || op == WB200_EW_SOFTPLUS;
+}
+
 wb200_status launch_elementwise_formal(int op, int in_format, int out_format, int input_count, const uint8_t *in0, const uint8_t *in1,
                                        uint8_t *dst, const LayoutMap &in_map, const LayoutMap &out_map, uint32_t *flags_word,
                                        cudaStream_t stream, RhsBroadcast rhs) {
   auto linear_layout = [](const LayoutMap &m) { return m.layout == WB200_LAYOUT_TENSOR || m.layout == WB200_LAYOUT_NTENSOR; };
-  const bool function_family = op == WB200_EW_SQRT || op == WB200_EW_RSQRT || (op >= WB200_EW_LOG2 && op <= WB200_EW_EXP) ||
-                               (op >= WB200_EW_SIN && op <= WB200_EW_SIGMOID) || op == WB200_EW_SOFTPLUS;
+  const bool function_family = is_function(op);
+  if (function_family && linear_layout(in_map) && linear_layout(out_map)) {
+    int64_t blocks = (out_map.element_count + kShortThreads - 1) / kShortThreads;
+    const int grid = static_cast<int>(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);
+    const bool single = in_format == WB200_F32 || in_format == WB200_TF32;
+#define WB200_FUNCTION(OP)                                                                                                              \
+  case OP:                                                                                                                              \
+    if (single) formal_function_kernel<OP, true><<<grid, kShortThreads, 0, stream>>>(in_format, in0, dst, out_map.element_count, flags_word); \
+    else formal_function_kernel<OP, false><<<grid, kShortThreads, 0, stream>>>(in_format, in0, dst, out_map.element_count, flags_word);      \
+    break;
+    switch (op) {
+      WB200_FUNCTION(WB200_EW_SQRT) WB200_FUNCTION(WB200_EW_RSQRT) WB200_FUNCTION(WB200_EW_LOG2) WB200_FUNCTION(WB200_EW_LN)
+      WB200_FUNCTION(WB200_EW_POW2) WB200_FUNCTION(WB200_EW_EXP) WB200_FUNCTION(WB200_EW_SIN) WB200_FUNCTION(WB200_EW_COS)
+      WB200_FUNCTION(WB200_EW_TANH) WB200_FUNCTION(WB200_EW_SIGMOID) WB200_FUNCTION(WB200_EW_SOFTPLUS)
+      default: return fail(WB200_ERR_UNSUPPORTED, "elementwise operation has no formal evaluation");
+    }
+#undef WB200_FUNCTION
+    WB200_CUDA_CHECK(cudaGetLastError());
+    return WB200_OK;
+  }
+  const bool short_vector = out_map.element_count > 0 && out_map.element_count <= kShortVector && linear_layout(in_map) && linear_layout(out_map) &&
+                            is_float_format(in_format) && is_float_format(out_format);
+  if (short_vector) {
+    const uint32_t count = static_cast<uint32_t>(out_map.element_count);
+    const int grid = static_cast<int>((count + kShortThreads - 1) / kShortThreads);
+#define WB200_SHORT_LAUNCH(OP, FORMAT) \
+  formal_elementwise_short_kernel<OP, FORMAT><<<grid, kShortThreads, 0, stream>>>(out_format, input_count, in0, in1, dst, count, rhs, flags_word)
+#define WB200_SHORT(OP)                                             \
+  case OP:                                                          \
+    if (in_format == WB200_F32) WB200_SHORT_LAUNCH(OP, WB200_F32);  \
+    else if (in_format == WB200_BF16) WB200_SHORT_LAUNCH(OP, WB200_BF16); \
+    else WB200_SHORT_LAUNCH(OP, WB200_F16);                         \
+    WB200_CUDA_CHECK(cudaGetLastError());                           \
+    return WB200_OK;
+    switch (op) {
+      WB200_SHORT(WB200_EW_ABS) WB200_SHORT(WB200_EW_NEG) WB200_SHORT(WB200_EW_RELU) WB200_SHORT(WB200_EW_RECIP) WB200_SHORT(WB200_EW_SQUARE)
+      WB200_SHORT(WB200_EW_MAX) WB200_SHORT(WB200_EW_MIN) WB200_SHORT(WB200_EW_ADD) WB200_SHORT(WB200_EW_SUB) WB200_SHORT(WB200_EW_MUL)
+      WB200_SHORT(WB200_EW_EQ) WB200_SHORT(WB200_EW_NE) WB200_SHORT(WB200_EW_GE) WB200_SHORT(WB200_EW_GT) WB200_SHORT(WB200_EW_LE)
+      WB200_SHORT(WB200_EW_LT)
+      default: break;
+    }
+#undef WB200_SHORT
+#undef WB200_SHORT_LAUNCH
+  }
   // a thread takes eight consecutive elements, or one at a time for the correctly rounded functions
   const int64_t groups = function_family ? out_map.element_count : (out_map.element_count + 7) / 8;
   int64_t blocks = (groups + kThreads - 1) / kThreads;
@@ -1355,13 +1543,21 @@ wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *f
   uintptr_t low_bits = reinterpret_cast<uintptr_t>(chain.lhs);
   for (int s = 0; s < chain.steps; ++s)
     low_bits |= reinterpret_cast<uintptr_t>(chain.step[s].dst) | (chain.step[s].rhs_mode == WB200_RHS_SAME ? reinterpret_cast<uintptr_t>(chain.step[s].rhs) : 0);
-  const int64_t groups = (chain.count + 7) / 8;
-  int64_t blocks = (groups + kThreads - 1) / kThreads;
+  bool one_each = chain.count <= kShortVector;
+  for (int s = 0; s < chain.steps; ++s) one_each |= is_function(chain.step[s].op);
+  const int per = one_each ? 1 : 8, threads = one_each ? kShortThreads : kThreads;
+  int64_t blocks = ((chain.count + per - 1) / per + threads - 1) / threads;
   blocks = blocks < 1 ? 1 : blocks > 148 * 32 ? 148 * 32 : blocks;
   const int grid = static_cast<int>(blocks), vector = (low_bits & 15) == 0;
-  if (chain.format == WB200_F32) formal_chain_kernel<WB200_F32><<<grid, kThreads, 0, stream>>>(chain, vector, flags_word);
-  else if (chain.format == WB200_BF16) formal_chain_kernel<WB200_BF16><<<grid, kThreads, 0, stream>>>(chain, vector, flags_word);
-  else formal_chain_kernel<WB200_F16><<<grid, kThreads, 0, stream>>>(chain, vector, flags_word);
+#define WB200_CHAIN(FORMAT)                                                                                          \
+  do {                                                                                                               \
+    if (one_each) formal_chain_kernel<FORMAT, 1><<<grid, threads, 0, stream>>>(chain, vector, flags_word);           \
+    else formal_chain_kernel<FORMAT, 8><<<grid, threads, 0, stream>>>(chain, vector, flags_word);                    \
+  } while (0)
+  if (chain.format == WB200_F32) WB200_CHAIN(WB200_F32);
+  else if (chain.format == WB200_BF16) WB200_CHAIN(WB200_BF16);
+  else WB200_CHAIN(WB200_F16);
+#undef WB200_CHAIN
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
 }

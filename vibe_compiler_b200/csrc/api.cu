@@ -51,6 +51,7 @@ void wb200_backend_destroy(wb200_backend *backend) {
   if (backend->stage) cudaFreeHost(backend->stage);
   for (cudaStream_t aux : backend->aux_stream)
     if (aux) { cudaStreamSynchronize(aux); cudaStreamDestroy(aux); }
+  for (cudaStream_t capture : backend->capture_stream) cudaStreamDestroy(capture);
   for (cudaEvent_t event : backend->aux_event)
     if (event) cudaEventDestroy(event);
   for (cudaEvent_t event : backend->pipeline_event) cudaEventDestroy(event);

@@ -66,6 +66,17 @@ struct wb200_backend {
     if (cudaEventElapsedTime(&ms, timing_event[0], timing_event[1]) != cudaSuccess) return 0;
     return static_cast<uint32_t>(ms * 1000.f + 0.5f);
   }
+  // Streams a Tile program's invocation is captured on, one per Tile (used during captures only, so the backend's programs
+  // share them; creating sixteen per program took milliseconds).
+  std::vector<cudaStream_t> capture_stream;
+  wb200_status capture_streams(size_t count) {
+    while (capture_stream.size() < count) {
+      cudaStream_t stream;
+      WB200_CUDA_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+      capture_stream.push_back(stream);
+    }
+    return WB200_OK;
+  }
   std::vector<cudaEvent_t> pipeline_event;   // edges of host-buffer pipelines, grown on demand
   uint32_t layer_timeline_parts = 0;         // parts of the last micro-batched decoder layer call (its events are still there)
   wb200_status pipeline_events(size_t count) {

@@ -22,6 +22,12 @@ class CommandIO {
   CommandIO(wb200_backend *backend, size_t expected) : backend_(backend), stream_(backend->stream) {
     status_ = backend->stage_reserve(expected);
   }
+  // A call that fails half way leaves copies in flight out of the area the next call will fill.
+  ~CommandIO() {
+    if (!finished_) cudaStreamSynchronize(stream_);
+  }
+  CommandIO(const CommandIO &) = delete;
+  CommandIO &operator=(const CommandIO &) = delete;
   wb200_status status() const { return status_; }
 
   // An operand. `reread`: the kernels read it more than once, so it belongs in device memory (slot `slot`).
@@ -72,8 +78,39 @@ class CommandIO {
     void *buffer;
     wb200_status st = backend_->buffer(slot, bytes, &buffer);
     if (st != WB200_OK) return st;
-    *device = device_ = static_cast<uint8_t *>(buffer);
+    *device = static_cast<uint8_t *>(buffer);
+    device_ = *device;
     return padded ? upload(buffer, storage_template, bytes) : WB200_OK;
+  }
+
+  // Host storage into device memory of the caller's.
+  wb200_status copy_in(void *device, const uint8_t *host, size_t bytes) {
+    if (!page_locked(host, bytes)) return upload(device, host, bytes);
+    WB200_CUDA_CHECK(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, stream_));
+    return WB200_OK;
+  }
+  // Device memory of the caller's to host storage: enqueued here, complete after finish() and deliver_copies().
+  wb200_status copy_out(uint8_t *host, const void *device, size_t bytes) {
+    uint8_t *area = host;
+    if (!page_locked(host, bytes)) {
+      if (!(area = take(bytes))) {   // larger than the area: piece by piece after the rest
+        late_.push_back({host, static_cast<const uint8_t *>(device), bytes});
+        return WB200_OK;
+      }
+      copies_.push_back({host, area, bytes});
+    }
+    WB200_CUDA_CHECK(cudaMemcpyAsync(area, device, bytes, cudaMemcpyDeviceToHost, stream_));
+    return WB200_OK;
+  }
+  wb200_status deliver_copies() {
+    for (const Copy &copy : copies_) memcpy(copy.host, copy.from, copy.bytes);
+    for (const Copy &copy : late_) {
+      device_ = copy.from;
+      bytes_ = copy.bytes;
+      wb200_status st = deliver(copy.host);
+      if (st != WB200_OK) return st;
+    }
+    return WB200_OK;
   }
 
   // A small device word (flags, refusals) to be read back with the result.
@@ -87,7 +124,10 @@ class CommandIO {
 
   // Ends the device part: everything enqueued has run, the status words are read (and cleared), words of read_back() are
   // there. *nan_flag as in read_device_status().
-  wb200_status finish(int *nan_flag) { return read_device_status(backend_, stream_, nan_flag); }
+  wb200_status finish(int *nan_flag) {
+    finished_ = true;
+    return read_device_status(backend_, stream_, nan_flag);
+  }
 
   // Copies the result to the caller (after finish(), and after the caller has accepted the status).
   wb200_status deliver(uint8_t *host) {
@@ -152,8 +192,11 @@ class CommandIO {
   wb200_backend *backend_;
   cudaStream_t stream_;
   wb200_status status_;
-  uint8_t *mapped_ = nullptr, *device_ = nullptr;
-  bool in_place_result_ = false;
+  struct Copy { uint8_t *host; const uint8_t *from; size_t bytes; };
+  std::vector<Copy> copies_, late_;
+  uint8_t *mapped_ = nullptr;
+  const uint8_t *device_ = nullptr;
+  bool in_place_result_ = false, finished_ = false;
   const uint8_t *in_place_[4];
   size_t in_place_bytes_[4];
   int in_place_count_ = 0;

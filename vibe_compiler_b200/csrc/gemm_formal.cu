@@ -9,6 +9,7 @@
 // keeps its order strictly k-ascending.
 #include "gemm_formal.cuh"
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -73,6 +74,8 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
       }
     }
   };
+  pdl_launch_dependents();
+  pdl_wait();
   float acc = 0.0f, partial = 0.0f;
   fetch(0);
   if (g.psum.base && owns) partial = __uint_as_float(load_element_bits(g.psum.base, small_at(g.psum, batch, row, col), WB200_F32));
@@ -137,6 +140,8 @@ __global__ void __launch_bounds__(256, 4) gemm_formal_tiled_kernel(const FormalP
   // banks, and every row stays 16-byte aligned for the 128-bit reads of the multiply loop
   __shared__ __align__(16) float lhs_panel[kPanelK][kBlockM + 4];   // [k][m]
   __shared__ __align__(16) float rhs_panel[kPanelK][kBlockN + 4];   // [k][n]
+  pdl_launch_dependents();
+  pdl_wait();
   gemm_formal_tile<kResolved, kSeparable, kWide>(p.a, blockIdx.z, blockIdx.y * kBlockM, blockIdx.x * kBlockN, threadIdx.x, true, lhs_panel,
                                                  rhs_panel);
 }
@@ -158,19 +163,19 @@ wb200_status launch_gemm_formal(const GemmFormalArgs &args, cudaStream_t stream)
   SmallGemm small{};
   if ((args.m < 32 || args.n < 32 || tiles <= kFewTiles) && small_gemm(args, &small)) {
     const dim3 grid((args.n + kTile - 1) / kTile, (args.m + kTile - 1) / kTile, args.batch);
-    gemm_formal_small_kernel<<<grid, 256, 0, stream>>>(small);
+    WB200_CUDA_CHECK(launch_dependent(gemm_formal_small_kernel, grid, 256, 0, stream, small));
     WB200_CUDA_CHECK(cudaGetLastError());
     return WB200_OK;
   }
   dim3 grid((args.n + kBlockN - 1) / kBlockN, (args.m + kBlockM - 1) / kBlockM, args.batch);
   if (wide)
-    gemm_formal_tiled_kernel<true, true, true><<<grid, 256, 0, stream>>>(p);
+    WB200_CUDA_CHECK(launch_dependent(gemm_formal_tiled_kernel<true, true, true>, grid, 256, 0, stream, p));
   else if (separable)
-    gemm_formal_tiled_kernel<true, true, false><<<grid, 256, 0, stream>>>(p);
+    WB200_CUDA_CHECK(launch_dependent(gemm_formal_tiled_kernel<true, true, false>, grid, 256, 0, stream, p));
   else if (all_resolved)
-    gemm_formal_tiled_kernel<true, false, false><<<grid, 256, 0, stream>>>(p);
+    WB200_CUDA_CHECK(launch_dependent(gemm_formal_tiled_kernel<true, false, false>, grid, 256, 0, stream, p));
   else
-    gemm_formal_tiled_kernel<false, false, false><<<grid, 256, 0, stream>>>(p);
+    WB200_CUDA_CHECK(launch_dependent(gemm_formal_tiled_kernel<false, false, false>, grid, 256, 0, stream, p));
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
 }

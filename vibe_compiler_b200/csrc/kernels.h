@@ -41,6 +41,24 @@ class PerDeviceOnce {
   bool done_[kMaxDevices] = {};
 };
 
+// Launches a kernel as a programmatic dependent of the one before it on the stream (an edge of that kind in a captured
+// graph): its blocks may be set up while that kernel drains. The kernel must call pdl_wait() before its first access to
+// memory another kernel may write (ptx_sm100.cuh).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 // ---- TMA descriptor encoding (driver entry point fetched at run time; libcuda is not linked)
 // `inner`/`outer`(/`batch`) are extents in elements, innermost first; the box is {box_inner,
 // box_outer(,1)} with 128-byte swizzle; 16-bit elements only.

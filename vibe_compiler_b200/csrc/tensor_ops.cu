@@ -6,6 +6,7 @@
 #include "gemm_formal.cuh"
 #include "kernels.h"
 #include "formal_functions_f32.cuh"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -688,6 +689,8 @@ formal_elementwise_short_kernel(int out_format, int input_count, const uint8_t *
                                 const RhsBroadcast rhs, uint32_t *flags_word) {
   const uint32_t i = blockIdx.x * kShortThreads + threadIdx.x;
   uint32_t flags = 0;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i < count) {
     const uint32_t a = load_element_bits(in0, i, kFormat), b = input_count > 1 ? rhs_bits(in1, rhs, i, kFormat) : 0u;
     store_element_bits(dst, i, out_format, formal_scalar(kOp, kFormat, out_format, a, b, &flags));
@@ -703,6 +706,8 @@ formal_function_kernel(int format, const uint8_t *in0, uint8_t *dst, int64_t cou
   uint32_t flags = 0;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kShortThreads;
   const int fixed = kSingle ? (format == WB200_TF32 ? WB200_TF32 : WB200_F32) : (format == WB200_BF16 ? WB200_BF16 : WB200_F16);
+  pdl_launch_dependents();
+  pdl_wait();
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * kShortThreads + threadIdx.x; i < count; i += stride) {
     uint32_t element_flags = 0;
     const uint32_t value = formal_mpfr_scalar(kOp, fixed, load_element_bits(in0, i, fixed), &element_flags);
@@ -751,6 +756,8 @@ __device__ __forceinline__ void chain_step(int op, uint32_t (&value)[kPer], cons
 template <int kFormat, int kPer>
 __global__ void __launch_bounds__(kPer == 1 ? kShortThreads : kThreads)
 formal_chain_kernel(const ElementwiseChain chain, int vector, uint32_t *flags_word) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int format = kFormat, bytes = kFormat == WB200_F32 ? 4 : 2;
   const int64_t total = chain.count, groups = (total + kPer - 1) / kPer;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -1031,6 +1038,8 @@ fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ Fol
   const int outputs = static_cast<int>(min(static_cast<int64_t>(kFoldOutputs), plan.dst.element_count - first_output));
   if (tid < outputs) fold_kept_coordinates(plan, first_output + tid, &kept_slice[tid], &kept_outer[tid], &kept_c[tid], &kept_dst[tid]);
   __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();
   auto place = [&](int i, int &out, uint32_t &step) {
     if (plan.along_steps) { step = (tid & 31) + 32 * (i & 1); out = (tid >> 5) + 8 * (i >> 1); }
     else { out = tid & 31; step = (tid >> 5) + 8 * i; }
@@ -1082,6 +1091,8 @@ fold_linear_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ Lin
   const uint32_t line = slice * f.src_slice + (blocked ? (c >> 6) * f.src_block : f.src_tail) + outer * width + in_row;
   const uint32_t line_step = f.slice_step ? f.slice_step : f.inner * width;
   const uint32_t dst_at = slice * f.dst_slice + (blocked ? (c >> 6) * f.dst_block : f.dst_tail) + kept * width + in_row;
+  pdl_launch_dependents();
+  pdl_wait();
   auto place = [&](int i, int &out, uint32_t &step) { out = lane; step = (tid >> 5) + 8 * i; };
   auto fetch = [&](uint32_t base, uint32_t (&v)[kFoldPerThread]) {
     const uint32_t first = base + (tid >> 5);
@@ -1402,8 +1413,8 @@ wb200_status launch_fold_staged(int op, int format, const uint8_t *src, uint8_t 
   }
 #define WB200_FOLD(COMBINE, FORMAT)                                                                                                      \
   do {                                                                                                                                  \
-    if (is_linear) fold_linear_kernel<kFormal, COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, linear, nan_flag, flags_word); \
-    else fold_staged_kernel<kFormal, COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, plan, nan_flag, flags_word);             \
+    if (is_linear) WB200_CUDA_CHECK(launch_dependent(fold_linear_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, linear, nan_flag, flags_word)); \
+    else WB200_CUDA_CHECK(launch_dependent(fold_staged_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, plan, nan_flag, flags_word));             \
   } while (0)
 #define WB200_FOLD_FORMATS(COMBINE)                                   \
   if (format == WB200_F32) WB200_FOLD(COMBINE, WB200_F32);            \
@@ -1466,8 +1477,8 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
     const bool single = in_format == WB200_F32 || in_format == WB200_TF32;
 #define WB200_FUNCTION(OP)                                                                                                              \
   case OP:                                                                                                                              \
-    if (single) formal_function_kernel<OP, true><<<grid, kShortThreads, 0, stream>>>(in_format, in0, dst, out_map.element_count, flags_word); \
-    else formal_function_kernel<OP, false><<<grid, kShortThreads, 0, stream>>>(in_format, in0, dst, out_map.element_count, flags_word);      \
+    if (single) WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, true>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, flags_word)); \
+    else WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, false>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, flags_word));      \
     break;
     switch (op) {
       WB200_FUNCTION(WB200_EW_SQRT) WB200_FUNCTION(WB200_EW_RSQRT) WB200_FUNCTION(WB200_EW_LOG2) WB200_FUNCTION(WB200_EW_LN)
@@ -1485,7 +1496,7 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
     const uint32_t count = static_cast<uint32_t>(out_map.element_count);
     const int grid = static_cast<int>((count + kShortThreads - 1) / kShortThreads);
 #define WB200_SHORT_LAUNCH(OP, FORMAT) \
-  formal_elementwise_short_kernel<OP, FORMAT><<<grid, kShortThreads, 0, stream>>>(out_format, input_count, in0, in1, dst, count, rhs, flags_word)
+  WB200_CUDA_CHECK(launch_dependent(formal_elementwise_short_kernel<OP, FORMAT>, grid, kShortThreads, 0, stream, out_format, input_count, in0, in1, dst, count, rhs, flags_word))
 #define WB200_SHORT(OP)                                             \
   case OP:                                                          \
     if (in_format == WB200_F32) WB200_SHORT_LAUNCH(OP, WB200_F32);  \
@@ -1551,8 +1562,8 @@ wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *f
   const int grid = static_cast<int>(blocks), vector = (low_bits & 15) == 0;
 #define WB200_CHAIN(FORMAT)                                                                                          \
   do {                                                                                                               \
-    if (one_each) formal_chain_kernel<FORMAT, 1><<<grid, threads, 0, stream>>>(chain, vector, flags_word);           \
-    else formal_chain_kernel<FORMAT, 8><<<grid, threads, 0, stream>>>(chain, vector, flags_word);                    \
+    if (one_each) WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 1>, grid, threads, 0, stream, chain, vector, flags_word));           \
+    else WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 8>, grid, threads, 0, stream, chain, vector, flags_word));                    \
   } while (0)
   if (chain.format == WB200_F32) WB200_CHAIN(WB200_F32);
   else if (chain.format == WB200_BF16) WB200_CHAIN(WB200_BF16);

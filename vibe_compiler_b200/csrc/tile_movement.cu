@@ -5,6 +5,7 @@
 // layout with payload byte p of the destination layout (lib/Wafer/Simulator/Kernel/TargetModelMovement.cpp:52-146).
 // HBM-bound byte work: algorithmic bytes = payload read once + written once.
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -12,6 +13,8 @@ namespace {
 template <typename Unit>
 __global__ void __launch_bounds__(256) strided_copy_kernel(const uint8_t *src, uint8_t *dst, StridedLayout from, StridedLayout to,
                                                             uint32_t units_per_segment, uint64_t total_units) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < total_units; u += stride) {
     // a command moves at most 4 GiB, so 32-bit division is enough (64-bit division is several times slower)
@@ -34,6 +37,8 @@ __global__ void __launch_bounds__(256) strided_copy_kernel(const uint8_t *src, u
 
 template <typename Element>
 __global__ void __launch_bounds__(256) fill_kernel(Element *dst, Element value, uint64_t count) {
+  pdl_launch_dependents();
+  pdl_wait();
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) dst[i] = value;
 }
@@ -103,11 +108,11 @@ wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, 
   const uint64_t bytes = segments * from.inner_bytes;
   const uintptr_t bases = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
   if (bases % 16 == 0 && layout_aligned(from, 16) && layout_aligned(to, 16)) {
-    strided_copy_kernel<uint4><<<grid_for(bytes / 16), 256, 0, stream>>>(src, dst, from, to, from.inner_bytes / 16, bytes / 16);
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint4>, grid_for(bytes / 16), 256, 0, stream, src, dst, from, to, from.inner_bytes / 16, bytes / 16));
   } else if (bases % 4 == 0 && layout_aligned(from, 4) && layout_aligned(to, 4)) {
-    strided_copy_kernel<uint32_t><<<grid_for(bytes / 4), 256, 0, stream>>>(src, dst, from, to, from.inner_bytes / 4, bytes / 4);
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint32_t>, grid_for(bytes / 4), 256, 0, stream, src, dst, from, to, from.inner_bytes / 4, bytes / 4));
   } else {
-    strided_copy_kernel<uint8_t><<<grid_for(bytes), 256, 0, stream>>>(src, dst, from, to, from.inner_bytes, bytes);
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint8_t>, grid_for(bytes), 256, 0, stream, src, dst, from, to, from.inner_bytes, bytes));
   }
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
@@ -117,9 +122,9 @@ wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int 
   if (count == 0) return WB200_OK;
   if (reinterpret_cast<uintptr_t>(dst) % element_bytes) return fail(WB200_ERR_INVALID_ARGUMENT, "fill destination is not element aligned");
   switch (element_bytes) {
-    case 1: fill_kernel<uint8_t><<<grid_for(count), 256, 0, stream>>>(dst, static_cast<uint8_t>(value_bits), count); break;
-    case 2: fill_kernel<uint16_t><<<grid_for(count), 256, 0, stream>>>(reinterpret_cast<uint16_t *>(dst), static_cast<uint16_t>(value_bits), count); break;
-    case 4: fill_kernel<uint32_t><<<grid_for(count), 256, 0, stream>>>(reinterpret_cast<uint32_t *>(dst), value_bits, count); break;
+    case 1: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint8_t>, grid_for(count), 256, 0, stream, dst, static_cast<uint8_t>(value_bits), count)); break;
+    case 2: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint16_t>, grid_for(count), 256, 0, stream, reinterpret_cast<uint16_t *>(dst), static_cast<uint16_t>(value_bits), count)); break;
+    case 4: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint32_t>, grid_for(count), 256, 0, stream, reinterpret_cast<uint32_t *>(dst), value_bits, count)); break;
     default: return fail(WB200_ERR_UNSUPPORTED, "fill takes 1, 2 or 4 byte elements");
   }
   WB200_CUDA_CHECK(cudaGetLastError());

@@ -15,7 +15,7 @@
 #include <utility>
 #include <vector>
 
-#include "backend.h"
+#include "command_io.h"
 
 namespace wb200 {
 namespace {
@@ -681,7 +681,8 @@ struct wb200_tile_program {
   uint32_t *numeric_words = nullptr;
   // Concurrent replay: one stream per Tile, Direct-DTE transfers as event edges, the whole invocation captured once
   // into a CUDA graph and relaunched on later runs.
-  std::vector<cudaStream_t> tile_streams;
+  std::vector<cudaStream_t> tile_streams;           // the backend's capture streams
+  uint8_t *images = nullptr;                        // every Tile's scratch-pad and staging area, one allocation
   std::vector<cudaEvent_t> edge_events;
   size_t edge_events_used = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};   // one captured invocation per GEMM policy
@@ -1500,6 +1501,11 @@ wb200_status run_all_tiles(wb200_tile_program *program) {
 namespace wb200 {
 namespace {
 
+cudaError_t reset_numeric_words(wb200_tile_program *program, cudaStream_t stream) {
+  const cudaError_t err = cudaMemsetAsync(program->numeric_words, 0, 8, stream);
+  return err != cudaSuccess ? err : cudaMemsetAsync(program->numeric_words + 2, 0xff, 8, stream);
+}
+
 // Interprets the invocation once while the backend stream and the Tile streams are being captured: every Tile's
 // commands land on its own stream, Direct-DTE transfers become event edges between streams, and the result is one
 // instantiated CUDA graph whose branches run concurrently on later launches.
@@ -1528,7 +1534,8 @@ wb200_status capture_invocation(wb200_tile_program *program) {
   wb200_status st = program_event(program, &fork);
   if (st != WB200_OK) return st;
   WB200_CUDA_CHECK(cudaStreamBeginCapture(origin, cudaStreamCaptureModeThreadLocal));
-  cudaError_t err = cudaEventRecord(fork, origin);
+  cudaError_t err = reset_numeric_words(program, origin);
+  if (err == cudaSuccess) err = cudaEventRecord(fork, origin);
   for (size_t t = 0; err == cudaSuccess && t < program->tile_streams.size(); ++t) err = cudaStreamWaitEvent(program->tile_streams[t], fork, 0);
   if (err == cudaSuccess) {
     st = run_all_tiles(program);
@@ -1595,19 +1602,21 @@ wb200_status wb200_tile_program_load(wb200_backend *backend, const char *const *
     WB200_CUDA_CHECK(cudaMalloc(&program->ddr.device, program->ddr_bytes));
     WB200_CUDA_CHECK(cudaMemsetAsync(program->ddr.device, 0, program->ddr_bytes, backend->stream));
     program->spm.assign(tile_count, wb200_spm_image{backend, 0, program->spm_bytes, nullptr});
-    for (uint32_t t = 0; t < tile_count; ++t) {
-      // the second half of each allocation is the Tile's private staging area for in-place gather / scatter
-      cudaError_t err = cudaMalloc(&program->spm[t].device, 2 * program->spm_bytes);
-      if (err == cudaSuccess) err = cudaMemsetAsync(program->spm[t].device, 0, 2 * program->spm_bytes, backend->stream);
-      cudaStream_t tile_stream = nullptr;
-      if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&tile_stream, cudaStreamNonBlocking);
-      if (err == cudaSuccess) program->tile_streams.push_back(tile_stream);
-      if (err != cudaSuccess) {
-        wb200_status failed = fail(WB200_ERR_CUDA, std::string("scratch-pad images: ") + cudaGetErrorString(err));
-        wb200_tile_program_destroy(program.release());
-        return failed;
-      }
+    // one allocation for all Tiles; the second half of each Tile's part is its private staging area for in-place gather / scatter
+    const uint64_t part = (2 * program->spm_bytes + 255) / 256 * 256;
+    cudaError_t err = cudaMalloc(&program->images, part * tile_count);
+    if (err == cudaSuccess) err = cudaMemsetAsync(program->images, 0, part * tile_count, backend->stream);
+    if (err == cudaSuccess && (st = backend->capture_streams(tile_count)) != WB200_OK) {
+      wb200_tile_program_destroy(program.release());
+      return st;
     }
+    if (err != cudaSuccess) {
+      wb200_status failed = fail(WB200_ERR_CUDA, std::string("scratch-pad images: ") + cudaGetErrorString(err));
+      wb200_tile_program_destroy(program.release());
+      return failed;
+    }
+    for (uint32_t t = 0; t < tile_count; ++t) program->spm[t].device = program->images + t * part;
+    program->tile_streams.assign(backend->capture_stream.begin(), backend->capture_stream.begin() + tile_count);
     WB200_CUDA_CHECK(cudaEventCreate(&program->begin));
     WB200_CUDA_CHECK(cudaEventCreate(&program->end));
     WB200_CUDA_CHECK(cudaMalloc(&program->numeric_words, 16));
@@ -1623,15 +1632,13 @@ void wb200_tile_program_destroy(wb200_tile_program *program) {
     cudaStreamSynchronize(program->backend->stream);
     if (program->ddr.device) cudaFree(program->ddr.device);
     if (program->numeric_words) cudaFree(program->numeric_words);
-    for (wb200_spm_image &image : program->spm)
-      if (image.device) cudaFree(image.device);
+    if (program->images) cudaFree(program->images);
     if (program->begin) cudaEventDestroy(program->begin);
     if (program->end) cudaEventDestroy(program->end);
     for (cudaGraphExec_t graph : program->graph)
       if (graph) cudaGraphExecDestroy(graph);
     for (uint8_t *staging : program->gemm_staging)
       if (staging) cudaFree(staging);
-    for (cudaStream_t tile_stream : program->tile_streams) cudaStreamDestroy(tile_stream);
     for (cudaEvent_t event : program->edge_events) cudaEventDestroy(event);
   }
   delete program;
@@ -1693,20 +1700,27 @@ wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *con
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
   wb200_status st;
+  for (size_t i = 0; i < program->outputs.size(); ++i)
+    if (!outputs[i]) return fail(WB200_ERR_INVALID_ARGUMENT, "null output tensor");
+  size_t host_bytes = 256;
+  for (const ExternalTensor &tensor : program->inputs) host_bytes += tensor.compact_bytes + 256;
+  for (const ExternalTensor &tensor : program->outputs) host_bytes += tensor.compact_bytes + 256;
+  CommandIO io(backend, host_bytes);
+  if ((st = io.status()) != WB200_OK) return st;
   for (size_t i = 0; i < program->inputs.size(); ++i) {
     const ExternalTensor &tensor = program->inputs[i];
     if (!inputs[i]) return fail(WB200_ERR_INVALID_ARGUMENT, "null input tensor");
     uint8_t *storage = program->ddr.device + (tensor.address - kDdrBase);
+    const uint8_t *host = static_cast<const uint8_t *>(inputs[i]);
     if (tensor.desc.layout == WB200_LAYOUT_TENSOR || tensor.desc.layout == WB200_LAYOUT_NTENSOR) {
-      WB200_CUDA_CHECK(cudaMemcpyAsync(storage, inputs[i], tensor.compact_bytes, cudaMemcpyHostToDevice, stream));
+      if ((st = io.copy_in(storage, host, tensor.compact_bytes)) != WB200_OK) return st;
     } else {
-      void *compact;
+      void *compact;   // one slot for all tensors: their copies and packs are in stream order
       if ((st = backend->buffer(10, tensor.compact_bytes, &compact)) != WB200_OK) return st;
-      WB200_CUDA_CHECK(cudaMemcpyAsync(compact, inputs[i], tensor.compact_bytes, cudaMemcpyHostToDevice, stream));
+      if ((st = io.copy_in(compact, host, tensor.compact_bytes)) != WB200_OK) return st;
       WB200_CUDA_CHECK(cudaMemsetAsync(storage, 0, tensor.physical_bytes, stream));
       if ((st = launch_pack(static_cast<const uint8_t *>(compact), storage, tensor.map, static_cast<int>(tensor.geometry.element_bytes), stream)) != WB200_OK) return st;
       backend->launches += 1;
-      WB200_CUDA_CHECK(cudaStreamSynchronize(stream));   // the staging slot is reused by the next tensor
     }
   }
   program->execute = true;
@@ -1718,8 +1732,7 @@ wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *con
   static const bool graph_enabled = [] { const char *env = getenv("WB200_REPLAY_GRAPH"); return !(env && env[0] == '0'); }();
   const bool concurrent = graph_enabled && !program->tile_streams.empty();
   if (concurrent && !program->graph[gemm_policy] && (st = capture_invocation(program)) != WB200_OK) return st;
-  WB200_CUDA_CHECK(cudaMemsetAsync(program->numeric_words, 0, 8, stream));
-  WB200_CUDA_CHECK(cudaMemsetAsync(program->numeric_words + 2, 0xff, 8, stream));
+  if (!concurrent) WB200_CUDA_CHECK(reset_numeric_words(program, stream));   // the captured graph begins with it
   WB200_CUDA_CHECK(cudaEventRecord(program->begin, stream));
   if (concurrent) {
     WB200_CUDA_CHECK(cudaGraphLaunch(program->graph[gemm_policy], stream));
@@ -1731,13 +1744,27 @@ wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *con
     if (st != WB200_OK) { cudaStreamSynchronize(stream); return st; }
   }
   WB200_CUDA_CHECK(cudaEventRecord(program->end, stream));
-  if ((st = read_device_status(backend, stream, nullptr)) != WB200_OK) return st;
+  const uint8_t *words;
+  if ((st = io.read_back(program->numeric_words, 16, &words)) != WB200_OK) return st;
+  for (size_t i = 0; i < program->outputs.size(); ++i) {
+    const ExternalTensor &tensor = program->outputs[i];
+    const uint8_t *storage = program->ddr.device + (tensor.address - kDdrBase);
+    const void *from = storage;
+    if (tensor.desc.layout != WB200_LAYOUT_TENSOR && tensor.desc.layout != WB200_LAYOUT_NTENSOR) {
+      void *compact;
+      if ((st = backend->buffer(12 + i, tensor.compact_bytes, &compact)) != WB200_OK) return st;
+      if ((st = launch_unpack(storage, static_cast<uint8_t *>(compact), tensor.map, static_cast<int>(tensor.geometry.element_bytes), stream)) != WB200_OK) return st;
+      backend->launches += 1;
+      from = compact;
+    }
+    if ((st = io.copy_out(static_cast<uint8_t *>(outputs[i]), from, tensor.compact_bytes)) != WB200_OK) return st;
+  }
+  if ((st = io.finish(nullptr)) != WB200_OK) return st;
   float elapsed = 0.f;
   WB200_CUDA_CHECK(cudaEventElapsedTime(&elapsed, program->begin, program->end));
   program->stats.device_ms = elapsed;
-  uint32_t numeric[4] = {0, 0, 0, 0};
-  WB200_CUDA_CHECK(cudaMemcpyAsync(numeric, program->numeric_words, sizeof(numeric), cudaMemcpyDeviceToHost, stream));
-  WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
+  uint32_t numeric[4];
+  memcpy(numeric, words, sizeof(numeric));
   unsigned long long refused;
   memcpy(&refused, numeric + 2, sizeof(refused));
   if (refused != ~0ull) {   // a failed command fails the invocation; outputs are not returned
@@ -1745,21 +1772,7 @@ wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *con
     return convert_refusal(refused);
   }
   program->stats.numeric_flags = numeric[0];
-  for (size_t i = 0; i < program->outputs.size(); ++i) {
-    const ExternalTensor &tensor = program->outputs[i];
-    if (!outputs[i]) return fail(WB200_ERR_INVALID_ARGUMENT, "null output tensor");
-    const uint8_t *storage = program->ddr.device + (tensor.address - kDdrBase);
-    if (tensor.desc.layout == WB200_LAYOUT_TENSOR || tensor.desc.layout == WB200_LAYOUT_NTENSOR) {
-      WB200_CUDA_CHECK(cudaMemcpyAsync(outputs[i], storage, tensor.compact_bytes, cudaMemcpyDeviceToHost, stream));
-    } else {
-      void *compact;
-      if ((st = backend->buffer(10, tensor.compact_bytes, &compact)) != WB200_OK) return st;
-      if ((st = launch_unpack(storage, static_cast<uint8_t *>(compact), tensor.map, static_cast<int>(tensor.geometry.element_bytes), stream)) != WB200_OK) return st;
-      backend->launches += 1;
-      WB200_CUDA_CHECK(cudaMemcpyAsync(outputs[i], compact, tensor.compact_bytes, cudaMemcpyDeviceToHost, stream));
-    }
-    WB200_CUDA_CHECK(cudaStreamSynchronize(stream));
-  }
+  if ((st = io.deliver_copies()) != WB200_OK) return st;
   if (stats) *stats = program->stats;
   return WB200_OK;
 }

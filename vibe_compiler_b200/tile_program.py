@@ -108,7 +108,7 @@ class TileProgram:
             if flat.size != info.compact_bytes:
                 raise ValueError(f"input of {flat.size} bytes where the program expects {info.compact_bytes}")
             held.append(flat)
-        outs = [np.empty(info.compact_bytes, dtype=np.uint8) for info in self.outputs]
+        outs = [B200TargetModelBackend._results.empty(info.compact_bytes) for info in self.outputs]
         in_ptrs = (C.c_void_p * len(held))(*[a.ctypes.data for a in held])
         out_ptrs = (C.c_void_p * len(outs))(*[a.ctypes.data for a in outs])
         stats = abi.ProgramStats()

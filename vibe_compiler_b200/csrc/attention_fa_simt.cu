@@ -1,6 +1,6 @@
 // Flash-attention prefill on CUDA cores, f32 arithmetic throughout: the path for f32 storage (where
 // the 1e-5 parity bound rules out tensor-core inputs narrower than f32) and for shapes the tcgen05
-// kernel does not take. One warp owns one query row and walks the keys in tiles of 32 that the block's sixteen
+// kernel does not take. In the general kernel one warp owns one query row and walks the keys in tiles of 32 that the block's sixteen
 // rows share through shared memory, applying the reference's online update literally
 // (lib/Wafer/Transforms/Linalg/OnlineAttentionDecomposition.cpp:568-594):
 //   s = (q.k)*scale (+mask); m' = max(m, max s); m_e = (m' == -inf ? 0 : m'); alpha = ExpLp(m - m_e);
@@ -8,6 +8,7 @@
 // and the finalize acc * (1/l) of OnlineAttentionMaterialization.cpp:196-262. ExpLp is
 // exp2(x * log2e) in f32 (lib/Wafer/Simulator/Reference/ManagedReferenceTargetModel.cpp:265-270).
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -154,6 +155,245 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) fa_simt_kernel(const Simt
   }
 }
 
+// ---------------------------------------------------------------- f32 storage, head_dim 64 or 128: register tiles
+// A block owns 32 query rows of one (batch, head). Its two groups of 128 threads walk the tiles of 64 keys in turn
+// (group g: tiles g, g + 2, ...), each with a state of its own; the states are merged once at the end. A thread holds
+// 4 rows x 4 keys of the scores (keys tx, tx + 16, ...) and 4 rows x D/16 columns of the accumulator, so 64 multiply-adds
+// follow on 8 shared-memory vectors; the 16 threads of a row are half a warp, which keeps the row statistics and P inside
+// the warp. K and V have a buffer each, refilled by cp.async as soon as the group has read it: K of the next tile travels
+// under the softmax and the PV product, V under the next scores.
+// Bound by the f32 multiply-adds (8 heads x 512 x 512 x 64: 0.27 G, 7 us at the rate of 148 SMs; 128 of them have a block)
+// and the shared-memory vectors that feed them: 73.7 us with a warp per row, 26.6 us now. The warp-per-row kernel stays for
+// other widths, 16-bit storage and unaligned buffers.
+constexpr int kTileRows = 32, kTileKeysWide = 64, kGroupThreads = 128, kGroups = 2;
+
+template <int kD>
+struct TiledSmem {
+  static constexpr int kKPitch = kD + 4;   // rows 16 bytes apart modulo the banks: eight lanes' vectors cover all banks
+  static constexpr int kPPitch = kTileKeysWide + 4;
+  static constexpr int kQ = 0;
+  static constexpr int kGroup0 = kTileRows * kKPitch;
+  static constexpr int kV = kTileKeysWide * kKPitch;                 // within a group
+  static constexpr int kP = kV + kTileKeysWide * kD;
+  static constexpr int kGroupFloats = kP + kTileRows * kPPitch;
+  static constexpr size_t kBytes = (kGroup0 + kGroups * kGroupFloats) * sizeof(float);
+};
+
+template <int kD>
+__global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const SimtParams p) {
+  using L = TiledSmem<kD>;
+  const AttentionArgs &a = p.a;
+  extern __shared__ float4 smem_vectors[];
+  float *smem = reinterpret_cast<float *>(smem_vectors);
+  const int group_id = threadIdx.x / kGroupThreads, tid = threadIdx.x % kGroupThreads;
+  const int tx = tid & 15, ty = tid >> 4;
+  const int row_block = static_cast<int>(gridDim.x - 1 - blockIdx.x) * kTileRows;   // causal: the longest rows first
+  const int bh = blockIdx.y;
+  const int b = bh / a.q_heads, h = bh % a.q_heads;
+  float *q_s = smem + L::kQ;
+  float *k_s = smem + L::kGroup0 + group_id * L::kGroupFloats, *v_s = k_s + L::kV, *p_s = k_s + L::kP;
+  const size_t kv_off = (static_cast<size_t>(b) * a.kv_heads + h / p.group) * static_cast<size_t>(a.kv_len) * kD;
+  const float *q = static_cast<const float *>(a.q) + (static_cast<size_t>(bh) * a.q_len + row_block) * kD;
+  const float *k = static_cast<const float *>(a.k) + kv_off, *v = static_cast<const float *>(a.v) + kv_off;
+
+  auto visible_of = [&](int r) {
+    long long last = static_cast<long long>(p.kv_visible) - 1;
+    if (a.causal && a.causal_offset + r < last) last = a.causal_offset + r;
+    return last < 0 ? 0 : static_cast<int>(last + 1);
+  };
+  const int rows = min(kTileRows, a.q_len - row_block);
+  const int block_visible = visible_of(row_block + rows - 1);   // the last row of the block sees the most keys
+  const int least_visible = visible_of(row_block);
+  int visible[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) visible[i] = ty * 4 + i < rows ? visible_of(row_block + ty * 4 + i) : 0;
+
+  auto fetch = [&](float *dst, int pitch, const float *src, int key0) {
+    const int count = min(kTileKeysWide, block_visible - key0);   // keys behind it are never used
+    for (int e = tid; e < count * (kD / 4); e += kGroupThreads) {
+      const int j = e / (kD / 4), d = e % (kD / 4) * 4;
+      cp_async16(smem_u32(dst + j * pitch + d), src + static_cast<size_t>(key0 + j) * kD + d, 16u);
+    }
+  };
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group_id), "n"(kGroupThreads) : "memory"); };
+
+  for (int e = threadIdx.x; e < kTileRows * (kD / 4); e += kGroups * kGroupThreads) {
+    const int r = e / (kD / 4), d = e % (kD / 4) * 4;
+    cp_async16(smem_u32(q_s + r * L::kKPitch + d), q + static_cast<size_t>(min(r, rows - 1)) * kD + d, 16u);
+  }
+  int key0 = group_id * kTileKeysWide;
+  if (key0 < block_visible) fetch(k_s, L::kKPitch, k, key0);
+  cp_async_commit();
+  if (key0 < block_visible) fetch(v_s, kD, v, key0);
+  cp_async_commit();
+  cp_async_wait<1>();
+  __syncthreads();   // every thread's part of Q (and of the first K) has landed
+
+  float m_run[4], l_run[4], acc[4][kD / 16];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m_run[i] = -INFINITY;
+    l_run[i] = 0.0f;
+#pragma unroll
+    for (int c = 0; c < kD / 16; ++c) acc[i][c] = 0.0f;
+  }
+
+  for (; key0 < block_visible; key0 += kGroups * kTileKeysWide) {
+    const int next = key0 + kGroups * kTileKeysWide;
+    cp_async_wait<1>();   // K of this tile (its V may still travel)
+    group_sync();
+    float s[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
+#pragma unroll 4
+    for (int d = 0; d < kD; d += 4) {
+      float4 qv[4], kv[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) qv[i] = *reinterpret_cast<const float4 *>(q_s + (ty * 4 + i) * L::kKPitch + d);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) kv[j] = *reinterpret_cast<const float4 *>(k_s + (tx + 16 * j) * L::kKPitch + d);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[i][j] = __fmaf_rn(qv[i].x, kv[j].x, s[i][j]);
+          s[i][j] = __fmaf_rn(qv[i].y, kv[j].y, s[i][j]);
+          s[i][j] = __fmaf_rn(qv[i].z, kv[j].z, s[i][j]);
+          s[i][j] = __fmaf_rn(qv[i].w, kv[j].w, s[i][j]);
+        }
+    }
+    group_sync();
+    if (next < block_visible) fetch(k_s, L::kKPitch, k, next);
+    cp_async_commit();
+
+    const bool masked = key0 + kTileKeysWide > least_visible;   // some row of the block does not see the whole tile
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float tile_max = -INFINITY;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s[i][j] = (masked && key0 + tx + 16 * j >= visible[i]) ? -INFINITY : __fmul_rn(s[i][j], a.scale);
+        tile_max = fmaxf(tile_max, s[i][j]);
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) tile_max = fmaxf(tile_max, __shfl_xor_sync(0xffffffffu, tile_max, off));
+      const float m_new = fmaxf(tile_max, m_run[i]);
+      const float m_exp = (m_new == -INFINITY) ? 0.0f : m_new;
+      const float alpha = exp_lp(__fsub_rn(m_run[i], m_exp));
+      float tile_sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float prob = exp_lp(__fsub_rn(s[i][j], m_exp));
+        tile_sum += prob;
+        p_s[(ty * 4 + i) * L::kPPitch + tx + 16 * j] = prob;
+      }
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) tile_sum += __shfl_xor_sync(0xffffffffu, tile_sum, off);
+      l_run[i] = __fadd_rn(__fmul_rn(l_run[i], alpha), tile_sum);
+      m_run[i] = m_new;
+#pragma unroll
+      for (int c = 0; c < kD / 16; ++c) acc[i][c] = __fmul_rn(acc[i][c], alpha);
+    }
+    cp_async_wait<1>();   // V of this tile (K of the next one may still travel)
+    group_sync();         // also: the half warp's P is written
+    if (!masked) {
+#pragma unroll 2
+      for (int j = 0; j < kTileKeysWide; j += 4) {
+        float4 pv[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(p_s + (ty * 4 + i) * L::kPPitch + j);
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+          for (int c = 0; c < kD / 64; ++c) {
+            const float4 vv = *reinterpret_cast<const float4 *>(v_s + (j + jj) * kD + c * 64 + tx * 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float pj = jj == 0 ? pv[i].x : jj == 1 ? pv[i].y : jj == 2 ? pv[i].z : pv[i].w;
+              acc[i][4 * c] = __fmaf_rn(pj, vv.x, acc[i][4 * c]);
+              acc[i][4 * c + 1] = __fmaf_rn(pj, vv.y, acc[i][4 * c + 1]);
+              acc[i][4 * c + 2] = __fmaf_rn(pj, vv.z, acc[i][4 * c + 2]);
+              acc[i][4 * c + 3] = __fmaf_rn(pj, vv.w, acc[i][4 * c + 3]);
+            }
+          }
+      }
+    } else {
+      // A key a row does not see takes no part in its product: 0 * V would turn an infinity there into a NaN.
+      const int count = min(kTileKeysWide, block_visible - key0);
+#pragma unroll 1
+      for (int j = 0; j < count; ++j) {
+        float vv[kD / 16];
+#pragma unroll
+        for (int c = 0; c < kD / 16; ++c) vv[c] = v_s[j * kD + (c / 4) * 64 + tx * 4 + c % 4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float pj = p_s[(ty * 4 + i) * L::kPPitch + j];
+          if (key0 + j < visible[i]) {
+#pragma unroll
+            for (int c = 0; c < kD / 16; ++c) acc[i][c] = __fmaf_rn(pj, vv[c], acc[i][c]);
+          }
+        }
+      }
+    }
+    group_sync();
+    if (next < block_visible) fetch(v_s, kD, v, next);
+    cp_async_commit();
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // Merge: group 1 leaves its states in its own K / V buffers, group 0 folds them in and finalizes.
+  float *state = smem + L::kGroup0 + L::kGroupFloats;   // [32][D], then m [32], l [32]
+  float *stats = state + kTileRows * kD;
+  if (group_id == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+      for (int c = 0; c < kD / 64; ++c)
+        *reinterpret_cast<float4 *>(state + (ty * 4 + i) * kD + c * 64 + tx * 4) =
+            make_float4(acc[i][4 * c], acc[i][4 * c + 1], acc[i][4 * c + 2], acc[i][4 * c + 3]);
+      if (tx == 0) {
+        stats[ty * 4 + i] = m_run[i];
+        stats[kTileRows + ty * 4 + i] = l_run[i];
+      }
+    }
+  }
+  __syncthreads();
+  if (group_id == 1) return;
+  float *out = static_cast<float *>(a.out);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = ty * 4 + i, row = row_block + r;
+    if (r >= rows) continue;
+    const float m_other = stats[r], l_other = stats[kTileRows + r];
+    const float m_all = fmaxf(m_run[i], m_other);
+    const float m_exp = (m_all == -INFINITY) ? 0.0f : m_all;
+    const float mine = exp_lp(__fsub_rn(m_run[i], m_exp)), other = exp_lp(__fsub_rn(m_other, m_exp));
+    const float l_all = __fadd_rn(__fmul_rn(l_run[i], mine), __fmul_rn(l_other, other));
+    float coefficient = __fdiv_rn(1.0f, l_all);
+    if (a.zero_fully_masked && l_all == 0.0f) coefficient = 0.0f;
+    float *dst = out + (a.out_token_major ? ((static_cast<size_t>(b) * a.q_len + row) * a.q_heads + h) * kD : (static_cast<size_t>(bh) * a.q_len + row) * kD);
+#pragma unroll
+    for (int c = 0; c < kD / 64; ++c) {
+      const float4 o = *reinterpret_cast<const float4 *>(state + r * kD + c * 64 + tx * 4);
+      const float others[4] = {o.x, o.y, o.z, o.w};
+      uint32_t w[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        w[e] = narrow_bits(__fmul_rn(__fmaf_rn(acc[i][4 * c + e], mine, __fmul_rn(others[e], other)), coefficient), WB200_F32);
+      *reinterpret_cast<uint4 *>(dst + c * 64 + tx * 4) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    if (tx == 0) {
+      const size_t stat = static_cast<size_t>(bh) * a.q_len + row;
+      if (a.lse) a.lse[stat] = (l_all == 0.0f) ? -INFINITY : m_all + logf(l_all);
+      if (a.row_max) a.row_max[stat] = m_all;
+      if (a.row_sum) a.row_sum[stat] = l_all;
+    }
+  }
+}
+
 }  // namespace
 
 wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t stream) {
@@ -167,6 +407,23 @@ wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t strea
   p.group = a.q_heads / a.kv_heads;
   int64_t visible = a.kv_valid < a.kv_len ? a.kv_valid : a.kv_len;
   p.kv_visible = visible < 0 ? 0 : static_cast<int>(visible);
+  // The register-tiled kernel takes every f32 request whose buffers allow 16-byte accesses.
+  const bool aligned = ((reinterpret_cast<uintptr_t>(a.q) | reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v) |
+                         reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0;
+  if (a.format == WB200_F32 && aligned && (a.head_dim == 64 || a.head_dim == 128)) {
+    static PerDeviceOnce attributes;
+    const wb200_status st = attributes.run([]() -> wb200_status {
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<64>::kBytes)));
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<128>::kBytes)));
+      return WB200_OK;
+    });
+    if (st != WB200_OK) return st;
+    const dim3 tiles((a.q_len + kTileRows - 1) / kTileRows, a.batch * a.q_heads);
+    if (a.head_dim == 64) fa_f32_kernel<64><<<tiles, kGroups * kGroupThreads, TiledSmem<64>::kBytes, stream>>>(p);
+    else fa_f32_kernel<128><<<tiles, kGroups * kGroupThreads, TiledSmem<128>::kBytes, stream>>>(p);
+    WB200_CUDA_CHECK(cudaGetLastError());
+    return WB200_OK;
+  }
   dim3 grid((a.q_len + kWarpsPerBlock - 1) / kWarpsPerBlock, a.batch * a.q_heads);
   const size_t smem_bytes = (static_cast<size_t>(kWarpsPerBlock) * a.head_dim + kTileKeys * (a.head_dim + 1) + kTileKeys * a.head_dim) * sizeof(float);
   // wide staging loads need 16-byte aligned K / V bases; head_dim % 32 == 0 keeps every row aligned

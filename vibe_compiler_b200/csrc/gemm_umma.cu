@@ -3,36 +3,44 @@
 // command (lib/Wafer/Transforms/Linalg/ContractionAccumulation.cpp:147-218; finalize
 // lib/Wafer/Simulator/Reference/Formal/FormalNumericGemm.cpp:115-157).
 //
-// Tile 128 x 256 x 64, 4-stage TMA ring, two 256-column TMEM accumulators so the epilogue of tile i
-// overlaps the main loop of tile i+1. Warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner,
-// warps 2-5 = epilogue (one TMEM lane quarter each). Roofline: tensor pipe; algorithmic work is
-// 2*M*N*K flop per launch.
+// Two kernels: CTA pairs on 256 x 256 tiles (persistent) for problems that fill the SMs with them, one tile of 64 or 128
+// columns per CTA for small and narrow ones. In both, warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps
+// 2-5 = epilogue (one TMEM lane quarter each). Roofline: tensor pipe, or the bytes of B when the rows are few; algorithmic
+// work is 2*M*N*K flop per launch.
+#include <algorithm>
+#include <cmath>
+
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 64, kStages = 4;
+constexpr int kBM = 128, kBN = 256, kBK = 64;
 constexpr int kABytes = kBM * kBK * 2;        // 16 KiB
-constexpr int kBBytes = kBN * kBK * 2;        // 32 KiB
-constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kTmemCols = 512;
 constexpr int kThreads = 192;
 constexpr int kGroupM = 8;
-constexpr size_t kSmemBytes = kStages * kStageBytes + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct GemmUmmaParams {
   int m, n, k;
   int out_format;
-  int a_mn_major, b_mn_major;
   int epilogue;
-  int bf16;
   const float *bias;
   void *out;
   int *status;
-  int num_m_tiles, num_n_tiles;
+  int num_n_tiles;
   int group_m;   // tile rows walked together (see tile_coords)
+};
+
+// How a problem is cut for the one-tile-per-CTA kernel (see choose_tile).
+constexpr int kMaxTileStages = 10;
+struct TilePlan {
+  int tile_cols;    // output columns per tile: 64 or 128
+  int tile_rows;    // output rows per tile: a multiple of 16 up to 256
+  int stages;       // TMA ring; a stage holds two 64-element blocks of K
+  int row_bytes;    // bytes of A per block of K
+  int tmem_cols;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int group_m, int &m_blk, int &n_blk) {
@@ -112,165 +120,208 @@ __device__ __forceinline__ void epilogue_chunk(const GemmUmmaParams &p, uint32_t
   }
 }
 
-template <bool kAMn, bool kBMn, bool kBf16>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_umma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const GemmUmmaParams p) {
+// ---------------------------------------------------------------- one tile per CTA: small and narrow problems
+// One CTA owns kCols (64 or 128) columns x tile_rows rows of the output over all of K. The output columns are the M side
+// of the instruction (B is its A operand) and the rows its N side (16 to 256), so a problem of few rows costs no products
+// on padding, and B is streamed by as many SMs as the columns give. K is not split: every element is one ascending chain
+// of products whatever the number of rows, so a row's bits do not depend on the batch it travels in.
+// The accumulator goes through shared memory to the epilogue, 8 columns of one row per thread.
+// Bound at few rows by the issue of instructions that each cover 2 or 4 KiB of B (about 75 clocks apiece, measured the same
+// for 64 and 128 columns and for 16 to 64 rows), hence 64-column tiles: twice as many SMs stream B. A stage holds two
+// blocks of K so that its barriers cost half as much (16 x 6144 x 4096: 15.9 -> 13.2 us, 8 x 4096 x 14336: 47 -> 37 us).
+// 16 x 6144 x 4096 bf16 in all: 29.7 us as one 128 x 256 tile per CTA (24 CTAs), 13.2 us now.
+// Epilogue of 8 accumulator columns [col, col + 8) of one row; col + 8 <= n.
+__device__ __forceinline__ void epilogue_row8(const GemmUmmaParams &p, float (&v)[8], int row, int col) {
+  if (p.epilogue == WB200_EPI_SWIGLU) {
+    uint32_t w[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float o[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float gate = v[4 * j + 2 * h], up = v[4 * j + 2 * h + 1];
+        o[h] = __fdividef(gate, 1.0f + __expf(-gate)) * up;
+      }
+      w[j] = narrow_bits(o[0], p.out_format) | (narrow_bits(o[1], p.out_format) << 16);
+    }
+    *reinterpret_cast<uint2 *>(reinterpret_cast<uint16_t *>(p.out) + static_cast<size_t>(row) * (p.n / 2) + col / 2) = make_uint2(w[0], w[1]);
+    return;
+  }
+  if (p.epilogue != WB200_EPI_NONE) {
+#pragma unroll
+    for (int i = 0; i < 8; i += 4) {
+      const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + col + i));
+      v[i] += b.x; v[i + 1] += b.y; v[i + 2] += b.z; v[i + 3] += b.w;
+    }
+    if (p.epilogue == WB200_EPI_BIAS_GELU) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = gelu_erf(v[i]);
+    }
+  }
+  if (p.out_format == WB200_F32) {
+    float *dst = reinterpret_cast<float *>(p.out) + static_cast<size_t>(row) * p.n + col;
+    *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4 *>(dst + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    return;
+  }
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) w[j] = narrow_bits(v[2 * j], p.out_format) | (narrow_bits(v[2 * j + 1], p.out_format) << 16);
+  *reinterpret_cast<uint4 *>(reinterpret_cast<uint16_t *>(p.out) + static_cast<size_t>(row) * p.n + col) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// kAMn: A[k, m] (m contiguous) instead of A[m, k]; kBMn: B[k, n] (n contiguous) instead of B[n, k].
+template <int kCols, bool kAMn, bool kBMn, bool kBf16>
+__global__ void __launch_bounds__(kThreads)
+gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                       const GemmUmmaParams p, const TilePlan plan) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t *smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
   const uint32_t smem_base = smem_u32(smem);
-
-  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + kStages * kStageBytes);
-  const uint32_t bar_base = smem_base + kStages * kStageBytes;
+  __shared__ uint64_t bars[2 * kMaxTileStages + 1];
+  __shared__ uint32_t tmem_slot_word;
+  __shared__ int abort_shared;
+  const uint32_t bar_base = smem_u32(bars);
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (kStages + s); };
-  auto tmem_full_bar = [&](int a) { return bar_base + 8u * (2 * kStages + a); };
-  auto tmem_empty_bar = [&](int a) { return bar_base + 8u * (2 * kStages + 2 + a); };
-  volatile uint32_t *tmem_slot = reinterpret_cast<volatile uint32_t *>(bars + 2 * kStages + 4);
-  volatile int *abort_word = reinterpret_cast<volatile int *>(bars + 2 * kStages + 5);
+  auto empty_bar = [&](int s) { return bar_base + 8u * (kMaxTileStages + s); };
+  const uint32_t acc_bar = bar_base + 8u * (2 * kMaxTileStages);
+  volatile int *abort_word = &abort_shared;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < plan.stages; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(tmem_full_bar(a), 1);
-      mbar_init(tmem_empty_bar(a), 128);
-    }
+    mbar_init(acc_bar, 1);
     *abort_word = 0;
     fence_mbar_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), kTmemCols);
+    tmem_alloc(smem_u32(&tmem_slot_word), plan.tmem_cols);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = *const_cast<volatile uint32_t *>(&tmem_slot_word);
+  pdl_wait();
 
-  const int num_tiles = p.num_m_tiles * p.num_n_tiles;
+  const int col_tiles = (p.n + kCols - 1) / kCols;
+  const int col0 = static_cast<int>(blockIdx.x) % col_tiles * kCols;
+  const int row0 = static_cast<int>(blockIdx.x) / col_tiles * plan.tile_rows;
   const int k_blocks = (p.k + kBK - 1) / kBK;
+  constexpr int kColBytes = kCols * kBK * 2;   // bytes of B per stage
+  const int block_bytes = kColBytes + plan.row_bytes;
 
   if (warp == 0) {
     if (lane == 0) {
       int stage = 0;
       uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-        int m_blk, n_blk;
-        tile_coords(tile, p.num_m_tiles, p.num_n_tiles, p.group_m, m_blk, n_blk);
-        const int m0 = m_blk * kBM, n0 = n_blk * kBN;
-        for (int kb = 0; kb < k_blocks; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word)) { ok = false; break; }
-          mbar_arrive_expect_tx(full_bar(stage), kStageBytes);
-          const uint32_t a_dst = smem_base + stage * kStageBytes;
-          const uint32_t b_dst = a_dst + kABytes;
-          const int k0 = kb * kBK;
-          if constexpr (!kAMn) {
-            tma_load_2d(a_dst, &tmap_a, full_bar(stage), k0, m0);            // box {64 k, 128 m}
-          } else {
-            tma_load_2d(a_dst, &tmap_a, full_bar(stage), m0, k0);            // box {64 m, 64 k}
-            tma_load_2d(a_dst + 8192, &tmap_a, full_bar(stage), m0 + 64, k0);
-          }
+      for (int kb = 0; kb < k_blocks; kb += 2) {
+        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word)) break;
+        const int blocks = min(2, k_blocks - kb);
+        mbar_arrive_expect_tx(full_bar(stage), blocks * block_bytes);
+        for (int half = 0; half < blocks; ++half) {
+          const uint32_t b_dst = smem_base + (2 * stage + half) * block_bytes;
+          const uint32_t a_dst = b_dst + kColBytes;
+          const int k0 = (kb + half) * kBK;
           if constexpr (kBMn) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)                                       // box {64 n, 64 k}
-              tma_load_2d(b_dst + i * 8192, &tmap_b, full_bar(stage), n0 + 64 * i, k0);
+            tma_load_2d(b_dst, &tmap_b, full_bar(stage), col0, k0);                // box {64 n, 64 k}
+            if constexpr (kCols == 128) tma_load_2d(b_dst + 8192, &tmap_b, full_bar(stage), col0 + 64, k0);
           } else {
-            tma_load_2d(b_dst, &tmap_b, full_bar(stage), k0, n0);            // box {64 k, 256 n}
+            tma_load_2d(b_dst, &tmap_b, full_bar(stage), k0, col0);                // box {64 k, kCols n}
           }
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if constexpr (kAMn) {
+            for (int i = 0; i * 8192 < plan.row_bytes; ++i)                        // box {64 m, 64 k}
+              tma_load_2d(a_dst + i * 8192, &tmap_a, full_bar(stage), row0 + 64 * i, k0);
+          } else {
+            tma_load_2d(a_dst, &tmap_a, full_bar(stage), k0, row0);                // box {64 k, tile_rows m}
+          }
         }
+        if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
       }
     }
   } else if (warp == 1) {
-    // The whole warp walks the loop (waits included) and one elected lane issues: with warp-uniform control flow the
-    // descriptor arithmetic stays on the uniform datapath, which keeps the issue cost per instruction well below the
-    // 128 clocks a 128 x 256 x 16 product occupies the tensor pipe (a loop run by a single diverged lane measured
-    // 171 clocks per instruction, the converged form 128).
-    constexpr uint32_t idesc = umma_idesc_f16(kBM, kBN, kBf16, kAMn, kBMn);
+    const uint32_t idesc = umma_idesc_f16(kCols, plan.tile_rows, kBf16, kBMn, kAMn);
     int stage = 0;
     uint32_t phase = 0;
-    int acc = 0;
-    uint32_t acc_phase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-      if (!mbar_wait(tmem_empty_bar(acc), acc_phase ^ 1u, abort_word)) { ok = false; break; }
+    for (int kb = 0; kb < k_blocks; kb += 2) {
+      if (!mbar_wait(full_bar(stage), phase, abort_word)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t d_tmem = tmem_base + acc * kBN;
-      for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait(full_bar(stage), phase, abort_word)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t a_src = smem_base + stage * kStageBytes;
-        const uint32_t b_src = a_src + kABytes;
-        const uint64_t adesc = kAMn ? umma_desc_mnmajor(a_src, 8192) : umma_desc_kmajor(a_src);
-        const uint64_t bdesc = kBMn ? umma_desc_mnmajor(b_src, 8192) : umma_desc_kmajor(b_src);
-        if (elect_one_sync()) {
+      const uint32_t b_src = smem_base + 2 * stage * block_bytes;
+      const uint32_t a_src = b_src + kColBytes;
+      const uint64_t bdesc = kBMn ? umma_desc_mnmajor(b_src, 8192) : umma_desc_kmajor(b_src);
+      const uint64_t adesc = kAMn ? umma_desc_mnmajor(a_src, 8192) : umma_desc_kmajor(a_src);
+      const uint64_t next = static_cast<uint32_t>(block_bytes) >> 4;
+      if (elect_one_sync()) {
+        constexpr uint64_t a_step = (kAMn ? 2048 : 32) >> 4, b_step = (kBMn ? 2048 : 32) >> 4;
 #pragma unroll
-          for (int ks = 0; ks < kBK / 16; ++ks) {
-            // a k-step of 16 advances the start address by 32 B in a K-major tile and by 2 KiB in an MN-major one
-            constexpr uint64_t a_step = (kAMn ? 2048 : 32) >> 4, b_step = (kBMn ? 2048 : 32) >> 4;
-            umma_f16_ss(d_tmem, adesc + ks * a_step, bdesc + ks * b_step, idesc, (kb | ks) != 0 ? 1u : 0u);
-          }
-          umma_commit(empty_bar(stage));
+        for (int ks = 0; ks < kBK / 16; ++ks)
+          umma_f16_ss(tmem_base, bdesc + ks * b_step, adesc + ks * a_step, idesc, (kb | ks) != 0 ? 1u : 0u);
+        if (kb + 1 < k_blocks) {
+#pragma unroll
+          for (int ks = 0; ks < kBK / 16; ++ks)
+            umma_f16_ss(tmem_base, bdesc + next + ks * b_step, adesc + next + ks * a_step, idesc, 1u);
         }
-        __syncwarp();
-        if (++stage == kStages) { stage = 0; phase ^= 1u; }
+        umma_commit(empty_bar(stage));
       }
-      if (!ok) break;
-      if (elect_one_sync()) umma_commit(tmem_full_bar(acc));
       __syncwarp();
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
+      if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
     }
+    if (ok && elect_one_sync()) umma_commit(acc_bar);
+    __syncwarp();
   } else {
+    // The ring is free once every product has finished: the accumulator goes over it as [tile_rows][kCols] f32.
+    // A 128-row accumulator fills the 32 lanes of each quarter, a 64-row one the first 16.
+    constexpr int kLanes = kCols / 4;
     const int quarter = warp & 3;
-    int acc = 0;
-    uint32_t acc_phase = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-      int m_blk, n_blk;
-      tile_coords(tile, p.num_m_tiles, p.num_n_tiles, p.group_m, m_blk, n_blk);
-      const int row = m_blk * kBM + quarter * 32 + lane;
-      const int n0 = n_blk * kBN;
-      if (!mbar_wait(tmem_full_bar(acc), acc_phase, abort_word)) { ok = false; break; }
+    if (mbar_wait(acc_bar, 0, abort_word)) {
       tc_fence_after();
-      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * kBN;
+      float *mine = reinterpret_cast<float *>(smem) + quarter * kLanes + lane;
+      const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
+      for (int c = 0; c < plan.tile_rows; c += 32) {   // tmem_cols is a multiple of 32
         uint32_t r[32];
-        tmem_ld_32x32(t_row + c * 32, r);
+        tmem_ld_32x32(t_row + c, r);
         tmem_wait_ld();
-        epilogue_chunk(p, r, row, n0 + c * 32);
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (lane < kLanes && c + i < plan.tile_rows) mine[(c + i) * kCols] = __uint_as_float(r[i]);
       }
       tc_fence_before();
-      mbar_arrive(tmem_empty_bar(acc));
-      acc ^= 1;
-      if (acc == 0) acc_phase ^= 1u;
     }
   }
 
   __syncthreads();
+  pdl_launch_dependents();
   if (*abort_word != 0) {
     // Give copies still in flight time to land before the shared memory is released.
     for (int i = 0; i < 64; ++i) __nanosleep(10000);
     if (threadIdx.x == 0) raise_status(p.status, *abort_word);
     __syncthreads();
   }
+  {
+    const int groups = min(plan.tile_rows, p.m - row0) * (kCols / 8);
+    for (int g = threadIdx.x; g < groups; g += kThreads) {
+      const int row = g / (kCols / 8), col = (g % (kCols / 8)) * 8;
+      if (col0 + col >= p.n) continue;
+      const float4 *src = reinterpret_cast<const float4 *>(smem) + (row * kCols + col) / 4;
+      const float4 lo = src[0], hi = src[1];
+      float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+      epilogue_row8(p, v, row0 + row, col0 + col);
+    }
+  }
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem_base, plan.tmem_cols);
   }
 }
-
 
 // ---------------------------------------------------------------- CTA-pair kernel: 256 x 256 x 64 tiles
 // Two CTAs of a cluster share one output tile: CTA r of the pair owns rows [128 r, 128 r + 128) of it (A rows,
@@ -474,21 +525,80 @@ bool gemm_umma_supports(const GemmUmmaArgs &a) {
 
 namespace {
 using GemmKernel = void (*)(const CUtensorMap, const CUtensorMap, const GemmUmmaParams);
-const GemmKernel kernels[8] = {
-    gemm_umma_kernel<false, false, false>, gemm_umma_kernel<false, false, true>, gemm_umma_kernel<false, true, false>,
-    gemm_umma_kernel<false, true, true>,   gemm_umma_kernel<true, false, false>, gemm_umma_kernel<true, false, true>,
-    gemm_umma_kernel<true, true, false>,   gemm_umma_kernel<true, true, true>};
+using TileKernel = void (*)(const CUtensorMap, const CUtensorMap, const GemmUmmaParams, const TilePlan);
+#define WB200_TILE_KERNELS(COLS)                                                                                        \
+  {gemm_umma_tile_kernel<COLS, false, false, false>, gemm_umma_tile_kernel<COLS, false, false, true>,                   \
+   gemm_umma_tile_kernel<COLS, false, true, false>,  gemm_umma_tile_kernel<COLS, false, true, true>,                    \
+   gemm_umma_tile_kernel<COLS, true, false, false>,  gemm_umma_tile_kernel<COLS, true, false, true>,                    \
+   gemm_umma_tile_kernel<COLS, true, true, false>,   gemm_umma_tile_kernel<COLS, true, true, true>}
+const TileKernel tile_kernels[2][8] = {WB200_TILE_KERNELS(64), WB200_TILE_KERNELS(128)};
+#undef WB200_TILE_KERNELS
 const GemmKernel pair_kernels[8] = {
     gemm_umma_pair_kernel<false, false, false>, gemm_umma_pair_kernel<false, false, true>, gemm_umma_pair_kernel<false, true, false>,
     gemm_umma_pair_kernel<false, true, true>,   gemm_umma_pair_kernel<true, false, false>, gemm_umma_pair_kernel<true, false, true>,
     gemm_umma_pair_kernel<true, true, false>,   gemm_umma_pair_kernel<true, true, true>};
+
+constexpr int kTileSmemShared = 108 * 1024;   // ring of a CTA that shares its SM with another one
+constexpr int kTileSmemAlone = 208 * 1024;
+
+int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// Fills in what follows from the tile's size.
+TilePlan make_tile(int tile_cols, int tile_rows, const GemmUmmaArgs &a, int sm_count) {
+  TilePlan plan;
+  plan.tile_cols = tile_cols;
+  plan.tile_rows = tile_rows;
+  plan.row_bytes = a.lhs_transposed ? ceil_div(tile_rows, 64) * 8192 : tile_rows * 128;
+  const int stage = 2 * (tile_cols * kBK * 2 + plan.row_bytes);
+  const bool alone = static_cast<int64_t>(ceil_div(a.n, tile_cols)) * ceil_div(a.m, tile_rows) <= sm_count || tile_rows > 64;
+  // the ring is also the accumulator's staging area; more stages than blocks of K would stay empty
+  const int need = std::max({ceil_div(a.k, 2 * kBK), ceil_div(tile_rows * tile_cols * 4, stage), 2});
+  plan.stages = std::min({(alone ? kTileSmemAlone : kTileSmemShared) / stage, kMaxTileStages, need});
+  plan.tmem_cols = 32;
+  while (plan.tmem_cols < tile_rows) plan.tmem_cols *= 2;
+  return plan;
+}
+
+// Estimated clocks of a launch of either kernel; the cheaper one runs. Measured at 1.9 GHz with cold caches (both sides in
+// us, launch included): a block of 64 of K costs a CTA four instructions of about 75 clocks however few rows or columns
+// they cover, or its products, or its operand bytes at about 52 per clock, whichever is more; a pair of CTAs needs about
+// 650 clocks for the same block of a 256 x 256 tile. Rows x columns x K: 16 x 6144 x 4096 pair 31 / tile 19, 128 x 4096 x
+// 4096 30 / 20, 512 x 4096 x 4096 32 / 28, 1024 x 1024 x 8192 49 / 34, 8192 x 256 x 2048 24 / 22; the pairs win once their
+// tiles fill the SMs: 1000 x 6144 x 4096 54 / 68, 512 x 28672 x 4096 101 / 165.
+double tile_cost(const TilePlan &plan, const GemmUmmaArgs &a, int sm_count) {
+  const double per_sm = std::ceil(static_cast<double>(ceil_div(a.n, plan.tile_cols)) * ceil_div(a.m, plan.tile_rows) / sm_count);
+  const double block = std::max({300.0, 2.0 * plan.tile_rows, (plan.tile_cols * kBK * 2 + plan.row_bytes) / 52.0});
+  return per_sm * ceil_div(a.k, kBK) * block + 5000.0 + 20.0 * plan.tile_rows;
+}
+double pair_cost(const GemmUmmaArgs &a, int sm_count) {
+  const double waves = std::ceil(static_cast<double>(ceil_div(a.m, 2 * kBM)) * ceil_div(a.n, kBN) / (sm_count / 2));
+  return waves * ceil_div(a.k, kBK) * 650.0 + 10000.0;
+}
+
+TilePlan choose_tile(const GemmUmmaArgs &a, int sm_count, double *cost) {
+  TilePlan best{};
+  *cost = 0;
+  int last_rows = 0;
+  for (const int limit : {256, 192, 128, 96, 64}) {
+    const int tile_rows = ceil_div(ceil_div(a.m, ceil_div(a.m, limit)), 16) * 16;
+    if (tile_rows == last_rows) continue;
+    last_rows = tile_rows;
+    for (const int tile_cols : {128, 64}) {
+      const TilePlan plan = make_tile(tile_cols, tile_rows, a, sm_count);
+      const double c = tile_cost(plan, a, sm_count);
+      if (best.tile_rows == 0 || c < *cost) { best = plan; *cost = c; }
+    }
+  }
+  return best;
+}
 }  // namespace
 
 wb200_status gemm_umma_prepare() {
   static PerDeviceOnce attributes;
   return attributes.run([]() -> wb200_status {
-    for (GemmKernel kernel : kernels)
-      WB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes)));
+    for (const auto &of_width : tile_kernels)
+      for (TileKernel kernel : of_width)
+        WB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemAlone + 1024));
     for (GemmKernel kernel : pair_kernels)
       WB200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes)));
     return WB200_OK;
@@ -498,53 +608,53 @@ wb200_status gemm_umma_prepare() {
 wb200_status launch_gemm_umma(const GemmUmmaArgs &a, int sm_count, int *device_status,
                               cudaStream_t stream) {
   if (!gemm_umma_supports(a)) return fail(WB200_ERR_UNSUPPORTED, "GEMM outside the tcgen05 kernel's domain");
-  // CTA pairs when the problem has at least one full 256 x 256 tile per pair of SMs to amortise the pairing; the
-  // single-CTA kernel otherwise (small or narrow problems, WB200_GEMM_PAIR=0).
-  static const bool pair_enabled = []() { const char *env = getenv("WB200_GEMM_PAIR"); return !(env && env[0] == '0'); }();
-  const int pair_tiles = ((a.m + 2 * kBM - 1) / (2 * kBM)) * ((a.n + kBN - 1) / kBN);
-  const bool use_pairs = pair_enabled && a.m >= 2 * kBM && a.n >= kBN && pair_tiles * 4 >= sm_count;
+  double tile_clocks;
+  const TilePlan tile = choose_tile(a, sm_count, &tile_clocks);
+  const bool use_pairs = pair_cost(a, sm_count) < tile_clocks;
   CUtensorMap tmap_a, tmap_b;
   wb200_status st;
   if (!a.lhs_transposed)  // A[m,k], k contiguous: K-major
-    st = encode_tmap_2d(&tmap_a, a.a, a.in_format, a.k, a.m, static_cast<uint64_t>(a.k) * 2, 64, kBM);
+    st = encode_tmap_2d(&tmap_a, a.a, a.in_format, a.k, a.m, static_cast<uint64_t>(a.k) * 2, 64, use_pairs ? kBM : tile.tile_rows);
   else                    // A[k,m], m contiguous: MN-major
     st = encode_tmap_2d(&tmap_a, a.a, a.in_format, a.m, a.k, static_cast<uint64_t>(a.m) * 2, 64, 64);
   if (st != WB200_OK) return st;
   if (!a.rhs_transposed)  // B[k,n], n contiguous: MN-major
     st = encode_tmap_2d(&tmap_b, a.b, a.in_format, a.n, a.k, static_cast<uint64_t>(a.n) * 2, 64, 64);
   else                    // B[n,k], k contiguous: K-major
-    st = encode_tmap_2d(&tmap_b, a.b, a.in_format, a.k, a.n, static_cast<uint64_t>(a.k) * 2, 64, use_pairs ? kBN / 2 : kBN);
+    st = encode_tmap_2d(&tmap_b, a.b, a.in_format, a.k, a.n, static_cast<uint64_t>(a.k) * 2, 64, use_pairs ? kBN / 2 : tile.tile_cols);
   if (st != WB200_OK) return st;
 
   GemmUmmaParams p;
   p.m = a.m; p.n = a.n; p.k = a.k;
   p.out_format = a.out_format;
-  p.a_mn_major = a.lhs_transposed ? 1 : 0;
-  p.b_mn_major = a.rhs_transposed ? 0 : 1;
   p.epilogue = a.epilogue;
-  p.bf16 = a.in_format == WB200_BF16;
   p.bias = a.bias;
   p.out = a.out;
   p.status = device_status;
-  p.num_m_tiles = (a.m + kBM - 1) / kBM;
   p.num_n_tiles = (a.n + kBN - 1) / kBN;
   static const int group_override = []() { const char *env = getenv("WB200_GEMM_GROUP_M"); return env ? atoi(env) : 0; }();
   p.group_m = group_override > 0 ? group_override : kGroupM;
 
   wb200_status st_attributes = gemm_umma_prepare();
   if (st_attributes != WB200_OK) return st_attributes;
-  const int variant = (p.a_mn_major ? 4 : 0) | (p.b_mn_major ? 2 : 0) | (p.bf16 ? 1 : 0);
+  const int variant = (a.lhs_transposed ? 4 : 0) | (a.rhs_transposed ? 0 : 2) | (a.in_format == WB200_BF16 ? 1 : 0);
   if (use_pairs) {
-    int clusters = sm_count / 2;
-    if (pair_tiles < clusters) clusters = pair_tiles;
+    const int clusters = std::min(sm_count / 2, ceil_div(a.m, 2 * kBM) * p.num_n_tiles);
     pair_kernels[variant]<<<2 * clusters, kThreads, kPairSmemBytes, stream>>>(tmap_a, tmap_b, p);
     WB200_CUDA_CHECK(cudaGetLastError());
     return WB200_OK;
   }
-  const int tiles = p.num_m_tiles * p.num_n_tiles;
-  const int grid = tiles < sm_count ? tiles : sm_count;
-  kernels[variant]<<<grid, kThreads, kSmemBytes, stream>>>(tmap_a, tmap_b, p);
-  WB200_CUDA_CHECK(cudaGetLastError());
+  cudaLaunchAttribute dependent;
+  dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  dependent.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(ceil_div(a.n, tile.tile_cols) * ceil_div(a.m, tile.tile_rows));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = 2 * tile.stages * (tile.tile_cols * kBK * 2 + tile.row_bytes) + 1024;
+  config.stream = stream;
+  config.attrs = &dependent;
+  config.numAttrs = 1;
+  WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, tile_kernels[tile.tile_cols == 128][variant], tmap_a, tmap_b, p, tile));
   return WB200_OK;
 }
 

@@ -79,37 +79,65 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const uint16_t *x
 // qkv is the projection output, token-major: row (b * seq + s) holds [q heads | k heads | v heads] x head_dim.
 // Writes head-major Q [B, Hq, S, D], K [B, Hkv, S, D], V [B, Hkv, S, D]; Q and K get the rotary embedding
 // (pairs (i, i + D/2), angle = (position_offset + s) * theta^(-2i/D), f32 math, one rounding).
-template <bool kBf16>
-__global__ void __launch_bounds__(256) rope_split_kernel(const uint16_t *qkv, uint16_t *q, uint16_t *k, uint16_t *v,
-                                                          int batch, int seq, int q_heads, int kv_heads, int head_dim,
-                                                          float log2_theta, int position_offset) {
+// One block per token: the sines and cosines of its D/2 angles are the same for every head, so they are computed once into
+// shared memory; with them per head the kernel was bound by sincosf. kVec = elements of either half per thread and step:
+// 8 (16-byte accesses; head_dim % 16 == 0) or 2.
+// 16384 tokens x 48 heads x 128 bf16 (403 MB, 61 us at the copy rate): 178 us with the angles per head, 64 us now; 1000 tokens 16.3 -> 7.5.
+constexpr int kRopeThreads = 128;
+constexpr int kRopeAngles = 512;   // angles in shared memory at a time
+
+template <bool kBf16, int kVec>
+__global__ void __launch_bounds__(kRopeThreads) rope_split_kernel(const uint16_t *qkv, uint16_t *q, uint16_t *k, uint16_t *v,
+                                                                   int seq, int q_heads, int kv_heads, int head_dim,
+                                                                   float log2_theta, int position_offset) {
+  __shared__ float2 angles[kRopeAngles];   // (sin, cos)
   const int token = blockIdx.x;
   const int b = token / seq, s = token % seq;
   const int heads = q_heads + 2 * kv_heads;
   const int half = head_dim / 2;
   const uint16_t *row = qkv + static_cast<size_t>(token) * heads * head_dim;
-  const int pairs_per_head = half / 2;   // each thread handles two adjacent rotation pairs (4 elements)
-  for (int idx = threadIdx.x; idx < heads * pairs_per_head; idx += blockDim.x) {
-    const int head = idx / pairs_per_head, i = (idx % pairs_per_head) * 2;
-    const uint16_t *src = row + static_cast<size_t>(head) * head_dim;
-    const float2 lo = unpack2<kBf16>(*reinterpret_cast<const uint32_t *>(src + i));
-    const float2 hi = unpack2<kBf16>(*reinterpret_cast<const uint32_t *>(src + i + half));
-    uint16_t *dst;
-    bool rotate = true;
-    if (head < q_heads) dst = q + ((static_cast<size_t>(b) * q_heads + head) * seq + s) * head_dim;
-    else if (head < q_heads + kv_heads) dst = k + ((static_cast<size_t>(b) * kv_heads + (head - q_heads)) * seq + s) * head_dim;
-    else { dst = v + ((static_cast<size_t>(b) * kv_heads + (head - q_heads - kv_heads)) * seq + s) * head_dim; rotate = false; }
-    float2 out_lo = lo, out_hi = hi;
-    if (rotate) {
-      const float position = static_cast<float>(position_offset + s);
-      float s0, c0, s1, c1;
-      sincosf(position * exp2f(-2.0f * static_cast<float>(i) / static_cast<float>(head_dim) * log2_theta), &s0, &c0);
-      sincosf(position * exp2f(-2.0f * static_cast<float>(i + 1) / static_cast<float>(head_dim) * log2_theta), &s1, &c1);
-      out_lo = make_float2(lo.x * c0 - hi.x * s0, lo.y * c1 - hi.y * s1);
-      out_hi = make_float2(hi.x * c0 + lo.x * s0, hi.y * c1 + lo.y * s1);
+  const float position = static_cast<float>(position_offset + s);
+  for (int first = 0; first < half; first += kRopeAngles) {
+    const int count = min(kRopeAngles, half - first);
+    if (first > 0) __syncthreads();
+    for (int i = threadIdx.x; i < count; i += kRopeThreads) {
+      float sine, cosine;
+      sincosf(position * exp2f(-2.0f * static_cast<float>(first + i) / static_cast<float>(head_dim) * log2_theta), &sine, &cosine);
+      angles[i] = make_float2(sine, cosine);
     }
-    *reinterpret_cast<uint32_t *>(dst + i) = pack2f<kBf16>(out_lo.x, out_lo.y);
-    *reinterpret_cast<uint32_t *>(dst + i + half) = pack2f<kBf16>(out_hi.x, out_hi.y);
+    __syncthreads();
+    const int groups = count / kVec;
+    for (int idx = threadIdx.x; idx < heads * groups; idx += kRopeThreads) {
+      const int head = idx / groups, at = (idx % groups) * kVec, i = first + at;
+      const uint16_t *src = row + static_cast<size_t>(head) * head_dim + i;
+      uint32_t lo[kVec / 2], hi[kVec / 2];
+      if constexpr (kVec == 8) {
+        *reinterpret_cast<uint4 *>(lo) = *reinterpret_cast<const uint4 *>(src);
+        *reinterpret_cast<uint4 *>(hi) = *reinterpret_cast<const uint4 *>(src + half);
+      } else {
+        lo[0] = *reinterpret_cast<const uint32_t *>(src);
+        hi[0] = *reinterpret_cast<const uint32_t *>(src + half);
+      }
+      uint16_t *dst;
+      if (head < q_heads) dst = q + ((static_cast<size_t>(b) * q_heads + head) * seq + s) * head_dim;
+      else if (head < q_heads + kv_heads) dst = k + ((static_cast<size_t>(b) * kv_heads + (head - q_heads)) * seq + s) * head_dim;
+      else dst = v + ((static_cast<size_t>(b) * kv_heads + (head - q_heads - kv_heads)) * seq + s) * head_dim;
+      const bool rotate = head < q_heads + kv_heads;
+#pragma unroll
+      for (int e = 0; e < kVec / 2; ++e) {
+        const float2 a0 = angles[at + 2 * e], a1 = angles[at + 2 * e + 1];
+        const float2 l = unpack2<kBf16>(lo[e]), h = unpack2<kBf16>(hi[e]);
+        lo[e] = rotate ? pack2f<kBf16>(l.x * a0.y - h.x * a0.x, l.y * a1.y - h.y * a1.x) : pack2f<kBf16>(l.x, l.y);
+        hi[e] = rotate ? pack2f<kBf16>(h.x * a0.y + l.x * a0.x, h.y * a1.y + l.y * a1.x) : pack2f<kBf16>(h.x, h.y);
+      }
+      if constexpr (kVec == 8) {
+        *reinterpret_cast<uint4 *>(dst + i) = *reinterpret_cast<const uint4 *>(lo);
+        *reinterpret_cast<uint4 *>(dst + i + half) = *reinterpret_cast<const uint4 *>(hi);
+      } else {
+        *reinterpret_cast<uint32_t *>(dst + i) = lo[0];
+        *reinterpret_cast<uint32_t *>(dst + i + half) = hi[0];
+      }
+    }
   }
 }
 
@@ -153,12 +181,12 @@ wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, vo
     return fail(WB200_ERR_INVALID_ARGUMENT, "invalid rope extents (head_dim % 4 == 0, theta > 0)");
   const int tokens = batch * seq;
   const float log2_theta = log2f(theta);
-  if (format == WB200_BF16)
-    rope_split_kernel<true><<<tokens, 256, 0, stream>>>(static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q), static_cast<uint16_t *>(k),
-                                                         static_cast<uint16_t *>(v), batch, seq, q_heads, kv_heads, head_dim, log2_theta, position_offset);
-  else
-    rope_split_kernel<false><<<tokens, 256, 0, stream>>>(static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q), static_cast<uint16_t *>(k),
-                                                          static_cast<uint16_t *>(v), batch, seq, q_heads, kv_heads, head_dim, log2_theta, position_offset);
+  const bool wide = head_dim % 16 == 0 && aligned16(qkv) && aligned16(q) && aligned16(k) && aligned16(v);
+  const bool bf16 = format == WB200_BF16;
+  const auto kernel = wide ? (bf16 ? rope_split_kernel<true, 8> : rope_split_kernel<false, 8>)
+                           : (bf16 ? rope_split_kernel<true, 2> : rope_split_kernel<false, 2>);
+  kernel<<<tokens, kRopeThreads, 0, stream>>>(static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q), static_cast<uint16_t *>(k),
+                                              static_cast<uint16_t *>(v), seq, q_heads, kv_heads, head_dim, log2_theta, position_offset);
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
 }

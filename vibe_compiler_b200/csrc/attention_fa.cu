@@ -255,6 +255,8 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();   // the next kernel's CTAs take over SM by SM as this grid drains
 
   // setmaxnreg.inc blocks until the CTA's own register pool can supply the request, so the totals after
   // reallocation (128 * 104 + 256 * 200) must not exceed what the CTA was launched with (384 * 168).
@@ -777,13 +779,13 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int 
   config.blockDim = dim3(kFaThreads);
   config.dynamicSmemBytes = FaSmem::kBytes;
   config.stream = stream;
-  cudaLaunchAttribute cluster;
-  cluster.id = cudaLaunchAttributeClusterDimension;
-  cluster.val.clusterDim.x = 2; cluster.val.clusterDim.y = 1; cluster.val.clusterDim.z = 1;
-  if (p.plan && grid % 2 == 0) {
-    config.attrs = &cluster;
-    config.numAttrs = 1;
-  }
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = 2; attrs[1].val.clusterDim.y = 1; attrs[1].val.clusterDim.z = 1;
+  config.attrs = attrs;
+  config.numAttrs = p.plan && grid % 2 == 0 ? 2 : 1;
   if (a.format == WB200_BF16)
     WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, fa_umma_kernel<true>, tq, tk, tv, p));
   else

@@ -217,6 +217,8 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const S
   };
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group_id), "n"(kGroupThreads) : "memory"); };
 
+  pdl_wait();
+  pdl_launch_dependents();
   for (int e = threadIdx.x; e < kTileRows * (kD / 4); e += kGroups * kGroupThreads) {
     const int r = e / (kD / 4), d = e % (kD / 4) * 4;
     cp_async16(smem_u32(q_s + r * L::kKPitch + d), q + static_cast<size_t>(min(r, rows - 1)) * kD + d, 16u);
@@ -419,9 +421,9 @@ wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t strea
     });
     if (st != WB200_OK) return st;
     const dim3 tiles((a.q_len + kTileRows - 1) / kTileRows, a.batch * a.q_heads);
-    if (a.head_dim == 64) fa_f32_kernel<64><<<tiles, kGroups * kGroupThreads, TiledSmem<64>::kBytes, stream>>>(p);
-    else fa_f32_kernel<128><<<tiles, kGroups * kGroupThreads, TiledSmem<128>::kBytes, stream>>>(p);
-    WB200_CUDA_CHECK(cudaGetLastError());
+    const bool narrow = a.head_dim == 64;
+    WB200_CUDA_CHECK(launch_dependent(narrow ? fa_f32_kernel<64> : fa_f32_kernel<128>, tiles, kGroups * kGroupThreads,
+                                      narrow ? TiledSmem<64>::kBytes : TiledSmem<128>::kBytes, stream, p));
     return WB200_OK;
   }
   dim3 grid((a.q_len + kWarpsPerBlock - 1) / kWarpsPerBlock, a.batch * a.q_heads);

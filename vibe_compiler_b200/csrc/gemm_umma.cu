@@ -379,6 +379,8 @@ gemm_umma_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   cluster_sync_all();     // both CTAs' barriers exist before either touches the partner's
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  pdl_launch_dependents();   // the next kernel's CTAs take over SM by SM as this grid drains
 
   const int num_pair_m = (p.m + 2 * kBM - 1) / (2 * kBM);
   const int num_tiles = num_pair_m * p.num_n_tiles;
@@ -640,21 +642,12 @@ wb200_status launch_gemm_umma(const GemmUmmaArgs &a, int sm_count, int *device_s
   const int variant = (a.lhs_transposed ? 4 : 0) | (a.rhs_transposed ? 0 : 2) | (a.in_format == WB200_BF16 ? 1 : 0);
   if (use_pairs) {
     const int clusters = std::min(sm_count / 2, ceil_div(a.m, 2 * kBM) * p.num_n_tiles);
-    pair_kernels[variant]<<<2 * clusters, kThreads, kPairSmemBytes, stream>>>(tmap_a, tmap_b, p);
-    WB200_CUDA_CHECK(cudaGetLastError());
+    WB200_CUDA_CHECK(launch_dependent(pair_kernels[variant], 2 * clusters, kThreads, kPairSmemBytes, stream, tmap_a, tmap_b, p));
     return WB200_OK;
   }
-  cudaLaunchAttribute dependent;
-  dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  dependent.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t config = {};
-  config.gridDim = dim3(ceil_div(a.n, tile.tile_cols) * ceil_div(a.m, tile.tile_rows));
-  config.blockDim = dim3(kThreads);
-  config.dynamicSmemBytes = 2 * tile.stages * (tile.tile_cols * kBK * 2 + tile.row_bytes) + 1024;
-  config.stream = stream;
-  config.attrs = &dependent;
-  config.numAttrs = 1;
-  WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, tile_kernels[tile.tile_cols == 128][variant], tmap_a, tmap_b, p, tile));
+  const int grid = ceil_div(a.n, tile.tile_cols) * ceil_div(a.m, tile.tile_rows);
+  const size_t smem = 2 * static_cast<size_t>(tile.stages) * (tile.tile_cols * kBK * 2 + tile.row_bytes) + 1024;
+  WB200_CUDA_CHECK(launch_dependent(tile_kernels[tile.tile_cols == 128][variant], grid, kThreads, smem, stream, tmap_a, tmap_b, p, tile));
   return WB200_OK;
 }
 

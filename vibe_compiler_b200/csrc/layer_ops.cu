@@ -5,6 +5,7 @@
 // (lib/Wafer/Simulator/Reference/ManagedReferenceTargetModel.cpp:230-342: decode to f32, operate, RNE encode).
 // All three are HBM-bound: algorithmic bytes = bytes read + bytes written once.
 #include "kernels.h"
+#include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
@@ -32,6 +33,8 @@ __device__ __forceinline__ uint32_t pack2f(float lo, float hi) {
 template <bool kBf16>
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(const uint16_t *x, const uint16_t *gamma, uint16_t *y,
                                                                 int rows, int dim, float eps) {
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x;
   const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<size_t>(row) * dim);
   const int chunks = dim / 8;
@@ -97,6 +100,7 @@ __global__ void __launch_bounds__(kRopeThreads) rope_split_kernel(const uint16_t
   const int half = head_dim / 2;
   const uint16_t *row = qkv + static_cast<size_t>(token) * heads * head_dim;
   const float position = static_cast<float>(position_offset + s);
+  pdl_launch_dependents();
   for (int first = 0; first < half; first += kRopeAngles) {
     const int count = min(kRopeAngles, half - first);
     if (first > 0) __syncthreads();
@@ -106,6 +110,7 @@ __global__ void __launch_bounds__(kRopeThreads) rope_split_kernel(const uint16_t
       angles[i] = make_float2(sine, cosine);
     }
     __syncthreads();
+    if (first == 0) pdl_wait();   // the angles need nothing of the kernel before this one
     const int groups = count / kVec;
     for (int idx = threadIdx.x; idx < heads * groups; idx += kRopeThreads) {
       const int head = idx / groups, at = (idx % groups) * kVec, i = first + at;
@@ -143,6 +148,8 @@ __global__ void __launch_bounds__(kRopeThreads) rope_split_kernel(const uint16_t
 
 template <bool kBf16>
 __global__ void __launch_bounds__(256) residual_add_kernel(const uint4 *a, const uint4 *b, uint4 *out, size_t chunks) {
+  pdl_wait();
+  pdl_launch_dependents();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   for (size_t c = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; c < chunks; c += stride) {
     const uint4 x = a[c], y = b[c];
@@ -166,11 +173,8 @@ wb200_status launch_rmsnorm(int format, const void *x, const void *gamma, void *
   if (format != WB200_BF16 && format != WB200_F16) return fail(WB200_ERR_UNSUPPORTED, "rmsnorm takes bf16 or f16 storage");
   if (rows <= 0 || dim <= 0 || dim % 8 != 0 || !aligned16(x) || !aligned16(gamma) || !aligned16(y))
     return fail(WB200_ERR_INVALID_ARGUMENT, "rmsnorm needs dim % 8 == 0 and 16-byte aligned buffers");
-  if (format == WB200_BF16)
-    rmsnorm_kernel<true><<<rows, kNormThreads, 0, stream>>>(static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(gamma), static_cast<uint16_t *>(y), rows, dim, eps);
-  else
-    rmsnorm_kernel<false><<<rows, kNormThreads, 0, stream>>>(static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(gamma), static_cast<uint16_t *>(y), rows, dim, eps);
-  WB200_CUDA_CHECK(cudaGetLastError());
+  WB200_CUDA_CHECK(launch_dependent(format == WB200_BF16 ? rmsnorm_kernel<true> : rmsnorm_kernel<false>, rows, kNormThreads, 0, stream,
+                                    static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(gamma), static_cast<uint16_t *>(y), rows, dim, eps));
   return WB200_OK;
 }
 
@@ -185,9 +189,9 @@ wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, vo
   const bool bf16 = format == WB200_BF16;
   const auto kernel = wide ? (bf16 ? rope_split_kernel<true, 8> : rope_split_kernel<false, 8>)
                            : (bf16 ? rope_split_kernel<true, 2> : rope_split_kernel<false, 2>);
-  kernel<<<tokens, kRopeThreads, 0, stream>>>(static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q), static_cast<uint16_t *>(k),
-                                              static_cast<uint16_t *>(v), seq, q_heads, kv_heads, head_dim, log2_theta, position_offset);
-  WB200_CUDA_CHECK(cudaGetLastError());
+  WB200_CUDA_CHECK(launch_dependent(kernel, tokens, kRopeThreads, 0, stream, static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q),
+                                    static_cast<uint16_t *>(k), static_cast<uint16_t *>(v), seq, q_heads, kv_heads, head_dim, log2_theta,
+                                    position_offset));
   return WB200_OK;
 }
 
@@ -198,11 +202,8 @@ wb200_status launch_residual_add(int format, const void *a, const void *b, void 
   const size_t chunks = elements / 8;
   size_t blocks = (chunks + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  if (format == WB200_BF16)
-    residual_add_kernel<true><<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const uint4 *>(a), static_cast<const uint4 *>(b), static_cast<uint4 *>(out), chunks);
-  else
-    residual_add_kernel<false><<<static_cast<int>(blocks), 256, 0, stream>>>(static_cast<const uint4 *>(a), static_cast<const uint4 *>(b), static_cast<uint4 *>(out), chunks);
-  WB200_CUDA_CHECK(cudaGetLastError());
+  WB200_CUDA_CHECK(launch_dependent(format == WB200_BF16 ? residual_add_kernel<true> : residual_add_kernel<false>, static_cast<unsigned>(blocks), 256, 0,
+                                    stream, static_cast<const uint4 *>(a), static_cast<const uint4 *>(b), static_cast<uint4 *>(out), chunks));
   return WB200_OK;
 }
 

@@ -87,22 +87,6 @@ template <int kRegs>
 __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
-// 2^x on the FMA pipe for x <= 0: x = n + f with n = round(x), f in [-0.5, 0.5]; 2^f by a degree-3 polynomial (maximum
-// relative error 7.5e-5, far below the rounding of P to 16 bits), 2^n by adding n to the exponent field. x is clamped at
-// -126, so the result is never exactly zero: tiles that hold masked (-inf) scores use the hardware ex2 throughout.
-#ifndef WB200_FA_POLY_PERIOD
-#define WB200_FA_POLY_PERIOD 4
-#endif
-constexpr int kPolyPeriod = WB200_FA_POLY_PERIOD;   // one pair of exponentials in kPolyPeriod runs on the FMA pipe
-__device__ __forceinline__ float ex2_poly(float x) {
-  x = fmaxf(x, -126.0f);
-  const float shifted = x + 12582912.0f;                 // 1.5 * 2^23: the low mantissa bits now hold n
-  const float f = x - (shifted - 12582912.0f);
-  float p = fmaf(0.0551716685295105f, f, 0.2426111251115799f);
-  p = fmaf(p, f, 0.6932609677314758f);
-  p = fmaf(p, f, 0.9999280571937561f);
-  return __int_as_float(__float_as_int(p) + (__float_as_int(shifted) << 23));
-}
 // Packed pairs of f32 (sm_100 has two-wide f32 fma / add): halves the issue slots of the scaling and of the row sums.
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
   unsigned long long r;
@@ -490,8 +474,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       // the first 64 exponentials, where it costs nothing.
       const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_m2 = pack_f32x2(-m_exp, -m_exp);
       unsigned long long sum2[4] = {0ull, 0ull, 0ull, 0ull};
-      auto exp_phase = [&](auto masked_tag) {
-      constexpr bool kMasked = decltype(masked_tag)::value;
+      auto exp_phase = [&]() {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t packed[16];
@@ -500,11 +483,10 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           const unsigned long long x2 = fma_f32x2(pack_f32x2(__uint_as_float(r[32 * c + i]), __uint_as_float(r[32 * c + i + 1])), scale2, neg_m2);
           float x0, x1;
           unpack_f32x2(x2, x0, x1);
-          // Every fourth pair of exponentials runs on the FMA pipe: the special-function pipe (ex2 and the 16-bit
-          // conversions) is the busiest unit of the softmax warps.
-          const bool poly = !kMasked && ((i >> 1) % kPolyPeriod) == kPolyPeriod - 1;
-          const float e0 = poly ? ex2_poly(x0) : ex2_approx(x0);
-          const float e1 = poly ? ex2_poly(x1) : ex2_approx(x1);
+          // All exponentials on the special-function pipe. A share of them as polynomials on the FMA pipe only adds
+          // instructions (and error): one pair in 4 / 6 / 16 / none measured 516 / 509 / 510 / 505 us at 4 x 32 heads x
+          // 4096 causal and 296 / 287 / 288 / 285 us at 8 x 32 / 8 heads x 2048.
+          const float e0 = ex2_approx(x0), e1 = ex2_approx(x1);
           sum2[(i >> 1) & 3] = add_f32x2(sum2[(i >> 1) & 3], pack_f32x2(e0, e1));
           if constexpr (kBf16) {
             __nv_bfloat162 v = __floats2bfloat162_rn(e0, e1);
@@ -537,8 +519,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
       }
       };
-      if (need_mask) exp_phase(std::true_type{});
-      else exp_phase(std::false_type{});
+      exp_phase();
       if (!ok) break;
       float s0, s1, s2, s3, s4, s5, s6, s7;
       unpack_f32x2(sum2[0], s0, s1); unpack_f32x2(sum2[1], s2, s3); unpack_f32x2(sum2[2], s4, s5); unpack_f32x2(sum2[3], s6, s7);

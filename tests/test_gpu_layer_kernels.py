@@ -23,3 +23,22 @@ def test_rope_split_widths(backend, hd, dtype):
     # bits, which is off by at most 2^-8 or 2^-11 of the value
     bound = want.abs().max().item() * ((2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) + 786 * 2.0 ** -22)
     assert (torch.cat((q, k), 1).double() - want).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("d_model", [128, 2056, 8320])
+def test_layer_with_the_add_inside_the_norm(backend, d_model):
+    # the fused layer adds the residual inside the second norm; the same layer from separate kernels has the same bits
+    # (rows below, at and beyond what the norm keeps in registers)
+    from vibe_compiler_b200.decoder_layer import LayerConfig, LayerWeights, ShardedDecoderLayer
+    cfg = LayerConfig(d_model=d_model, q_heads=2, kv_heads=1, ffn=256)
+    gen = torch.Generator(device="cuda").manual_seed(d_model)
+    w = lambda *shape: (torch.randn(shape, device="cuda", generator=gen) * 0.02).bfloat16()
+    hd = cfg.head_dim
+    weights = LayerWeights(norm1=1 + w(d_model), wq=w(d_model, 2 * hd), wk=w(d_model, hd), wv=w(d_model, hd), wo=w(2 * hd, d_model),
+                           norm2=1 + w(d_model), wgate=w(d_model, 256), wup=w(d_model, 256), wdown=w(256, d_model))
+    layer = ShardedDecoderLayer(backend, cfg, weights)
+    x = torch.randn(2, 36, d_model, device="cuda", generator=gen).bfloat16()
+    fused, separate = layer.forward_fused(x), layer.forward(x)
+    torch.cuda.synchronize()
+    backend.poll()
+    assert torch.equal(fused, separate)

@@ -1,5 +1,5 @@
 // wb200_decoder_layer: one rank's shard of a Llama-style decoder layer forward as a single C-ABI call.
-// The ten kernels are the library's own regions (RMSNorm, tcgen05 GEMM with NONE / SwiGLU epilogues, rotary +
+// The nine kernels are the library's own regions (RMSNorm, tcgen05 GEMM with NONE / SwiGLU epilogues, rotary +
 // head-major split, tcgen05 flash attention, residual add); the two sums over shards are delegated to the caller's
 // all-reduce callback, which stands where the reference places its Tile collectives
 // (lib/Wafer/Transforms/Tile/DistributedCollectiveMovement.cpp:675-735).
@@ -205,11 +205,12 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
   auto ffn_phase = [&](const Part &part) -> wb200_status {
     wb200_status s;
     if ((s = await_sum(part, 0)) != WB200_OK) return s;
-    if (!fused_residual) {
-      if ((s = launch_residual_add(fmt, part.x, part.partial, part.x1, static_cast<size_t>(tokens) * d, part.stream)) != WB200_OK) return s;
-      backend->launches += 1;
+    if (fused_residual) {
+      s = launch_rmsnorm(fmt, part.x1, p->norm2, part.h, tokens, d, p->eps, part.stream);
+    } else {   // x1 = x + attention on the way into the norm
+      s = launch_rmsnorm(fmt, part.x, p->norm2, part.h, tokens, d, p->eps, part.stream, part.partial, part.x1);
     }
-    if ((s = launch_rmsnorm(fmt, part.x1, p->norm2, part.h, tokens, d, p->eps, part.stream)) != WB200_OK) return s;
+    if (s != WB200_OK) return s;
     backend->launches += 1;
     if ((s = gemm(part.stream, part.h, p->wgu, part.act, tokens, 2 * static_cast<int>(p->ffn), d, WB200_EPI_SWIGLU)) != WB200_OK) return s;
     if ((s = gemm(part.stream, part.act, p->wdown, part.partial, tokens, d, static_cast<int>(p->ffn), WB200_EPI_NONE)) != WB200_OK) return s;

@@ -250,8 +250,9 @@ wb200_status launch_switch_sum(void *multicast, uint64_t elements, int format, i
 
 
 // ---- decoder-layer pieces (layer_ops.cu); device pointers, bf16 / f16 storage
+// With `addend` and `sum`: the norm of round(x + addend), which is stored to `sum`.
 wb200_status launch_rmsnorm(int format, const void *x, const void *gamma, void *y, int rows, int dim, float eps,
-                            cudaStream_t stream);
+                            cudaStream_t stream, const void *addend = nullptr, void *sum = nullptr);
 wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, void *v, int batch, int seq, int q_heads,
                                int kv_heads, int head_dim, float theta, int position_offset, cudaStream_t stream);
 wb200_status launch_residual_add(int format, const void *a, const void *b, void *out, size_t elements, cudaStream_t stream);

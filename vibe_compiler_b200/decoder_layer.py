@@ -139,7 +139,7 @@ class ShardedDecoderLayer:
 
     def forward_fused(self, x: torch.Tensor, position_offset: int = 0, micro_batches: Optional[int] = None,
                       reserved_sms: Optional[int] = None) -> torch.Tensor:
-        """Same computation through the single C-ABI call (wb200_decoder_layer): ten kernels per part enqueued by one call,
+        """Same computation through the single C-ABI call (wb200_decoder_layer): nine kernels per part enqueued by one call,
         the two sums through a callback into torch.distributed, intermediates in one reused workspace. With several
         shards the batch is cut into `micro_batches` parts whose sums run on a second stream while the following parts
         compute; `reserved_sms` SMs stay free for the sum's kernel. The sums are done by the NVSwitch through the

@@ -6,6 +6,7 @@ import torch
 
 from vibe_compiler_b200 import _abi as abi
 from vibe_compiler_b200.backend import B200TargetModelBackend, NumericTensor, PhysicalTensorDescriptor, WB200Error
+from vibe_compiler_b200.tile_program import TileProgram
 
 pytestmark = pytest.mark.gpu
 LAYOUTS = {"tensor": abi.LAYOUT_TENSOR, "cx": abi.LAYOUT_CX, "ncx": abi.LAYOUT_NCX}
@@ -92,3 +93,39 @@ def test_storage_in_place_and_in_pieces(backend, elements):
     key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [elements])
     got = backend.execute_elementwise("add", [NumericTensor(key, x), NumericTensor(key, y)], NumericTensor(key, np.zeros(4 * elements, np.uint8)))
     assert np.array_equal(got.destination.storage.view(np.float32), x + y)
+
+
+MIB = 1 << 20
+
+
+# operands that fill the 32 MiB transfer area to its last byte, once and one and a half times over
+@pytest.mark.parametrize("each", [16 * MIB, 24 * MIB])
+def test_flags_are_read_back_behind_operands_that_fill_the_transfer_area(backend, each):
+    key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [each // 4])
+    x = np.arange(each // 4, dtype=np.float32)
+    got = backend.execute_elementwise("add", [NumericTensor(key, x), NumericTensor(key, x)], NumericTensor(key, np.zeros(each, np.uint8)), formal=True)
+    assert np.array_equal(got.destination.storage.view(np.float32), x + x) and got.evidence.flags == 0
+    key, out_key = (PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [rows, each // 128]) for rows in (64, 1))
+    x = np.arange(each // 2, dtype=np.float32) % 127
+    got = backend.execute_reduce("sum", "trailing1", NumericTensor(key, x), NumericTensor(out_key, np.zeros(each // 32, np.uint8)), formal=True)
+    assert np.array_equal(got.destination.storage.view(np.float32), x.reshape(64, -1).sum(0)) and got.evidence.flags == 0   # small integers: exact
+
+
+def test_program_with_inputs_that_fill_the_transfer_area(backend):
+    rows = [f'!{{i64 {i}, !"external-{kind}", i64 0, !"", !"f32", !"tensor", i64 {count * 4}, i64 {count}, !"{access}-only", i64 {count // 64}, i64 64, i64 0}}'
+            for i, (kind, count, access) in enumerate((("input", 8 * MIB, "read"), ("output", 256, "write")))]
+    module = f"""define void @entry(i64 %0, i64 %1) {{
+  %src = add i64 %0, {32 * MIB - 1024}
+  call void @wafer_tx81_rdma(i64 %src, i64 0, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)
+  call void @wafer_tx81_wdma(i64 0, i64 %1, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)
+  ret void
+}}
+!wafer.target.tile_id = !{{!2}}
+!wafer.target.entry_arguments = !{{!10, !11}}
+!2 = !{{i64 0}}
+!10 = {rows[0]}
+!11 = {rows[1]}
+"""
+    x = np.arange(8 * MIB, dtype=np.float32).reshape(-1, 64)
+    (out,), _ = TileProgram([module], backend, spm_bytes=1 << 16).run([x])
+    assert np.array_equal(out.view(np.float32).reshape(-1), x.reshape(-1)[-256:])

@@ -20,8 +20,9 @@ struct wb200_backend {
   // [0] bounded-wait status, [1] NaN flag: pinned host memory the kernels store to when something is wrong, so that reading
   // it takes no copy (d_status: its device address).
   int *h_status = nullptr, *d_status = nullptr;
-  // Pinned, device-mapped staging area of the command calls (command_io.h), grown on demand up to kMaxStageBytes.
-  static constexpr size_t kMaxStageBytes = size_t(32) << 20;
+  // Pinned, device-mapped staging area of the command calls (command_io.h), grown on demand up to kMaxStageBytes. Behind its
+  // `stage_bytes` lie kStageWordBytes for the words a call reads back, which no operand can crowd out.
+  static constexpr size_t kMaxStageBytes = size_t(32) << 20, kStageWordBytes = 256;
   uint8_t *stage = nullptr;
   size_t stage_bytes = 0, stage_low = 0, stage_high = 0;
   wb200_status stage_reserve(size_t expected) {
@@ -33,7 +34,7 @@ struct wb200_backend {
       stage = nullptr;
       stage_bytes = 0;
       void *area;
-      WB200_CUDA_CHECK(cudaHostAlloc(&area, wanted, cudaHostAllocMapped));
+      WB200_CUDA_CHECK(cudaHostAlloc(&area, wanted + kStageWordBytes, cudaHostAllocMapped));
       stage = static_cast<uint8_t *>(area);
       stage_bytes = wanted;
     }

@@ -113,10 +113,10 @@ class CommandIO {
     return WB200_OK;
   }
 
-  // A small device word (flags, refusals) to be read back with the result.
+  // The device words (flags, refusals) a call reads back with its result: at most kStageWordBytes, once per call. Their place
+  // lies behind the operands' area, which uploads may have filled to the last byte.
   wb200_status read_back(const void *device_word, size_t bytes, const uint8_t **host) {
-    uint8_t *area = take(bytes);
-    if (!area) return fail(WB200_ERR_LIMIT, "command staging area exhausted");
+    uint8_t *area = backend_->stage + backend_->stage_bytes;
     WB200_CUDA_CHECK(cudaMemcpyAsync(area, device_word, bytes, cudaMemcpyDeviceToHost, stream_));
     *host = area;
     return WB200_OK;

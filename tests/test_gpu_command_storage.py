@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from vibe_compiler_b200 import _abi as abi
-from vibe_compiler_b200.backend import B200TargetModelBackend, NumericTensor, PhysicalTensorDescriptor, WB200Error
+from vibe_compiler_b200.backend import B200TargetModelBackend, FormalGemmOperation, NumericTensor, PhysicalTensorDescriptor, WB200Error
 from vibe_compiler_b200.tile_program import TileProgram
 
 pytestmark = pytest.mark.gpu
@@ -129,3 +129,36 @@ def test_program_with_inputs_that_fill_the_transfer_area(backend):
     x = np.arange(8 * MIB, dtype=np.float32).reshape(-1, 64)
     (out,), _ = TileProgram([module], backend, spm_bytes=1 << 16).run([x])
     assert np.array_equal(out.view(np.float32).reshape(-1), x.reshape(-1)[-256:])
+
+
+def pinned(data):
+    """A page-locked copy of `data`'s bytes."""
+    return torch.from_numpy(data.view(np.uint8).reshape(-1)).pin_memory().numpy()
+
+
+def into(monkeypatch, storage):
+    """Makes the next command write its result to `storage`, as a C caller may name any destination."""
+    monkeypatch.setattr(B200TargetModelBackend._results, "empty", lambda size: storage[:size])
+
+
+# Results over their own page-locked operands, in layouts whose padding comes from the template: the operands are read first.
+def test_padded_result_over_a_page_locked_operand(backend, monkeypatch):
+    rng = np.random.default_rng(5)
+    square = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_CX, [321, 321])
+    lhs, rhs = (physical(backend, square, rng.standard_normal(321 * 321).astype(np.float32).view(np.uint32)) for _ in range(2))
+    blank = NumericTensor(square, np.full(B200TargetModelBackend.physical_bytes(square), 0x11, np.uint8))
+    operation = FormalGemmOperation(square, square, square, 321, 321, 321)
+    halves = [PhysicalTensorDescriptor(f, abi.LAYOUT_CX, [300, 97]) for f in (abi.BF16, abi.F16)]
+    source = physical(backend, halves[0], rng.integers(0x3f00, 0x4100, 300 * 97).astype(np.uint16))
+    spare = NumericTensor(halves[1], np.full(B200TargetModelBackend.physical_bytes(halves[1]), 0x11, np.uint8))
+
+    def commands(lhs, rhs, source):
+        yield lhs, lambda: backend.try_execute(operation, NumericTensor(square, lhs), NumericTensor(square, rhs), blank, policy=abi.GEMM_FORMAL)
+        yield rhs, lambda: backend.try_execute(operation, NumericTensor(square, lhs), NumericTensor(square, rhs), blank, policy=abi.GEMM_FORMAL)
+        yield source, lambda: backend.execute_convert(154, NumericTensor(halves[0], source), spare, formal=True)
+    for index in range(3):
+        want = list(commands(lhs, rhs, source))[index][1]().destination.storage.copy()
+        with monkeypatch.context() as patch:
+            over, command = list(commands(pinned(lhs), pinned(rhs), pinned(source)))[index]
+            into(patch, over)
+            assert np.array_equal(command().destination.storage, want)

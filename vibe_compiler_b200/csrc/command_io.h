@@ -33,9 +33,11 @@ class CommandIO {
   // An operand. `reread`: the kernels read it more than once, so it belongs in device memory (slot `slot`).
   wb200_status input(size_t slot, const uint8_t *host, size_t bytes, const uint8_t **device, bool reread = false) {
     const bool pinned = page_locked(host, bytes);
+    if (pinned) {   // read by the kernels or by a copy in flight, in either case after output() has run
+      held_[held_count_] = host;
+      held_bytes_[held_count_++] = bytes;
+    }
     if (pinned && !reread) {
-      in_place_[in_place_count_] = host;
-      in_place_bytes_[in_place_count_++] = bytes;
       *device = host;
       return WB200_OK;
     }
@@ -63,7 +65,7 @@ class CommandIO {
   wb200_status output(size_t slot, const uint8_t *storage_template, uint8_t *host, size_t bytes, bool padded, uint8_t **device) {
     bytes_ = bytes;
     bool overlaps = false;
-    for (int i = 0; i < in_place_count_; ++i) overlaps |= host < in_place_[i] + in_place_bytes_[i] && in_place_[i] < host + bytes;
+    for (int i = 0; i < held_count_; ++i) overlaps |= host < held_[i] + held_bytes_[i] && held_[i] < host + bytes;
     if (!overlaps && page_locked(host, bytes)) {
       if (padded && host != storage_template) memmove(host, storage_template, bytes);
       *device = host;
@@ -197,9 +199,9 @@ class CommandIO {
   uint8_t *mapped_ = nullptr;
   const uint8_t *device_ = nullptr;
   bool in_place_result_ = false, finished_ = false;
-  const uint8_t *in_place_[4];
-  size_t in_place_bytes_[4];
-  int in_place_count_ = 0;
+  const uint8_t *held_[4];      // page-locked operands: a result that overlaps one is written only after they have been read
+  size_t held_bytes_[4];
+  int held_count_ = 0;
   size_t bytes_ = 0;
 };
 

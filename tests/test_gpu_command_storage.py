@@ -162,3 +162,20 @@ def test_padded_result_over_a_page_locked_operand(backend, monkeypatch):
             over, command = list(commands(pinned(lhs), pinned(rhs), pinned(source)))[index]
             into(patch, over)
             assert np.array_equal(command().destination.storage, want)
+
+
+@pytest.mark.parametrize("start", [0, 1 << 17])
+def test_storage_of_which_only_a_part_is_registered(backend, start):
+    elements = 1 << 16
+    room = np.zeros(4 * elements + 4096, np.uint8)
+    lead = -room.ctypes.data % 4096
+    x = room[lead:lead + 4 * elements].view(np.float32)
+    x[:] = np.arange(elements)
+    runtime = torch.cuda.cudart()
+    assert runtime.cudaHostRegister(x.ctypes.data + start, 1 << 17, 0) == runtime.cudaError.success   # half of the operand
+    try:
+        key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [elements])
+        got = backend.execute_elementwise("add", [NumericTensor(key, x), NumericTensor(key, x)], NumericTensor(key, np.zeros(4 * elements, np.uint8)))
+        assert np.array_equal(got.destination.storage.view(np.float32), x + x)
+    finally:
+        runtime.cudaHostUnregister(x.ctypes.data + start)

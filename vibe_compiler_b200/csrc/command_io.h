@@ -160,13 +160,10 @@ class CommandIO {
   }
 
  private:
-  // Page-locked by the CUDA runtime and addressable by the device at the same, 16-byte aligned address. Small operands are
-  // not worth the query.
+  // Page-locked from the first byte to the last (a caller may have registered only a part) and 16-byte aligned. Small
+  // operands are not worth the query.
   static bool page_locked(const void *host, size_t bytes) {
-    if (bytes < 16384 || (reinterpret_cast<uintptr_t>(host) & 15u)) return false;
-    cudaPointerAttributes attributes;
-    if (cudaPointerGetAttributes(&attributes, host) != cudaSuccess) { cudaGetLastError(); return false; }
-    return attributes.type == cudaMemoryTypeHost && attributes.devicePointer == host;
+    return bytes >= 16384 && (reinterpret_cast<uintptr_t>(host) & 15u) == 0 && page_locked_range(host, bytes);
   }
   // What kernels access in place lies at the end of the area, pieces on their way to device memory at its start.
   uint8_t *take(size_t bytes) {

@@ -69,6 +69,9 @@ wb200_status encode_tmap_3d(CUtensorMap *map, const void *base, int format, uint
                             uint64_t outer, uint64_t batch, uint64_t row_pitch_bytes,
                             uint64_t batch_pitch_bytes, uint32_t box_inner, uint32_t box_outer);
 
+// All of [host, host + bytes) lies in one page-locked allocation or registration, which the device addresses alike.
+bool page_locked_range(const void *host, size_t bytes);
+
 // ---- tcgen05 GEMM with fused epilogue (gemm_umma.cu)
 struct GemmUmmaArgs {
   int m, n, k;

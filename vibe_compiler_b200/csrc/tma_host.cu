@@ -1,7 +1,5 @@
-// Host-side construction of TMA tensor maps. cuTensorMapEncodeTiled is looked up through the
-// runtime's driver-entry-point query, so the library has no link-time dependency on libcuda.
-#include <mutex>
-
+// Host-side calls of the driver: construction of TMA tensor maps, extent of page-locked memory. The functions are looked
+// up through the runtime's driver-entry-point query, so the library has no link-time dependency on libcuda.
 #include "kernels.h"
 
 namespace wb200 {
@@ -12,17 +10,17 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_
                                    const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+using PointerAttributesFn = CUresult (*)(unsigned int, CUpointer_attribute *, void **, CUdeviceptr);
+
+void *driver_function(const char *name) {
+  void *entry = nullptr;
+  cudaDriverEntryPointQueryResult query;
+  if (cudaGetDriverEntryPoint(name, &entry, cudaEnableDefault, &query) != cudaSuccess || query != cudaDriverEntryPointSuccess) return nullptr;
+  return entry;
+}
+
 EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void *entry = nullptr;
-    cudaDriverEntryPointQueryResult query;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &entry, cudaEnableDefault, &query) ==
-            cudaSuccess &&
-        query == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(entry);
-  });
+  static const EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(driver_function("cuTensorMapEncodeTiled"));
   return fn;
 }
 
@@ -66,6 +64,20 @@ wb200_status encode_tmap_3d(CUtensorMap *map, const void *base, int format, uint
   const cuuint64_t strides[2] = {row_pitch_bytes, batch_pitch_bytes};
   const cuuint32_t box[3] = {box_inner, box_outer, 1};
   return encode(map, base, format, 3, dims, strides, box);
+}
+
+bool page_locked_range(const void *host, size_t bytes) {
+  static const PointerAttributesFn fn = reinterpret_cast<PointerAttributesFn>(driver_function("cuPointerGetAttributes"));
+  if (!fn) return false;
+  unsigned int type = 0;   // stays 0 for memory the driver does not know
+  CUdeviceptr device = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute names[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void *values[4] = {&type, &device, &start, &size};
+  const CUdeviceptr address = reinterpret_cast<CUdeviceptr>(host);
+  if (fn(4, names, values, address) != CUDA_SUCCESS) return false;
+  return type == CU_MEMORYTYPE_HOST && device == address && start <= address && address - start <= size && bytes <= size - (address - start);
 }
 
 }  // namespace wb200

@@ -312,7 +312,9 @@ wb200_status wb200_attention_fa(wb200_backend *backend, const wb200_attention_pa
  * The split-KV partial records of this entry and of wb200_attention_fd_partial / _exchange live in a grow-only scratch
  * buffer of the backend: a call that needs more than every call before it frees and reallocates that buffer (cudaFree
  * waits for the device's outstanding work first), so a CUDA graph that captured an earlier decode call would replay
- * with a dangling address. Run the largest shape once before capturing. */
+ * with a dangling address. Run the largest shape once before capturing. All calls of a backend share that scratch: the
+ * results of calls whose kernels overlap on the GPU (different streams) are undefined, so serialise them, or give each
+ * stream a backend of its own. Calls that follow an overlap in order are not affected by it. */
 wb200_status wb200_attention_fd(wb200_backend *backend, const wb200_attention_params *params,
                                 uint32_t kv_splits);
 
@@ -327,7 +329,8 @@ wb200_status wb200_attention_fd(wb200_backend *backend, const wb200_attention_pa
  * batch * q_heads * kv_splits * (head_dim + 2) <= 4 194 304 floats, otherwise WB200_ERR_LIMIT
  * (kv_splits == 0 takes the split count wb200_attention_fd would choose and halves it until it fits). The first call on a device looks up the
  * array's device address; make that call before any stream capture begins. All calls share the one
- * array: two calls whose kernels overlap on the GPU (different streams) race on it, so serialise them.
+ * array, whatever backend they go through: the results of calls whose kernels overlap on the GPU (different streams) are
+ * undefined, so serialise them. Calls that follow an overlap in order are not affected by it.
  * Nothing in the array has to be cleared between calls (every record read is written first). */
 wb200_status wb200_attention_fd_static(wb200_backend *backend, const wb200_attention_params *params,
                                        uint32_t kv_splits);

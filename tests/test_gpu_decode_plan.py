@@ -32,3 +32,37 @@ def test_decode_plans_match_float64(backend, shape, dtype):
     assert (lse.double() - torch.logsumexp(scores, -1)).abs().max().item() <= 2e-4
     assert (m.double() - scores.amax(-1)).abs().max().item() <= 1e-4
     assert torch.allclose(m.double() + l.double().log(), lse.double(), atol=1e-5)
+
+
+@pytest.mark.parametrize("static", [False, True])
+def test_decode_is_right_after_calls_that_overlapped(backend, static):
+    """Calls that share the scratch and overlap on two streams have no defined result, but the calls after them do, eager and
+    replayed from a graph, with every number of records."""
+    gen = torch.Generator(device="cuda").manual_seed(17)
+    q, k, v = (torch.randn(2, h, n, 128, device="cuda", generator=gen).bfloat16() for h, n in ((8, 1), (2, 30000), (2, 30000)))
+    kk, vv = (t.double().repeat_interleave(4, 1) for t in (k, v))
+    want = torch.softmax(q.double() @ kk.transpose(-1, -2) * 128 ** -0.5, -1) @ vv
+    decode = backend.attention_fd_static if static else backend.attention_fd
+
+    def run(splits, **more):
+        return decode(q, k, v, 128 ** -0.5, kv_splits=splits, **more)
+    run(16)   # the scratch has its size
+    torch.cuda.synchronize()
+    graph, replayed = torch.cuda.CUDAGraph(), torch.empty_like(q)
+    with torch.cuda.graph(graph):
+        run(6, out=replayed)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    spare = [torch.empty_like(q) for _ in streams]
+    for turn in range(4):
+        for _ in range(8):
+            for stream, splits, out in zip(streams, (3 + turn, 7), spare):
+                run(splits, stream=stream.cuda_stream, out=out)
+        torch.cuda.synchronize()
+        for splits in (2, 7, 16):
+            got = run(splits, out=torch.full_like(q, float("nan")))
+            assert helpers.max_rel_err(got.double().cpu().numpy(), want.cpu().numpy()) <= 2 ** -7
+        replayed.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert helpers.max_rel_err(replayed.double().cpu().numpy(), want.cpu().numpy()) <= 2 ** -7
+    backend.poll()

@@ -101,7 +101,7 @@ struct FdTailParams {
   int rank, world;
   float *peer[kMaxExchangeRanks];    // exchange buffers of all ranks, [rank] = this rank's own
   unsigned int *epoch;               // this rank's {epoch, finished rows}, zero-initialised
-  unsigned int *arrivals;            // [batch * kv_heads] finished stage-1 CTAs, zero-initialised, reset by the last one
+  unsigned int *arrivals;            // [batch * kv_heads] of fd_arrive(), zero-initialised
   int out_format, zero_fully_masked;
   void *out;
   float *lse, *row_max, *row_sum;
@@ -210,6 +210,14 @@ __device__ void fd_local_rows(const FdTailParams &x, const float *records, int s
     fd_fold_records(records + static_cast<size_t>(row) * splits * kRecord, splits, lane, m, l, a);
     fd_deliver_row(x, row, lane, m, l, a);
   }
+}
+// Counts the arrival of cluster `index` of a (batch, kv head) unit's `clusters`; true for the last one. The shares of a launch
+// add up to 2^32, that is to nothing, and are added whatever the word holds: the word is back at zero after every launch, also
+// after launches that wrongly overlapped on one scratch, which can spoil each other's results but not those of later ones.
+// The sum is zero only at the last arrival: the others give 1 each, the first cluster 1 - clusters.
+__device__ __forceinline__ bool fd_arrive(unsigned int *word, unsigned int index, unsigned int clusters) {
+  const unsigned int share = index == 0u ? 1u - clusters : 1u;
+  return atomicAdd(word, share) + share == 0u;
 }
 // Swizzled byte offset of 16-byte chunk `c` of row `r` inside a 16 x 256-byte tile.
 __device__ __forceinline__ uint32_t tile_offset(int r, int c) {
@@ -471,9 +479,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) fd_partial_kernel(const FdPara
     __syncthreads();
     if (threadIdx.x == 0) {
       __threadfence();      // cumulative over the CTA's record stores, which the barrier ordered before it
-      unsigned int *arrivals = tail.arrivals + b * p.kv_heads + hk;
-      const unsigned int last = static_cast<unsigned int>(p.splits) - 1u;
-      last_of_head = atomicInc(arrivals, last) == last;   // wraps to zero, ready for the next launch
+      last_of_head = fd_arrive(tail.arrivals + b * p.kv_heads + hk, static_cast<unsigned int>(cluster_index), static_cast<unsigned int>(p.splits));
       __threadfence();
     }
     __syncthreads();
@@ -843,7 +849,7 @@ namespace {
 
 constexpr size_t kStaticScratchFloats = size_t(4) << 20;   // 16 MiB, held by every GPU that loads the library
 static __device__ __align__(256) float g_fd_static_scratch[kStaticScratchFloats];
-// Arrival counters of the (batch, kv head) units, left at zero by every launch; a unit has at least one row of at least one record.
+// Arrival words of the (batch, kv head) units (fd_arrive); a unit has at least one row of at least one record.
 constexpr size_t kStaticArrivals = kStaticScratchFloats / kRecord;
 static __device__ unsigned int g_fd_static_arrivals[kStaticArrivals];
 

@@ -220,7 +220,9 @@ wb200_status launch_attention_fa_simt(const AttentionArgs &args, cudaStream_t st
 
 // Flash-decoding. `partials` is scratch of fd_partial_floats(args, plan.records) floats.
 // The keys of a (batch, kv head) are cut over `records` clusters of `cluster` CTAs. Every cluster writes one (acc[D], m, l)
-// record per query head; the last cluster of a (batch, kv head) folds them (with one record it finalizes directly). `arrivals` is batch * kv_heads zero-initialised words, which the kernel leaves zeroed.
+// record per query head; the last cluster of a (batch, kv head) folds them (with one record it finalizes directly).
+// `arrivals` is batch * kv_heads words for that count, zero when they are made. Launches that share `partials` and `arrivals`
+// must not overlap; if they do, the results of those launches are undefined, later ones are not touched.
 // With `state_out` the merged state goes there instead of out / lse.
 bool attention_fd_supports(const AttentionArgs &args);
 struct FdPlan { uint32_t cluster, records; };
@@ -234,8 +236,8 @@ wb200_status launch_attention_fd_merge(const AttentionArgs &args, const float *s
 // Sequence-sharded decode with the exchange inside the kernel: stage 1, then one kernel that folds this rank's splits,
 // writes the state into every rank's exchange buffer (peer-mapped memory), waits for the world's states and merges
 // them in ascending rank order. `peer_buffers` holds `world` buffers of fd_exchange_floats() floats, zero-initialised;
-// `epoch` is this rank's pair of zero-initialised words. With `arrivals` (batch * kv_heads zero-initialised words that the
-// kernel leaves zeroed) the fold, exchange and merge run in the last stage-1 CTA of every (batch, kv head): one launch.
+// `epoch` is this rank's pair of zero-initialised words. With `arrivals` (as above) the fold,
+// exchange and merge run in the last stage-1 CTA of every (batch, kv head): one launch.
 size_t fd_exchange_floats(int rows, int world);
 wb200_status launch_attention_fd_exchange(const AttentionArgs &args, FdPlan plan, float *partials, int rank, int world,
                                           void *const *peer_buffers, unsigned int *epoch, unsigned int *arrivals,

@@ -7,6 +7,7 @@
 #include "kernels.h"
 #include "formal_functions_f32.cuh"
 #include "ptx_sm100.cuh"
+#include "storage_walk.cuh"
 
 namespace wb200 {
 namespace {
@@ -43,52 +44,10 @@ __device__ __forceinline__ float apply_elementwise(int op, float x, float y) {
   }
 }
 
-// A walk over physical storage in groups of eight elements, for commands whose operands are placed alike: linear layouts,
-// and Cx / NCx tensors of one shape (channel blocks of 64, then the aligned tail; slices padded to bank lines). The
-// alternative, an element per thread through the row-major-to-physical map, spends its time on 64-bit divisions and moves
-// two or four bytes per access (a 256 x 520 Cx convert took 8 us).
-struct StorageWalk {
-  int dense;                      // every physical element is a logical one (no padding): `count` consecutive elements
-  int64_t count;
-  uint32_t slices;                // else: NCx leading slices,
-  int64_t groups;                 //   groups of a slice,
-  int64_t src_stride, dst_stride; //   elements between slices,
-  int64_t full;                   //   elements of a slice's full channel blocks,
-  int64_t used;                   //   elements of a slice before its end padding,
-  uint32_t block_elements;        //   elements of a channel block (outer extent x 64),
-  uint32_t channels, full_channels, tail;   //   logical channels, channels of the full blocks, width of the tail
-};
-__device__ __forceinline__ uint32_t walk_valid(const StorageWalk &w, int64_t offset) {
-  // bit e: element `offset` + e of a slice is a logical element
-  if (offset < w.full) {
-    const uint32_t block = offset < 0x80000000ll ? static_cast<uint32_t>(offset) / w.block_elements : static_cast<uint32_t>(offset / w.block_elements);
-    const int left = static_cast<int>(w.channels) - static_cast<int>(block * 64u + static_cast<uint32_t>(offset & 63));
-    return left >= 8 ? 0xffu : left <= 0 ? 0u : (1u << left) - 1u;
-  }
-  uint32_t mask = 0;
-  const uint32_t keep = w.channels - w.full_channels;   // logical channels of the tail (its width is a power of two)
-#pragma unroll
-  for (int e = 0; e < 8; ++e)
-    if (offset + e < w.used && static_cast<uint32_t>((offset - w.full + e) & (w.tail - 1)) < keep) mask |= 1u << e;
-  return mask;
-}
-// Calls visit(src element, dst element, valid mask, wide) for this thread's groups; `wide`: all eight are there and valid.
+// Calls visit(src element, dst element, valid mask) for this thread's groups.
 template <typename Visit>
 __device__ __forceinline__ void walk_groups(const StorageWalk &w, Visit &&visit) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (w.dense) {
-    for (int64_t g = first; g * 8 < w.count; g += stride) {
-      const int64_t left = w.count - g * 8;
-      visit(g * 8, g * 8, left >= 8 ? 0xffu : (1u << static_cast<int>(left)) - 1u);
-    }
-  } else {
-    for (uint32_t slice = 0; slice < w.slices; ++slice)
-      for (int64_t g = first; g < w.groups; g += stride) {
-        const uint32_t valid = walk_valid(w, g * 8);
-        if (valid) visit(slice * w.src_stride + g * 8, slice * w.dst_stride + g * 8, valid);
-      }
-  }
+  walk_groups(w, static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x, static_cast<int64_t>(gridDim.x) * blockDim.x, visit);
 }
 __device__ __forceinline__ void walk_load(const uint8_t *base, int64_t at, uint32_t valid, int format, uint32_t (&v)[8]) {
   if (valid == 0xffu) {
@@ -1336,25 +1295,6 @@ wb200_status launch_codec(const uint8_t *src, uint8_t *dst, const LayoutMap &map
   return WB200_OK;
 }
 
-// `src` and `dst` describe tensors of one shape and layout (their formats, and so their slice strides, may differ).
-StorageWalk storage_walk(const LayoutMap &src, const LayoutMap &dst) {
-  StorageWalk w{};
-  w.dense = src.physical_elements == src.element_count && dst.physical_elements == dst.element_count;
-  w.count = src.element_count;
-  if (w.dense) return w;
-  const bool sliced = src.layout == WB200_LAYOUT_NCX && src.rank > 1;
-  w.slices = sliced ? static_cast<uint32_t>(src.shape[0]) : 1u;
-  w.src_stride = src.outer_slice_stride;
-  w.dst_stride = dst.outer_slice_stride;
-  w.block_elements = static_cast<uint32_t>(src.block_outer_elements * src.c_block);
-  w.channels = static_cast<uint32_t>(src.shape[src.rank - 1]);
-  w.full_channels = static_cast<uint32_t>(src.cx_blocks * src.c_block);
-  w.tail = static_cast<uint32_t>(src.c0);
-  w.full = src.cx_blocks * src.block_outer_elements * src.c_block;
-  w.used = w.full + src.block_outer_elements * src.c0;
-  w.groups = (w.used + 7) / 8;
-  return w;
-}
 int walk_grid(const StorageWalk &w) {
   const int64_t groups = w.dense ? (w.count + 7) / 8 : w.groups;
   const int64_t blocks = (groups + kThreads - 1) / kThreads;

@@ -47,6 +47,13 @@ static void check_all(int from, int to, int layout, const std::vector<uint64_t> 
   for (int64_t at = 0; at < src.physical_elements; ++at) expect(place[at] < 0, "padding visited", shape, at);
 }
 
+// Groups are spread over threads across the slices: a thread per group as long as the machine has room for them.
+static void check_threads(int layout, const std::vector<uint64_t> &shape) {
+  const LayoutMap map = map_of(WB200_BF16, layout, shape);
+  const int64_t groups = map.physical_elements / 8, threads = 256ll * walk_blocks(storage_walk(map, map), 256);
+  expect(threads >= (groups < 256 * 148 * 32 ? map.element_count / 8 : 256 * 148 * 32), "too few threads", shape, threads);
+}
+
 // Samples of a tensor too large to hold.
 static void check_some(int layout, const std::vector<uint64_t> &shape) {
   const LayoutMap map = map_of(WB200_BF16, layout, shape);
@@ -71,6 +78,8 @@ int main() {
     for (const auto &shape : shapes)
       for (int from : formats)
         for (int to : formats) check_all(from, to, layout, shape);
+  for (const auto &shape : std::vector<std::vector<uint64_t>>{{4096, 1, 64}, {4096, 1, 40}, {512, 7, 97}, {1, 1 << 20, 3}, {1 << 20, 1, 130}})
+    check_threads(WB200_LAYOUT_NCX, shape);
   const uint64_t outer = 1ull << 26;   // 64 * outer passes 32 bits
   check_some(WB200_LAYOUT_CX, {outer - 1, 130});
   check_some(WB200_LAYOUT_CX, {outer, 130});

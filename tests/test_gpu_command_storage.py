@@ -23,7 +23,7 @@ def logical(backend, key, storage, dtype):
 
 
 @pytest.mark.parametrize("layout,shape", [("tensor", [7]), ("tensor", [1003]), ("cx", [3, 5]), ("cx", [5, 66]), ("cx", [7, 97]), ("cx", [33, 64]),
-                                          ("ncx", [2, 3, 65]), ("ncx", [3, 2, 5, 129]), ("cx", [1031, 263]), ("tensor", [700001])])
+                                          ("ncx", [2, 3, 65]), ("ncx", [3, 2, 5, 129]), ("ncx", [2049, 1, 64]), ("ncx", [300, 2, 97]), ("cx", [1031, 263]), ("tensor", [700001])])
 def test_elementwise_and_convert_keep_padding_and_match_numpy(backend, layout, shape):
     rng = np.random.default_rng(sum(shape))
     count = int(np.prod(shape))

@@ -9,6 +9,7 @@
 namespace wb200 {
 
 struct StorageWalk {
+  int64_t units;                  // groups in all: a thread takes them one by one, whichever slice they belong to
   int dense;                      // every physical element is a logical one (no padding): `count` consecutive elements
   int64_t count;
   int64_t slices;                 // else: NCx leading slices,
@@ -26,6 +27,7 @@ inline StorageWalk storage_walk(const LayoutMap &src, const LayoutMap &dst) {
   StorageWalk w{};
   w.dense = src.physical_elements == src.element_count && dst.physical_elements == dst.element_count;
   w.count = src.element_count;
+  w.units = (w.count + 7) / 8;
   if (w.dense) return w;
   const bool sliced = src.layout == WB200_LAYOUT_NCX && src.rank > 1;
   w.slices = sliced ? src.shape[0] : 1;
@@ -38,7 +40,14 @@ inline StorageWalk storage_walk(const LayoutMap &src, const LayoutMap &dst) {
   w.full = src.cx_blocks * src.block_outer_elements * src.c_block;
   w.used = w.full + src.block_outer_elements * src.c0;
   w.groups = (w.used + 7) / 8;
+  w.units = w.slices * w.groups;
   return w;
+}
+
+// Blocks of `threads` that give every group a thread, up to 32 per SM of 148.
+inline int walk_blocks(const StorageWalk &w, int threads) {
+  const int64_t blocks = (w.units + threads - 1) / threads;
+  return static_cast<int>(blocks < 1 ? 1 : blocks > 148 * 32 ? 148 * 32 : blocks);
 }
 
 // Bit e: element `offset` + e of a slice is a logical element.
@@ -60,17 +69,19 @@ __host__ __device__ inline uint32_t walk_valid(const StorageWalk &w, int64_t off
 #pragma nv_exec_check_disable   // a kernel's visitor is device code
 template <typename Visit>
 __host__ __device__ inline void walk_groups(const StorageWalk &w, int64_t first, int64_t stride, Visit &&visit) {
-  if (w.dense) {
-    for (int64_t g = first; g * 8 < w.count; g += stride) {
-      const int64_t left = w.count - g * 8;
-      visit(g * 8, g * 8, left >= 8 ? 0xffu : (1u << static_cast<int>(left)) - 1u);
+  for (int64_t u = first; u < w.units; u += stride) {
+    if (w.dense) {
+      const int64_t left = w.count - u * 8;
+      visit(u * 8, u * 8, left >= 8 ? 0xffu : (1u << static_cast<int>(left)) - 1u);
+      continue;
     }
-  } else {
-    for (int64_t slice = 0; slice < w.slices; ++slice)
-      for (int64_t g = first; g < w.groups; g += stride) {
-        const uint32_t valid = walk_valid(w, g * 8);
-        if (valid) visit(slice * w.src_stride + g * 8, slice * w.dst_stride + g * 8, valid);
-      }
+    int64_t slice = 0, at = u * 8;
+    if (w.slices > 1) {
+      slice = w.units < (1ll << 32) ? static_cast<uint32_t>(u) / static_cast<uint32_t>(w.groups) : u / w.groups;
+      at = (u - slice * w.groups) * 8;
+    }
+    const uint32_t valid = walk_valid(w, at);
+    if (valid) visit(slice * w.src_stride + at, slice * w.dst_stride + at, valid);
   }
 }
 

@@ -1295,12 +1295,6 @@ wb200_status launch_codec(const uint8_t *src, uint8_t *dst, const LayoutMap &map
   return WB200_OK;
 }
 
-int walk_grid(const StorageWalk &w) {
-  const int64_t groups = w.dense ? (w.count + 7) / 8 : w.groups;
-  const int64_t blocks = (groups + kThreads - 1) / kThreads;
-  return static_cast<int>(blocks < 1 ? 1 : blocks > 148 * 32 ? 148 * 32 : blocks);
-}
-
 // Few outputs cannot fill the machine with one thread each; the staged fold spreads their loads over 8 threads per output.
 constexpr int64_t kManyOutputs = 65536;
 template <bool kFormal>
@@ -1381,7 +1375,7 @@ wb200_status launch_elementwise(int op, int format, int input_count, const uint8
                                 uint8_t *dst, const LayoutMap &map, int *nan_flag, cudaStream_t stream) {
   if (!all_aligned16(in0, in1, dst)) return fail(WB200_ERR_INVALID_ARGUMENT, "elementwise storage must be 16-byte aligned on the device");
   const StorageWalk walk = storage_walk(map, map);
-  const int grid = walk_grid(walk);
+  const int grid = walk_blocks(walk, kThreads);
 #define WB200_MEW(OP)                                                                                                                     \
   case OP:                                                                                                                                \
     if (format == WB200_F32) elementwise_walk_kernel<OP, WB200_F32><<<grid, kThreads, 0, stream>>>(input_count, in0, in1, dst, walk, nan_flag);        \
@@ -1591,7 +1585,7 @@ wb200_status launch_convert(int src_format, int dst_format, const uint8_t *src, 
   if (!is_float_format(src_format) || !is_float_format(dst_format) || src_map.layout != dst_map.layout || !all_aligned16(src, dst))
     return fail(WB200_ERR_INVALID_ARGUMENT, "convert takes float formats of one layout, 16-byte aligned on the device");
   const StorageWalk walk = storage_walk(src_map, dst_map);
-  const int grid = walk_grid(walk);
+  const int grid = walk_blocks(walk, kThreads);
 #define WB200_MCV(SRC, DST) convert_walk_kernel<SRC, DST><<<grid, kThreads, 0, stream>>>(src, dst, walk, nan_flag)
 #define WB200_MCV_TO(SRC)                                        \
   if (dst_format == WB200_F32) WB200_MCV(SRC, WB200_F32);        \

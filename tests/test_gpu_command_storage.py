@@ -1,5 +1,7 @@
 """Command calls on host storage around the sizes where their paths change: element groups against padded channel tails and
 bank-line padding, folds of a few long chains, storage read in place (up to 1 MiB) against storage copied in pieces."""
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -179,3 +181,21 @@ def test_storage_of_which_only_a_part_is_registered(backend, start):
         assert np.array_equal(got.destination.storage.view(np.float32), x + x)
     finally:
         runtime.cudaHostUnregister(x.ctypes.data + start)
+
+
+def test_ragged_product_under_the_tensor_policy_reads_its_operands_on_the_device(backend):
+    """A product the tensor-core kernel does not take runs on the bit-exact kernel, which reads operands many times: the same bits,
+    in about the time of the bit-exact policy (read over PCIe instead, this one took six times as long)."""
+    m, k, n = 4001, 1005, 4003
+    lhs_key, rhs_key, out_key = (PhysicalTensorDescriptor(abi.BF16, abi.LAYOUT_CX, shape) for shape in ([m, k], [k, n], [m, n]))
+    rng = np.random.default_rng(2)
+    lhs, rhs = (NumericTensor(key, pinned(physical(backend, key, rng.integers(0x3e00, 0x4000, key.element_count).astype(np.uint16)))) for key in (lhs_key, rhs_key))
+    blank = NumericTensor(out_key, np.zeros(B200TargetModelBackend.physical_bytes(out_key), np.uint8))
+    operation = FormalGemmOperation(lhs_key, rhs_key, out_key, m, k, n)
+    best, results = {}, {}
+    for policy in (abi.GEMM_FORMAL, abi.GEMM_TENSOR) * 4:
+        begin = time.perf_counter()
+        results[policy] = backend.try_execute(operation, lhs, rhs, blank, policy=policy).destination.storage
+        best[policy] = min(best.get(policy, 1e9), time.perf_counter() - begin)
+    assert np.array_equal(results[abi.GEMM_FORMAL], results[abi.GEMM_TENSOR])
+    assert best[abi.GEMM_TENSOR] < 2 * best[abi.GEMM_FORMAL], best

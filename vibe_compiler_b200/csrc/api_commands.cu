@@ -17,6 +17,22 @@ struct DeviceGemm {
   uint8_t *dst;                     // device, physical storage (pre-filled with the template)
 };
 
+// Whether the tensor-core kernel takes a command under `policy`, its compact operands being 16-byte aligned; *args describes one
+// matrix of the batch then.
+bool tensor_gemm(const DeviceGemm &g, int policy, GemmUmmaArgs *args) {
+  if (policy != WB200_GEMM_TENSOR || g.has_psum || (g.in_format != WB200_BF16 && g.in_format != WB200_F16)) return false;
+  const size_t in_bytes = 2, out_bytes = g.out_format == WB200_F32 ? 4 : 2;
+  // Per-batch operand offsets must keep 16-byte alignment for TMA.
+  if (g.batch != 1 && ((static_cast<size_t>(g.m) * g.k * in_bytes) % 16 != 0 || (static_cast<size_t>(g.k) * g.n * in_bytes) % 16 != 0 ||
+                       (static_cast<size_t>(g.m) * g.n * out_bytes) % 16 != 0))
+    return false;
+  args->m = g.m; args->n = g.n; args->k = g.k;
+  args->in_format = g.in_format; args->out_format = g.out_format;
+  args->lhs_transposed = g.lhs_transposed; args->rhs_transposed = g.rhs_transposed;
+  args->epilogue = WB200_EPI_NONE;
+  return gemm_umma_supports(*args);
+}
+
 // Runs one GEMM command whose operands already sit on the device. `scratch_slot` is the first of
 // three backend staging slots the tensor path may use for compact operands.
 // `private_staging` (three areas of `private_each` bytes) replaces the backend slots when given: commands of different
@@ -25,22 +41,12 @@ struct DeviceGemm {
 wb200_status run_device_gemm(wb200_backend *backend, const DeviceGemm &g, int policy, size_t scratch_slot,
                              cudaStream_t stream, const char **implementation, bool host_operands, uint8_t *private_staging = nullptr,
                              size_t private_each = 0) {
-  const bool tensor_domain = policy == WB200_GEMM_TENSOR && !g.has_psum &&
-                             (g.in_format == WB200_BF16 || g.in_format == WB200_F16);
-  if (tensor_domain) {
+  GemmUmmaArgs probe{};
+  if (tensor_gemm(g, policy, &probe)) {
     const size_t in_bytes = 2;
     const size_t out_bytes = g.out_format == WB200_F32 ? 4 : 2;
     const size_t lhs_count = static_cast<size_t>(g.batch) * g.m * g.k, rhs_count = static_cast<size_t>(g.batch) * g.k * g.n;
     const size_t dst_count = static_cast<size_t>(g.batch) * g.m * g.n;
-    GemmUmmaArgs probe{};
-    probe.m = g.m; probe.n = g.n; probe.k = g.k;
-    probe.in_format = g.in_format; probe.out_format = g.out_format;
-    probe.lhs_transposed = g.lhs_transposed; probe.rhs_transposed = g.rhs_transposed;
-    probe.epilogue = WB200_EPI_NONE;
-    // Per-batch operand offsets must keep 16-byte alignment for TMA.
-    const bool batch_aligned = g.batch == 1 || ((static_cast<size_t>(g.m) * g.k * in_bytes) % 16 == 0 &&
-                                                (static_cast<size_t>(g.k) * g.n * in_bytes) % 16 == 0 &&
-                                                (static_cast<size_t>(g.m) * g.n * out_bytes) % 16 == 0);
     void *c_lhs, *c_rhs, *c_dst;
     wb200_status st;
     if (private_staging) {
@@ -53,7 +59,7 @@ wb200_status run_device_gemm(wb200_backend *backend, const DeviceGemm &g, int po
       if ((st = backend->buffer(scratch_slot + 2, dst_count * out_bytes, &c_dst)) != WB200_OK) return st;
     }
     probe.a = c_lhs; probe.b = c_rhs; probe.out = c_dst;
-    if (batch_aligned && gemm_umma_supports(probe)) {
+    if (gemm_umma_supports(probe)) {   // the private areas may lie less than 16-byte aligned
       int unpacks = 2;
       if (host_operands) {
         st = launch_unpack_pair(g.lhs, static_cast<uint8_t *>(c_lhs), g.lhs_map, g.rhs, static_cast<uint8_t *>(c_rhs), g.rhs_map, 2, &unpacks, stream);
@@ -136,8 +142,13 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   }
   DeviceGuard guard(backend->device);
   cudaStream_t stream = backend->stream;
-  // The tensor policy unpacks each operand once; the bit-exact kernel reads operands (and nothing else) again per output tile.
-  const bool reread = r->policy == WB200_GEMM_FORMAL;
+  g.m = r->m; g.k = r->k; g.n = r->n; g.batch = r->batch_count;
+  g.in_format = r->lhs.format; g.out_format = r->destination.format;
+  g.lhs_transposed = lt; g.rhs_transposed = rt; g.has_psum = r->has_psum ? 1 : 0;
+  // The tensor path unpacks each operand once; the bit-exact kernel, which also runs the tensor policy's ragged products, reads
+  // operands (and nothing else) again per output tile: 4001 x 4003 x 1005 from page-locked memory took 36.0 ms over PCIe.
+  GemmUmmaArgs unused{};
+  const bool reread = !tensor_gemm(g, r->policy, &unused);
   CommandIO io(backend, r->lhs_bytes + r->rhs_bytes + r->destination_bytes + (r->has_psum ? r->psum_bytes : 0));
   if ((st = io.status()) != WB200_OK) return st;
   const uint8_t *d_lhs, *d_rhs, *d_psum = nullptr;
@@ -146,9 +157,6 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   if ((st = io.input(1, r->rhs_storage, r->rhs_bytes, &d_rhs, reread)) != WB200_OK) return st;
   if (r->has_psum && (st = io.input(3, r->psum_storage, r->psum_bytes, &d_psum)) != WB200_OK) return st;
   if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(g.dst_map), &d_dst)) != WB200_OK) return st;
-  g.m = r->m; g.k = r->k; g.n = r->n; g.batch = r->batch_count;
-  g.in_format = r->lhs.format; g.out_format = r->destination.format;
-  g.lhs_transposed = lt; g.rhs_transposed = rt; g.has_psum = r->has_psum ? 1 : 0;
   g.lhs = d_lhs; g.rhs = d_rhs;
   g.psum = d_psum; g.dst = d_dst;
   const uint64_t launches_before = backend->launches;

@@ -199,3 +199,51 @@ def test_ragged_product_under_the_tensor_policy_reads_its_operands_on_the_device
         best[policy] = min(best.get(policy, 1e9), time.perf_counter() - begin)
     assert np.array_equal(results[abi.GEMM_FORMAL], results[abi.GEMM_TENSOR])
     assert best[abi.GEMM_TENSOR] < 2 * best[abi.GEMM_FORMAL], best
+
+
+@pytest.mark.parametrize("m,n", [(33, 17), (256, 321), (700, 1001), (2049, 1003)])   # results staged, page-locked, in pieces
+def test_bit_exact_product_returns_through_every_kind_of_result_storage(backend, monkeypatch, m, n):
+    """The same bits and the template's padding, whether the result's storage is page-locked or pageable, apart from the template or
+    the template itself."""
+    k = 65
+    lhs_key, rhs_key, out_key = (PhysicalTensorDescriptor(abi.BF16, abi.LAYOUT_CX, shape) for shape in ([m, k], [k, n], [m, n]))
+    rng = np.random.default_rng(m)
+    a, b = (rng.integers(-8, 9, shape).astype(np.float32) for shape in ((m, k), (k, n)))   # small integers: every sum is exact
+    half = lambda x: torch.from_numpy(x.reshape(-1)).bfloat16().view(torch.int16).numpy().view(np.uint16)
+    lhs, rhs = NumericTensor(lhs_key, physical(backend, lhs_key, half(a))), NumericTensor(rhs_key, physical(backend, rhs_key, half(b)))
+    operation = FormalGemmOperation(lhs_key, rhs_key, out_key, m, k, n)
+    size = B200TargetModelBackend.physical_bytes(out_key)
+    want = backend.pack(out_key, half(a @ b), np.full(size, 0x33, np.uint8))
+    for storage in (pinned(np.zeros(size, np.uint8)), np.zeros(size, np.uint8)):
+        for template in (np.full(size, 0x33, np.uint8), storage):
+            storage[:] = 0x33
+            with monkeypatch.context() as patch:
+                into(patch, storage)
+                got = backend.try_execute(operation, lhs, rhs, NumericTensor(out_key, template), policy=abi.GEMM_FORMAL)
+            assert np.array_equal(got.destination.storage, want)
+
+
+def scattered_commands(backend):
+    """Commands whose kernels store one element at a time, with a result of 4 MB: name -> (descriptor, command)."""
+    key, other = (PhysicalTensorDescriptor(f, abi.LAYOUT_CX, [2000, 1030]) for f in (abi.BF16, abi.F16))
+    blank, other_blank = (NumericTensor(k, np.zeros(B200TargetModelBackend.physical_bytes(k), np.uint8)) for k in (key, other))
+    thin, wide = (PhysicalTensorDescriptor(abi.BF16, abi.LAYOUT_CX, shape) for shape in ([2000, 64], [64, 1030]))
+    lhs, rhs = (NumericTensor(k, np.zeros(B200TargetModelBackend.physical_bytes(k), np.uint8)) for k in (thin, wide))
+    product = FormalGemmOperation(thin, wide, key, 2000, 64, 1030)
+    return {"gemm": (key, lambda: backend.try_execute(product, lhs, rhs, blank, policy=abi.GEMM_FORMAL))}
+
+
+@pytest.mark.parametrize("name", ["gemm"])
+def test_page_locked_results_of_element_wise_stores_are_not_slower(backend, monkeypatch, name):
+    """A large result goes through device memory and one copy whatever its storage (stored over PCIe it took three times as long
+    with page-locked storage as with pageable storage)."""
+    key, command = scattered_commands(backend)[name]
+    size, best = B200TargetModelBackend.physical_bytes(key), {}
+    for _ in range(4):
+        for kind, storage in (("pageable", np.zeros(size, np.uint8)), ("page-locked", pinned(np.zeros(size, np.uint8)))):
+            with monkeypatch.context() as patch:
+                into(patch, storage)
+                begin = time.perf_counter()
+                command()
+                best[kind] = min(best.get(kind, 1e9), time.perf_counter() - begin)
+    assert best["page-locked"] < 1.5 * best["pageable"], best

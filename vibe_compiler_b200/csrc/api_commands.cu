@@ -148,7 +148,7 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   // The tensor path unpacks each operand once; the bit-exact kernel, which also runs the tensor policy's ragged products, reads
   // operands (and nothing else) again per output tile: 4001 x 4003 x 1005 from page-locked memory took 36.0 ms over PCIe.
   GemmUmmaArgs unused{};
-  const bool reread = !tensor_gemm(g, r->policy, &unused);
+  const bool reread = !tensor_gemm(g, r->policy, &unused);   // it also stores element by element
   CommandIO io(backend, r->lhs_bytes + r->rhs_bytes + r->destination_bytes + (r->has_psum ? r->psum_bytes : 0));
   if ((st = io.status()) != WB200_OK) return st;
   const uint8_t *d_lhs, *d_rhs, *d_psum = nullptr;
@@ -156,7 +156,7 @@ wb200_status wb200_gemm(wb200_backend *backend, const wb200_gemm_request *r, int
   if ((st = io.input(0, r->lhs_storage, r->lhs_bytes, &d_lhs, reread)) != WB200_OK) return st;
   if ((st = io.input(1, r->rhs_storage, r->rhs_bytes, &d_rhs, reread)) != WB200_OK) return st;
   if (r->has_psum && (st = io.input(3, r->psum_storage, r->psum_bytes, &d_psum)) != WB200_OK) return st;
-  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(g.dst_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(g.dst_map), &d_dst, reread ? g.dst_map.element_count : 0)) != WB200_OK) return st;
   g.lhs = d_lhs; g.rhs = d_rhs;
   g.psum = d_psum; g.dst = d_dst;
   const uint64_t launches_before = backend->launches;

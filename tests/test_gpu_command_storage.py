@@ -230,10 +230,12 @@ def scattered_commands(backend):
     thin, wide = (PhysicalTensorDescriptor(abi.BF16, abi.LAYOUT_CX, shape) for shape in ([2000, 64], [64, 1030]))
     lhs, rhs = (NumericTensor(k, np.zeros(B200TargetModelBackend.physical_bytes(k), np.uint8)) for k in (thin, wide))
     product = FormalGemmOperation(thin, wide, key, 2000, 64, 1030)
-    return {"gemm": (key, lambda: backend.try_execute(product, lhs, rhs, blank, policy=abi.GEMM_FORMAL))}
+    return {"gemm": (key, lambda: backend.try_execute(product, lhs, rhs, blank, policy=abi.GEMM_FORMAL)),
+            "add": (key, lambda: backend.execute_elementwise("add", [blank, blank], blank, formal=True)),
+            "convert": (other, lambda: backend.execute_convert(154, blank, other_blank, formal=True))}
 
 
-@pytest.mark.parametrize("name", ["gemm"])
+@pytest.mark.parametrize("name", ["gemm", "add", "convert"])
 def test_page_locked_results_of_element_wise_stores_are_not_slower(backend, monkeypatch, name):
     """A large result goes through device memory and one copy whatever its storage (stored over PCIe it took three times as long
     with page-locked storage as with pageable storage)."""

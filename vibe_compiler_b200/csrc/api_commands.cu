@@ -275,10 +275,12 @@ wb200_status wb200_elementwise_formal(wb200_backend *backend, const wb200_elemen
   const uint8_t *d_in[2] = {nullptr, nullptr}, *h_flags;
   uint8_t *d_dst;
   void *d_flags;
+  // outside the linear layouts the kernel loads and stores element by element
+  const int64_t scattered = is_linear(in_map) && is_linear(out_map) ? 0 : out_map.element_count;
   for (int i = 0; i < arity; ++i)
-    if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i])) != WB200_OK) return st;
+    if ((st = io.input(i, r->input_storage[i], r->input_bytes[i], &d_in[i], scattered > CommandIO::kScattered)) != WB200_OK) return st;
   // bit-packed results keep the template's bits behind the last element
-  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, bool_out || has_padding(out_map), &d_dst)) != WB200_OK) return st;
+  if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, bool_out || has_padding(out_map), &d_dst, scattered)) != WB200_OK) return st;
   if ((st = backend->buffer(3, sizeof(uint32_t), &d_flags)) != WB200_OK) return st;
   WB200_CUDA_CHECK(cudaMemsetAsync(d_flags, 0, sizeof(uint32_t), stream));
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;

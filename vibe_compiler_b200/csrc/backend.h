@@ -208,6 +208,7 @@ inline wb200_status check_storage(const wb200_tensor_desc &desc, uint64_t bytes,
 
 // The physical storage of `map` holds bytes that belong to no element (they keep the destination template's values).
 inline bool has_padding(const LayoutMap &map) { return map.physical_elements != map.element_count; }
+inline bool is_linear(const LayoutMap &map) { return map.layout == WB200_LAYOUT_TENSOR || map.layout == WB200_LAYOUT_NTENSOR; }
 
 inline bool same_shape(const wb200_tensor_desc &a, const wb200_tensor_desc &b) {
   if (a.rank != b.rank) return false;

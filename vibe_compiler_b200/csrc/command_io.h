@@ -17,7 +17,7 @@ class CommandIO {
  public:
   static constexpr size_t kMappedBytes = size_t(1) << 20;
   static constexpr size_t kPieceBytes = size_t(1) << 20;
-  static constexpr int64_t kScattered = 12 << 10;
+  static constexpr int64_t kScattered = 4 << 10;
 
   // `expected` bytes of host storage will pass through the call (sizes the pinned area, up to its limit).
   CommandIO(wb200_backend *backend, size_t expected) : backend_(backend), stream_(backend->stream) {
@@ -64,7 +64,7 @@ class CommandIO {
   // The result, after all operands. `padded`: its layout has bytes that are no element, which keep the template's values.
   // `host` is where deliver() puts it. `scattered`: elements the kernel stores one by one, at about 1.3 ns each over PCIe, so that
   // a larger result goes through device memory and one copy from there (bit-exact GEMM, 1001 x 1003 bf16: 1783 against 619 us
-  // in all, 256 x 520 f32 429 against 290; 65 x 130 f32 45 against 54).
+  // in all, 256 x 520 f32 429 against 290; a formal convert of 2 x 5 x 7 x 97 83 against 70; 64 x 64 f32 GEMM 38 against 44).
   wb200_status output(size_t slot, const uint8_t *storage_template, uint8_t *host, size_t bytes, bool padded, uint8_t **device, int64_t scattered = 0) {
     bytes_ = bytes;
     if (scattered > kScattered) {

@@ -100,7 +100,7 @@ def test_storage_in_place_and_in_pieces(backend, elements):
 MIB = 1 << 20
 
 
-# operands that fill the 32 MiB transfer area to its last byte, once and one and a half times over
+# operands of as many bytes as the 32 MiB transfer area holds, once and one and a half times over
 @pytest.mark.parametrize("each", [16 * MIB, 24 * MIB])
 def test_flags_are_read_back_behind_operands_that_fill_the_transfer_area(backend, each):
     key = PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [each // 4])
@@ -114,22 +114,18 @@ def test_flags_are_read_back_behind_operands_that_fill_the_transfer_area(backend
 
 
 def test_program_with_inputs_that_fill_the_transfer_area(backend):
-    rows = [f'!{{i64 {i}, !"external-{kind}", i64 0, !"", !"f32", !"tensor", i64 {count * 4}, i64 {count}, !"{access}-only", i64 {count // 64}, i64 64, i64 0}}'
-            for i, (kind, count, access) in enumerate((("input", 8 * MIB, "read"), ("output", 256, "write")))]
-    module = f"""define void @entry(i64 %0, i64 %1) {{
-  %src = add i64 %0, {32 * MIB - 1024}
-  call void @wafer_tx81_rdma(i64 %src, i64 0, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)
-  call void @wafer_tx81_wdma(i64 0, i64 %1, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)
-  ret void
-}}
-!wafer.target.tile_id = !{{!2}}
-!wafer.target.entry_arguments = !{{!10, !11}}
-!2 = !{{i64 0}}
-!10 = {rows[0]}
-!11 = {rows[1]}
-"""
-    x = np.arange(8 * MIB, dtype=np.float32).reshape(-1, 64)
-    (out,), _ = TileProgram([module], backend, spm_bytes=1 << 16).run([x])
+    count = 32   # of 1 MiB, the largest that go through the area
+    rows = [f'!{{i64 {i}, !"external-input", i64 {i}, !"", !"f32", !"tensor", i64 {MIB}, i64 {MIB // 4}, !"read-only", i64 {MIB // 256}, i64 64, i64 0}}'
+            for i in range(count)]
+    rows.append(f'!{{i64 {count}, !"external-output", i64 0, !"", !"f32", !"tensor", i64 1024, i64 256, !"write-only", i64 4, i64 64, i64 0}}')
+    lines = [f"define void @entry({', '.join(f'i64 %{i}' for i in range(count + 1))}) {{", f"  %src = add i64 %{count - 1}, {MIB - 1024}",
+             "  call void @wafer_tx81_rdma(i64 %src, i64 0, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)",
+             f"  call void @wafer_tx81_wdma(i64 0, i64 %{count}, i32 1024, i32 1024, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)",
+             "  ret void", "}", "!wafer.target.tile_id = !{!2}",
+             f"!wafer.target.entry_arguments = !{{{', '.join(f'!{10 + i}' for i in range(count + 1))}}}", "!2 = !{i64 0}"]
+    module = "\n".join(lines + [f"!{10 + i} = {row}" for i, row in enumerate(rows)]) + "\n"
+    x = np.arange(count * MIB // 4, dtype=np.float32).reshape(count, -1, 64)
+    (out,), _ = TileProgram([module], backend, spm_bytes=1 << 16).run(list(x))
     assert np.array_equal(out.view(np.float32).reshape(-1), x.reshape(-1)[-256:])
 
 

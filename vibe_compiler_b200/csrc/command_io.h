@@ -1,9 +1,11 @@
 // Host storage in and out of one command call. The reference hands commands over as pageable host vectors; a pageable
 // cudaMemcpyAsync costs 10-40 us each (driver staging and, for results, a synchronisation of its own), more than the
 // commands themselves. Storage goes through one pinned, device-mapped area of the backend instead:
-//   up to kMappedBytes per operand (or result) the kernel reads (writes) the area directly over PCIe - every command
-//   kernel but the formal GEMM touches a byte once - so there is no copy command at all;
-//   larger storage is copied through the area in pieces, so that the CPU copy of a piece overlaps the DMA of the one before.
+//   up to kMappedBytes per operand (or result) the kernel reads (writes) the area directly over PCIe, where it
+//   touches a byte once and in whole groups, so there is no copy command at all;
+//   storage in device memory (operands read several times, results stored element by element, anything larger) is copied
+//   through the area up to kPieceBytes, larger operands by the driver; larger results come back through the area in pieces, so
+//   that the CPU copy of a piece overlaps the DMA of the next.
 // Storage that is page-locked already (the results the Python layer hands out, see ResultPool; a caller's own pinned
 // memory) is read and written where it lies, so a chain of commands copies nothing between its calls.
 // One synchronisation ends the call. A result is copied to the caller only after the call's status words are known.
@@ -191,19 +193,22 @@ class CommandIO {
     device_ = result_ = *device;
     return padded ? upload(buffer, storage_template, bytes) : WB200_OK;
   }
+  // Through the area up to kPieceBytes; beyond, the driver's own copy of pageable memory is faster (reduce of 8 / 32 MB 422 / 1423
+  // us in all against 540 / 2060 in pieces of 1 MB; 64 KB 99 against 65). Either has read `host` when it returns.
   wb200_status upload(void *device, const uint8_t *host, size_t bytes) {
-    for (size_t at = 0; at < bytes; at += kPieceBytes) {
-      const size_t count = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
-      if (backend_->stage_low + count > backend_->stage_high) {
-        WB200_CUDA_CHECK(cudaStreamSynchronize(stream_));   // the pieces have left the area
-        backend_->stage_low = 0;
-        if (count > backend_->stage_high) return fail(WB200_ERR_LIMIT, "command staging area exhausted");
-      }
-      uint8_t *piece = backend_->stage + backend_->stage_low;
-      backend_->stage_low += count;
-      memcpy(piece, host + at, count);
-      WB200_CUDA_CHECK(cudaMemcpyAsync(static_cast<uint8_t *>(device) + at, piece, count, cudaMemcpyHostToDevice, stream_));
+    if (bytes > kPieceBytes) {
+      WB200_CUDA_CHECK(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, stream_));
+      return WB200_OK;
     }
+    if (backend_->stage_low + bytes > backend_->stage_high) {
+      WB200_CUDA_CHECK(cudaStreamSynchronize(stream_));   // the pieces have left the area
+      backend_->stage_low = 0;
+      if (bytes > backend_->stage_high) return fail(WB200_ERR_LIMIT, "command staging area exhausted");
+    }
+    uint8_t *piece = backend_->stage + backend_->stage_low;
+    backend_->stage_low += bytes;
+    memcpy(piece, host, bytes);
+    WB200_CUDA_CHECK(cudaMemcpyAsync(device, piece, bytes, cudaMemcpyHostToDevice, stream_));
     return WB200_OK;
   }
 

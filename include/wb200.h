@@ -158,8 +158,9 @@ wb200_status wb200_pack(wb200_backend *backend, const wb200_tensor_desc *desc,
 /* All storage pointers are HOST pointers to full physical storage, as the reference's
  * TargetModelNumericTensor::storage vectors are. `destination_out` receives the full physical
  * storage of the result, padding bytes copied from `destination_template`. Page-locked storage is read and written where
- * it lies, without a copy; when a call fails with WB200_ERR_NAN_DOMAIN the contents of a page-locked `destination_out` are
- * unspecified (pageable storage is left as it was). */
+ * it lies, without a copy; when an elementwise, convert or reduce call of the managed domain fails with
+ * WB200_ERR_NAN_DOMAIN, or any call with WB200_ERR_DEVICE_TIMEOUT or WB200_ERR_CUDA, the contents of a page-locked
+ * `destination_out` are unspecified. Calls refused before that write nothing, and pageable storage is left as it was. */
 
 typedef struct wb200_gemm_request { /* FormalGemmOperation + TargetModelNumericOperands */
   wb200_tensor_desc lhs, rhs, destination, psum;
@@ -648,7 +649,7 @@ wb200_status wb200_tile_program_trace(wb200_tile_program *program, wb200_program
 const char *wb200_program_command_name(uint32_t kind);
 /* Runs the invocation: host compact row-major inputs are packed into their physical DDR layout, all Tiles execute,
  * outputs are unpacked to `outputs`. `gemm_policy`: wb200_gemm_policy for psum-free, untransposed GEMM commands
- * (commands with a partial sum always take the bit-exact sequential-k path). */
+ * (commands with a partial sum always take the bit-exact sequential-k path). A run that fails writes no output. */
 wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *const *inputs, void *const *outputs,
                                     uint32_t gemm_policy, wb200_program_stats *stats);
 

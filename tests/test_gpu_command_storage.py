@@ -245,3 +245,50 @@ def test_page_locked_results_of_element_wise_stores_are_not_slower(backend, monk
                 command()
                 best[kind] = min(best.get(kind, 1e9), time.perf_counter() - begin)
     assert best["page-locked"] < 1.5 * best["pageable"], best
+
+
+@pytest.mark.parametrize("shape,layout", [([512, 5], "cx"), ([300, 97], "cx"), ([30000], "tensor")])
+def test_refused_formal_convert_leaves_page_locked_storage(backend, monkeypatch, shape, layout):
+    key, out_key = (PhysicalTensorDescriptor(f, LAYOUTS[layout], shape) for f in (abi.F32, abi.I32))
+    values = np.ones(key.element_count, np.float32)
+    values[7] = np.inf
+    storage = pinned(np.full(B200TargetModelBackend.physical_bytes(out_key), 0x77, np.uint8))
+    source, template = NumericTensor(key, physical(backend, key, values)), NumericTensor(out_key, np.zeros(storage.size, np.uint8))
+    opcode = 165   # F32 -> I32
+    into(monkeypatch, storage)
+    with pytest.raises(WB200Error, match="float-to-integer-non-finite"):
+        backend.execute_convert(opcode, source, template, formal=True)
+    assert (storage == 0x77).all()
+    values[7] = 3
+    got = backend.execute_convert(opcode, NumericTensor(key, physical(backend, key, values)), template, formal=True)
+    assert np.array_equal(logical(backend, out_key, got.destination.storage, np.int32), values.astype(np.int32))
+
+
+def test_refused_program_leaves_page_locked_outputs(backend, monkeypatch):
+    rows = [f'!{{i64 {i}, !"external-{kind}", i64 0, !"", !"{form}", !"tensor", i64 32768, i64 8192, !"{access}-only", i64 128, i64 64, i64 0}}'
+            for i, (kind, form, access) in enumerate((("input", "f32", "read"), ("output", "i32", "write")))]
+    module = f"""define void @entry(i64 %0, i64 %1) {{
+  call void @wafer_tx81_rdma(i64 %0, i64 0, i32 32768, i32 32768, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0)
+  call void @wafer_tx81_convert_fp32_int32(i64 0, i64 32768, i32 8192, i32 0, i32 0, i32 1)
+  call void @wafer_tx81_wdma(i64 32768, i64 %1, i32 32768, i32 32768, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 4, i32 0)
+  ret void
+}}
+!wafer.target.tile_id = !{{!2}}
+!wafer.target.entry_arguments = !{{!10, !11}}
+!2 = !{{i64 0}}
+!10 = {rows[0]}
+!11 = {rows[1]}
+"""
+    program = TileProgram([module], backend, spm_bytes=1 << 17)
+    values = np.arange(8192, dtype=np.float32).reshape(128, 64)
+    storage = pinned(np.full(32768, 0x77, np.uint8))
+    into(monkeypatch, storage)
+    for _ in range(2):   # the second run relaunches the graph
+        values[3, 1] = np.nan
+        storage[:] = 0x77
+        with pytest.raises(WB200Error, match="float-to-integer-non-finite"):
+            program.run([values])
+        assert (storage == 0x77).all()
+        values[3, 1] = 5.0
+        (out,), _ = program.run([values])
+        assert np.array_equal(out.view(np.int32), values.astype(np.int32))

@@ -103,20 +103,25 @@ class CommandIO {
     WB200_CUDA_CHECK(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, stream_));
     return WB200_OK;
   }
-  // Device memory of the caller's to host storage: enqueued here, complete after finish() and deliver_copies().
+  // Device memory of the caller's to host storage that is written by deliver_copies() alone, after the caller has accepted what
+  // finish() brought: storage that is not page-locked is fetched into the area ahead of it, the rest is copied then.
   wb200_status copy_out(uint8_t *host, const void *device, size_t bytes) {
-    uint8_t *area = host;
-    if (!page_locked(host, bytes)) {
-      if (!(area = take(bytes))) {   // larger than the area: piece by piece after the rest
-        late_.push_back({host, static_cast<const uint8_t *>(device), bytes});
-        return WB200_OK;
-      }
-      copies_.push_back({host, area, bytes});
+    const uint8_t *from = static_cast<const uint8_t *>(device);
+    if (page_locked(host, bytes)) {
+      direct_.push_back({host, from, bytes});
+      return WB200_OK;
     }
+    uint8_t *area = take(bytes);
+    if (!area) {   // larger than the area: piece by piece after the rest
+      late_.push_back({host, from, bytes});
+      return WB200_OK;
+    }
+    copies_.push_back({host, area, bytes});
     WB200_CUDA_CHECK(cudaMemcpyAsync(area, device, bytes, cudaMemcpyDeviceToHost, stream_));
     return WB200_OK;
   }
   wb200_status deliver_copies() {
+    for (const Copy &copy : direct_) WB200_CUDA_CHECK(cudaMemcpyAsync(copy.host, copy.from, copy.bytes, cudaMemcpyDeviceToHost, stream_));
     for (const Copy &copy : copies_) memcpy(copy.host, copy.from, copy.bytes);
     for (const Copy &copy : late_) {
       device_ = copy.from;
@@ -124,6 +129,7 @@ class CommandIO {
       wb200_status st = deliver(copy.host);
       if (st != WB200_OK) return st;
     }
+    if (!direct_.empty()) WB200_CUDA_CHECK(cudaStreamSynchronize(stream_));
     return WB200_OK;
   }
 
@@ -216,7 +222,7 @@ class CommandIO {
   cudaStream_t stream_;
   wb200_status status_;
   struct Copy { uint8_t *host; const uint8_t *from; size_t bytes; };
-  std::vector<Copy> copies_, late_;
+  std::vector<Copy> direct_, copies_, late_;
   uint8_t *mapped_ = nullptr;                              // the result in the area,
   const uint8_t *device_ = nullptr;                        // or in device memory, to be brought in pieces
   const uint8_t *result_ = nullptr;                        // where the kernels put a result of device_output(),

@@ -459,7 +459,7 @@ wb200_status wb200_convert_formal(wb200_backend *backend, const wb200_convert_re
   uint8_t *d_dst;
   if ((st = io.input(0, r->source_storage, r->source_bytes, &d_src, true)) != WB200_OK) return st;   // validated, then converted
   if ((st = io.output(2, r->destination_template, r->destination_out, r->destination_bytes, has_padding(dst_map), &d_dst,
-                      is_linear(dst_map) ? 0 : dst_map.element_count)) != WB200_OK) return st;   // stored element by element
+                      is_linear(dst_map) ? 0 : dst_map.element_count + CommandIO::kScattered)) != WB200_OK) return st;   // a refused command writes no template either
   uint32_t flags = 0;
   const uint64_t before = backend->launches;
   if ((st = backend->timing_begin(stream)) != WB200_OK) return st;

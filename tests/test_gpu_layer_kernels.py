@@ -42,3 +42,21 @@ def test_layer_with_the_add_inside_the_norm(backend, d_model):
     torch.cuda.synchronize()
     backend.poll()
     assert torch.equal(fused, separate)
+
+
+@pytest.mark.parametrize("seq", [32, 136])
+def test_parts_with_kept_sms_equal_one_pass(backend, seq):
+    """Parts of few tokens with SMs kept for the sums: the gate/up projection has more tiles than SMs to use and goes to CTA pairs of
+    which the rows fill a part, where one pass takes the tile kernel. The bits are the same."""
+    from vibe_compiler_b200.decoder_layer import LayerConfig, ShardedDecoderLayer, random_weights
+    cfg = LayerConfig(d_model=512, q_heads=4, kv_heads=2, ffn=14336)
+    layer = ShardedDecoderLayer(backend, cfg, random_weights(cfg))
+    x = torch.randn(2, seq, cfg.d_model, generator=torch.Generator().manual_seed(seq)).bfloat16().cuda()
+    kwargs = dict(norm1=layer.norm1, wqkv=layer.wqkv, wo=layer.wo, norm2=layer.norm2, wgu=layer.wgu, wdown=layer.wdown, q_heads=layer.hq,
+                  kv_heads=layer.hkv, head_dim=cfg.head_dim, eps=cfg.eps, rope_theta=cfg.rope_theta, allreduce=lambda tensor: None)
+    one, _ = backend.decoder_layer(x, **kwargs)
+    for reserved in (4, 16):
+        parts, _ = backend.decoder_layer(x, micro_batches=2, reserved_sms=reserved, **kwargs)
+        torch.cuda.synchronize()
+        backend.poll()
+        assert torch.equal(one, parts)

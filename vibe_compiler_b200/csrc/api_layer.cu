@@ -92,6 +92,8 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
   backend->layer_timeline_parts = 0;
   if (parts > 1) WB200_CUDA_CHECK(cudaEventRecord(backend->pipeline_event[4 * parts], user_stream));   // timeline origin
   cudaStream_t comm_stream = parts > 1 ? backend->aux_stream[0] : user_stream;
+  // a sum's kernel on the communication stream runs beside the kernels of the parts (see launch_gemm_umma)
+  const bool beside = parts > 1;
   int compute_sms = backend->sm_count;
   if (parts > 1 && p->reserved_sms > 0 && static_cast<int>(p->reserved_sms) < backend->sm_count / 2)
     compute_sms = backend->sm_count - static_cast<int>(p->reserved_sms);
@@ -135,7 +137,7 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
     g.in_format = fmt; g.out_format = fmt;
     g.epilogue = epilogue;
     g.a = a; g.b = b; g.out = out;
-    wb200_status s = launch_gemm_umma(g, compute_sms, backend->d_status, stream);
+    wb200_status s = launch_gemm_umma(g, compute_sms, backend->d_status, stream, beside);
     if (s == WB200_OK) backend->launches += 1;
     return s;
   };
@@ -181,11 +183,11 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
   // RMSNorm -> QKV -> rotary split -> attention -> output projection -> [sum over shards]
   auto attention_phase = [&](const Part &part) -> wb200_status {
     wb200_status s;
-    if ((s = launch_rmsnorm(fmt, part.x, p->norm1, part.h, tokens, d, p->eps, part.stream)) != WB200_OK) return s;
+    if ((s = launch_rmsnorm(fmt, part.x, p->norm1, part.h, tokens, d, p->eps, part.stream, nullptr, nullptr, beside)) != WB200_OK) return s;
     backend->launches += 1;
     if ((s = gemm(part.stream, part.h, p->wqkv, part.qkv, tokens, static_cast<int>(plan.qkv_cols), d, WB200_EPI_NONE)) != WB200_OK) return s;
     if ((s = launch_rope_split(fmt, part.qkv, part.q, part.k, part.v, part_batch, p->seq, p->q_heads, p->kv_heads, p->head_dim, p->rope_theta,
-                               static_cast<int>(p->position_offset), part.stream)) != WB200_OK) return s;
+                               static_cast<int>(p->position_offset), part.stream, beside)) != WB200_OK) return s;
     backend->launches += 1;
     AttentionArgs a{};
     a.batch = part_batch; a.q_heads = p->q_heads; a.kv_heads = p->kv_heads; a.q_len = p->seq; a.kv_len = p->seq; a.head_dim = p->head_dim;
@@ -194,7 +196,7 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
     a.causal_offset = 0; a.kv_valid = p->seq;
     a.q = part.q; a.k = part.k; a.v = part.v; a.out = part.attn;
     a.out_token_major = 1;
-    s = attention_fa_umma_supports(a) ? launch_attention_fa_umma(a, compute_sms, backend->d_status, part.stream)
+    s = attention_fa_umma_supports(a) ? launch_attention_fa_umma(a, compute_sms, backend->d_status, part.stream, beside)
                                       : launch_attention_fa_simt(a, part.stream);
     if (s != WB200_OK) return s;
     backend->launches += 1;
@@ -206,9 +208,9 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
     wb200_status s;
     if ((s = await_sum(part, 0)) != WB200_OK) return s;
     if (fused_residual) {
-      s = launch_rmsnorm(fmt, part.x1, p->norm2, part.h, tokens, d, p->eps, part.stream);
+      s = launch_rmsnorm(fmt, part.x1, p->norm2, part.h, tokens, d, p->eps, part.stream, nullptr, nullptr, beside);
     } else {   // x1 = x + attention on the way into the norm
-      s = launch_rmsnorm(fmt, part.x, p->norm2, part.h, tokens, d, p->eps, part.stream, part.partial, part.x1);
+      s = launch_rmsnorm(fmt, part.x, p->norm2, part.h, tokens, d, p->eps, part.stream, part.partial, part.x1, beside);
     }
     if (s != WB200_OK) return s;
     backend->launches += 1;
@@ -223,7 +225,7 @@ wb200_status wb200_decoder_layer(wb200_backend *backend, const wb200_decoder_lay
       WB200_CUDA_CHECK(cudaMemcpyAsync(part.out, part.partial, static_cast<size_t>(tokens) * d * e, cudaMemcpyDeviceToDevice, part.stream));
       return WB200_OK;
     }
-    if ((s = launch_residual_add(fmt, part.x1, part.partial, part.out, static_cast<size_t>(tokens) * d, part.stream)) != WB200_OK) return s;
+    if ((s = launch_residual_add(fmt, part.x1, part.partial, part.out, static_cast<size_t>(tokens) * d, part.stream, beside)) != WB200_OK) return s;
     backend->launches += 1;
     return WB200_OK;
   };

@@ -695,7 +695,7 @@ bool attention_fa_umma_supports(const AttentionArgs &a) {
 }
 
 wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int *device_status,
-                                      cudaStream_t stream) {
+                                      cudaStream_t stream, bool beside) {
   if (sm_count <= 0) sm_count = 148;
   if (!attention_fa_umma_supports(a))
     return fail(WB200_ERR_UNSUPPORTED, "attention request outside the tcgen05 prefill kernel's domain");
@@ -762,7 +762,7 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int 
   config.stream = stream;
   cudaLaunchAttribute attrs[2];
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[0].val.programmaticStreamSerializationAllowed = beside ? 0 : 1;
   attrs[1].id = cudaLaunchAttributeClusterDimension;
   attrs[1].val.clusterDim.x = 2; attrs[1].val.clusterDim.y = 1; attrs[1].val.clusterDim.z = 1;
   config.attrs = attrs;

@@ -7,16 +7,12 @@
 // columns per CTA for small and narrow ones. In both, warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner, warps
 // 2-5 = epilogue (one TMEM lane quarter each). Roofline: tensor pipe, or the bytes of B when the rows are few; algorithmic
 // work is 2*M*N*K flop per launch.
-#include <algorithm>
-#include <cmath>
-
-#include "kernels.h"
+#include "gemm_plan.h"
 #include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
 
-constexpr int kBM = 128, kBN = 256, kBK = 64;
 constexpr int kABytes = kBM * kBK * 2;        // 16 KiB
 constexpr int kTmemCols = 512;
 constexpr int kThreads = 192;
@@ -31,16 +27,6 @@ struct GemmUmmaParams {
   int *status;
   int num_n_tiles;
   int group_m;   // tile rows walked together (see tile_coords)
-};
-
-// How a problem is cut for the one-tile-per-CTA kernel (see choose_tile).
-constexpr int kMaxTileStages = 10;
-struct TilePlan {
-  int tile_cols;    // output columns per tile: 64 or 128
-  int tile_rows;    // output rows per tile: a multiple of 16 up to 256
-  int stages;       // TMA ring; a stage holds two 64-element blocks of K
-  int row_bytes;    // bytes of A per block of K
-  int tmem_cols;
 };
 
 __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int group_m, int &m_blk, int &n_blk) {
@@ -539,60 +525,6 @@ const GemmKernel pair_kernels[8] = {
     gemm_umma_pair_kernel<false, false, false>, gemm_umma_pair_kernel<false, false, true>, gemm_umma_pair_kernel<false, true, false>,
     gemm_umma_pair_kernel<false, true, true>,   gemm_umma_pair_kernel<true, false, false>, gemm_umma_pair_kernel<true, false, true>,
     gemm_umma_pair_kernel<true, true, false>,   gemm_umma_pair_kernel<true, true, true>};
-
-constexpr int kTileSmemShared = 108 * 1024;   // ring of a CTA that shares its SM with another one
-constexpr int kTileSmemAlone = 208 * 1024;
-
-int ceil_div(int a, int b) { return (a + b - 1) / b; }
-
-// Fills in what follows from the tile's size.
-TilePlan make_tile(int tile_cols, int tile_rows, const GemmUmmaArgs &a, int sm_count) {
-  TilePlan plan;
-  plan.tile_cols = tile_cols;
-  plan.tile_rows = tile_rows;
-  plan.row_bytes = a.lhs_transposed ? ceil_div(tile_rows, 64) * 8192 : tile_rows * 128;
-  const int stage = 2 * (tile_cols * kBK * 2 + plan.row_bytes);
-  const bool alone = static_cast<int64_t>(ceil_div(a.n, tile_cols)) * ceil_div(a.m, tile_rows) <= sm_count || tile_rows > 64;
-  // the ring is also the accumulator's staging area; more stages than blocks of K would stay empty
-  const int need = std::max({ceil_div(a.k, 2 * kBK), ceil_div(tile_rows * tile_cols * 4, stage), 2});
-  plan.stages = std::min({(alone ? kTileSmemAlone : kTileSmemShared) / stage, kMaxTileStages, need});
-  plan.tmem_cols = 32;
-  while (plan.tmem_cols < tile_rows) plan.tmem_cols *= 2;
-  return plan;
-}
-
-// Estimated clocks of a launch of either kernel; the cheaper one runs. Measured at 1.9 GHz with cold caches (both sides in
-// us, launch included): a block of 64 of K costs a CTA four instructions of about 75 clocks however few rows or columns
-// they cover, or its products, or its operand bytes at about 52 per clock, whichever is more; a pair of CTAs needs about
-// 650 clocks for the same block of a 256 x 256 tile. Rows x columns x K: 16 x 6144 x 4096 pair 31 / tile 19, 128 x 4096 x
-// 4096 30 / 20, 512 x 4096 x 4096 32 / 28, 1024 x 1024 x 8192 49 / 34, 8192 x 256 x 2048 24 / 22; the pairs win once their
-// tiles fill the SMs: 1000 x 6144 x 4096 54 / 68, 512 x 28672 x 4096 101 / 165.
-double tile_cost(const TilePlan &plan, const GemmUmmaArgs &a, int sm_count) {
-  const double per_sm = std::ceil(static_cast<double>(ceil_div(a.n, plan.tile_cols)) * ceil_div(a.m, plan.tile_rows) / sm_count);
-  const double block = std::max({300.0, 2.0 * plan.tile_rows, (plan.tile_cols * kBK * 2 + plan.row_bytes) / 52.0});
-  return per_sm * ceil_div(a.k, kBK) * block + 5000.0 + 20.0 * plan.tile_rows;
-}
-double pair_cost(const GemmUmmaArgs &a, int sm_count) {
-  const double waves = std::ceil(static_cast<double>(ceil_div(a.m, 2 * kBM)) * ceil_div(a.n, kBN) / (sm_count / 2));
-  return waves * ceil_div(a.k, kBK) * 650.0 + 10000.0;
-}
-
-TilePlan choose_tile(const GemmUmmaArgs &a, int sm_count, double *cost) {
-  TilePlan best{};
-  *cost = 0;
-  int last_rows = 0;
-  for (const int limit : {256, 192, 128, 96, 64}) {
-    const int tile_rows = ceil_div(ceil_div(a.m, ceil_div(a.m, limit)), 16) * 16;
-    if (tile_rows == last_rows) continue;
-    last_rows = tile_rows;
-    for (const int tile_cols : {128, 64}) {
-      const TilePlan plan = make_tile(tile_cols, tile_rows, a, sm_count);
-      const double c = tile_cost(plan, a, sm_count);
-      if (best.tile_rows == 0 || c < *cost) { best = plan; *cost = c; }
-    }
-  }
-  return best;
-}
 }  // namespace
 
 wb200_status gemm_umma_prepare() {
@@ -608,11 +540,11 @@ wb200_status gemm_umma_prepare() {
 }
 
 wb200_status launch_gemm_umma(const GemmUmmaArgs &a, int sm_count, int *device_status,
-                              cudaStream_t stream) {
+                              cudaStream_t stream, bool beside) {
   if (!gemm_umma_supports(a)) return fail(WB200_ERR_UNSUPPORTED, "GEMM outside the tcgen05 kernel's domain");
-  double tile_clocks;
-  const TilePlan tile = choose_tile(a, sm_count, &tile_clocks);
-  const bool use_pairs = pair_cost(a, sm_count) < tile_clocks;
+  const GemmPlan plan = plan_gemm(a, sm_count, beside);
+  const TilePlan &tile = plan.tile;
+  const bool use_pairs = plan.pairs;
   CUtensorMap tmap_a, tmap_b;
   wb200_status st;
   if (!a.lhs_transposed)  // A[m,k], k contiguous: K-major
@@ -641,13 +573,11 @@ wb200_status launch_gemm_umma(const GemmUmmaArgs &a, int sm_count, int *device_s
   if (st_attributes != WB200_OK) return st_attributes;
   const int variant = (a.lhs_transposed ? 4 : 0) | (a.rhs_transposed ? 0 : 2) | (a.in_format == WB200_BF16 ? 1 : 0);
   if (use_pairs) {
-    const int clusters = std::min(sm_count / 2, ceil_div(a.m, 2 * kBM) * p.num_n_tiles);
-    WB200_CUDA_CHECK(launch_dependent(pair_kernels[variant], 2 * clusters, kThreads, kPairSmemBytes, stream, tmap_a, tmap_b, p));
+    WB200_CUDA_CHECK(launch_ordered(pair_kernels[variant], plan.grid, kThreads, kPairSmemBytes, stream, !beside, tmap_a, tmap_b, p));
     return WB200_OK;
   }
-  const int grid = ceil_div(a.n, tile.tile_cols) * ceil_div(a.m, tile.tile_rows);
   const size_t smem = 2 * static_cast<size_t>(tile.stages) * (tile.tile_cols * kBK * 2 + tile.row_bytes) + 1024;
-  WB200_CUDA_CHECK(launch_dependent(tile_kernels[tile.tile_cols == 128][variant], grid, kThreads, smem, stream, tmap_a, tmap_b, p, tile));
+  WB200_CUDA_CHECK(launch_ordered(tile_kernels[tile.tile_cols == 128][variant], plan.grid, kThreads, smem, stream, !beside, tmap_a, tmap_b, p, tile));
   return WB200_OK;
 }
 

@@ -44,8 +44,9 @@ class PerDeviceOnce {
 // Launches a kernel as a programmatic dependent of the one before it on the stream (an edge of that kind in a captured
 // graph): its blocks may be set up while that kernel drains. The kernel must call pdl_wait() before its first access to
 // memory another kernel may write (ptx_sm100.cuh).
+// With `dependent` = false it starts after that kernel, as any other.
 template <typename... Params, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+cudaError_t launch_ordered(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool dependent, Args &&...args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = grid;
   config.blockDim = block;
@@ -55,8 +56,12 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
-  config.numAttrs = 1;
+  config.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+  return launch_ordered(kernel, grid, block, smem, stream, true, static_cast<Args &&>(args)...);
 }
 
 // ---- TMA descriptor encoding (driver entry point fetched at run time; libcuda is not linked)
@@ -87,8 +92,11 @@ bool gemm_umma_supports(const GemmUmmaArgs &args);
 // Sets the kernels' per-device launch attributes (also done lazily by the first launch): call before a stream capture that
 // will contain tensor-core GEMM launches.
 wb200_status gemm_umma_prepare();
+// `beside` (here and below): a kernel of another stream runs beside this one, on the SMs that sm_count leaves out. No more CTAs
+// than sm_count are launched then, and not as programmatic dependents: those would sit on the free SMs while they wait for the
+// kernel before them.
 wb200_status launch_gemm_umma(const GemmUmmaArgs &args, int sm_count, int *device_status,
-                              cudaStream_t stream);
+                              cudaStream_t stream, bool beside = false);
 
 // ---- bit-exact sequential-k GEMM on physical or compact storage (gemm_formal.cu)
 struct GemmFormalArgs {
@@ -215,7 +223,7 @@ struct AttentionArgs {
 };
 bool attention_fa_umma_supports(const AttentionArgs &args);
 wb200_status launch_attention_fa_umma(const AttentionArgs &args, int sm_count, int *device_status,
-                                      cudaStream_t stream);
+                                      cudaStream_t stream, bool beside = false);
 wb200_status launch_attention_fa_simt(const AttentionArgs &args, cudaStream_t stream);
 
 // Flash-decoding. `partials` is scratch of fd_partial_floats(args, plan.records) floats.
@@ -257,10 +265,10 @@ wb200_status launch_switch_sum(void *multicast, uint64_t elements, int format, i
 // ---- decoder-layer pieces (layer_ops.cu); device pointers, bf16 / f16 storage
 // With `addend` and `sum`: the norm of round(x + addend), which is stored to `sum`.
 wb200_status launch_rmsnorm(int format, const void *x, const void *gamma, void *y, int rows, int dim, float eps,
-                            cudaStream_t stream, const void *addend = nullptr, void *sum = nullptr);
+                            cudaStream_t stream, const void *addend = nullptr, void *sum = nullptr, bool beside = false);
 wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, void *v, int batch, int seq, int q_heads,
-                               int kv_heads, int head_dim, float theta, int position_offset, cudaStream_t stream);
-wb200_status launch_residual_add(int format, const void *a, const void *b, void *out, size_t elements, cudaStream_t stream);
+                               int kv_heads, int head_dim, float theta, int position_offset, cudaStream_t stream, bool beside = false);
+wb200_status launch_residual_add(int format, const void *a, const void *b, void *out, size_t elements, cudaStream_t stream, bool beside = false);
 
 // ---- movement commands on device-resident memory images (tile_movement.cu)
 struct StridedLayout {

@@ -197,20 +197,20 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 }  // namespace
 
 wb200_status launch_rmsnorm(int format, const void *x, const void *gamma, void *y, int rows, int dim, float eps,
-                            cudaStream_t stream, const void *addend, void *sum) {
+                            cudaStream_t stream, const void *addend, void *sum, bool beside) {
   if (format != WB200_BF16 && format != WB200_F16) return fail(WB200_ERR_UNSUPPORTED, "rmsnorm takes bf16 or f16 storage");
   if (rows <= 0 || dim <= 0 || dim % 8 != 0 || !aligned16(x) || !aligned16(gamma) || !aligned16(y) || !aligned16(addend) || !aligned16(sum))
     return fail(WB200_ERR_INVALID_ARGUMENT, "rmsnorm needs dim % 8 == 0 and 16-byte aligned buffers");
   const bool bf16 = format == WB200_BF16;
   const auto kernel = addend ? (bf16 ? rmsnorm_kernel<true, true> : rmsnorm_kernel<false, true>)
                              : (bf16 ? rmsnorm_kernel<true, false> : rmsnorm_kernel<false, false>);
-  WB200_CUDA_CHECK(launch_dependent(kernel, rows, kNormThreads, 0, stream, static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(addend),
+  WB200_CUDA_CHECK(launch_ordered(kernel, rows, kNormThreads, 0, stream, !beside, static_cast<const uint16_t *>(x), static_cast<const uint16_t *>(addend),
                                     static_cast<uint16_t *>(sum), static_cast<const uint16_t *>(gamma), static_cast<uint16_t *>(y), dim, eps));
   return WB200_OK;
 }
 
 wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, void *v, int batch, int seq, int q_heads,
-                               int kv_heads, int head_dim, float theta, int position_offset, cudaStream_t stream) {
+                               int kv_heads, int head_dim, float theta, int position_offset, cudaStream_t stream, bool beside) {
   if (format != WB200_BF16 && format != WB200_F16) return fail(WB200_ERR_UNSUPPORTED, "rope takes bf16 or f16 storage");
   if (batch <= 0 || seq <= 0 || q_heads <= 0 || kv_heads <= 0 || head_dim <= 0 || head_dim % 4 != 0 || !(theta > 0.f))
     return fail(WB200_ERR_INVALID_ARGUMENT, "invalid rope extents (head_dim % 4 == 0, theta > 0)");
@@ -220,21 +220,21 @@ wb200_status launch_rope_split(int format, const void *qkv, void *q, void *k, vo
   const bool bf16 = format == WB200_BF16;
   const auto kernel = wide ? (bf16 ? rope_split_kernel<true, 8> : rope_split_kernel<false, 8>)
                            : (bf16 ? rope_split_kernel<true, 2> : rope_split_kernel<false, 2>);
-  WB200_CUDA_CHECK(launch_dependent(kernel, tokens, kRopeThreads, 0, stream, static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q),
+  WB200_CUDA_CHECK(launch_ordered(kernel, tokens, kRopeThreads, 0, stream, !beside, static_cast<const uint16_t *>(qkv), static_cast<uint16_t *>(q),
                                     static_cast<uint16_t *>(k), static_cast<uint16_t *>(v), seq, q_heads, kv_heads, head_dim, log2_theta,
                                     position_offset));
   return WB200_OK;
 }
 
-wb200_status launch_residual_add(int format, const void *a, const void *b, void *out, size_t elements, cudaStream_t stream) {
+wb200_status launch_residual_add(int format, const void *a, const void *b, void *out, size_t elements, cudaStream_t stream, bool beside) {
   if (format != WB200_BF16 && format != WB200_F16) return fail(WB200_ERR_UNSUPPORTED, "residual add takes bf16 or f16 storage");
   if (elements == 0 || elements % 8 != 0 || !aligned16(a) || !aligned16(b) || !aligned16(out))
     return fail(WB200_ERR_INVALID_ARGUMENT, "residual add needs a multiple of 8 elements and 16-byte aligned buffers");
   const size_t chunks = elements / 8;
   size_t blocks = (chunks + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
-  WB200_CUDA_CHECK(launch_dependent(format == WB200_BF16 ? residual_add_kernel<true> : residual_add_kernel<false>, static_cast<unsigned>(blocks), 256, 0,
-                                    stream, static_cast<const uint4 *>(a), static_cast<const uint4 *>(b), static_cast<uint4 *>(out), chunks));
+  WB200_CUDA_CHECK(launch_ordered(format == WB200_BF16 ? residual_add_kernel<true> : residual_add_kernel<false>, static_cast<unsigned>(blocks), 256, 0,
+                                    stream, !beside, static_cast<const uint4 *>(a), static_cast<const uint4 *>(b), static_cast<uint4 *>(out), chunks));
   return WB200_OK;
 }
 

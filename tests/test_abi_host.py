@@ -95,3 +95,12 @@ def test_microbenchmarks_import_and_parse_their_arguments():
     replay = importlib.import_module("vibe_compiler_b200.microbench.replay")
     with pytest.raises(SystemExit):
         replay.main([])            # --fixture is required: no default into the test tree
+
+
+def test_a_descriptor_hands_out_c_forms_of_its_own():
+    from vibe_compiler_b200.backend import PhysicalTensorDescriptor
+    first, second = (PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, [4, 6]) for _ in range(2))
+    changed = first.c()
+    changed.shape[0] = 99
+    assert list(first.c().shape[:2]) == [4, 6] and list(second.c().shape[:2]) == [4, 6]
+    assert list(PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, np.array([4.0, 6.0])).c().shape[:2]) == [4, 6]

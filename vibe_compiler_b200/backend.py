@@ -59,8 +59,8 @@ class PhysicalTensorDescriptor:
     shape: Sequence[int]
 
     def c(self) -> abi.TensorDesc:
-        """The C form (shared between equal descriptors: copy it before changing it)."""
-        return _c_descriptor(self.format, self.layout, tuple(self.shape))
+        """The C form, the caller's own."""
+        return abi.TensorDesc.from_buffer_copy(_c_descriptor(self.format, self.layout, tuple(map(int, self.shape))))
 
     @property
     def element_count(self) -> int:

@@ -104,3 +104,13 @@ def test_a_descriptor_hands_out_c_forms_of_its_own():
     changed.shape[0] = 99
     assert list(first.c().shape[:2]) == [4, 6] and list(second.c().shape[:2]) == [4, 6]
     assert list(PhysicalTensorDescriptor(abi.F32, abi.LAYOUT_TENSOR, np.array([4.0, 6.0])).c().shape[:2]) == [4, 6]
+
+
+@pytest.mark.parametrize("scale", [0.125, 1, np.float64(0.1), 1e39, -1e39, float("nan")])
+def test_attention_requests_round_the_scale_to_f32(scale):
+    import torch
+    from vibe_compiler_b200.backend import B200TargetModelBackend
+    q = torch.zeros(1, 2, 1, 128)
+    p = B200TargetModelBackend._attention_params(None, q, q, q, q, scale, False, False, 0, 0, 0, None, None, None, 0)
+    with np.errstate(over="ignore"):
+        assert np.array_equal(np.float32(p.scale), np.float32(scale), equal_nan=True)

@@ -347,7 +347,7 @@ class B200TargetModelBackend:
         _, kv_heads, kv_len, _ = k.shape
         return abi.AttentionParams.from_buffer_copy(_ATTENTION_PACK(
             batch, q_heads, kv_heads, q_len, kv_len, head_dim, _TORCH_FORMATS[dtype], bool(causal), bool(zero_fully_masked),
-            abi.MEM_DEVICE if on_device else abi.MEM_HOST, scale, int(query_start), int(key_start), int(key_end),
+            abi.MEM_DEVICE if on_device else abi.MEM_HOST, C.c_float(scale).value, int(query_start), int(key_start), int(key_end),
             q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr() if lse is not None else 0,
             row_max.data_ptr() if row_max is not None else 0, row_sum.data_ptr() if row_sum is not None else 0, stream or 0,
             abi.OUT_TOKEN_MAJOR if token_major_out else abi.OUT_HEAD_MAJOR, 0))

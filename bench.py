@@ -38,7 +38,7 @@ SEED = 20260803
 TRAFFIC = {
     "fa": 2 * (214.2e6 + 46.1e6),      # profiles/fa_umma_kernel_cfg2.md: batch 2 of 4 captured
     "fd": 8 * (1.073832e9 + 6.2e6),    # profiles/fd_partial_kernel_cfg3.md: batch 8 of 64 captured
-    "layer": 8.259e9 + 1.472e9,        # profiles/decoder_layer_tp1_dram.md: the ten kernels of one full-size forward on one GPU
+    "layer": 8.125e9 + 1.472e9,        # profiles/decoder_layer_tp1_dram.md: one full-size forward on one GPU, less the read that the fused add saves
     "gemm": 1.118e9 + 0.124e9,         # profiles/gemm_umma_pair_kernel_cfg4.md: the full 8192^3 launch, one-pass capture
 }
 
@@ -535,9 +535,9 @@ def main():
         lv = torch.randn(1, FD_LONG["kv_heads"], hi - lo, FD_LONG["head_dim"], device=device, generator=gen).bfloat16()
         lout = torch.empty_like(lq)
         group = None
-        # One step = stage 1 over this rank's KV shard + one kernel that folds the splits, exchanges the per-head states
-        # with plain peer stores over NVLink and merges them in ascending shard order. No collective library call, so
-        # the two launches replay as one CUDA graph at every world size.
+        # One step = one launch: stage 1 over this rank's KV shard, whose last clusters fold the records, exchange the per-head
+        # states with plain peer stores over NVLink and merge them in ascending shard order. No collective library call, so it
+        # replays as a CUDA graph at every world size.
         from vibe_compiler_b200.sharding import PeerExchange
         exchange = PeerExchange(backend, 1, FD_LONG["q_heads"], group, device)
         long_lse = torch.empty(1, FD_LONG["q_heads"], 1, device=device)

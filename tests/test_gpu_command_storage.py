@@ -295,3 +295,17 @@ def test_refused_program_leaves_page_locked_outputs(backend, monkeypatch):
         values[3, 1] = 5.0
         (out,), _ = program.run([values])
         assert np.array_equal(out.view(np.int32), values.astype(np.int32))
+
+
+def test_padded_result_over_a_page_locked_operand_that_is_not_aligned(backend, monkeypatch):
+    """Such an operand is copied, asynchronously beyond 1 MiB, and its storage counts as an operand's all the same."""
+    key, out_key = (PhysicalTensorDescriptor(f, abi.LAYOUT_CX, [1500, 1030]) for f in (abi.F32, abi.BF16))
+    size, out_size = (B200TargetModelBackend.physical_bytes(k) for k in (key, out_key))
+    source = physical(backend, key, np.random.default_rng(4).standard_normal(key.element_count).astype(np.float32).view(np.uint32))
+    blank = NumericTensor(out_key, np.full(out_size, 0x11, np.uint8))
+    want = backend.execute_convert(167, NumericTensor(key, source), blank).destination.storage.copy()
+    room = pinned(np.zeros(size + 4096, np.uint8))
+    room[8:8 + size] = source
+    into(monkeypatch, room)   # the result begins 8 bytes before the operand
+    got = backend.execute_convert(167, NumericTensor(key, room[8:8 + size]), blank)
+    assert np.array_equal(got.destination.storage, want)

@@ -36,10 +36,8 @@ class CommandIO {
   // An operand. `reread`: the kernels read it more than once, so it belongs in device memory (slot `slot`).
   wb200_status input(size_t slot, const uint8_t *host, size_t bytes, const uint8_t **device, bool reread = false) {
     const bool pinned = page_locked(host, bytes);
-    if (pinned) {   // read by the kernels or by a copy in flight, in either case after output() has run
-      held_[held_count_] = host;
-      held_bytes_[held_count_++] = bytes;
-    }
+    held_[held_count_] = host;   // it may be read by the kernels or by a copy in flight after output() has run
+    held_bytes_[held_count_++] = bytes;
     if (pinned && !reread) {
       *device = host;
       return WB200_OK;
@@ -200,7 +198,8 @@ class CommandIO {
     return padded ? upload(buffer, storage_template, bytes) : WB200_OK;
   }
   // Through the area up to kPieceBytes; beyond, the driver's own copy of pageable memory is faster (reduce of 8 / 32 MB 422 / 1423
-  // us in all against 540 / 2060 in pieces of 1 MB; 64 KB 99 against 65). Either has read `host` when it returns.
+  // us in all against 540 / 2060 in pieces of 1 MB; 64 KB 99 against 65). Either has read pageable
+  // `host` when it returns.
   wb200_status upload(void *device, const uint8_t *host, size_t bytes) {
     if (bytes > kPieceBytes) {
       WB200_CUDA_CHECK(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, stream_));
@@ -228,7 +227,7 @@ class CommandIO {
   const uint8_t *result_ = nullptr;                        // where the kernels put a result of device_output(),
   uint8_t *copied_result_ = nullptr;                       // and where finish() copies it
   bool in_place_result_ = false, finished_ = false;
-  const uint8_t *held_[4];      // page-locked operands: a result that overlaps one is written only after they have been read
+  const uint8_t *held_[4];      // the operands: a page-locked result that overlaps one is written only after they have been read
   size_t held_bytes_[4];
   int held_count_ = 0;
   size_t bytes_ = 0;

@@ -616,7 +616,7 @@ typedef struct wb200_program_stats {
   uint64_t gemm_commands, movement_commands, fill_commands, transfer_commands, sync_commands;
   uint64_t gemm_fused_multiply_adds;  /* sum of m * k * n * batch */
   uint64_t bytes_moved;               /* payload bytes of DMA, gather / scatter, fill and Direct-DTE transfers */
-  uint64_t gpu_launches;
+  uint64_t gpu_launches;              /* a launch that serves a command of several Tiles counts once per Tile */
   float device_ms;                    /* command stream only (CUDA events); excludes host <-> device tensor copies */
   uint32_t numeric_flags;             /* OR of the IEEE flags of all elementwise / convert / reduce / pool commands (bit 0 invalid .. bit 4 inexact) */
 } wb200_program_stats;

@@ -1,0 +1,60 @@
+"""Tiles that run one program on different data are replayed in step, one launch per command for all of them: the bits, flags
+and counts must be those of the same modules run one Tile at a time (whose replay is compared with the CPU's elsewhere)."""
+import numpy as np
+import pytest
+
+from vibe_compiler_b200.tile_program import TileProgram
+
+pytestmark = pytest.mark.gpu
+
+
+def _module(tile, tiles, count, scale, gap):
+    """`count` f32 values of the Tile (4 * gap bytes between the Tiles' blocks): a constant vector, a product, exp, a repeated
+    unit, a reduction over [1, 1, count / 64, 64], a 64 x 64 x 64 product when there are enough values, a transposing copy."""
+    step, flat = 4 * (count + gap), "i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0"
+    size = (4 * count + 255) // 256 * 256
+    a, b, c, d, moved, product, folded = (i * size for i in range(7))
+    vector, same, unit = f"i32 {count}, i32 5", "i32 0, i32 0, i32 0, i32 1", "i32 64, i32 0, i32 0, i32 1"
+    call = "  call void @wafer_tx81_"
+    body = [f"  %in = add i64 %0, {tile * step}", f"  %out = add i64 %1, {tile * step}", f"  %sums = add i64 %2, {tile * 256}",
+            f"{call}rdma(i64 %in, i64 {a}, i32 {4 * count}, i32 {4 * count}, {flat})",
+            f"{call}memset(i64 {b}, i32 {scale}, {vector}, i32 0)",
+            f"{call}elementwise_mul(i64 {a}, i64 {b}, i64 {c}, {vector}, {same})", f"{call}elementwise_exp(i64 {c}, i64 {c}, {vector}, i32 1)",
+            f"{call}elementwise_sub(i64 {c}, i64 {a}, i64 {d}, {vector}, {unit})",
+            f"{call}gather_scatter(i64 {d}, i64 {moved}, i32 {4 * count}, i32 4, i32 256, i32 4, i32 0, i32 {count // 64}, i32 64, i32 1, "
+            f"i32 4, i32 {count // 64 * 4}, i32 0, i32 {count // 64}, i32 64, i32 1, i32 0)",
+            f"{call}ncc_join(i32 1)"]
+    if count >= 4096:
+        body += [f"{call}gemm_oriented(i64 {moved}, i64 {a}, i64 {product}, i64 {d}, i32 64, i32 64, i32 64, i32 1, i32 5, i32 5, i32 5, i32 1, i32 0, i32 0)",
+                 f"{call}elementwise_max(i64 {product}, i64 {d}, i64 {moved}, i32 4096, i32 5, {same})"]
+    body += [f"{call}reduce_sum(i64 {moved}, i64 {folded}, i32 1, i32 1, i32 1, i32 {count // 64}, i32 64, i32 5, i32 1)",
+             f"{call}wdma(i64 {moved}, i64 %out, i32 {4 * count}, i32 {4 * count}, {flat})", f"{call}wdma(i64 {folded}, i64 %sums, i32 256, i32 256, {flat})"]
+    total = tiles * (count + gap)
+    rows = [f'!{{i64 0, !"external-input", i64 0, !"", !"f32", !"tensor", i64 {4 * total}, i64 {total}, !"read-only", i64 {total}, i64 0}}',
+            f'!{{i64 1, !"external-output", i64 0, !"", !"f32", !"tensor", i64 {4 * total}, i64 {total}, !"write-only", i64 {total}, i64 0}}',
+            f'!{{i64 2, !"external-output", i64 1, !"", !"f32", !"tensor", i64 {256 * tiles}, i64 {64 * tiles}, !"write-only", i64 {64 * tiles}, i64 0}}']
+    meta = "\n".join(f"!{10 + i} = {row}" for i, row in enumerate(rows))
+    return ("define void @entry(i64 %0, i64 %1, i64 %2) {\n" + "\n".join(body) + "\n  ret void\n}\n!wafer.target.tile_id = !{!2}\n"
+            f"!wafer.target.entry_arguments = !{{!10, !11, !12}}\n!2 = !{{i64 {tile}}}\n{meta}\n")
+
+
+# the last two are replayed Tile by Tile: too long for the launches that serve several Tiles; Tiles that differ
+@pytest.mark.parametrize("tiles,count,gap,differ", [(2, 64, 0, False), (3, 192, 1, False), (16, 4096, 0, False), (5, 4160, 3, False),
+                                                    (2, 36864, 0, False), (3, 128, 0, True)])
+def test_tiles_in_step_match_the_tiles_alone(backend, tiles, count, gap, differ):
+    scale = [0x3f000000 + (0x10000 * t if differ else 0) for t in range(tiles)]
+    program = TileProgram([_module(t, tiles, count, scale[t], gap) for t in range(tiles)], backend, spm_bytes=1 << 20)
+    alone = [TileProgram([_module(0, 1, count, scale[t], gap)], backend, spm_bytes=1 << 20) for t in range(tiles)]
+    for seed in range(2):   # the first run captures, the second relaunches on other data
+        blocks = np.random.default_rng(seed).standard_normal((tiles, count + gap)).astype(np.float32)
+        (out, sums), stats = program.run([blocks.reshape(-1)])
+        singles = [one.run([blocks[t]]) for t, one in enumerate(alone)]
+        for t, ((want_out, want_sums), _) in enumerate(singles):
+            assert np.array_equal(out.reshape(tiles, -1)[t, :count], want_out.reshape(-1)[:count])
+            assert np.array_equal(sums.reshape(tiles, 64)[t], want_sums.reshape(-1))
+        for name in ("commands", "gpu_launches", "bytes_moved", "gemm_commands", "movement_commands", "fill_commands"):
+            assert stats[name] == sum(one[name] for _, one in singles), name
+        flags = 0
+        for _, one in singles:
+            flags |= one["numeric_flags"]
+        assert stats["numeric_flags"] == flags

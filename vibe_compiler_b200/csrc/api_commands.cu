@@ -553,17 +553,23 @@ wb200_status enqueue_image_gemm(wb200_spm_image *image, uint64_t lhs, uint64_t r
   g.dst = image->device + (dst - image->base);
   const char *implementation = "";
   const int effective_policy = (policy == WB200_GEMM_TENSOR && !has_psum && !lt && !rt) ? WB200_GEMM_TENSOR : WB200_GEMM_FORMAL;
-  if (defer && deferred && effective_policy == WB200_GEMM_FORMAL) {
-    RunCommand command;
-    command.kind = WB200_RUN_GEMM;
-    GemmFormalArgs &f = command.u.gemm;
-    f = GemmFormalArgs{};
+  const bool several = image->batch.tiles > 1;
+  if (several && effective_policy != WB200_GEMM_FORMAL) return fail(WB200_ERR_UNSUPPORTED, "tensor-core GEMM commands are issued Tile by Tile");
+  if (several || (defer && deferred && effective_policy == WB200_GEMM_FORMAL)) {
+    GemmFormalArgs f{};
     f.m = g.m; f.k = g.k; f.n = g.n; f.batch = g.batch;
     f.in_format = g.in_format; f.out_format = g.out_format;
     f.lhs_transposed = g.lhs_transposed; f.rhs_transposed = g.rhs_transposed;
     f.has_psum = g.has_psum;
     f.lhs = g.lhs; f.rhs = g.rhs; f.psum = g.psum; f.dst = g.dst;
     f.lhs_map = g.lhs_map; f.rhs_map = g.rhs_map; f.psum_map = g.psum_map; f.dst_map = g.dst_map;
+    if (several) {
+      if ((st = launch_gemm_formal(f, image->work_stream(), image->batch)) == WB200_OK) backend->launches += 1;
+      return st;
+    }
+    RunCommand command;
+    command.kind = WB200_RUN_GEMM;
+    command.u.gemm = f;
     command.variant = formal_gemm_variant(f);
     *defer = command;
     *deferred = formal_run_admits(command);
@@ -661,7 +667,7 @@ wb200_status enqueue_image_elementwise(wb200_spm_image *image, uint32_t operatio
     return WB200_OK;
   }
   st = launch_elementwise_formal(operation, format, out_format, arity, d_lhs, d_rhs, image->device + (dst - image->base), in_map,
-                                 out_map, d_flags, image->work_stream(), rhs);
+                                 out_map, d_flags, image->work_stream(), rhs, image->batch);
   if (st == WB200_OK) backend->launches += 1;
   return st;
 }
@@ -707,7 +713,7 @@ wb200_status enqueue_image_reduce(wb200_spm_image *image, uint32_t operation, ui
   }
   DeviceGuard guard(image->backend->device);
   st = launch_reduce_formal(operation, format, image->device + (source - image->base), image->device + (destination - image->base), in_map,
-                            dst_map, mask, d_flags, image->work_stream());
+                            dst_map, mask, d_flags, image->work_stream(), image->batch);
   if (st == WB200_OK) image->backend->launches += 1;
   return st;
 }

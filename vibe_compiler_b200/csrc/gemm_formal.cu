@@ -18,6 +18,8 @@ constexpr int kTile = 16;
 
 struct FormalParams {
   GemmFormalArgs a;
+  uint32_t tiled;         // blockIdx.z is the Tile (one matrix each), not the matrix of a batch
+  uint64_t tile_stride;   // bytes between the Tiles' operands
 };
 
 // Commands with few output tiles (a Tile's attention step is one 64 x 64 x 64 product): the register-tiled kernel would put
@@ -36,6 +38,8 @@ struct SmallOperand {
 struct SmallGemm {
   int m, k, n, in_format, out_format, lhs_transposed, rhs_transposed;
   SmallOperand lhs, rhs, dst, psum;  // psum.base null: none
+  uint32_t tiled;                    // as FormalParams
+  uint64_t tile_stride;
 };
 __device__ __forceinline__ uint32_t small_at(const SmallOperand &o, uint32_t batch, uint32_t row, uint32_t col) {
   if (col < o.full) return batch * o.batch + row * o.row + (col >> 6) * o.block + (col & 63u);
@@ -45,7 +49,9 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
   __shared__ float lhs_panel[kSmallPanelK][kTile + 1];   // [k][m]
   __shared__ float rhs_panel[kSmallPanelK][kTile + 1];   // [k][n]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int batch = blockIdx.z, row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+  const int batch = g.tiled ? 0 : blockIdx.z, row0 = blockIdx.y * kTile, col0 = blockIdx.x * kTile;
+  const uint64_t tile_offset = g.tiled ? blockIdx.z * g.tile_stride : 0;
+  const uint8_t *lhs = g.lhs.base + tile_offset, *rhs = g.rhs.base + tile_offset;
   // staging roles: consecutive threads take consecutive elements of the operand's fastest dimension
   const int l_kk = g.lhs_transposed ? tid >> 4 : tid & 63, l_r = g.lhs_transposed ? tid & 15 : tid >> 6;
   const int l_dk = g.lhs_transposed ? 16 : 0, l_dr = g.lhs_transposed ? 0 : 4;
@@ -61,7 +67,7 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
       lv[e] = 0.0f;
       if (k < g.k && r < g.m) {
         const uint32_t at = small_at(g.lhs, batch, g.lhs_transposed ? k : r, g.lhs_transposed ? r : k);
-        lv[e] = widen_bits(load_element_bits(g.lhs.base, at, g.in_format), g.in_format);
+        lv[e] = widen_bits(load_element_bits(lhs, at, g.in_format), g.in_format);
       }
     }
 #pragma unroll
@@ -70,7 +76,7 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
       rv[e] = 0.0f;
       if (k < g.k && c < g.n) {
         const uint32_t at = small_at(g.rhs, batch, g.rhs_transposed ? c : k, g.rhs_transposed ? k : c);
-        rv[e] = widen_bits(load_element_bits(g.rhs.base, at, g.in_format), g.in_format);
+        rv[e] = widen_bits(load_element_bits(rhs, at, g.in_format), g.in_format);
       }
     }
   };
@@ -78,7 +84,7 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
   pdl_wait();
   float acc = 0.0f, partial = 0.0f;
   fetch(0);
-  if (g.psum.base && owns) partial = __uint_as_float(load_element_bits(g.psum.base, small_at(g.psum, batch, row, col), WB200_F32));
+  if (g.psum.base && owns) partial = __uint_as_float(load_element_bits(g.psum.base + tile_offset, small_at(g.psum, batch, row, col), WB200_F32));
   for (int k0 = 0; k0 < g.k; k0 += kSmallPanelK) {
     if (k0) __syncthreads();   // the previous panel has been multiplied
 #pragma unroll
@@ -94,7 +100,7 @@ __global__ void __launch_bounds__(256) gemm_formal_small_kernel(const __grid_con
   }
   if (owns) {
     if (g.psum.base) acc = __fadd_rn(acc, partial);
-    store_element_bits(const_cast<uint8_t *>(g.dst.base), small_at(g.dst, batch, row, col), g.out_format, narrow_bits(acc, g.out_format));
+    store_element_bits(const_cast<uint8_t *>(g.dst.base) + tile_offset, small_at(g.dst, batch, row, col), g.out_format, narrow_bits(acc, g.out_format));
   }
 }
 // Fills `o` for a logical [batch, rows, cols] operand; false when its placement needs more than 32 bits or the general map.
@@ -142,32 +148,42 @@ __global__ void __launch_bounds__(256, 4) gemm_formal_tiled_kernel(const FormalP
   __shared__ __align__(16) float rhs_panel[kPanelK][kBlockN + 4];   // [k][n]
   pdl_launch_dependents();
   pdl_wait();
-  gemm_formal_tile<kResolved, kSeparable, kWide>(p.a, blockIdx.z, blockIdx.y * kBlockM, blockIdx.x * kBlockN, threadIdx.x, true, lhs_panel,
-                                                 rhs_panel);
+  GemmFormalArgs a = p.a;
+  const uint64_t offset = p.tiled ? blockIdx.z * p.tile_stride : 0;
+  a.lhs += offset;
+  a.rhs += offset;
+  a.psum += offset;   // read only where there is one
+  a.dst += offset;
+  gemm_formal_tile<kResolved, kSeparable, kWide>(a, p.tiled ? 0 : blockIdx.z, blockIdx.y * kBlockM, blockIdx.x * kBlockN, threadIdx.x, true,
+                                                 lhs_panel, rhs_panel);
 }
 
 }  // namespace
 
 int formal_gemm_variant(const GemmFormalArgs &args) { return gemm_formal_variant(args); }
 
-wb200_status launch_gemm_formal(const GemmFormalArgs &args, cudaStream_t stream) {
+wb200_status launch_gemm_formal(const GemmFormalArgs &args, cudaStream_t stream, TileBatch batch) {
   if (!is_float_format(args.in_format) || !is_float_format(args.out_format))
     return fail(WB200_ERR_UNSUPPORTED, "formal GEMM admits f16, bf16 and f32 only");
   if (args.m <= 0 || args.n <= 0 || args.k < 0 || args.batch <= 0)
     return fail(WB200_ERR_INVALID_ARGUMENT, "GEMM extents must be positive");
   if (args.batch > 65535) return fail(WB200_ERR_UNSUPPORTED, "batch count above 65535");
-  FormalParams p{args};
+  const bool tiled = batch.tiles > 1;
+  if (tiled && (args.batch != 1 || batch.stride % 16)) return fail(WB200_ERR_UNSUPPORTED, "a GEMM of several Tiles has one matrix each, 16-byte aligned strides");
+  FormalParams p{args, tiled, batch.stride};
   const int variant = gemm_formal_variant(args);
   const bool wide = variant == 3, separable = variant >= 2, all_resolved = variant >= 1;
   const int64_t tiles = static_cast<int64_t>((args.n + kBlockN - 1) / kBlockN) * ((args.m + kBlockM - 1) / kBlockM) * args.batch;
   SmallGemm small{};
   if ((args.m < 32 || args.n < 32 || tiles <= kFewTiles) && small_gemm(args, &small)) {
-    const dim3 grid((args.n + kTile - 1) / kTile, (args.m + kTile - 1) / kTile, args.batch);
+    const dim3 grid((args.n + kTile - 1) / kTile, (args.m + kTile - 1) / kTile, tiled ? batch.tiles : args.batch);
+    small.tiled = tiled;
+    small.tile_stride = batch.stride;
     WB200_CUDA_CHECK(launch_dependent(gemm_formal_small_kernel, grid, 256, 0, stream, small));
     WB200_CUDA_CHECK(cudaGetLastError());
     return WB200_OK;
   }
-  dim3 grid((args.n + kBlockN - 1) / kBlockN, (args.m + kBlockM - 1) / kBlockM, args.batch);
+  dim3 grid((args.n + kBlockN - 1) / kBlockN, (args.m + kBlockM - 1) / kBlockM, tiled ? batch.tiles : args.batch);
   if (wide)
     WB200_CUDA_CHECK(launch_dependent(gemm_formal_tiled_kernel<true, true, true>, grid, 256, 0, stream, p));
   else if (separable)

@@ -64,6 +64,13 @@ cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, s
   return launch_ordered(kernel, grid, block, smem, stream, true, static_cast<Args &&>(args)...);
 }
 
+// One command of several Tiles in one launch: their scratch-pad images lie `stride` bytes apart, and blockIdx.z = t works on
+// the operands t * stride behind the given ones (Tile 0's).
+struct TileBatch {
+  uint32_t tiles = 1;
+  uint64_t stride = 0;
+};
+
 // ---- TMA descriptor encoding (driver entry point fetched at run time; libcuda is not linked)
 // `inner`/`outer`(/`batch`) are extents in elements, innermost first; the box is {box_inner,
 // box_outer(,1)} with 128-byte swizzle; 16-bit elements only.
@@ -108,7 +115,7 @@ struct GemmFormalArgs {
   uint8_t *dst;
   LayoutMap lhs_map, rhs_map, psum_map, dst_map;  // physical placement of every operand
 };
-wb200_status launch_gemm_formal(const GemmFormalArgs &args, cudaStream_t stream);
+wb200_status launch_gemm_formal(const GemmFormalArgs &args, cudaStream_t stream, TileBatch tiles = TileBatch());
 
 // ---- managed-reference tensor commands (tensor_ops.cu)
 // `nan_flag` is set to 1 by the kernel if any input or result is NaN (the contract rejects those).
@@ -128,7 +135,7 @@ struct PoolWindow {
 };
 wb200_status launch_elementwise_formal(int op, int in_format, int out_format, int input_count, const uint8_t *in0, const uint8_t *in1,
                                        uint8_t *dst, const LayoutMap &in_map, const LayoutMap &out_map, uint32_t *flags_word,
-                                       cudaStream_t stream, RhsBroadcast rhs = RhsBroadcast());
+                                       cudaStream_t stream, RhsBroadcast rhs = RhsBroadcast(), TileBatch tiles = TileBatch());
 // A run of formal elementwise commands over 1-D Tensor vectors of one format and element count in which every command's
 // first operand is the previous command's destination: one launch carries the value in registers from step to step and
 // still writes every step's destination. Second operands are a full vector (WB200_RHS_SAME), immediate bits
@@ -146,7 +153,7 @@ struct ElementwiseChain {
   const uint8_t *lhs;
   ChainStep step[kMaxChainSteps];
 };
-wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream);
+wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles = TileBatch());
 // A run of formal commands of one Tile - GEMMs (one matrix, formal policy), elementwise commands over 1-D vectors and
 // NCx [n, h, w, c] reductions in any order, e.g. the scores, running maximum, probabilities, running sum and PV product
 // of an online-attention step - executed by ONE launch: a single thread block walks the commands in issue order with a
@@ -189,7 +196,7 @@ int formal_gemm_variant(const GemmFormalArgs &args);   // gemm_formal.cu
 wb200_status launch_formal_run(const FormalRun &run, uint32_t *flags_word, cudaStream_t stream);
 // Formal reduction: NaN-canonicalising, flag-raising fold in row-major input order (bit d of `reduced_mask` = dimension d reduced).
 wb200_status launch_reduce_formal(int op, int format, const uint8_t *src, uint8_t *dst, const LayoutMap &src_map, const LayoutMap &dst_map,
-                                  uint32_t reduced_mask, uint32_t *flags_word, cudaStream_t stream);
+                                  uint32_t reduced_mask, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles = TileBatch());
 // Plain pooling over NCx [n, h, w, c] tensors: `combine` is WB200_EW_MAX, WB200_EW_MIN or WB200_EW_ADD.
 wb200_status launch_pool_formal(int combine, int format, const uint8_t *src, uint8_t *dst, const LayoutMap &src_map,
                                 const LayoutMap &dst_map, PoolWindow window, uint32_t *flags_word, cudaStream_t stream);
@@ -278,9 +285,11 @@ struct StridedLayout {
 };
 uint64_t strided_segments(const StridedLayout &layout);
 uint64_t strided_span(const StridedLayout &layout);   // bytes from the first to one past the last byte touched
+// `tiles` copies at once, their sources and destinations so many bytes apart.
 wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to,
-                                 cudaStream_t stream);
-wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int element_bytes, cudaStream_t stream);
+                                 cudaStream_t stream, uint32_t tiles = 1, int64_t src_step = 0, int64_t dst_step = 0);
+wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int element_bytes, cudaStream_t stream,
+                         TileBatch tiles = TileBatch());
 // Packed Bool -> 1.0 / 0 of `format`; masked element move (store = 0: validate only; *first_refused = smallest element << 8 | 4
 // whose mask is neither 0 nor 1.0).
 wb200_status launch_bit2fp(const uint8_t *src, uint8_t *dst, uint32_t count, int format, cudaStream_t stream);

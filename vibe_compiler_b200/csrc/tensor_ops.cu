@@ -645,9 +645,13 @@ __device__ __forceinline__ uint32_t rhs_bits(const uint8_t *in1, const RhsBroadc
 template <int kOp, int kFormat>
 __global__ void __launch_bounds__(kShortThreads)
 formal_elementwise_short_kernel(int out_format, int input_count, const uint8_t *in0, const uint8_t *in1, uint8_t *dst, uint32_t count,
-                                const RhsBroadcast rhs, uint32_t *flags_word) {
+                                const RhsBroadcast rhs, uint64_t tile_stride, uint32_t *flags_word) {
   const uint32_t i = blockIdx.x * kShortThreads + threadIdx.x;
   uint32_t flags = 0;
+  const uint64_t tile_offset = blockIdx.z * tile_stride;
+  in0 += tile_offset;
+  in1 += tile_offset;   // read only where there is one
+  dst += tile_offset;
   pdl_launch_dependents();
   pdl_wait();
   if (i < count) {
@@ -661,8 +665,10 @@ formal_elementwise_short_kernel(int out_format, int input_count, const uint8_t *
 // evaluator instead of eleven behind a switch, so a block's code fits the instruction cache. kSingle: binary32 and TF32.
 template <int kOp, bool kSingle>
 __global__ void __launch_bounds__(kShortThreads)
-formal_function_kernel(int format, const uint8_t *in0, uint8_t *dst, int64_t count, uint32_t *flags_word) {
+formal_function_kernel(int format, const uint8_t *in0, uint8_t *dst, int64_t count, uint64_t tile_stride, uint32_t *flags_word) {
   uint32_t flags = 0;
+  in0 += blockIdx.z * tile_stride;
+  dst += blockIdx.z * tile_stride;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kShortThreads;
   const int fixed = kSingle ? (format == WB200_TF32 ? WB200_TF32 : WB200_F32) : (format == WB200_BF16 ? WB200_BF16 : WB200_F16);
   pdl_launch_dependents();
@@ -714,9 +720,11 @@ __device__ __forceinline__ void chain_step(int op, uint32_t (&value)[kPer], cons
 // made a 64-element subtract - exp - multiply chain take 67 us; it takes 4).
 template <int kFormat, int kPer>
 __global__ void __launch_bounds__(kPer == 1 ? kShortThreads : kThreads)
-formal_chain_kernel(const ElementwiseChain chain, int vector, uint32_t *flags_word) {
+formal_chain_kernel(const ElementwiseChain chain, int vector, uint64_t tile_stride, uint32_t *flags_word) {
   pdl_launch_dependents();
   pdl_wait();
+  const uint64_t tile_offset = blockIdx.z * tile_stride;
+  const uint8_t *const lhs = chain.lhs + tile_offset;
   constexpr int format = kFormat, bytes = kFormat == WB200_F32 ? 4 : 2;
   const int64_t total = chain.count, groups = (total + kPer - 1) / kPer;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -727,15 +735,15 @@ formal_chain_kernel(const ElementwiseChain chain, int vector, uint32_t *flags_wo
     const bool wide = kPer == 8 && vector && count == 8;
     uint32_t value[kPer], b[kPer];
     if (wide) {
-      if constexpr (kPer == 8) load_group8(chain.lhs, g, bytes, value);
+      if constexpr (kPer == 8) load_group8(lhs, g, bytes, value);
     } else {
 #pragma unroll
-      for (int e = 0; e < kPer; ++e) value[e] = e < count ? load_element_bits(chain.lhs, first + e, format) : 0u;
+      for (int e = 0; e < kPer; ++e) value[e] = e < count ? load_element_bits(lhs, first + e, format) : 0u;
     }
 #pragma unroll 1
     for (int s = 0; s < chain.steps; ++s) {
-      const uint8_t *rhs = chain.step[s].rhs;
-      uint8_t *dst = chain.step[s].dst;
+      const uint8_t *rhs = chain.step[s].rhs + tile_offset;   // read only where there is one
+      uint8_t *dst = chain.step[s].dst + tile_offset;
       if (chain.step[s].rhs_mode == WB200_RHS_SAME) {
         if (wide) {
           if constexpr (kPer == 8) load_group8(rhs, g, bytes, b);
@@ -990,7 +998,10 @@ __device__ __forceinline__ uint32_t fold_block(uint32_t steps, int outputs, Fetc
 // Any rank, layout and set of reduced dimensions.
 template <bool kFormal, int kCombine, int kFormat>
 __global__ void __launch_bounds__(kThreads)
-fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ FoldPlan plan, int *nan_flag, uint32_t *flags_word) {
+fold_staged_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ FoldPlan plan, uint64_t tile_stride, int *nan_flag,
+                   uint32_t *flags_word) {
+  src += blockIdx.z * tile_stride;
+  dst += blockIdx.z * tile_stride;
   __shared__ int64_t kept_slice[kFoldOutputs], kept_outer[kFoldOutputs], kept_c[kFoldOutputs], kept_dst[kFoldOutputs];
   const int tid = threadIdx.x;
   const int64_t first_output = static_cast<int64_t>(blockIdx.x) * kFoldOutputs;
@@ -1037,7 +1048,10 @@ struct LinearFold {
 };
 template <bool kFormal, int kCombine, int kFormat>
 __global__ void __launch_bounds__(kThreads)
-fold_linear_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ LinearFold f, int *nan_flag, uint32_t *flags_word) {
+fold_linear_kernel(const uint8_t *src, uint8_t *dst, const __grid_constant__ LinearFold f, uint64_t tile_stride, int *nan_flag,
+                   uint32_t *flags_word) {
+  src += blockIdx.z * tile_stride;
+  dst += blockIdx.z * tile_stride;
   const int tid = threadIdx.x, lane = tid & 31;
   const uint32_t output = blockIdx.x * kFoldOutputs + lane;
   const int outputs = static_cast<int>(min(static_cast<uint32_t>(kFoldOutputs), f.outputs - blockIdx.x * kFoldOutputs));
@@ -1299,7 +1313,7 @@ wb200_status launch_codec(const uint8_t *src, uint8_t *dst, const LayoutMap &map
 constexpr int64_t kManyOutputs = 65536;
 template <bool kFormal>
 wb200_status launch_fold_staged(int op, int format, const uint8_t *src, uint8_t *dst, const LayoutMap &src_map, const LayoutMap &dst_map,
-                                uint32_t reduced_mask, int *nan_flag, uint32_t *flags_word, cudaStream_t stream) {
+                                uint32_t reduced_mask, int *nan_flag, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles = TileBatch()) {
   FoldPlan plan{};
   plan.src = src_map; plan.dst = dst_map; plan.reduced_mask = reduced_mask;
   const int rank = src_map.rank;
@@ -1321,7 +1335,7 @@ wb200_status launch_fold_staged(int op, int format, const uint8_t *src, uint8_t 
   plan.along_steps = (reduced_mask >> (rank - 1)) & 1u;
   const int64_t blocks = (dst_map.element_count + kFoldOutputs - 1) / kFoldOutputs;
   if (blocks >= (1ll << 31)) return fail(WB200_ERR_LIMIT, "reduction output too large");
-  const int grid = static_cast<int>(blocks < 1 ? 1 : blocks);
+  const dim3 grid(static_cast<unsigned>(blocks < 1 ? 1 : blocks), 1, tiles.tiles);
   LinearFold linear{};
   const bool is_linear = plan.count == 1 && plan.kind[0] != 2 && dst_map.element_count > 0 && steps > 0 && src_map.physical_elements < (1ll << 31);
   if (is_linear) {
@@ -1347,8 +1361,8 @@ wb200_status launch_fold_staged(int op, int format, const uint8_t *src, uint8_t 
   }
 #define WB200_FOLD(COMBINE, FORMAT)                                                                                                      \
   do {                                                                                                                                  \
-    if (is_linear) WB200_CUDA_CHECK(launch_dependent(fold_linear_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, linear, nan_flag, flags_word)); \
-    else WB200_CUDA_CHECK(launch_dependent(fold_staged_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, plan, nan_flag, flags_word));             \
+    if (is_linear) WB200_CUDA_CHECK(launch_dependent(fold_linear_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, linear, tiles.stride, nan_flag, flags_word)); \
+    else WB200_CUDA_CHECK(launch_dependent(fold_staged_kernel<kFormal, COMBINE, FORMAT>, grid, kThreads, 0, stream, src, dst, plan, tiles.stride, nan_flag, flags_word));             \
   } while (0)
 #define WB200_FOLD_FORMATS(COMBINE)                                   \
   if (format == WB200_F32) WB200_FOLD(COMBINE, WB200_F32);            \
@@ -1402,17 +1416,17 @@ static bool is_function(int op) {
 
 wb200_status launch_elementwise_formal(int op, int in_format, int out_format, int input_count, const uint8_t *in0, const uint8_t *in1,
                                        uint8_t *dst, const LayoutMap &in_map, const LayoutMap &out_map, uint32_t *flags_word,
-                                       cudaStream_t stream, RhsBroadcast rhs) {
+                                       cudaStream_t stream, RhsBroadcast rhs, TileBatch tiles) {
   auto linear_layout = [](const LayoutMap &m) { return m.layout == WB200_LAYOUT_TENSOR || m.layout == WB200_LAYOUT_NTENSOR; };
   const bool function_family = is_function(op);
   if (function_family && linear_layout(in_map) && linear_layout(out_map)) {
     int64_t blocks = (out_map.element_count + kShortThreads - 1) / kShortThreads;
-    const int grid = static_cast<int>(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks);
+    const dim3 grid(static_cast<unsigned>(blocks < 1 ? 1 : blocks > 148 * 16 ? 148 * 16 : blocks), 1, tiles.tiles);
     const bool single = in_format == WB200_F32 || in_format == WB200_TF32;
 #define WB200_FUNCTION(OP)                                                                                                              \
   case OP:                                                                                                                              \
-    if (single) WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, true>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, flags_word)); \
-    else WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, false>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, flags_word));      \
+    if (single) WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, true>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, tiles.stride, flags_word)); \
+    else WB200_CUDA_CHECK(launch_dependent(formal_function_kernel<OP, false>, grid, kShortThreads, 0, stream, in_format, in0, dst, out_map.element_count, tiles.stride, flags_word));      \
     break;
     switch (op) {
       WB200_FUNCTION(WB200_EW_SQRT) WB200_FUNCTION(WB200_EW_RSQRT) WB200_FUNCTION(WB200_EW_LOG2) WB200_FUNCTION(WB200_EW_LN)
@@ -1428,9 +1442,9 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
                             is_float_format(in_format) && is_float_format(out_format);
   if (short_vector) {
     const uint32_t count = static_cast<uint32_t>(out_map.element_count);
-    const int grid = static_cast<int>((count + kShortThreads - 1) / kShortThreads);
+    const dim3 grid((count + kShortThreads - 1) / kShortThreads, 1, tiles.tiles);
 #define WB200_SHORT_LAUNCH(OP, FORMAT) \
-  WB200_CUDA_CHECK(launch_dependent(formal_elementwise_short_kernel<OP, FORMAT>, grid, kShortThreads, 0, stream, out_format, input_count, in0, in1, dst, count, rhs, flags_word))
+  WB200_CUDA_CHECK(launch_dependent(formal_elementwise_short_kernel<OP, FORMAT>, grid, kShortThreads, 0, stream, out_format, input_count, in0, in1, dst, count, rhs, tiles.stride, flags_word))
 #define WB200_SHORT(OP)                                             \
   case OP:                                                          \
     if (in_format == WB200_F32) WB200_SHORT_LAUNCH(OP, WB200_F32);  \
@@ -1448,6 +1462,7 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
 #undef WB200_SHORT
 #undef WB200_SHORT_LAUNCH
   }
+  if (tiles.tiles > 1) return fail(WB200_ERR_UNSUPPORTED, "no elementwise kernel for several Tiles at these sizes and formats");
   // a thread takes eight consecutive elements, or one at a time for the correctly rounded functions
   const int64_t groups = function_family ? out_map.element_count : (out_map.element_count + 7) / 8;
   int64_t blocks = (groups + kThreads - 1) / kThreads;
@@ -1482,10 +1497,10 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
   return WB200_OK;
 }
 
-wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream) {
+wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles) {
   if (chain.steps < 1 || chain.steps > kMaxChainSteps || chain.count < 1 || !is_float_format(chain.format))
     return fail(WB200_ERR_INVALID_ARGUMENT, "malformed elementwise chain");
-  uintptr_t low_bits = reinterpret_cast<uintptr_t>(chain.lhs);
+  uintptr_t low_bits = reinterpret_cast<uintptr_t>(chain.lhs) | (tiles.tiles > 1 ? static_cast<uintptr_t>(tiles.stride) : 0);
   for (int s = 0; s < chain.steps; ++s)
     low_bits |= reinterpret_cast<uintptr_t>(chain.step[s].dst) | (chain.step[s].rhs_mode == WB200_RHS_SAME ? reinterpret_cast<uintptr_t>(chain.step[s].rhs) : 0);
   bool one_each = chain.count <= kShortVector;
@@ -1493,11 +1508,12 @@ wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *f
   const int per = one_each ? 1 : 8, threads = one_each ? kShortThreads : kThreads;
   int64_t blocks = ((chain.count + per - 1) / per + threads - 1) / threads;
   blocks = blocks < 1 ? 1 : blocks > 148 * 32 ? 148 * 32 : blocks;
-  const int grid = static_cast<int>(blocks), vector = (low_bits & 15) == 0;
+  const dim3 grid(static_cast<unsigned>(blocks), 1, tiles.tiles);
+  const int vector = (low_bits & 15) == 0;
 #define WB200_CHAIN(FORMAT)                                                                                          \
   do {                                                                                                               \
-    if (one_each) WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 1>, grid, threads, 0, stream, chain, vector, flags_word));           \
-    else WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 8>, grid, threads, 0, stream, chain, vector, flags_word));                    \
+    if (one_each) WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 1>, grid, threads, 0, stream, chain, vector, tiles.stride, flags_word));           \
+    else WB200_CUDA_CHECK(launch_dependent(formal_chain_kernel<FORMAT, 8>, grid, threads, 0, stream, chain, vector, tiles.stride, flags_word));                    \
   } while (0)
   if (chain.format == WB200_F32) WB200_CHAIN(WB200_F32);
   else if (chain.format == WB200_BF16) WB200_CHAIN(WB200_BF16);
@@ -1535,9 +1551,10 @@ wb200_status launch_formal_run(const FormalRun &run, uint32_t *flags_word, cudaS
 }
 
 wb200_status launch_reduce_formal(int op, int format, const uint8_t *src, uint8_t *dst, const LayoutMap &src_map, const LayoutMap &dst_map,
-                                  uint32_t reduced_mask, uint32_t *flags_word, cudaStream_t stream) {
+                                  uint32_t reduced_mask, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles) {
   if (!reduce_one_thread_per_output(src_map, dst_map))
-    return launch_fold_staged<true>(op, format, src, dst, src_map, dst_map, reduced_mask, nullptr, flags_word, stream);
+    return launch_fold_staged<true>(op, format, src, dst, src_map, dst_map, reduced_mask, nullptr, flags_word, stream, tiles);
+  if (tiles.tiles > 1) return fail(WB200_ERR_UNSUPPORTED, "no reduction of several Tiles with so many outputs");
   const int grid = static_cast<int>((dst_map.element_count + kThreads - 1) / kThreads);
 #define WB200_RED_LAUNCH(COMBINE, FORMAT) formal_reduce_nhwc_kernel<COMBINE, FORMAT><<<grid, kThreads, 0, stream>>>(src, dst, src_map, dst_map, reduced_mask, flags_word)
 #define WB200_RED_FORMATS(COMBINE)                                              \

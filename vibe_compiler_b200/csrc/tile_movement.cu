@@ -12,9 +12,12 @@ namespace {
 
 template <typename Unit>
 __global__ void __launch_bounds__(256) strided_copy_kernel(const uint8_t *src, uint8_t *dst, StridedLayout from, StridedLayout to,
-                                                            uint32_t units_per_segment, uint64_t total_units) {
+                                                            uint32_t units_per_segment, uint64_t total_units, int64_t src_step,
+                                                            int64_t dst_step) {
   pdl_launch_dependents();
   pdl_wait();
+  src += blockIdx.z * src_step;
+  dst += blockIdx.z * dst_step;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < total_units; u += stride) {
     // a command moves at most 4 GiB, so 32-bit division is enough (64-bit division is several times slower)
@@ -36,9 +39,10 @@ __global__ void __launch_bounds__(256) strided_copy_kernel(const uint8_t *src, u
 }
 
 template <typename Element>
-__global__ void __launch_bounds__(256) fill_kernel(Element *dst, Element value, uint64_t count) {
+__global__ void __launch_bounds__(256) fill_kernel(Element *dst, Element value, uint64_t count, uint64_t tile_stride) {
   pdl_launch_dependents();
   pdl_wait();
+  dst += blockIdx.z * (tile_stride / sizeof(Element));
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
   for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) dst[i] = value;
 }
@@ -98,7 +102,7 @@ uint64_t strided_span(const StridedLayout &layout) {
 }
 
 wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, uint32_t tiles, int64_t src_step, int64_t dst_step) {
   if (from.inner_bytes == 0 || from.inner_bytes != to.inner_bytes)
     return fail(WB200_ERR_INVALID_ARGUMENT, "strided copy needs equal, non-zero inner byte counts");
   for (int d = 0; d < 3; ++d)
@@ -106,25 +110,27 @@ wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, 
   const uint64_t segments = strided_segments(from);
   if (segments != strided_segments(to)) return fail(WB200_ERR_INVALID_ARGUMENT, "source and destination segment counts differ");
   const uint64_t bytes = segments * from.inner_bytes;
-  const uintptr_t bases = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
+  // every Tile's addresses have to allow the unit
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) |
+                          (tiles > 1 ? static_cast<uintptr_t>(src_step) | static_cast<uintptr_t>(dst_step) : 0);
   if (bases % 16 == 0 && layout_aligned(from, 16) && layout_aligned(to, 16)) {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint4>, grid_for(bytes / 16), 256, 0, stream, src, dst, from, to, from.inner_bytes / 16, bytes / 16));
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint4>, dim3(grid_for(bytes / 16), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes / 16, bytes / 16, src_step, dst_step));
   } else if (bases % 4 == 0 && layout_aligned(from, 4) && layout_aligned(to, 4)) {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint32_t>, grid_for(bytes / 4), 256, 0, stream, src, dst, from, to, from.inner_bytes / 4, bytes / 4));
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint32_t>, dim3(grid_for(bytes / 4), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes / 4, bytes / 4, src_step, dst_step));
   } else {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint8_t>, grid_for(bytes), 256, 0, stream, src, dst, from, to, from.inner_bytes, bytes));
+    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint8_t>, dim3(grid_for(bytes), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes, bytes, src_step, dst_step));
   }
   WB200_CUDA_CHECK(cudaGetLastError());
   return WB200_OK;
 }
 
-wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int element_bytes, cudaStream_t stream) {
+wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int element_bytes, cudaStream_t stream, TileBatch tiles) {
   if (count == 0) return WB200_OK;
-  if (reinterpret_cast<uintptr_t>(dst) % element_bytes) return fail(WB200_ERR_INVALID_ARGUMENT, "fill destination is not element aligned");
+  if (reinterpret_cast<uintptr_t>(dst) % element_bytes || (tiles.tiles > 1 && tiles.stride % element_bytes)) return fail(WB200_ERR_INVALID_ARGUMENT, "fill destination is not element aligned");
   switch (element_bytes) {
-    case 1: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint8_t>, grid_for(count), 256, 0, stream, dst, static_cast<uint8_t>(value_bits), count)); break;
-    case 2: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint16_t>, grid_for(count), 256, 0, stream, reinterpret_cast<uint16_t *>(dst), static_cast<uint16_t>(value_bits), count)); break;
-    case 4: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint32_t>, grid_for(count), 256, 0, stream, reinterpret_cast<uint32_t *>(dst), value_bits, count)); break;
+    case 1: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint8_t>, dim3(grid_for(count), 1, tiles.tiles), 256, 0, stream, dst, static_cast<uint8_t>(value_bits), count, tiles.stride)); break;
+    case 2: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint16_t>, dim3(grid_for(count), 1, tiles.tiles), 256, 0, stream, reinterpret_cast<uint16_t *>(dst), static_cast<uint16_t>(value_bits), count, tiles.stride)); break;
+    case 4: WB200_CUDA_CHECK(launch_dependent(fill_kernel<uint32_t>, dim3(grid_for(count), 1, tiles.tiles), 256, 0, stream, reinterpret_cast<uint32_t *>(dst), value_bits, count, tiles.stride)); break;
     default: return fail(WB200_ERR_UNSUPPORTED, "fill takes 1, 2 or 4 byte elements");
   }
   WB200_CUDA_CHECK(cudaGetLastError());

@@ -14,7 +14,7 @@
 // pipe works on one tile while the other tile's softmax runs. A persistent grid of one CTA per SM walks
 // a host-made plan of items, so the loads and first scores of an item overlap the softmax tail and
 // write-out of the previous one and every CTA ends at nearly the same time. Warp 0 = TMA producer (per
-// item: Q, then K0 V0 K1 V1 ... through a ring of five 32 KiB slots that runs on across items), warp 1 =
+// item: Q, then K0 V0 K1 V1 ... through a ring of four 32 KiB slots that runs on across items), warp 1 =
 // MMA issuer and TMEM owner (the whole warp walks the loop, one elected lane issues), warps 4-7 / 8-11 =
 // softmax + rescale + epilogue for Q tile 0 / 1 (thread = query row, so row max and row sum need no
 // shuffles; setmaxnreg moves registers from warpgroup 0 to the softmax warpgroups). All mbarriers are
@@ -42,16 +42,18 @@ constexpr int kTileM = 128;       // query rows per Q tile (TMEM lanes)
 constexpr int kTileN = 128;       // keys per KV tile
 constexpr int kTileBytesFa = kTileN * kHd * 2;  // 32 KiB: two 64-element column blocks of 128 rows
 constexpr int kBlockBytes = 128 * 128;          // one [128 rows][128 B] swizzled block
+constexpr int kOutStageBytes = 32 * 128;        // one softmax warp's 32 rows x 64 columns of output
 constexpr int kFaThreads = 384;          // warpgroup 0: TMA + MMA warps; warpgroups 1, 2: softmax of Q tile 0, 1
-constexpr int kPParts = 2;               // P of a tile is published in two halves so PV starts on the first
-constexpr int kChunksPerPart = 2;        // 32-key chunks per half
+constexpr int kPParts = 2;               // P of a tile is published in two parts so PV starts on the first
+constexpr int kFirstChunks = 3;          // 32-key chunks of the first part, of 4: the products behind the last one are few
 constexpr uint32_t kColS0 = 0, kColO0 = 256;    // S_t at t*128, O_t at 256 + t*128
 
 struct FaSmem {
-  static constexpr int kSlots = 5;         // K / V ring
+  static constexpr int kSlots = 4;         // K / V ring
   static constexpr int kQOff = 0;
   static constexpr int kRingOff = 2 * kTileBytesFa;
-  static constexpr int kBarOff = kRingOff + kSlots * kTileBytesFa;
+  static constexpr int kOutOff = kRingOff + kSlots * kTileBytesFa;     // a stage per softmax warp
+  static constexpr int kBarOff = kOutOff + 8 * kOutStageBytes;
   static constexpr size_t kBytes = kBarOff + 256 + 1024;
 };
 
@@ -154,13 +156,14 @@ struct FaItem {
   int n_max;
   __device__ __forceinline__ int tiles(int t) const { return t ? n1 : n0; }
 };
-__device__ __forceinline__ FaItem fa_item(const FaParams &p, int k) {
+__device__ __forceinline__ int fa_item_id(const FaParams &p, int k) {
+  if (p.plan) return p.plan[static_cast<size_t>(blockIdx.x) * p.plan_stride + k];
+  return k == 0 ? static_cast<int>(blockIdx.x) : -1;   // no plan: CTA b runs item b only
+}
+__device__ __forceinline__ FaItem fa_decode(const FaParams &p, int id) {
   FaItem item;
   // 32-bit arithmetic only: a 64-bit division is an out-of-line call, and a call inside the MMA warp's code costs
   // about 8 % per KV step of its issue loop.
-  int id;
-  if (p.plan) id = p.plan[static_cast<size_t>(blockIdx.x) * p.plan_stride + k];
-  else id = k == 0 ? static_cast<int>(blockIdx.x) : -1;   // no plan: CTA b runs item b only
   const unsigned g = static_cast<unsigned>(id);
   const unsigned bh_count = static_cast<unsigned>(p.batch * p.q_heads);
   item.valid = id >= 0;
@@ -182,7 +185,7 @@ __device__ __forceinline__ FaItem fa_item(const FaParams &p, int k) {
 // warps alone); advances k past it.
 __device__ __forceinline__ FaItem fa_next_working_item(const FaParams &p, int &k) {
   while (true) {
-    const FaItem item = fa_item(p, k++);
+    const FaItem item = fa_decode(p, fa_item_id(p, k++));
     if (!item.valid || item.n_max > 0) return item;
   }
 }
@@ -190,7 +193,7 @@ __device__ __forceinline__ FaItem fa_next_working_item(const FaParams &p, int &k
 template <bool kBf16>
 __global__ void __launch_bounds__(kFaThreads, 1)
 fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-               const __grid_constant__ CUtensorMap tmap_v, const FaParams p) {
+               const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_out, const FaParams p) {
   using L = FaSmem;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -202,7 +205,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
   auto kv_empty = [&](int s) { return bar_base + 8u * (L::kSlots + s); };
   const uint32_t q_full = bar_base + 8u * (2 * L::kSlots);
   auto s_full = [&](int t) { return bar_base + 8u * (2 * L::kSlots + 1 + t); };
-  // P of one tile is published in two halves (keys 0-63, 64-127) so PV can start on the first half.
+  // P of one tile is published in two parts (keys 0-95, 96-127) so PV can start on the first.
   auto p_part = [&](int t, int part) { return bar_base + 8u * (2 * L::kSlots + 3 + kPParts * t + part); };
   auto o_done = [&](int t) { return bar_base + 8u * (2 * L::kSlots + 3 + 2 * kPParts + t); };
   const uint32_t q_empty = bar_base + 8u * (2 * L::kSlots + 5 + 2 * kPParts);   // every S product of an item has finished
@@ -222,7 +225,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     mbar_init(q_empty, 1);
     for (int t = 0; t < 2; ++t) {
       mbar_init(s_full(t), 1);
-      for (int part = 0; part < kPParts; ++part) mbar_init(p_part(t, part), kTileM);
+      for (int part = 0; part < kPParts; ++part) mbar_init(p_part(t, part), kTileM / 32);   // one arrival per softmax warp
       mbar_init(o_done(t), 1);
     }
     *abort_word = 0;
@@ -230,6 +233,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_v);
+    tma_prefetch_desc(&tmap_out);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), 512);
@@ -320,7 +324,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         const uint32_t d_tmem = tmem_base + kColO0 + t * 128;
         if (elect_one_sync()) {
 #pragma unroll
-          for (int ks = (8 / kPParts) * part; ks < (8 / kPParts) * (part + 1); ++ks) {
+          for (int ks = part ? 2 * kFirstChunks : 0; ks < (part ? 8 : 2 * kFirstChunks); ++ks) {
             const uint64_t bdesc = v_desc + static_cast<uint32_t>((ks * 2048) >> 4);
             const uint32_t acc = (accumulate || ks != 0) ? 1u : 0u;
             umma_f16_ts(d_tmem, tmem_base + kColS0 + t * 128 + ks * 8, bdesc, idesc_o, acc);
@@ -372,11 +376,9 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
               if (!mbar_wait_spin(p_part(t, 0), (tile_base + j) & 1u, abort_word)) { ok = false; return; }
               tc_fence_after();
               issue_pv_part(tile_tag, std::integral_constant<int, 0>{}, v_slot, j > 0);
-              if constexpr (kPParts > 1) {
-                if (!mbar_wait_spin(p_part(t, kPParts - 1), (tile_base + j) & 1u, abort_word)) { ok = false; return; }
-                tc_fence_after();
-                issue_pv_part(tile_tag, std::integral_constant<int, kPParts - 1>{}, v_slot, j > 0);
-              }
+              if (!mbar_wait_spin(p_part(t, 1), (tile_base + j) & 1u, abort_word)) { ok = false; return; }
+              tc_fence_after();
+              issue_pv_part(tile_tag, std::integral_constant<int, 1>{}, v_slot, j > 0);
             }
             if (j + 1 < n_tiles) {
               if (!k_ready) {
@@ -411,13 +413,17 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const uint32_t o_addr = tmem_base + lane_sel + kColO0 + t * 128;
     uint32_t tiles_done = 0;   // S tiles of this Q-tile slot consumed so far, over all items (barrier parities)
     bool ok = true;
+    const uint32_t out_stage = smem_base + L::kOutOff + (warp - 4) * kOutStageBytes;
+    int next_id = fa_item_id(p, 0);
     for (int item_index = 0; ok; ++item_index) {
+    const int id = next_id;
+    if (id < 0) break;
+    next_id = fa_item_id(p, item_index + 1);   // on its way while this item is worked on
     // Only the row, the tile count and the mask limit stay live through the tile loop; the output coordinates are
     // recomputed after it (the softmax threads need every register for the 128 scores they hold).
     int row_base, my_tiles;
     {
-      const FaItem item = fa_item(p, item_index);
-      if (!item.valid) break;
+      const FaItem item = fa_decode(p, id);
       row_base = item.row_base;
       my_tiles = item.tiles(t);
     }
@@ -464,14 +470,15 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       const float raw_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
       m_true = fmaxf(m_true, raw_max * p.scale_log2);     // scale > 0, so max commutes with the scaling
       float alpha = 1.0f;
-      if (m_true - m_ref > kRescaleThreshold) {           // also taken when m_ref is still -inf
+      const bool moves = m_true - m_ref > kRescaleThreshold, any_moves = __any_sync(0xffffffffu, moves);
+      if (moves) {           // also when m_ref is still -inf
         alpha = exp2f(m_ref - m_true);
         m_ref = m_true;
       }
       const float m_exp = (m_ref == -INFINITY) ? 0.f : m_ref;
-      // acc' = acc * alpha (rare) needs the PV product of the previous tile in TMEM and has to land before any PV of
-      // this tile is issued, i.e. before the first half of P is published; the wait for that product sits there, behind
-      // the first 64 exponentials, where it costs nothing.
+      // acc' = acc * alpha (rare) has to land before any PV of this tile is issued, i.e. before the first part of P is
+      // published. It needs no wait: the previous PV products were issued by the same thread before these scores, whose
+      // commit therefore covers them.
       const unsigned long long scale2 = pack_f32x2(p.scale_log2, p.scale_log2), neg_m2 = pack_f32x2(-m_exp, -m_exp);
       unsigned long long sum2[4] = {0ull, 0ull, 0ull, 0ull};
       auto exp_phase = [&]() {
@@ -497,25 +504,22 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
           }
         }
         tmem_st_32x16(s_addr + c * 16, packed);   // P aliases the first 64 columns of S
-        if (c == kChunksPerPart - 1 && j > 0) {
-          if (!mbar_wait(o_done(t), (tiles_done - 1) & 1u, abort_word, 112 + t)) { ok = false; return; }
-          if (__any_sync(0xffffffffu, alpha != 1.0f)) {
-            tc_fence_after();
+        if (c == kFirstChunks - 1 && j > 0 && any_moves) {
 #pragma unroll 1
-            for (int oc = 0; oc < 4; ++oc) {
-              uint32_t o[32];
-              tmem_ld_32x32(o_addr + oc * 32, o);
-              tmem_wait_ld();
+          for (int oc = 0; oc < 4; ++oc) {
+            uint32_t o[32];
+            tmem_ld_32x32(o_addr + oc * 32, o);
+            tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st_32x32(o_addr + oc * 32, o);
-            }
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32(o_addr + oc * 32, o);
           }
         }
-        if ((c + 1) % kChunksPerPart == 0) {   // a half of P is complete: publish it
+        if (c == kFirstChunks - 1 || c == 3) {   // a part of P is complete: publish it
           tmem_wait_st();
           tc_fence_before();
-          mbar_arrive(p_part(t, c / kChunksPerPart));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_part(t, c == 3 ? 1 : 0));
         }
       }
       };
@@ -532,27 +536,30 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       tc_fence_after();
       float coefficient = 1.0f / l_run;
       if (p.zero_fully_masked && l_run == 0.f) coefficient = 0.f;
-      const FaItem where = fa_item(p, item_index);
-      const int bh = where.bh, b = where.b, h = where.h;
-      const size_t out_row = p.out_token_major
-                                 ? ((static_cast<size_t>(b) * p.q_len + row) * p.q_heads + h) * kHd
-                                 : (static_cast<size_t>(bh) * p.q_len + row) * kHd;
-      uint32_t r[128];
-      if (my_tiles > 0) {
+      const FaItem where = fa_decode(p, id);
+      const int bh = where.bh;
+      const int warp_row = row_base + t * kTileM + quarter * 32;
+      // 0 * (1/0): a row that saw no key and is not zero-filled is the canonical quiet NaN of the format.
+      const bool nan_row = !(coefficient == coefficient) || (l_run == 0.f && !p.zero_fully_masked);
+      const uint32_t nan_pair = kBf16 ? 0x7fc07fc0u : 0x7e007e00u;
+      // Written out through shared memory, 32 rows x 64 columns of a warp at a time (the tensor map's 128-byte swizzle; rows
+      // behind q_len are clipped). With a row per thread every 16-byte store of a warp touches 32 lines, and the 2000 clocks
+      // those take per tile hold up the other tile's barriers and TMEM traffic.
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
+        uint32_t r[64];
+        if (my_tiles > 0) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld_32x32(o_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32 * c]));
-        tmem_wait_ld();
-      } else {
+          for (int c = 0; c < 2; ++c) tmem_ld_32x32(o_addr + half * 64 + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32 * c]));
+          tmem_wait_ld();
+        } else {
 #pragma unroll
-        for (int i = 0; i < 128; ++i) r[i] = 0u;
-      }
-      if (row < p.q_len) {
-        uint16_t *dst = reinterpret_cast<uint16_t *>(p.out) + out_row;
-        // 0 * (1/0): a row that saw no key and is not zero-filled is the canonical quiet NaN of the format.
-        const bool nan_row = !(coefficient == coefficient) || (l_run == 0.f && !p.zero_fully_masked);
-        const uint32_t nan_pair = kBf16 ? 0x7fc07fc0u : 0x7e007e00u;
+          for (int i = 0; i < 64; ++i) r[i] = 0u;
+        }
+        if (lane == 0) tma_store_wait_read();   // the stage's previous contents have been read
+        __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 128; i += 8) {
+        for (int i = 0; i < 64; i += 8) {
           uint32_t w[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -566,7 +573,13 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             }
             if (nan_row) w[k] = nan_pair;
           }
-          *reinterpret_cast<uint4 *>(dst + i) = make_uint4(w[0], w[1], w[2], w[3]);
+          st_shared_v4(out_stage + lane * 128 + (((i >> 3) ^ (lane & 7)) << 4), w);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (warp_row < p.q_len) tma_store_4d(&tmap_out, out_stage, half * 64, warp_row, where.h, where.b);
+          tma_store_commit();
         }
       }
       if (row < p.q_len) {
@@ -579,6 +592,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
       }
     }
     }   // items
+    if (lane == 0) tma_store_wait_read();   // the staging area outlives the copies out of it
   }
 
   tc_fence_before();
@@ -711,6 +725,14 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int 
                       row_pitch * a.kv_len, 64, kTileN);
   if (st != WB200_OK) return st;
 
+  // The output as [batch][head][row][column], whichever of head and row is the outer one in memory.
+  CUtensorMap to;
+  const uint64_t out_row_pitch = a.out_token_major ? row_pitch * a.q_heads : row_pitch;
+  const uint64_t out_head_pitch = a.out_token_major ? row_pitch : row_pitch * a.q_len;
+  st = encode_tmap_4d(&to, a.out, a.format, kHd, a.q_len, a.q_heads, a.batch, out_row_pitch, out_head_pitch,
+                      row_pitch * a.q_len * a.q_heads, 64, 32);
+  if (st != WB200_OK) return st;
+
   FaParams p;
   p.batch = a.batch; p.q_heads = a.q_heads; p.kv_heads = a.kv_heads; p.group = a.q_heads / a.kv_heads;
   p.q_len = a.q_len; p.kv_len = a.kv_len;
@@ -768,9 +790,9 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int 
   config.attrs = attrs;
   config.numAttrs = p.plan && grid % 2 == 0 ? 2 : 1;
   if (a.format == WB200_BF16)
-    WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, fa_umma_kernel<true>, tq, tk, tv, p));
+    WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, fa_umma_kernel<true>, tq, tk, tv, to, p));
   else
-    WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, fa_umma_kernel<false>, tq, tk, tv, p));
+    WB200_CUDA_CHECK(cudaLaunchKernelEx(&config, fa_umma_kernel<false>, tq, tk, tv, to, p));
   return WB200_OK;
 }
 

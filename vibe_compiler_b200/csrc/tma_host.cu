@@ -35,7 +35,7 @@ wb200_status encode(CUtensorMap *map, const void *base, int format, uint32_t ran
   for (uint32_t i = 0; i + 1 < rank; ++i)
     if (strides[i] % 16 != 0)
       return fail(WB200_ERR_INVALID_ARGUMENT, "TMA strides must be multiples of 16 bytes");
-  const cuuint32_t element_strides[3] = {1, 1, 1};
+  const cuuint32_t element_strides[4] = {1, 1, 1, 1};
   CUresult result =
       fn(map, format == WB200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
          rank, const_cast<void *>(base), dims, strides, box, element_strides,
@@ -64,6 +64,15 @@ wb200_status encode_tmap_3d(CUtensorMap *map, const void *base, int format, uint
   const cuuint64_t strides[2] = {row_pitch_bytes, batch_pitch_bytes};
   const cuuint32_t box[3] = {box_inner, box_outer, 1};
   return encode(map, base, format, 3, dims, strides, box);
+}
+
+wb200_status encode_tmap_4d(CUtensorMap *map, const void *base, int format, uint64_t inner, uint64_t extent1, uint64_t extent2,
+                            uint64_t extent3, uint64_t pitch1_bytes, uint64_t pitch2_bytes, uint64_t pitch3_bytes, uint32_t box_inner,
+                            uint32_t box_extent1) {
+  const cuuint64_t dims[4] = {inner, extent1, extent2, extent3};
+  const cuuint64_t strides[3] = {pitch1_bytes, pitch2_bytes, pitch3_bytes};
+  const cuuint32_t box[4] = {box_inner, box_extent1, 1, 1};
+  return encode(map, base, format, 4, dims, strides, box);
 }
 
 bool page_locked_range(const void *host, size_t bytes) {

@@ -39,3 +39,22 @@ def test_tile_edges_match_float64(backend, shape, token_major):
     assert (lse.double() - torch.logsumexp(scores, -1)).abs().max().item() <= 1e-5
     assert (m.double() - scores.amax(-1)).abs().max().item() <= 1e-5
     assert torch.allclose(m.double() + l.double().log(), lse.double(), atol=1e-5)
+
+
+@pytest.mark.parametrize("keys", [1, 64, 65, 128, 192, 193, 256, 257, 320, 513])
+@pytest.mark.parametrize("causal", [False, True])
+def test_key_tiles_over_the_groups_match_float64(backend, keys, causal):
+    # 64-key tiles go to four groups of threads in turn: none, some or all of them with a tile, whole, ragged or on the diagonal
+    rows, d = min(keys, 70), 64
+    gen = torch.Generator(device="cuda").manual_seed(keys)
+    q, k, v = (torch.randn(2, 3, n, d, device="cuda", generator=gen) for n in (rows, keys, keys))
+    lse = torch.empty(2, 3, rows, device="cuda")
+    out = backend.attention_fa(q, k, v, d ** -0.5, causal, lse=lse, query_start=keys - rows)
+    torch.cuda.synchronize()
+    backend.poll()
+    scores = q.double() @ k.double().transpose(-1, -2) * d ** -0.5
+    if causal:
+        scores = scores.masked_fill(~torch.ones(rows, keys, dtype=torch.bool, device="cuda").tril(keys - rows), float("-inf"))
+    want = torch.softmax(scores, -1) @ v.double()
+    assert helpers.max_rel_err(out.double().cpu().numpy(), want.cpu().numpy()) <= 1e-5   # the f32 bound of the path
+    assert (lse.double() - torch.logsumexp(scores, -1)).abs().max().item() <= 1e-5

@@ -156,19 +156,21 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) fa_simt_kernel(const Simt
 }
 
 // ---------------------------------------------------------------- f32 storage, head_dim 64 or 128: register tiles
-// A block owns 32 query rows of one (batch, head). Its two groups of 128 threads walk the tiles of 64 keys in turn
-// (group g: tiles g, g + 2, ...), each with a state of its own; the states are merged once at the end. A thread holds
+// A block owns 32 query rows of one (batch, head). Its groups of 128 threads (four at head_dim 64, two at 128: what shared
+// memory holds) walk the tiles of 64 keys in turn, each with a state of its own; the states are merged once at the end. A thread holds
 // 4 rows x 4 keys of the scores (keys tx, tx + 16, ...) and 4 rows x D/16 columns of the accumulator, so 64 multiply-adds
 // follow on 8 shared-memory vectors; the 16 threads of a row are half a warp, which keeps the row statistics and P inside
 // the warp. K and V have a buffer each, refilled by cp.async as soon as the group has read it: K of the next tile travels
 // under the softmax and the PV product, V under the next scores.
 // Bound by the f32 multiply-adds (8 heads x 512 x 512 x 64: 0.27 G, 7 us at the rate of 148 SMs; 128 of them have a block)
-// and the shared-memory vectors that feed them: 73.7 us with a warp per row, 26.6 us now. The warp-per-row kernel stays for
-// other widths, 16-bit storage and unaligned buffers.
-constexpr int kTileRows = 32, kTileKeysWide = 64, kGroupThreads = 128, kGroups = 2;
+// and the shared-memory vectors that feed them: 73.7 us with a warp per row, 23.8 us with two groups, 22.2 us with four (16
+// warps hide more of the latency of loads, shuffles and exponentials). The warp-per-row kernel stays for other widths, 16-bit
+// storage and unaligned buffers.
+constexpr int kTileRows = 32, kTileKeysWide = 64, kGroupThreads = 128;
 
 template <int kD>
 struct TiledSmem {
+  static constexpr int kGroups = kD == 64 ? 4 : 2;   // as many as shared memory holds
   static constexpr int kKPitch = kD + 4;   // rows 16 bytes apart modulo the banks: eight lanes' vectors cover all banks
   static constexpr int kPPitch = kTileKeysWide + 4;
   static constexpr int kQ = 0;
@@ -180,8 +182,9 @@ struct TiledSmem {
 };
 
 template <int kD>
-__global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const SimtParams p) {
+__global__ void __launch_bounds__(TiledSmem<kD>::kGroups * kGroupThreads) fa_f32_kernel(const SimtParams p) {
   using L = TiledSmem<kD>;
+  constexpr int kGroups = L::kGroups;
   const AttentionArgs &a = p.a;
   extern __shared__ float4 smem_vectors[];
   float *smem = reinterpret_cast<float *>(smem_vectors);
@@ -300,9 +303,11 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const S
     }
     cp_async_wait<1>();   // V of this tile (K of the next one may still travel)
     group_sync();         // also: the half warp's P is written
-    if (!masked) {
+    // keys that every row of the block sees, in fours
+    const int common = masked ? max(least_visible - key0, 0) & ~3 : kTileKeysWide;
+    {
 #pragma unroll 2
-      for (int j = 0; j < kTileKeysWide; j += 4) {
+      for (int j = 0; j < common; j += 4) {
         float4 pv[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) pv[i] = *reinterpret_cast<const float4 *>(p_s + (ty * 4 + i) * L::kPPitch + j);
@@ -321,11 +326,12 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const S
             }
           }
       }
-    } else {
+    }
+    if (masked) {
       // A key a row does not see takes no part in its product: 0 * V would turn an infinity there into a NaN.
       const int count = min(kTileKeysWide, block_visible - key0);
 #pragma unroll 1
-      for (int j = 0; j < count; ++j) {
+      for (int j = common; j < count; ++j) {
         float vv[kD / 16];
 #pragma unroll
         for (int c = 0; c < kD / 16; ++c) vv[c] = v_s[j * kD + (c / 4) * 64 + tx * 4 + c % 4];
@@ -346,10 +352,10 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const S
   cp_async_wait<0>();
   __syncthreads();
 
-  // Merge: group 1 leaves its states in its own K / V buffers, group 0 folds them in and finalizes.
-  float *state = smem + L::kGroup0 + L::kGroupFloats;   // [32][D], then m [32], l [32]
-  float *stats = state + kTileRows * kD;
-  if (group_id == 1) {
+  // Merge: the other groups leave their states in their own K / V buffers, group 0 folds them in and finalizes.
+  auto state_of = [&](int g) { return smem + L::kGroup0 + g * L::kGroupFloats; };   // [32][D], then m [32], l [32]
+  if (group_id > 0) {
+    float *state = state_of(group_id), *stats = state + kTileRows * kD;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
 #pragma unroll
@@ -363,28 +369,40 @@ __global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const S
     }
   }
   __syncthreads();
-  if (group_id == 1) return;
+  if (group_id > 0) return;
   float *out = static_cast<float *>(a.out);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = ty * 4 + i, row = row_block + r;
     if (r >= rows) continue;
-    const float m_other = stats[r], l_other = stats[kTileRows + r];
-    const float m_all = fmaxf(m_run[i], m_other);
+    float m_all = m_run[i];
+#pragma unroll
+    for (int g = 1; g < kGroups; ++g) m_all = fmaxf(m_all, state_of(g)[kTileRows * kD + r]);
     const float m_exp = (m_all == -INFINITY) ? 0.0f : m_all;
-    const float mine = exp_lp(__fsub_rn(m_run[i], m_exp)), other = exp_lp(__fsub_rn(m_other, m_exp));
-    const float l_all = __fadd_rn(__fmul_rn(l_run[i], mine), __fmul_rn(l_other, other));
+    const float mine = exp_lp(__fsub_rn(m_run[i], m_exp));
+    float l_all = __fmul_rn(l_run[i], mine), other[kGroups];
+#pragma unroll
+    for (int g = 1; g < kGroups; ++g) {
+      const float *stats = state_of(g) + kTileRows * kD;
+      other[g] = exp_lp(__fsub_rn(stats[r], m_exp));
+      l_all = __fadd_rn(l_all, __fmul_rn(stats[kTileRows + r], other[g]));
+    }
     float coefficient = __fdiv_rn(1.0f, l_all);
     if (a.zero_fully_masked && l_all == 0.0f) coefficient = 0.0f;
     float *dst = out + (a.out_token_major ? ((static_cast<size_t>(b) * a.q_len + row) * a.q_heads + h) * kD : (static_cast<size_t>(bh) * a.q_len + row) * kD);
 #pragma unroll
     for (int c = 0; c < kD / 64; ++c) {
-      const float4 o = *reinterpret_cast<const float4 *>(state + r * kD + c * 64 + tx * 4);
-      const float others[4] = {o.x, o.y, o.z, o.w};
+      float sum[4];
+#pragma unroll
+      for (int g = 1; g < kGroups; ++g) {
+        const float4 o = *reinterpret_cast<const float4 *>(state_of(g) + r * kD + c * 64 + tx * 4);
+        const float others[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sum[e] = g == 1 ? __fmul_rn(others[e], other[g]) : __fmaf_rn(others[e], other[g], sum[e]);
+      }
       uint32_t w[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        w[e] = narrow_bits(__fmul_rn(__fmaf_rn(acc[i][4 * c + e], mine, __fmul_rn(others[e], other)), coefficient), WB200_F32);
+      for (int e = 0; e < 4; ++e) w[e] = narrow_bits(__fmul_rn(__fmaf_rn(acc[i][4 * c + e], mine, sum[e]), coefficient), WB200_F32);
       *reinterpret_cast<uint4 *>(dst + c * 64 + tx * 4) = make_uint4(w[0], w[1], w[2], w[3]);
     }
     if (tx == 0) {
@@ -422,7 +440,7 @@ wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t strea
     if (st != WB200_OK) return st;
     const dim3 tiles((a.q_len + kTileRows - 1) / kTileRows, a.batch * a.q_heads);
     const bool narrow = a.head_dim == 64;
-    WB200_CUDA_CHECK(launch_dependent(narrow ? fa_f32_kernel<64> : fa_f32_kernel<128>, tiles, kGroups * kGroupThreads,
+    WB200_CUDA_CHECK(launch_dependent(narrow ? fa_f32_kernel<64> : fa_f32_kernel<128>, tiles, (narrow ? TiledSmem<64>::kGroups : TiledSmem<128>::kGroups) * kGroupThreads,
                                       narrow ? TiledSmem<64>::kBytes : TiledSmem<128>::kBytes, stream, p));
     return WB200_OK;
   }

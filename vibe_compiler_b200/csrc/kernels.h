@@ -140,21 +140,21 @@ struct PoolWindow {
 wb200_status launch_elementwise_formal(int op, int in_format, int out_format, int input_count, const uint8_t *in0, const uint8_t *in1,
                                        uint8_t *dst, const LayoutMap &in_map, const LayoutMap &out_map, uint32_t *flags_word,
                                        cudaStream_t stream, RhsBroadcast rhs = RhsBroadcast(), TileBatch tiles = TileBatch());
-// A run of formal elementwise commands over 1-D Tensor vectors of one format and element count in which every command's
-// first operand is the previous command's destination: one launch carries the value in registers from step to step and
-// still writes every step's destination. Second operands are a full vector (WB200_RHS_SAME), immediate bits
-// (WB200_RHS_SCALAR) or absent (unary; scalar = 0).
+// A run of formal elementwise commands over 1-D Tensor vectors of one format and element count: one launch, in which a
+// thread takes the same elements through every command, reads what an earlier step stored there and stores every step's
+// destination. A step's first operand is a vector, or null for the previous step's result, which stays in registers; its
+// second operand a full vector (WB200_RHS_SAME), a unit of `scalar` elements repeated (WB200_RHS_UNIT; no destination of the
+// chain overlaps it), immediate bits (WB200_RHS_SCALAR) or absent (unary; scalar = 0).
 constexpr int kMaxChainSteps = 8;
 struct ChainStep {
   int32_t op;
   uint32_t rhs_mode, scalar, reserved;
-  const uint8_t *rhs;
+  const uint8_t *lhs, *rhs;
   uint8_t *dst;
 };
 struct ElementwiseChain {
   int32_t steps, format;
   int64_t count;
-  const uint8_t *lhs;
   ChainStep step[kMaxChainSteps];
 };
 wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles = TileBatch());
@@ -289,6 +289,20 @@ struct StridedLayout {
 };
 uint64_t strided_segments(const StridedLayout &layout);
 uint64_t strided_span(const StridedLayout &layout);   // bytes from the first to one past the last byte touched
+// A copy as the kernel takes it; units of 16, 4 or 1 bytes.
+struct CopyJob {
+  const uint8_t *src;
+  uint8_t *dst;
+  StridedLayout from, to;
+  uint32_t units_per_segment, unit;
+  uint64_t total_units;
+  int64_t src_step, dst_step;   // bytes between the Tiles' sources and destinations
+};
+constexpr int kMaxCopyJobs = 4;
+wb200_status make_copy_job(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to, uint32_t tiles, int64_t src_step,
+                           int64_t dst_step, CopyJob *job);
+// Up to kMaxCopyJobs copies of one unit that do not depend on one another, for `tiles` Tiles, in one launch.
+wb200_status launch_copy_jobs(const CopyJob *jobs, int count, uint32_t tiles, cudaStream_t stream);
 // `tiles` copies at once, their sources and destinations so many bytes apart.
 wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to,
                                  cudaStream_t stream, uint32_t tiles = 1, int64_t src_step = 0, int64_t dst_step = 0);

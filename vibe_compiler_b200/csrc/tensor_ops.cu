@@ -724,7 +724,6 @@ formal_chain_kernel(const ElementwiseChain chain, int vector, uint64_t tile_stri
   pdl_launch_dependents();
   pdl_wait();
   const uint64_t tile_offset = blockIdx.z * tile_stride;
-  const uint8_t *const lhs = chain.lhs + tile_offset;
   constexpr int format = kFormat, bytes = kFormat == WB200_F32 ? 4 : 2;
   const int64_t total = chain.count, groups = (total + kPer - 1) / kPer;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -734,14 +733,17 @@ formal_chain_kernel(const ElementwiseChain chain, int vector, uint64_t tile_stri
     const int count = total - first < kPer ? static_cast<int>(total - first) : kPer;
     const bool wide = kPer == 8 && vector && count == 8;
     uint32_t value[kPer], b[kPer];
-    if (wide) {
-      if constexpr (kPer == 8) load_group8(lhs, g, bytes, value);
-    } else {
-#pragma unroll
-      for (int e = 0; e < kPer; ++e) value[e] = e < count ? load_element_bits(lhs, first + e, format) : 0u;
-    }
 #pragma unroll 1
     for (int s = 0; s < chain.steps; ++s) {
+      if (chain.step[s].lhs) {
+        const uint8_t *lhs = chain.step[s].lhs + tile_offset;
+        if (wide) {
+          if constexpr (kPer == 8) load_group8(lhs, g, bytes, value);
+        } else {
+#pragma unroll
+          for (int e = 0; e < kPer; ++e) value[e] = e < count ? load_element_bits(lhs, first + e, format) : 0u;
+        }
+      }
       const uint8_t *rhs = chain.step[s].rhs + tile_offset;   // read only where there is one
       uint8_t *dst = chain.step[s].dst + tile_offset;
       if (chain.step[s].rhs_mode == WB200_RHS_SAME) {
@@ -751,6 +753,10 @@ formal_chain_kernel(const ElementwiseChain chain, int vector, uint64_t tile_stri
 #pragma unroll
           for (int e = 0; e < kPer; ++e) b[e] = e < count ? load_element_bits(rhs, first + e, format) : 0u;
         }
+      } else if (chain.step[s].rhs_mode == WB200_RHS_UNIT) {
+#pragma unroll
+        for (int e = 0; e < kPer; ++e)   // a command has fewer than 2^32 elements
+          b[e] = e < count ? load_element_bits(rhs, static_cast<uint32_t>(first + e) % chain.step[s].scalar, format) : 0u;
       } else {
 #pragma unroll
         for (int e = 0; e < kPer; ++e) b[e] = chain.step[s].scalar;
@@ -1500,9 +1506,10 @@ wb200_status launch_elementwise_formal(int op, int in_format, int out_format, in
 wb200_status launch_elementwise_chain(const ElementwiseChain &chain, uint32_t *flags_word, cudaStream_t stream, TileBatch tiles) {
   if (chain.steps < 1 || chain.steps > kMaxChainSteps || chain.count < 1 || !is_float_format(chain.format))
     return fail(WB200_ERR_INVALID_ARGUMENT, "malformed elementwise chain");
-  uintptr_t low_bits = reinterpret_cast<uintptr_t>(chain.lhs) | (tiles.tiles > 1 ? static_cast<uintptr_t>(tiles.stride) : 0);
+  if (!chain.step[0].lhs) return fail(WB200_ERR_INVALID_ARGUMENT, "malformed elementwise chain");
+  uintptr_t low_bits = tiles.tiles > 1 ? static_cast<uintptr_t>(tiles.stride) : 0;
   for (int s = 0; s < chain.steps; ++s)
-    low_bits |= reinterpret_cast<uintptr_t>(chain.step[s].dst) | (chain.step[s].rhs_mode == WB200_RHS_SAME ? reinterpret_cast<uintptr_t>(chain.step[s].rhs) : 0);
+    low_bits |= reinterpret_cast<uintptr_t>(chain.step[s].dst) | reinterpret_cast<uintptr_t>(chain.step[s].lhs) | (chain.step[s].rhs_mode == WB200_RHS_SAME ? reinterpret_cast<uintptr_t>(chain.step[s].rhs) : 0);
   bool one_each = chain.count <= kShortVector;
   for (int s = 0; s < chain.steps; ++s) one_each |= is_function(chain.step[s].op);
   const int per = one_each ? 1 : 8, threads = one_each ? kShortThreads : kThreads;

@@ -4,22 +4,30 @@
 // (lib/Wafer/Simulator/Memory/TargetModelStridedMemory.cpp:121-152). A copy pairs payload byte p of the source
 // layout with payload byte p of the destination layout (lib/Wafer/Simulator/Kernel/TargetModelMovement.cpp:52-146).
 // HBM-bound byte work: algorithmic bytes = payload read once + written once.
+#include <algorithm>
+
 #include "kernels.h"
 #include "ptx_sm100.cuh"
 
 namespace wb200 {
 namespace {
 
-template <typename Unit>
-__global__ void __launch_bounds__(256) strided_copy_kernel(const uint8_t *src, uint8_t *dst, StridedLayout from, StridedLayout to,
-                                                            uint32_t units_per_segment, uint64_t total_units, int64_t src_step,
-                                                            int64_t dst_step) {
+// blockIdx.y = copy, blockIdx.z = Tile.
+template <int kJobs>
+struct CopyJobs {
+  CopyJob job[kJobs];
+};
+template <typename Unit, int kJobs>
+__global__ void __launch_bounds__(256) strided_copy_kernel(const __grid_constant__ CopyJobs<kJobs> jobs) {
+  const CopyJob &job = jobs.job[kJobs == 1 ? 0 : blockIdx.y];
+  const StridedLayout &from = job.from, &to = job.to;
+  const uint32_t units_per_segment = job.units_per_segment;
   pdl_launch_dependents();
   pdl_wait();
-  src += blockIdx.z * src_step;
-  dst += blockIdx.z * dst_step;
+  const uint8_t *src = job.src + blockIdx.z * job.src_step;
+  uint8_t *dst = job.dst + blockIdx.z * job.dst_step;
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < total_units; u += stride) {
+  for (uint64_t u = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < job.total_units; u += stride) {
     // a command moves at most 4 GiB, so 32-bit division is enough (64-bit division is several times slower)
     const uint32_t unit = static_cast<uint32_t>(u);
     const uint32_t segment = unit / units_per_segment;
@@ -101,27 +109,54 @@ uint64_t strided_span(const StridedLayout &layout) {
   return span;
 }
 
-wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to,
-                                 cudaStream_t stream, uint32_t tiles, int64_t src_step, int64_t dst_step) {
+wb200_status make_copy_job(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to, uint32_t tiles, int64_t src_step,
+                           int64_t dst_step, CopyJob *job) {
   if (from.inner_bytes == 0 || from.inner_bytes != to.inner_bytes)
     return fail(WB200_ERR_INVALID_ARGUMENT, "strided copy needs equal, non-zero inner byte counts");
   for (int d = 0; d < 3; ++d)
     if (from.iterations[d] == 0 || to.iterations[d] == 0) return fail(WB200_ERR_INVALID_ARGUMENT, "strided copy iteration counts must be positive");
   const uint64_t segments = strided_segments(from);
   if (segments != strided_segments(to)) return fail(WB200_ERR_INVALID_ARGUMENT, "source and destination segment counts differ");
-  const uint64_t bytes = segments * from.inner_bytes;
   // every Tile's addresses have to allow the unit
   const uintptr_t bases = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) |
                           (tiles > 1 ? static_cast<uintptr_t>(src_step) | static_cast<uintptr_t>(dst_step) : 0);
-  if (bases % 16 == 0 && layout_aligned(from, 16) && layout_aligned(to, 16)) {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint4>, dim3(grid_for(bytes / 16), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes / 16, bytes / 16, src_step, dst_step));
-  } else if (bases % 4 == 0 && layout_aligned(from, 4) && layout_aligned(to, 4)) {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint32_t>, dim3(grid_for(bytes / 4), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes / 4, bytes / 4, src_step, dst_step));
-  } else {
-    WB200_CUDA_CHECK(launch_dependent(strided_copy_kernel<uint8_t>, dim3(grid_for(bytes), 1, tiles), 256, 0, stream, src, dst, from, to, from.inner_bytes, bytes, src_step, dst_step));
-  }
-  WB200_CUDA_CHECK(cudaGetLastError());
+  const uint32_t unit = bases % 16 == 0 && layout_aligned(from, 16) && layout_aligned(to, 16) ? 16
+                        : bases % 4 == 0 && layout_aligned(from, 4) && layout_aligned(to, 4)  ? 4
+                                                                                              : 1;
+  *job = {src, dst, from, to, from.inner_bytes / unit, unit, segments * from.inner_bytes / unit, src_step, dst_step};
   return WB200_OK;
+}
+
+namespace {
+template <int kJobs>
+cudaError_t launch_copies(const CopyJob *jobs, int count, uint32_t tiles, cudaStream_t stream) {
+  CopyJobs<kJobs> args{};
+  uint64_t longest = 0;
+  for (int i = 0; i < count; ++i) {
+    args.job[i] = jobs[i];
+    longest = std::max(longest, jobs[i].total_units);
+  }
+  const dim3 grid(grid_for(longest), count, tiles);
+  if (jobs[0].unit == 16) return launch_dependent(strided_copy_kernel<uint4, kJobs>, grid, 256, 0, stream, args);
+  if (jobs[0].unit == 4) return launch_dependent(strided_copy_kernel<uint32_t, kJobs>, grid, 256, 0, stream, args);
+  return launch_dependent(strided_copy_kernel<uint8_t, kJobs>, grid, 256, 0, stream, args);
+}
+}  // namespace
+
+wb200_status launch_copy_jobs(const CopyJob *jobs, int count, uint32_t tiles, cudaStream_t stream) {
+  if (count < 1 || count > kMaxCopyJobs) return fail(WB200_ERR_INVALID_ARGUMENT, "unsupported number of copies");
+  for (int i = 1; i < count; ++i)
+    if (jobs[i].unit != jobs[0].unit) return fail(WB200_ERR_INVALID_ARGUMENT, "copies of one launch have one unit");
+  if (count == 1) WB200_CUDA_CHECK(launch_copies<1>(jobs, count, tiles, stream));
+  else WB200_CUDA_CHECK(launch_copies<kMaxCopyJobs>(jobs, count, tiles, stream));
+  return WB200_OK;
+}
+
+wb200_status launch_strided_copy(const uint8_t *src, const StridedLayout &from, uint8_t *dst, const StridedLayout &to,
+                                 cudaStream_t stream, uint32_t tiles, int64_t src_step, int64_t dst_step) {
+  CopyJob job;
+  const wb200_status st = make_copy_job(src, from, dst, to, tiles, src_step, dst_step, &job);
+  return st != WB200_OK ? st : launch_copy_jobs(&job, 1, tiles, stream);
 }
 
 wb200_status launch_fill(uint8_t *dst, uint32_t value_bits, uint64_t count, int element_bytes, cudaStream_t stream, TileBatch tiles) {

@@ -633,9 +633,8 @@ struct PreparedSend {
 // Elementwise commands of one Tile that are held back while the following command may extend them into one fused launch.
 struct PendingChain {
   ElementwiseChain chain{};                 // device pointers; chain.steps == 0 when nothing is pending
-  uint64_t bytes = 0, lhs_address = 0;
-  uint64_t rhs_address[kMaxChainSteps] = {0}, dst_address[kMaxChainSteps] = {0};
-  bool rhs_vector[kMaxChainSteps] = {false};
+  uint64_t lhs_address[kMaxChainSteps] = {0}, rhs_address[kMaxChainSteps] = {0}, dst_address[kMaxChainSteps] = {0};
+  uint64_t rhs_bytes[kMaxChainSteps] = {0};   // 0: no second vector
   uint64_t first_args[8] = {0};             // the first command as issued: a chain that stays one command long runs unfused
   uint32_t first_operation = 0;
   int first_command = 0;
@@ -651,8 +650,19 @@ struct PendingRun {
   int first_command = 0;
 };
 
+// DMA commands of one Tile that are held back while the following command may join them in one launch: the loads of a block's
+// operands follow one another, and a launch of a few KiB costs its start.
+struct PendingCopies {
+  int count = 0;
+  CopyJob job[kMaxCopyJobs];
+  // what each reads and writes, as (image, first byte, last byte + 1)
+  const void *source_image[kMaxCopyJobs], *destination_image[kMaxCopyJobs];
+  uint64_t source[kMaxCopyJobs][2], destination[kMaxCopyJobs][2];
+};
+
 struct TileState {
   PendingChain chain;
+  PendingCopies copies;
   PendingRun run;
   std::vector<uint64_t> regs;
   int block = 0, previous = -1;
@@ -1009,9 +1019,51 @@ wb200_status flush_run(wb200_tile_program *program, int tile_index) {
   return st;
 }
 
-// Launches what the Tile holds back (a command run or an elementwise chain, never both): one fused kernel for two or
-// more commands, the ordinary kernel for one.
+// Launches the Tile's held-back DMA commands.
+wb200_status flush_copies(wb200_tile_program *program, int tile_index) {
+  PendingCopies &pending = program->state[tile_index].copies;
+  if (pending.count == 0) return WB200_OK;
+  DeviceGuard guard(program->backend->device);
+  wb200_spm_image &spm = program->spm[tile_index];
+  const wb200_status st = launch_copy_jobs(pending.job, pending.count, spm.batch.tiles, spm.work_stream());
+  program->backend->launches += 1;
+  program->stats.gpu_launches += pending.count;   // counted per command
+  pending.count = 0;
+  return st;
+}
+
+// Holds a DMA command back, behind those already held if neither depends on the other. Validation has passed.
+wb200_status defer_copy(wb200_tile_program *program, int tile_index, wb200_spm_image *from_image, uint64_t source, const StridedLayout &from,
+                        wb200_spm_image *to_image, uint64_t destination, const StridedLayout &to, int64_t ddr_step) {
+  PendingCopies &pending = program->state[tile_index].copies;
+  const wb200_spm_image &spm = program->spm[tile_index];
+  const int64_t image_step = static_cast<int64_t>(spm.batch.stride);
+  CopyJob job;
+  wb200_status st = make_copy_job(from_image->device + (source - from_image->base), from, to_image->device + (destination - to_image->base), to,
+                                  spm.batch.tiles, from_image == &spm ? image_step : ddr_step, to_image == &spm ? image_step : ddr_step, &job);
+  if (st != WB200_OK) return st;
+  const uint64_t reads[2] = {source, source + strided_span(from)}, writes[2] = {destination, destination + strided_span(to)};
+  auto touch = [](const void *a, const uint64_t x[2], const void *b, const uint64_t y[2]) { return a == b && x[0] < y[1] && y[0] < x[1]; };
+  bool joins = pending.count < kMaxCopyJobs;
+  for (int i = 0; joins && i < pending.count; ++i)
+    joins = pending.job[i].unit == job.unit && !touch(to_image, writes, pending.source_image[i], pending.source[i]) &&
+            !touch(to_image, writes, pending.destination_image[i], pending.destination[i]) &&
+            !touch(from_image, reads, pending.destination_image[i], pending.destination[i]);
+  // Several Tiles: what one Tile's command writes to DDR may be what another one's reads, so loads and stores do not mix.
+  for (int i = 0; joins && i < pending.count; ++i) joins = (pending.destination_image[i] == &spm) == (to_image == &spm);
+  if (!joins && (st = flush_copies(program, tile_index)) != WB200_OK) return st;
+  const int i = pending.count++;
+  pending.job[i] = job;
+  pending.source_image[i] = from_image;
+  pending.destination_image[i] = to_image;
+  for (int e = 0; e < 2; ++e) { pending.source[i][e] = reads[e]; pending.destination[i][e] = writes[e]; }
+  return WB200_OK;
+}
+
+// Launches what the Tile holds back (copies, a command run or an elementwise chain, one of them at a time): one fused kernel
+// for two or more commands, the ordinary kernel for one.
 wb200_status flush_chain(wb200_tile_program *program, int tile_index) {
+  if (wb200_status copy_status = flush_copies(program, tile_index)) return copy_status;
   if (wb200_status run_status = flush_run(program, tile_index)) return run_status;
   PendingChain &pending = program->state[tile_index].chain;
   if (pending.chain.steps == 0) return WB200_OK;
@@ -1028,38 +1080,39 @@ wb200_status flush_chain(wb200_tile_program *program, int tile_index) {
   return st;
 }
 
-// Two equally long byte ranges may both take part in a chain when they coincide or do not touch: a thread of the fused
-// kernel owns the same elements of every vector, so only a shifted overlap would cross threads.
-bool ranges_compatible(uint64_t x, uint64_t y, uint64_t bytes) { return x == y || x + bytes <= y || y + bytes <= x; }
+// May a chain store to [destination, + bytes) and read [address, + read)? Equally long ranges, when they coincide or do not
+// touch: a thread of the fused kernel owns the same elements of every vector, so only a shifted overlap would cross threads.
+// A repeated unit, which is shorter, is read by all threads and must not be stored to.
+bool ranges_compatible(uint64_t destination, uint64_t bytes, uint64_t address, uint64_t read) {
+  return (destination == address && read == bytes) || destination + bytes <= address || address + read <= destination;
+}
 
-// Holds an arithmetic / function elementwise command back as a chain step, extending the pending chain when the
-// command's first operand is the pending chain's last destination. Validation has already passed.
+// Holds an arithmetic / function elementwise command back as a chain step, extending the pending chain when the command has
+// its format and length and nothing that either stores is read by other threads. Validation has already passed.
 wb200_status defer_elementwise(wb200_tile_program *program, int tile_index, int command, uint32_t operation, const uint64_t *a) {
   PendingChain &pending = program->state[tile_index].chain;
   wb200_spm_image *spm = &program->spm[tile_index];
   const bool unary = command == kElementwiseUnary;
-  const bool rhs_vector = !unary && a[6] == 0;
   const uint64_t lhs = a[0], rhs = unary ? 0 : a[1], destination = unary ? a[1] : a[2], count = unary ? a[2] : a[3], format = unary ? a[3] : a[4];
-  const uint64_t bytes = count * (format_bits(static_cast<int>(format)) / 8);
+  const uint64_t element = format_bits(static_cast<int>(format)) / 8, bytes = count * element;
+  const bool rhs_vector = !unary && a[6] == 0;
+  // a unit as long as the vector is an ordinary second operand (so is a longer one, of which the first elements are read)
+  const bool unit = rhs_vector && a[5] != 0 && a[5] < count;
+  const uint64_t rhs_bytes = !rhs_vector ? 0 : unit ? a[5] * element : bytes;
   wb200_status st;
-  bool extend = pending.chain.steps > 0 && pending.chain.steps < kMaxChainSteps && pending.chain.format == static_cast<int32_t>(format) &&
-                pending.chain.count == static_cast<int64_t>(count) && lhs == pending.dst_address[pending.chain.steps - 1];
-  if (extend) {
-    extend = ranges_compatible(destination, pending.lhs_address, bytes) && (!rhs_vector || ranges_compatible(destination, rhs, bytes));
-    for (int s = 0; extend && s < pending.chain.steps; ++s)
-      extend = ranges_compatible(destination, pending.dst_address[s], bytes) &&
-               (!pending.rhs_vector[s] || ranges_compatible(destination, pending.rhs_address[s], bytes)) &&
-               (!rhs_vector || ranges_compatible(rhs, pending.dst_address[s], bytes));
-  }
+  const bool alone = !ranges_compatible(destination, bytes, lhs, bytes) || (rhs_vector && !ranges_compatible(destination, bytes, rhs, rhs_bytes));
+  bool extend = !alone && pending.chain.steps > 0 && pending.chain.steps < kMaxChainSteps && pending.chain.format == static_cast<int32_t>(format) &&
+                pending.chain.count == static_cast<int64_t>(count);
+  for (int s = 0; extend && s < pending.chain.steps; ++s)
+    extend = ranges_compatible(destination, bytes, pending.lhs_address[s], bytes) && ranges_compatible(destination, bytes, pending.dst_address[s], bytes) &&
+             (!pending.rhs_bytes[s] || ranges_compatible(destination, bytes, pending.rhs_address[s], pending.rhs_bytes[s])) &&
+             ranges_compatible(pending.dst_address[s], bytes, lhs, bytes) &&
+             (!rhs_vector || ranges_compatible(pending.dst_address[s], bytes, rhs, rhs_bytes));
   if (!extend) {
     if ((st = flush_chain(program, tile_index)) != WB200_OK) return st;
-    if (!ranges_compatible(destination, lhs, bytes) || (rhs_vector && !ranges_compatible(destination, rhs, bytes)))
-      return issue_elementwise(program, spm, command, operation, a, true);   // shifted in-place command: never part of a chain
+    if (alone) return issue_elementwise(program, spm, command, operation, a, true);   // shifted in-place command: never part of a chain
     pending.chain.format = static_cast<int32_t>(format);
     pending.chain.count = static_cast<int64_t>(count);
-    pending.chain.lhs = spm->device + (lhs - spm->base);
-    pending.bytes = bytes;
-    pending.lhs_address = lhs;
     pending.first_command = command;
     pending.first_operation = operation;
     for (int i = 0; i < 8; ++i) pending.first_args[i] = a[i];
@@ -1067,13 +1120,15 @@ wb200_status defer_elementwise(wb200_tile_program *program, int tile_index, int 
   const int s = pending.chain.steps++;
   ChainStep &step = pending.chain.step[s];
   step.op = static_cast<int32_t>(operation);
-  step.rhs_mode = rhs_vector ? WB200_RHS_SAME : WB200_RHS_SCALAR;
-  step.scalar = unary ? 0u : static_cast<uint32_t>(rhs);
+  step.rhs_mode = unit ? WB200_RHS_UNIT : rhs_vector ? WB200_RHS_SAME : WB200_RHS_SCALAR;
+  step.scalar = unary ? 0u : unit ? static_cast<uint32_t>(a[5]) : static_cast<uint32_t>(rhs);
   step.reserved = 0;
+  step.lhs = s > 0 && lhs == pending.dst_address[s - 1] ? nullptr : spm->device + (lhs - spm->base);
   step.rhs = rhs_vector ? spm->device + (rhs - spm->base) : nullptr;
   step.dst = spm->device + (destination - spm->base);
-  pending.rhs_vector[s] = rhs_vector;
+  pending.lhs_address[s] = lhs;
   pending.rhs_address[s] = rhs_vector ? rhs : 0;
+  pending.rhs_bytes[s] = rhs_bytes;
   pending.dst_address[s] = destination;
   return WB200_OK;
 }
@@ -1148,7 +1203,11 @@ wb200_status execute_call(wb200_tile_program *program, int tile_index, const Ins
   const bool runs = program->execute && program->fuse_chains && program->fuse_runs;
   // Held-back commands precede this one, unless it may join them: a GEMM or a reduction joins (or opens) a command run,
   // an elementwise command joins an open run or the elementwise chain.
-  if (!elementwise && !(run_starter && runs && tile.run.run.count > 0) && (st = flush_chain(program, tile_index)) != WB200_OK) return st;
+  const bool dma = inst.command == kRdma || inst.command == kWdma;
+  if (elementwise && (st = flush_copies(program, tile_index)) != WB200_OK) return st;
+  const bool holds_copies_only = tile.copies.count > 0;   // then nothing else is held back
+  if (!elementwise && !(dma && holds_copies_only) && !(run_starter && runs && tile.run.run.count > 0) &&
+      (st = flush_chain(program, tile_index)) != WB200_OK) return st;
   switch (inst.command) {
     case kNccJoin:
       if (a[0] == 0 || (a[0] & ~0xFull)) return program_error(program, tile_index, "NCC join mask is empty or outside the worker domain");
@@ -1255,8 +1314,13 @@ wb200_status execute_call(wb200_tile_program *program, int tile_index, const Ins
       program->stats.movement_commands += 1;
       program->stats.bytes_moved += a[2];
       const int64_t ddr_step = spm->batch.tiles > 1 ? program->ddr_steps[program->next_ddr_step++] : 0;
-      if (inst.command == kRdma) return enqueue_image_copy(ddr, a[0], strided, spm, a[1], flat, program->execute, &program->stats.gpu_launches, ddr_step);
-      return enqueue_image_copy(spm, a[0], flat, ddr, a[1], strided, program->execute, &program->stats.gpu_launches, ddr_step);
+      const bool load = inst.command == kRdma;
+      wb200_spm_image *from_image = load ? ddr : spm, *to_image = load ? spm : ddr;
+      const StridedLayout &from = load ? strided : flat, &to = load ? flat : strided;
+      if (!program->execute || !program->fuse_chains)
+        return enqueue_image_copy(from_image, a[0], from, to_image, a[1], to, program->execute, &program->stats.gpu_launches, ddr_step);
+      if ((st = enqueue_image_copy(from_image, a[0], from, to_image, a[1], to, false, nullptr)) != WB200_OK) return st;   // validation only
+      return defer_copy(program, tile_index, from_image, a[0], from, to_image, a[1], to, ddr_step);
     }
     case kGatherScatter: {
       // (source, destination, byte_count, inner_bytes, src strides[3], src iterations[3], dst strides[3], dst iterations[3])
@@ -1290,8 +1354,9 @@ wb200_status execute_call(wb200_tile_program *program, int tile_index, const Ins
       }
       const uint32_t op = inst.operation;
       const bool arithmetic = op == WB200_EW_MAX || op == WB200_EW_MIN || op == WB200_EW_ADD || op == WB200_EW_SUB || op == WB200_EW_MUL;
-      // same-index or immediate second operands only; relations, logic and the repeated-unit / grouped forms run unfused
-      const bool chainable = unary ? op != WB200_EW_LOGIC_NOT : (full && arithmetic && (a[6] != 0 || (a[5] == 0 && a[7] == 0)));
+      // same-index, repeated-unit or immediate second operands; relations, logic and the grouped form run unfused
+      const bool chainable = is_float_format(static_cast<int>(format)) &&
+                             (unary ? op != WB200_EW_LOGIC_NOT : (full && arithmetic && (a[6] != 0 || a[7] == 0)));
       if (chainable) return defer_elementwise(program, tile_index, inst.command, op, a);
       if ((st = flush_chain(program, tile_index)) != WB200_OK) return st;
       return issue_elementwise(program, spm, inst.command, op, a, true);

@@ -205,11 +205,13 @@ gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const int block_bytes = kColBytes + plan.row_bytes;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int kb = 0; kb < k_blocks; kb += 2) {
-        if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_word)) break;
+    // The whole warp walks the loop and one elected lane issues: in a loop that a single lane walks every copy costs about 150
+    // clocks of issue (16 x 6144 x 4096 13.2 -> 11.7 us, 8 x 4096 x 14336 38.2 -> 31.9).
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int kb = 0; kb < k_blocks; kb += 2) {
+      if (!__all_sync(0xffffffffu, mbar_wait(empty_bar(stage), phase ^ 1u, abort_word))) break;
+      if (elect_one_sync()) {
         const int blocks = min(2, k_blocks - kb);
         mbar_arrive_expect_tx(full_bar(stage), blocks * block_bytes);
         for (int half = 0; half < blocks; ++half) {
@@ -217,20 +219,21 @@ gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const uint32_t a_dst = b_dst + kColBytes;
           const int k0 = (kb + half) * kBK;
           if constexpr (kBMn) {
-            tma_load_2d(b_dst, &tmap_b, full_bar(stage), col0, k0);                // box {64 n, 64 k}
+            tma_load_2d(b_dst, &tmap_b, full_bar(stage), col0, k0);              // box {64 n, 64 k}
             if constexpr (kCols == 128) tma_load_2d(b_dst + 8192, &tmap_b, full_bar(stage), col0 + 64, k0);
           } else {
-            tma_load_2d(b_dst, &tmap_b, full_bar(stage), k0, col0);                // box {64 k, kCols n}
+            tma_load_2d(b_dst, &tmap_b, full_bar(stage), k0, col0);              // box {64 k, kCols n}
           }
           if constexpr (kAMn) {
-            for (int i = 0; i * 8192 < plan.row_bytes; ++i)                        // box {64 m, 64 k}
+            for (int i = 0; i * 8192 < plan.row_bytes; ++i)                    // box {64 m, 64 k}
               tma_load_2d(a_dst + i * 8192, &tmap_a, full_bar(stage), row0 + 64 * i, k0);
           } else {
-            tma_load_2d(a_dst, &tmap_a, full_bar(stage), k0, row0);                // box {64 k, tile_rows m}
+            tma_load_2d(a_dst, &tmap_a, full_bar(stage), k0, row0);              // box {64 k, tile_rows m}
           }
         }
-        if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
       }
+      __syncwarp();
+      if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
     }
   } else if (warp == 1) {
     const uint32_t idesc = umma_idesc_f16(kCols, plan.tile_rows, kBf16, kBMn, kAMn);

@@ -45,3 +45,18 @@ def test_rows_do_not_depend_on_the_batch(backend, epilogue, out_dtype, m, n, k):
     torch.cuda.synchronize()
     backend.poll()
     assert torch.equal(part.view(torch.uint8), whole[:m].contiguous().view(torch.uint8))
+
+
+@pytest.mark.parametrize("k", [1016, 1024, 1032, 1088, 1096, 1152, 1216, 1280, 1288, 2056, 4096])
+@pytest.mark.parametrize("rt", [False, True])
+@pytest.mark.parametrize("m,n", [(8, 72), (16, 192)])
+def test_stages_of_four_blocks_are_exact_on_integers(backend, m, n, k, rt):
+    # Rings of at least eight stages are walked four 64-element blocks of K at a time: whole and ragged last stages and last
+    # blocks. Sums of products of small integers are exact in f32, so the result is.
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    a = torch.randint(-4, 5, (m, k), device="cuda", generator=gen).bfloat16()
+    b = torch.randint(-4, 5, (n, k) if rt else (k, n), device="cuda", generator=gen).bfloat16()
+    out = backend.gemm_epilogue(a, b, rhs_transposed=rt, out_dtype=torch.float32)
+    torch.cuda.synchronize()
+    backend.poll()
+    assert torch.equal(out.double(), a.double() @ (b.double().T if rt else b.double()))

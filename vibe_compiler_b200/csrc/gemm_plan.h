@@ -16,6 +16,7 @@ struct TilePlan {
   int tile_cols;    // output columns per tile: 64 or 128
   int tile_rows;    // output rows per tile: a multiple of 16 up to 256
   int stages;       // TMA ring; a stage holds two 64-element blocks of K
+  int wide;         // 1: two stages serve as one of four blocks
   int row_bytes;    // bytes of A per block of K
   int tmem_cols;
 };
@@ -38,15 +39,19 @@ inline TilePlan make_tile(int tile_cols, int tile_rows, const GemmUmmaArgs &a, i
   // the ring is also the accumulator's staging area; more stages than blocks of K would stay empty
   const int need = std::max({ceil_div(a.k, 2 * kBK), ceil_div(tile_rows * tile_cols * 4, stage), 2});
   plan.stages = std::min({(alone ? kTileSmemAlone : kTileSmemShared) / stage, kMaxTileStages, need});
+  // A stage costs the issuing warp about 310 clocks besides its products (the wait, descriptors, election, commit), which take
+  // 28 clocks each at 64 columns: four blocks of K to a stage where at least four such stages fit.
+  plan.wide = plan.stages >= 8;
+  if (plan.wide) plan.stages &= ~1;
   plan.tmem_cols = 32;
   while (plan.tmem_cols < tile_rows) plan.tmem_cols *= 2;
   return plan;
 }
 
 // Estimated clocks of a launch of either kernel; the cheaper one runs. Measured at 1.9 GHz with cold caches (both sides in
-// us, the launch on an idle stream included, so more than the 13.2 that 16 x 6144 x 4096 takes among other launches): a block of
-// 64 of K costs a CTA four instructions of about 75 clocks however few rows or columns they cover, or its products, or its
-// operand bytes at about 52 per clock, whichever is more; a pair of CTAs needs about 650 clocks for the same block of a
+// us, the launch on an idle stream included): a block of 64 of K costs a CTA about 300 clocks however few rows or columns it
+// covers (measured with a slower loader and two blocks to a stage; about 190 now with four, which moves no line between the
+// kernels that was measured), or its products, or its operand bytes at about 52 per clock, whichever is more; a pair of CTAs needs about 650 clocks for the same block of a
 // 256 x 256 tile. Rows x columns x K: 16 x 6144 x 4096 pair 31 / tile 19, 128 x 4096 x 4096 30 / 20, 512 x 4096 x 4096 32 / 28,
 // 1024 x 1024 x 8192 49 / 34, 8192 x 256 x 2048 24 / 22; the pairs win once their tiles fill the SMs: 1000 x 6144 x 4096
 // 54 / 68, 512 x 28672 x 4096 101 / 165.

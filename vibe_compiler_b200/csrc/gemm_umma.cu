@@ -112,10 +112,10 @@ __device__ __forceinline__ void epilogue_chunk(const GemmUmmaParams &p, uint32_t
 // on padding, and B is streamed by as many SMs as the columns give. K is not split: every element is one ascending chain
 // of products whatever the number of rows, so a row's bits do not depend on the batch it travels in.
 // The accumulator goes through shared memory to the epilogue, 8 columns of one row per thread.
-// Bound at few rows by the issue of instructions that each cover 2 or 4 KiB of B (about 75 clocks apiece, measured the same
-// for 64 and 128 columns and for 16 to 64 rows), hence 64-column tiles: twice as many SMs stream B. A stage holds two
-// blocks of K so that its barriers cost half as much (16 x 6144 x 4096: 15.9 -> 13.2 us, 8 x 4096 x 14336: 47 -> 37 us).
-// 16 x 6144 x 4096 bf16 in all: 29.7 us as one 128 x 256 tile per CTA (24 CTAs), 13.2 us now.
+// Bound at few rows by the bytes of B, hence 64-column tiles: twice as many SMs stream them. The products themselves take 28
+// clocks each (64 columns x 16 rows); what a stage costs besides, about 310 clocks, is why a stage holds two blocks of K, or four
+// where the ring stays long enough (make_tile): 16 x 6144 x 4096 15.9 us with one, 11.7 with two, 11.2 with four; 8 x 4096 x
+// 14336 31.8 -> 23.1 with four, 8 x 4096 x 4096 11.2 -> 8.9. As one 128 x 256 tile per CTA the first took 29.7.
 // Epilogue of 8 accumulator columns [col, col + 8) of one row; col + 8 <= n.
 __device__ __forceinline__ void epilogue_row8(const GemmUmmaParams &p, float (&v)[8], int row, int col) {
   if (p.epilogue == WB200_EPI_SWIGLU) {
@@ -203,19 +203,20 @@ gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const int k_blocks = (p.k + kBK - 1) / kBK;
   constexpr int kColBytes = kCols * kBK * 2;   // bytes of B per stage
   const int block_bytes = kColBytes + plan.row_bytes;
+  const int per_stage = plan.wide ? 4 : 2, stages = plan.wide ? plan.stages / 2 : plan.stages;   // blocks of K, stages
 
   if (warp == 0) {
     // The whole warp walks the loop and one elected lane issues: in a loop that a single lane walks every copy costs about 150
-    // clocks of issue (16 x 6144 x 4096 13.2 -> 11.7 us, 8 x 4096 x 14336 38.2 -> 31.9).
+    // clocks of issue (16 x 6144 x 4096 13.2 -> 11.7 us, 8 x 4096 x 14336 38.2 -> 31.8, stages of two blocks).
     int stage = 0;
     uint32_t phase = 0;
-    for (int kb = 0; kb < k_blocks; kb += 2) {
+    for (int kb = 0; kb < k_blocks; kb += per_stage) {
       if (!__all_sync(0xffffffffu, mbar_wait(empty_bar(stage), phase ^ 1u, abort_word))) break;
       if (elect_one_sync()) {
-        const int blocks = min(2, k_blocks - kb);
+        const int blocks = min(per_stage, k_blocks - kb);
         mbar_arrive_expect_tx(full_bar(stage), blocks * block_bytes);
         for (int half = 0; half < blocks; ++half) {
-          const uint32_t b_dst = smem_base + (2 * stage + half) * block_bytes;
+          const uint32_t b_dst = smem_base + (per_stage * stage + half) * block_bytes;
           const uint32_t a_dst = b_dst + kColBytes;
           const int k0 = (kb + half) * kBK;
           if constexpr (kBMn) {
@@ -233,17 +234,17 @@ gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
       }
       __syncwarp();
-      if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
+      if (++stage == stages) { stage = 0; phase ^= 1u; }
     }
   } else if (warp == 1) {
     const uint32_t idesc = umma_idesc_f16(kCols, plan.tile_rows, kBf16, kBMn, kAMn);
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (int kb = 0; kb < k_blocks; kb += 2) {
+    for (int kb = 0; kb < k_blocks; kb += per_stage) {
       if (!mbar_wait(full_bar(stage), phase, abort_word)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t b_src = smem_base + 2 * stage * block_bytes;
+      const uint32_t b_src = smem_base + per_stage * stage * block_bytes;
       const uint32_t a_src = b_src + kColBytes;
       const uint64_t bdesc = kBMn ? umma_desc_mnmajor(b_src, 8192) : umma_desc_kmajor(b_src);
       const uint64_t adesc = kAMn ? umma_desc_mnmajor(a_src, 8192) : umma_desc_kmajor(a_src);
@@ -253,15 +254,19 @@ gemm_umma_tile_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
         for (int ks = 0; ks < kBK / 16; ++ks)
           umma_f16_ss(tmem_base, bdesc + ks * b_step, adesc + ks * a_step, idesc, (kb | ks) != 0 ? 1u : 0u);
-        if (kb + 1 < k_blocks) {
+        const int blocks = min(per_stage, k_blocks - kb);
 #pragma unroll
-          for (int ks = 0; ks < kBK / 16; ++ks)
-            umma_f16_ss(tmem_base, bdesc + next + ks * b_step, adesc + next + ks * a_step, idesc, 1u);
+        for (int block = 1; block < 4; ++block) {
+          if (block < blocks) {
+#pragma unroll
+            for (int ks = 0; ks < kBK / 16; ++ks)
+              umma_f16_ss(tmem_base, bdesc + block * next + ks * b_step, adesc + block * next + ks * a_step, idesc, 1u);
+          }
         }
         umma_commit(empty_bar(stage));
       }
       __syncwarp();
-      if (++stage == plan.stages) { stage = 0; phase ^= 1u; }
+      if (++stage == stages) { stage = 0; phase ^= 1u; }
     }
     if (ok && elect_one_sync()) umma_commit(acc_bar);
     __syncwarp();

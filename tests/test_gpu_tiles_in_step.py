@@ -58,3 +58,24 @@ def test_tiles_in_step_match_the_tiles_alone(backend, tiles, count, gap, differ)
         for _, one in singles:
             flags |= one["numeric_flags"]
         assert stats["numeric_flags"] == flags
+
+
+def test_stores_of_two_steps_keep_their_order(backend):
+    # Tile t stores to slot 2t and then to slot 1 + t: apart for Tile 0, one slot for Tile 1, whose second store has to win.
+    tiles, size = 3, 1 << 16
+    flat = f"i32 {size}, i32 {size}, i32 0, i32 0, i32 0, i32 1, i32 1, i32 1, i32 5, i32 0"
+
+    def module(t):
+        call = "  call void @wafer_tx81_"
+        rows = [f'!{{i64 {i}, !"external-{kind}", i64 0, !"", !"f32", !"tensor", i64 {slots * size}, i64 {slots * size // 4}, '
+                f'!"{access}-only", i64 {slots * size // 4}, i64 0}}' for i, (kind, slots, access) in enumerate((("input", 6, "read"), ("output", 5, "write")))]
+        body = [f"  %a = add i64 %0, {2 * t * size}", f"  %b = add i64 %a, {size}", f"  %first = add i64 %1, {2 * t * size}",
+                f"  %second = add i64 %1, {(1 + t) * size}", f"{call}rdma(i64 %a, i64 0, {flat})", f"{call}rdma(i64 %b, i64 {size}, {flat})",
+                f"{call}wdma(i64 0, i64 %first, {flat})", f"{call}wdma(i64 {size}, i64 %second, {flat})", "  ret void"]
+        return ("define void @entry(i64 %0, i64 %1) {\n" + "\n".join(body) + "\n}\n!wafer.target.tile_id = !{!2}\n"
+                f"!wafer.target.entry_arguments = !{{!10, !11}}\n!2 = !{{i64 {t}}}\n" + "\n".join(f"!{10 + i} = {row}" for i, row in enumerate(rows)) + "\n")
+    program = TileProgram([module(t) for t in range(tiles)], backend, spm_bytes=2 * size)
+    for seed in range(3):
+        slots = np.random.default_rng(seed).standard_normal((6, size // 4)).astype(np.float32)
+        (out,), _ = program.run([slots.reshape(-1)])
+        assert np.array_equal(out.view(np.float32).reshape(5, -1), slots[[0, 1, 3, 5, 4]])

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "command_io.h"
+#include "replay_rules.h"
 
 namespace wb200 {
 namespace {
@@ -655,9 +656,7 @@ struct PendingRun {
 struct PendingCopies {
   int count = 0;
   CopyJob job[kMaxCopyJobs];
-  // what each reads and writes, as (image, first byte, last byte + 1)
-  const void *source_image[kMaxCopyJobs], *destination_image[kMaxCopyJobs];
-  uint64_t source[kMaxCopyJobs][2], destination[kMaxCopyJobs][2];
+  ReplayCopy rule[kMaxCopyJobs];
 };
 
 struct TileState {
@@ -1042,21 +1041,15 @@ wb200_status defer_copy(wb200_tile_program *program, int tile_index, wb200_spm_i
   wb200_status st = make_copy_job(from_image->device + (source - from_image->base), from, to_image->device + (destination - to_image->base), to,
                                   spm.batch.tiles, from_image == &spm ? image_step : ddr_step, to_image == &spm ? image_step : ddr_step, &job);
   if (st != WB200_OK) return st;
-  const uint64_t reads[2] = {source, source + strided_span(from)}, writes[2] = {destination, destination + strided_span(to)};
-  auto touch = [](const void *a, const uint64_t x[2], const void *b, const uint64_t y[2]) { return a == b && x[0] < y[1] && y[0] < x[1]; };
-  bool joins = pending.count < kMaxCopyJobs;
-  for (int i = 0; joins && i < pending.count; ++i)
-    joins = pending.job[i].unit == job.unit && !touch(to_image, writes, pending.source_image[i], pending.source[i]) &&
-            !touch(to_image, writes, pending.destination_image[i], pending.destination[i]) &&
-            !touch(from_image, reads, pending.destination_image[i], pending.destination[i]);
-  // Several Tiles: what one Tile's command writes to DDR may be what another one's reads, so loads and stores do not mix.
-  for (int i = 0; joins && i < pending.count; ++i) joins = (pending.destination_image[i] == &spm) == (to_image == &spm);
-  if (!joins && (st = flush_copies(program, tile_index)) != WB200_OK) return st;
-  const int i = pending.count++;
-  pending.job[i] = job;
-  pending.source_image[i] = from_image;
-  pending.destination_image[i] = to_image;
-  for (int e = 0; e < 2; ++e) { pending.source[i][e] = reads[e]; pending.destination[i][e] = writes[e]; }
+  const ReplayCopy copy{{from_image, source, source + strided_span(from), from_image == &spm ? 0 : ddr_step},
+                        {to_image, destination, destination + strided_span(to), to_image == &spm ? 0 : ddr_step},
+                        job.unit,
+                        to_image == &spm};
+  if ((pending.count == kMaxCopyJobs || !copies_join(pending.rule, pending.count, copy, spm.batch.tiles)) &&
+      (st = flush_copies(program, tile_index)) != WB200_OK)
+    return st;
+  pending.job[pending.count] = job;
+  pending.rule[pending.count++] = copy;
   return WB200_OK;
 }
 

@@ -616,7 +616,10 @@ typedef struct wb200_program_stats {
   uint64_t gemm_commands, movement_commands, fill_commands, transfer_commands, sync_commands;
   uint64_t gemm_fused_multiply_adds;  /* sum of m * k * n * batch */
   uint64_t bytes_moved;               /* payload bytes of DMA, gather / scatter, fill and Direct-DTE transfers */
-  uint64_t gpu_launches;              /* a launch that serves a command of several Tiles counts once per Tile */
+  /* Launches that the commands take Tile by Tile with every DMA command on its own; a fused elementwise chain or command
+   * run counts once. A launch that serves several Tiles or DMA commands counts for each of them: the kernels that ran are the
+   * difference of wb200_backend_launch_count. */
+  uint64_t gpu_launches;
   float device_ms;                    /* command stream only (CUDA events); excludes host <-> device tensor copies */
   uint32_t numeric_flags;             /* OR of the IEEE flags of all elementwise / convert / reduce / pool commands (bit 0 invalid .. bit 4 inexact) */
 } wb200_program_stats;

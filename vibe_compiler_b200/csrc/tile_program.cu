@@ -696,6 +696,7 @@ struct wb200_tile_program {
   size_t edge_events_used = 0;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};   // one captured invocation per GEMM policy
   wb200_program_stats graph_stats[2] = {};
+  uint64_t graph_launches[2] = {0, 0};             // kernels that a relaunch of the graph starts
   // Replay in step (plan_in_step): per DMA command of a Tile, the bytes between the Tiles' DDR addresses.
   std::vector<int64_t> ddr_steps;
   size_t next_ddr_step = 0;
@@ -1025,8 +1026,10 @@ wb200_status flush_copies(wb200_tile_program *program, int tile_index) {
   DeviceGuard guard(program->backend->device);
   wb200_spm_image &spm = program->spm[tile_index];
   const wb200_status st = launch_copy_jobs(pending.job, pending.count, spm.batch.tiles, spm.work_stream());
-  program->backend->launches += 1;
-  program->stats.gpu_launches += pending.count;   // counted per command
+  if (st == WB200_OK) {
+    program->backend->launches += 1;
+    program->stats.gpu_launches += pending.count;   // counted per command
+  }
   pending.count = 0;
   return st;
 }
@@ -1648,9 +1651,10 @@ wb200_status capture_in_step(wb200_tile_program *program, wb200_program_stats st
     st = WB200_ERR_CUDA;
   }
   if (graph) cudaGraphDestroy(graph);
+  program->graph_launches[policy] = backend->launches - launches_before;
+  backend->launches = launches_before;   // captured, not launched
   if (st != WB200_OK || err != cudaSuccess) {
     cudaGetLastError();
-    backend->launches = launches_before;
     return st != WB200_OK ? st : WB200_ERR_CUDA;
   }
   stats.gpu_launches = program->stats.gpu_launches * program->tiles.size();   // counted per Tile, as when they are issued Tile by Tile
@@ -1684,6 +1688,7 @@ wb200_status capture_invocation(wb200_tile_program *program) {
     program->spm[t].gemm_staging = policy == WB200_GEMM_TENSOR ? program->gemm_staging[t] : nullptr;
   }
   program->edge_events_used = 0;
+  const uint64_t launches_before = backend->launches;
   cudaEvent_t fork;
   wb200_status st = program_event(program, &fork);
   if (st != WB200_OK) return st;
@@ -1702,6 +1707,8 @@ wb200_status capture_invocation(wb200_tile_program *program) {
   }
   cudaGraph_t graph = nullptr;
   const cudaError_t end_error = cudaStreamEndCapture(origin, &graph);   // always leave capture mode
+  program->graph_launches[policy] = backend->launches - launches_before;
+  backend->launches = launches_before;   // captured, not launched
   if (st == WB200_OK && err != cudaSuccess) st = fail(WB200_ERR_CUDA, std::string("capturing the invocation: ") + cudaGetErrorString(err));
   if (st == WB200_OK && end_error != cudaSuccess) st = fail(WB200_ERR_CUDA, std::string("ending the capture: ") + cudaGetErrorString(end_error));
   if (st != WB200_OK) {
@@ -1892,7 +1899,7 @@ wb200_status wb200_tile_program_run(wb200_tile_program *program, const void *con
   if (concurrent) {
     WB200_CUDA_CHECK(cudaGraphLaunch(program->graph[gemm_policy], stream));
     program->stats = program->graph_stats[gemm_policy];
-    backend->launches += program->stats.gpu_launches;
+    backend->launches += program->graph_launches[gemm_policy];
   } else {
     for (wb200_spm_image &image : program->spm) { image.stream = nullptr; image.staging = nullptr; image.gemm_staging = nullptr; }
     st = run_all_tiles(program);

@@ -59,10 +59,12 @@ constexpr int kBlockM = 64, kBlockN = 64, kPanelK = 16;
 // rhs along n - instead of eight 2-byte loads with eight addresses.
 // One 64 x 64 output tile by 256 threads (`tid` 0 .. 255) through the caller's two shared-memory panels. Every thread of
 // the block must make the call (it contains block barriers); threads with `active` false only take part in the barriers,
-// which lets a larger block work on several tiles side by side, each 256-thread group with panels of its own.
+// which lets a larger block work on several tiles side by side, each 256-thread group with panels of its own. `shift`: bytes
+// behind the given operands at which the caller's lie (a parameter of its own: a shifted copy of the arguments does not fit the
+// registers).
 template <bool kResolved, bool kSeparable, bool kWide>
 __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int batch, int row0, int col0, int tid, bool active,
-                                                 float (*lhs_panel)[kBlockM + 4], float (*rhs_panel)[kBlockN + 4]) {
+                                                 float (*lhs_panel)[kBlockM + 4], float (*rhs_panel)[kBlockN + 4], uint64_t shift = 0) {
   const int tx = tid & 15, ty = tid >> 4;
   const int m_extent = active ? a.m : 0, n_extent = active ? a.n : 0;   // an inactive thread finds every element out of range
   float acc[4][4];   // outputs (row0 + ty * 4 + i, col0 + tx * 4 + j)
@@ -99,7 +101,7 @@ __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int ba
       if (wide_lhs) {
         const int k = k0 + wide_off;
         if (row0 + wide_row < m_extent && k < a.k)
-          raw = *reinterpret_cast<const uint4 *>(a.lhs + (wide_fixed + col_part(a.lhs_map, k)) * 2);
+          raw = *reinterpret_cast<const uint4 *>(a.lhs + shift + (wide_fixed + col_part(a.lhs_map, k)) * 2);
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -109,7 +111,7 @@ __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int ba
       } else {
         const int k = k0 + wide_row;
         if (col0 + wide_off < n_extent && k < a.k)
-          raw = *reinterpret_cast<const uint4 *>(a.rhs + (wide_fixed + row_part(a.rhs_map, batch, a.k, k, a.n)) * 2);
+          raw = *reinterpret_cast<const uint4 *>(a.rhs + shift + (wide_fixed + row_part(a.rhs_map, batch, a.k, k, a.n)) * 2);
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
         float4 lo, hi;
         lo.x = widen_bits(w[0] & 0xffffu, a.in_format); lo.y = widen_bits(w[0] >> 16, a.in_format);
@@ -129,7 +131,7 @@ __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int ba
           if (kSeparable) at = l_fixed[e] + (a.lhs_transposed ? row_part(a.lhs_map, batch, a.k, k, a.m) : col_part(a.lhs_map, k));
           else at = a.lhs_transposed ? operand_index<kResolved>(a.lhs_map, batch, a.k, k, a.m, row0 + l_r[e])
                                      : operand_index<kResolved>(a.lhs_map, batch, a.m, row0 + l_r[e], a.k, k);
-          value = widen_bits(load_element_bits(a.lhs, at, a.in_format), a.in_format);
+          value = widen_bits(load_element_bits(a.lhs + shift, at, a.in_format), a.in_format);
         }
         lhs_panel[l_kk[e]][l_r[e]] = value;
       }
@@ -142,7 +144,7 @@ __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int ba
           if (kSeparable) at = r_fixed[e] + (a.rhs_transposed ? col_part(a.rhs_map, k) : row_part(a.rhs_map, batch, a.k, k, a.n));
           else at = a.rhs_transposed ? operand_index<kResolved>(a.rhs_map, batch, a.n, col0 + r_c[e], a.k, k)
                                      : operand_index<kResolved>(a.rhs_map, batch, a.k, k, a.n, col0 + r_c[e]);
-          value = widen_bits(load_element_bits(a.rhs, at, a.in_format), a.in_format);
+          value = widen_bits(load_element_bits(a.rhs + shift, at, a.in_format), a.in_format);
         }
         rhs_panel[r_kk[e]][r_c[e]] = value;
       }
@@ -167,8 +169,8 @@ __device__ __forceinline__ void gemm_formal_tile(const GemmFormalArgs &a, int ba
       const int row = row0 + ty * 4 + i, col = col0 + tx * 4 + j;
       if (row < m_extent && col < n_extent) {
         float value = acc[i][j];
-        if (a.has_psum) value = __fadd_rn(value, __uint_as_float(load_element_bits(a.psum, operand_index<kResolved>(a.psum_map, batch, a.m, row, a.n, col), WB200_F32)));
-        store_element_bits(a.dst, operand_index<kResolved>(a.dst_map, batch, a.m, row, a.n, col), a.out_format, narrow_bits(value, a.out_format));
+        if (a.has_psum) value = __fadd_rn(value, __uint_as_float(load_element_bits(a.psum + shift, operand_index<kResolved>(a.psum_map, batch, a.m, row, a.n, col), WB200_F32)));
+        store_element_bits(a.dst + shift, operand_index<kResolved>(a.dst_map, batch, a.m, row, a.n, col), a.out_format, narrow_bits(value, a.out_format));
       }
     }
 }

@@ -1583,14 +1583,28 @@ cudaError_t reset_numeric_words(wb200_tile_program *program, cudaStream_t stream
   return err != cudaSuccess ? err : cudaMemsetAsync(program->numeric_words + 2, 0xff, 8, stream);
 }
 
+// Commands whose kernels have a form for several Tiles (for some sizes and policies only, which their launch tells).
+bool serves_several_tiles(int command) {
+  switch (command) {
+    case kRdma: case kWdma: case kNccJoin: case kGatherScatter: case kMemset: case kElementwiseUnary: case kElementwiseBinary:
+    case kElementwiseLogic: case kReduce: case kGemm: case kGemmOriented: return true;
+    default: return false;
+  }
+}
+
 // Tiles that run one program on different data (same commands on the same scratch-pad addresses, no transfers between
 // Tiles, and DDR addresses that differ by one step from Tile to Tile) can be replayed in step: one launch per command for
 // all Tiles. With a branch of the graph per Tile every node costs its start, about a third of a microsecond: 16 Tiles x 107
 // launches of an attention program took 569 us a run that way and 419 in step, where one Tile alone takes 340.
-// Interprets all Tiles without executing; *stats are the invocation's (but for the launches).
+// Interprets all Tiles without executing; *stats are the invocation's (but for the launches). Modules that name a command
+// without a form for several Tiles are not interpreted: their capture does that once more.
 bool plan_in_step(wb200_tile_program *program, wb200_program_stats *stats) {
   const size_t tiles = program->tiles.size();
   if (tiles < 2 || tiles > 65535 || program->fuse_runs) return false;
+  for (const Module &module : program->tiles)
+    for (const Block &block : module.blocks)
+      for (const Inst &inst : block.insts)
+        if (inst.op == Op::Call && !serves_several_tiles(inst.command)) return false;
   std::vector<wb200_program_command> trace;
   program->execute = false;
   program->trace = &trace;
@@ -1604,14 +1618,7 @@ bool plan_in_step(wb200_tile_program *program, wb200_program_stats *stats) {
   program->ddr_steps.clear();
   for (size_t i = 0; i < length; ++i) {
     const wb200_program_command &first = trace[i];
-    int ddr_arg = -1;
-    switch (first.kind) {
-      case kRdma: ddr_arg = 0; break;
-      case kWdma: ddr_arg = 1; break;
-      case kNccJoin: case kGatherScatter: case kMemset: case kElementwiseUnary: case kElementwiseBinary: case kElementwiseLogic:
-      case kReduce: case kGemm: case kGemmOriented: break;
-      default: return false;
-    }
+    const int ddr_arg = first.kind == kRdma ? 0 : first.kind == kWdma ? 1 : -1;
     int64_t step = 0;
     for (size_t t = 0; t < tiles; ++t) {
       const wb200_program_command &other = trace[t * length + i];

@@ -76,6 +76,15 @@ def test_tiles_in_step_match_the_tiles_alone(backend, tiles, count, gap, differ)
         assert stats["numeric_flags"] == flags
 
 
+def test_fusing_off_issues_every_command_of_every_tile(backend, monkeypatch):
+    monkeypatch.setenv("WB200_REPLAY_FUSE", "0")   # read when a program is loaded
+    program = TileProgram([_module(t, 3, 192, 0x3f000000, 0) for t in range(3)], backend, spm_bytes=1 << 20)
+    values = np.random.default_rng(1).standard_normal(3 * 192).astype(np.float32)
+    for _ in range(2):
+        (_, stats), launched = _launched(backend, lambda: program.run([values]))
+        assert launched == stats["gpu_launches"] == stats["commands"] - stats["sync_commands"]
+
+
 def test_stores_of_two_steps_keep_their_order(backend):
     # Tile t stores to slot 2t and then to slot 1 + t: apart for Tile 0, one slot for Tile 1, whose second store has to win.
     tiles, size = 3, 1 << 16

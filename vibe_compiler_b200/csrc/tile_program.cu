@@ -1600,7 +1600,7 @@ bool serves_several_tiles(int command) {
 // without a form for several Tiles are not interpreted: their capture does that once more.
 bool plan_in_step(wb200_tile_program *program, wb200_program_stats *stats) {
   const size_t tiles = program->tiles.size();
-  if (tiles < 2 || tiles > 65535 || program->fuse_runs) return false;
+  if (tiles < 2 || tiles > 65535 || !program->fuse_chains || program->fuse_runs) return false;
   for (const Module &module : program->tiles)
     for (const Block &block : module.blocks)
       for (const Inst &inst : block.insts)

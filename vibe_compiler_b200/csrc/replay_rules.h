@@ -40,4 +40,37 @@ inline bool copies_join(const ReplayCopy *held, int count, const ReplayCopy &nex
   return true;
 }
 
+// The operands of an elementwise command of `bytes` bytes of results. The second one has rhs_bytes: none or an immediate (0), a
+// vector like the first (`bytes`) or a shorter unit that is repeated.
+struct ChainOperands {
+  uint64_t lhs, rhs, destination, bytes, rhs_bytes;
+};
+
+// May a chain store to [destination, + bytes) and read [address, + read)? Equally long ranges, when they coincide or do not
+// touch: a thread of the fused kernel owns the same elements of every vector, so only a shifted overlap would cross threads.
+// A repeated unit, which is shorter, is read by all threads and must not be stored to.
+inline bool ranges_compatible(uint64_t destination, uint64_t bytes, uint64_t address, uint64_t read) {
+  return (destination == address && read == bytes) || destination + bytes <= address || address + read <= destination;
+}
+
+// A command whose own operands rule it out of every chain.
+inline bool chain_refuses(const ChainOperands &c) {
+  return !ranges_compatible(c.destination, c.bytes, c.lhs, c.bytes) || (c.rhs_bytes && !ranges_compatible(c.destination, c.bytes, c.rhs, c.rhs_bytes));
+}
+
+// May `next` follow the held commands, of its format and length, in one launch? Nothing that either stores is read, or stored
+// to, by other threads.
+inline bool chain_extends(const ChainOperands *held, int count, const ChainOperands &next) {
+  if (chain_refuses(next)) return false;
+  for (int s = 0; s < count; ++s) {
+    const ChainOperands &c = held[s];
+    if (!ranges_compatible(next.destination, next.bytes, c.lhs, c.bytes) || !ranges_compatible(next.destination, next.bytes, c.destination, c.bytes) ||
+        (c.rhs_bytes && !ranges_compatible(next.destination, next.bytes, c.rhs, c.rhs_bytes)) ||
+        !ranges_compatible(c.destination, c.bytes, next.lhs, next.bytes) ||
+        (next.rhs_bytes && !ranges_compatible(c.destination, c.bytes, next.rhs, next.rhs_bytes)))
+      return false;
+  }
+  return true;
+}
+
 }  // namespace wb200

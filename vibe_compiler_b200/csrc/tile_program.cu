@@ -634,8 +634,7 @@ struct PreparedSend {
 // Elementwise commands of one Tile that are held back while the following command may extend them into one fused launch.
 struct PendingChain {
   ElementwiseChain chain{};                 // device pointers; chain.steps == 0 when nothing is pending
-  uint64_t lhs_address[kMaxChainSteps] = {0}, rhs_address[kMaxChainSteps] = {0}, dst_address[kMaxChainSteps] = {0};
-  uint64_t rhs_bytes[kMaxChainSteps] = {0};   // 0: no second vector
+  ChainOperands operands[kMaxChainSteps] = {};
   uint64_t first_args[8] = {0};             // the first command as issued: a chain that stays one command long runs unfused
   uint32_t first_operation = 0;
   int first_command = 0;
@@ -1076,13 +1075,6 @@ wb200_status flush_chain(wb200_tile_program *program, int tile_index) {
   return st;
 }
 
-// May a chain store to [destination, + bytes) and read [address, + read)? Equally long ranges, when they coincide or do not
-// touch: a thread of the fused kernel owns the same elements of every vector, so only a shifted overlap would cross threads.
-// A repeated unit, which is shorter, is read by all threads and must not be stored to.
-bool ranges_compatible(uint64_t destination, uint64_t bytes, uint64_t address, uint64_t read) {
-  return (destination == address && read == bytes) || destination + bytes <= address || address + read <= destination;
-}
-
 // Holds an arithmetic / function elementwise command back as a chain step, extending the pending chain when the command has
 // its format and length and nothing that either stores is read by other threads. Validation has already passed.
 wb200_status defer_elementwise(wb200_tile_program *program, int tile_index, int command, uint32_t operation, const uint64_t *a) {
@@ -1094,19 +1086,13 @@ wb200_status defer_elementwise(wb200_tile_program *program, int tile_index, int 
   const bool rhs_vector = !unary && a[6] == 0;
   // a unit as long as the vector is an ordinary second operand (so is a longer one, of which the first elements are read)
   const bool unit = rhs_vector && a[5] != 0 && a[5] < count;
-  const uint64_t rhs_bytes = !rhs_vector ? 0 : unit ? a[5] * element : bytes;
+  const ChainOperands operands{lhs, rhs_vector ? rhs : 0, destination, bytes, !rhs_vector ? 0 : unit ? a[5] * element : bytes};
   wb200_status st;
-  const bool alone = !ranges_compatible(destination, bytes, lhs, bytes) || (rhs_vector && !ranges_compatible(destination, bytes, rhs, rhs_bytes));
-  bool extend = !alone && pending.chain.steps > 0 && pending.chain.steps < kMaxChainSteps && pending.chain.format == static_cast<int32_t>(format) &&
-                pending.chain.count == static_cast<int64_t>(count);
-  for (int s = 0; extend && s < pending.chain.steps; ++s)
-    extend = ranges_compatible(destination, bytes, pending.lhs_address[s], bytes) && ranges_compatible(destination, bytes, pending.dst_address[s], bytes) &&
-             (!pending.rhs_bytes[s] || ranges_compatible(destination, bytes, pending.rhs_address[s], pending.rhs_bytes[s])) &&
-             ranges_compatible(pending.dst_address[s], bytes, lhs, bytes) &&
-             (!rhs_vector || ranges_compatible(pending.dst_address[s], bytes, rhs, rhs_bytes));
+  const bool extend = pending.chain.steps > 0 && pending.chain.steps < kMaxChainSteps && pending.chain.format == static_cast<int32_t>(format) &&
+                      pending.chain.count == static_cast<int64_t>(count) && chain_extends(pending.operands, pending.chain.steps, operands);
   if (!extend) {
     if ((st = flush_chain(program, tile_index)) != WB200_OK) return st;
-    if (alone) return issue_elementwise(program, spm, command, operation, a, true);   // shifted in-place command: never part of a chain
+    if (chain_refuses(operands)) return issue_elementwise(program, spm, command, operation, a, true);   // shifted in-place command: never part of a chain
     pending.chain.format = static_cast<int32_t>(format);
     pending.chain.count = static_cast<int64_t>(count);
     pending.first_command = command;
@@ -1119,13 +1105,10 @@ wb200_status defer_elementwise(wb200_tile_program *program, int tile_index, int 
   step.rhs_mode = unit ? WB200_RHS_UNIT : rhs_vector ? WB200_RHS_SAME : WB200_RHS_SCALAR;
   step.scalar = unary ? 0u : unit ? static_cast<uint32_t>(a[5]) : static_cast<uint32_t>(rhs);
   step.reserved = 0;
-  step.lhs = s > 0 && lhs == pending.dst_address[s - 1] ? nullptr : spm->device + (lhs - spm->base);
+  step.lhs = s > 0 && lhs == pending.operands[s - 1].destination ? nullptr : spm->device + (lhs - spm->base);
   step.rhs = rhs_vector ? spm->device + (rhs - spm->base) : nullptr;
   step.dst = spm->device + (destination - spm->base);
-  pending.lhs_address[s] = lhs;
-  pending.rhs_address[s] = rhs_vector ? rhs : 0;
-  pending.rhs_bytes[s] = rhs_bytes;
-  pending.dst_address[s] = destination;
+  pending.operands[s] = operands;
   return WB200_OK;
 }
 

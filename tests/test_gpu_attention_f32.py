@@ -58,3 +58,21 @@ def test_key_tiles_over_the_groups_match_float64(backend, keys, causal):
     want = torch.softmax(scores, -1) @ v.double()
     assert helpers.max_rel_err(out.double().cpu().numpy(), want.cpu().numpy()) <= 1e-5   # the f32 bound of the path
     assert (lse.double() - torch.logsumexp(scores, -1)).abs().max().item() <= 1e-5
+
+
+@pytest.mark.parametrize("batch,heads,rows,keys", [(1, 37, 128, 129), (1, 37, 129, 129), (5, 4, 256, 257), (3, 7, 256, 257), (2, 75, 33, 500), (2, 37, 33, 65)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_either_number_of_groups_matches_float64(backend, batch, heads, rows, keys, causal):
+    # launches on both sides of the lines between two and four groups: 148 blocks of 32 rows, 20 causal heads, 128 keys
+    gen = torch.Generator(device="cuda").manual_seed(heads + keys)
+    q, k, v = (torch.randn(batch, heads, n, 64, device="cuda", generator=gen) for n in (rows, keys, keys))
+    lse = torch.empty(batch, heads, rows, device="cuda")
+    out = backend.attention_fa(q, k, v, 64 ** -0.5, causal, lse=lse, query_start=keys - rows)
+    torch.cuda.synchronize()
+    backend.poll()
+    scores = q.double() @ k.double().transpose(-1, -2) * 64 ** -0.5
+    if causal:
+        scores = scores.masked_fill(~torch.ones(rows, keys, dtype=torch.bool, device="cuda").tril(keys - rows), float("-inf"))
+    want = torch.softmax(scores, -1) @ v.double()
+    assert helpers.max_rel_err(out.double().cpu().numpy(), want.cpu().numpy()) <= 1e-5   # the f32 bound of the path
+    assert (lse.double() - torch.logsumexp(scores, -1)).abs().max().item() <= 1e-5

@@ -156,21 +156,20 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) fa_simt_kernel(const Simt
 }
 
 // ---------------------------------------------------------------- f32 storage, head_dim 64 or 128: register tiles
-// A block owns 32 query rows of one (batch, head). Its groups of 128 threads (four at head_dim 64, two at 128: what shared
-// memory holds) walk the tiles of 64 keys in turn, each with a state of its own; the states are merged once at the end. A thread holds
+// A block owns 32 query rows of one (batch, head). Its two or four groups of 128 threads (f32_groups below) walk the tiles of
+// 64 keys in turn, each with a state of its own; the states are merged once at the end. A thread holds
 // 4 rows x 4 keys of the scores (keys tx, tx + 16, ...) and 4 rows x D/16 columns of the accumulator, so 64 multiply-adds
 // follow on 8 shared-memory vectors; the 16 threads of a row are half a warp, which keeps the row statistics and P inside
 // the warp. K and V have a buffer each, refilled by cp.async as soon as the group has read it: K of the next tile travels
 // under the softmax and the PV product, V under the next scores.
 // Bound by the f32 multiply-adds (8 heads x 512 x 512 x 64: 0.27 G, 7 us at the rate of 148 SMs; 128 of them have a block)
-// and the shared-memory vectors that feed them: 73.7 us with a warp per row, 23.8 us with two groups, 22.2 us with four (16
+// and the shared-memory vectors that feed them: 73.7 us with a warp per row, 24.4 us with two groups, 22.4 us with four (16
 // warps hide more of the latency of loads, shuffles and exponentials). The warp-per-row kernel stays for other widths, 16-bit
 // storage and unaligned buffers.
 constexpr int kTileRows = 32, kTileKeysWide = 64, kGroupThreads = 128;
 
-template <int kD>
+template <int kD, int kGroups>
 struct TiledSmem {
-  static constexpr int kGroups = kD == 64 ? 4 : 2;   // as many as shared memory holds
   static constexpr int kKPitch = kD + 4;   // rows 16 bytes apart modulo the banks: eight lanes' vectors cover all banks
   static constexpr int kPPitch = kTileKeysWide + 4;
   static constexpr int kQ = 0;
@@ -181,10 +180,9 @@ struct TiledSmem {
   static constexpr size_t kBytes = (kGroup0 + kGroups * kGroupFloats) * sizeof(float);
 };
 
-template <int kD>
-__global__ void __launch_bounds__(TiledSmem<kD>::kGroups * kGroupThreads) fa_f32_kernel(const SimtParams p) {
-  using L = TiledSmem<kD>;
-  constexpr int kGroups = L::kGroups;
+template <int kD, int kGroups>
+__global__ void __launch_bounds__(kGroups * kGroupThreads) fa_f32_kernel(const SimtParams p) {
+  using L = TiledSmem<kD, kGroups>;
   const AttentionArgs &a = p.a;
   extern __shared__ float4 smem_vectors[];
   float *smem = reinterpret_cast<float *>(smem_vectors);
@@ -414,6 +412,18 @@ __global__ void __launch_bounds__(TiledSmem<kD>::kGroups * kGroupThreads) fa_f32
   }
 }
 
+// Key groups of a block. At head_dim 64 shared memory holds four, one block to an SM, or two blocks of two groups each; at 128
+// two. Four are for blocks that would have an SM to themselves with two: where no more blocks than SMs are launched, and on
+// causal requests of few heads, whose long blocks outlast the short ones beside them. With no more than two tiles of keys half
+// of them would idle. us with two / four groups, 64 columns, heads x rows (= keys): all keys 8 x 512 24.4 / 22.4, 8 x 1024
+// 74.6 / 78.9, 32 x 256 21.4 / 24.6, 512 x 128 75.0 / 105.8, 512 x 512 1016 / 1169; causal 10 x 512 37.4 / 23.9, 8 x 1024
+// 72.0 / 62.0, 20 x 1024 125 / 121, 20 x 512 42.8 / 42.6, 24 x 1024 139 / 140, 32 x 256 21.4 / 23.6. A row's bits depend on the
+// number of groups, and so on the heads and sequences beside it.
+int f32_groups(const AttentionArgs &a, int kv_visible, int64_t blocks) {
+  const bool few = blocks <= 148 || (a.causal && a.batch * static_cast<int64_t>(a.q_heads) <= 20);
+  return a.head_dim == 64 && kv_visible > 2 * kTileKeysWide && few ? 4 : 2;
+}
+
 }  // namespace
 
 wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t stream) {
@@ -433,15 +443,17 @@ wb200_status launch_attention_fa_simt(const AttentionArgs &a, cudaStream_t strea
   if (a.format == WB200_F32 && aligned && (a.head_dim == 64 || a.head_dim == 128)) {
     static PerDeviceOnce attributes;
     const wb200_status st = attributes.run([]() -> wb200_status {
-      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<64>::kBytes)));
-      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<128>::kBytes)));
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<64, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<64, 2>::kBytes)));
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<64, 4>::kBytes)));
+      WB200_CUDA_CHECK(cudaFuncSetAttribute(fa_f32_kernel<128, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(TiledSmem<128, 2>::kBytes)));
       return WB200_OK;
     });
     if (st != WB200_OK) return st;
     const dim3 tiles((a.q_len + kTileRows - 1) / kTileRows, a.batch * a.q_heads);
-    const bool narrow = a.head_dim == 64;
-    WB200_CUDA_CHECK(launch_dependent(narrow ? fa_f32_kernel<64> : fa_f32_kernel<128>, tiles, (narrow ? TiledSmem<64>::kGroups : TiledSmem<128>::kGroups) * kGroupThreads,
-                                      narrow ? TiledSmem<64>::kBytes : TiledSmem<128>::kBytes, stream, p));
+    const int groups = f32_groups(a, p.kv_visible, static_cast<int64_t>(tiles.x) * tiles.y);
+    if (a.head_dim == 128) WB200_CUDA_CHECK(launch_dependent(fa_f32_kernel<128, 2>, tiles, 2 * kGroupThreads, TiledSmem<128, 2>::kBytes, stream, p));
+    else if (groups == 4) WB200_CUDA_CHECK(launch_dependent(fa_f32_kernel<64, 4>, tiles, 4 * kGroupThreads, TiledSmem<64, 4>::kBytes, stream, p));
+    else WB200_CUDA_CHECK(launch_dependent(fa_f32_kernel<64, 2>, tiles, 2 * kGroupThreads, TiledSmem<64, 2>::kBytes, stream, p));
     return WB200_OK;
   }
   dim3 grid((a.q_len + kWarpsPerBlock - 1) / kWarpsPerBlock, a.batch * a.q_heads);

@@ -316,8 +316,9 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         }
         __syncwarp();
       };
-      // PV over the keys of one published part of P.
-      auto issue_pv_part = [&](auto tile_tag, auto part_tag, int v_slot, bool accumulate) {
+      // PV over the keys of one published part of P. Behind the item's last product o_done completes, once per item: the
+      // softmax warps wait for it once per item, and a barrier that could be a phase further would fool their parity.
+      auto issue_pv_part = [&](auto tile_tag, auto part_tag, int v_slot, bool accumulate, bool last) {
         constexpr int t = decltype(tile_tag)::value;
         constexpr int part = decltype(part_tag)::value;
         const uint64_t v_desc = ring_v_desc + static_cast<uint32_t>(v_slot) * kSlotStep;
@@ -329,7 +330,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             const uint32_t acc = (accumulate || ks != 0) ? 1u : 0u;
             umma_f16_ts(d_tmem, tmem_base + kColS0 + t * 128 + ks * 8, bdesc, idesc_o, acc);
           }
-          if (part == kPParts - 1) umma_commit(o_done(t));
+          if (part == kPParts - 1 && last) umma_commit(o_done(t));
         }
         __syncwarp();
       };
@@ -375,10 +376,10 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
             if (j < n_tiles) {
               if (!mbar_wait_spin(p_part(t, 0), (tile_base + j) & 1u, abort_word)) { ok = false; return; }
               tc_fence_after();
-              issue_pv_part(tile_tag, std::integral_constant<int, 0>{}, v_slot, j > 0);
+              issue_pv_part(tile_tag, std::integral_constant<int, 0>{}, v_slot, j > 0, false);
               if (!mbar_wait_spin(p_part(t, 1), (tile_base + j) & 1u, abort_word)) { ok = false; return; }
               tc_fence_after();
-              issue_pv_part(tile_tag, std::integral_constant<int, 1>{}, v_slot, j > 0);
+              issue_pv_part(tile_tag, std::integral_constant<int, 1>{}, v_slot, j > 0, j + 1 == n_tiles);
             }
             if (j + 1 < n_tiles) {
               if (!k_ready) {
@@ -411,7 +412,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     const uint32_t lane_sel = static_cast<uint32_t>(quarter * 32) << 16;
     const uint32_t s_addr = tmem_base + lane_sel + kColS0 + t * 128;
     const uint32_t o_addr = tmem_base + lane_sel + kColO0 + t * 128;
-    uint32_t tiles_done = 0;   // S tiles of this Q-tile slot consumed so far, over all items (barrier parities)
+    uint32_t tiles_done = 0, items_done = 0;   // S tiles and items with any of this Q-tile slot so far (barrier parities)
     bool ok = true;
     const uint32_t out_stage = smem_base + L::kOutOff + (warp - 4) * kOutStageBytes;
     int next_id = fa_item_id(p, 0);
@@ -531,7 +532,7 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
     }
 
     // Finalize: out = acc * (1 / l), rounded once to the storage type.
-    if (ok && my_tiles > 0) ok = mbar_wait(o_done(t), (tiles_done - 1) & 1u, abort_word, 114 + t);
+    if (ok && my_tiles > 0) ok = mbar_wait(o_done(t), items_done++ & 1u, abort_word, 114 + t);
     if (ok && row_base + t * kTileM < p.q_len) {
       tc_fence_after();
       float coefficient = 1.0f / l_run;

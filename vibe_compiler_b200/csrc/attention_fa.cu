@@ -579,7 +579,8 @@ fa_umma_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) {
-          if (warp_row < p.q_len) tma_store_4d(&tmap_out, out_stage, half * 64, warp_row, where.h, where.b);
+          if (warp_row < p.q_len)
+            tma_store_4d(&tmap_out, out_stage, half * 64, p.out_token_major ? where.h : warp_row, p.out_token_major ? warp_row : where.h, where.b);
           tma_store_commit();
         }
       }
@@ -726,12 +727,11 @@ wb200_status launch_attention_fa_umma(const AttentionArgs &a, int sm_count, int 
                       row_pitch * a.kv_len, 64, kTileN);
   if (st != WB200_OK) return st;
 
-  // The output as [batch][head][row][column], whichever of head and row is the outer one in memory.
+  // The output, its dimensions in the order they have in memory; a store covers 32 rows of one head.
   CUtensorMap to;
-  const uint64_t out_row_pitch = a.out_token_major ? row_pitch * a.q_heads : row_pitch;
-  const uint64_t out_head_pitch = a.out_token_major ? row_pitch : row_pitch * a.q_len;
-  st = encode_tmap_4d(&to, a.out, a.format, kHd, a.q_len, a.q_heads, a.batch, out_row_pitch, out_head_pitch,
-                      row_pitch * a.q_len * a.q_heads, 64, 32);
+  const uint64_t rows = a.q_len, heads = a.q_heads, batch = a.batch;
+  st = a.out_token_major ? encode_tmap_4d_dense(&to, a.out, a.format, {kHd, heads, rows, batch}, {64, 1, 32, 1})
+                         : encode_tmap_4d_dense(&to, a.out, a.format, {kHd, rows, heads, batch}, {64, 32, 1, 1});
   if (st != WB200_OK) return st;
 
   FaParams p;

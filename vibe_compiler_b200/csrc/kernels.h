@@ -80,10 +80,8 @@ wb200_status encode_tmap_2d(CUtensorMap *map, const void *base, int format, uint
 wb200_status encode_tmap_3d(CUtensorMap *map, const void *base, int format, uint64_t inner,
                             uint64_t outer, uint64_t batch, uint64_t row_pitch_bytes,
                             uint64_t batch_pitch_bytes, uint32_t box_inner, uint32_t box_outer);
-// Four dimensions with a pitch each, in any order in memory; the box is {box_inner, box_extent1, 1, 1}.
-wb200_status encode_tmap_4d(CUtensorMap *map, const void *base, int format, uint64_t inner, uint64_t extent1, uint64_t extent2,
-                            uint64_t extent3, uint64_t pitch1_bytes, uint64_t pitch2_bytes, uint64_t pitch3_bytes, uint32_t box_inner,
-                            uint32_t box_extent1);
+// Four dimensions without gaps, innermost first, and the box in the same order.
+wb200_status encode_tmap_4d_dense(CUtensorMap *map, const void *base, int format, const uint64_t (&extents)[4], const uint32_t (&box_extents)[4]);
 
 // All of [host, host + bytes) lies in one page-locked allocation or registration, which the device addresses alike.
 bool page_locked_range(const void *host, size_t bytes);

@@ -32,9 +32,12 @@ wb200_status encode(CUtensorMap *map, const void *base, int format, uint32_t ran
     return fail(WB200_ERR_UNSUPPORTED, "TMA maps are built for 16-bit float formats only");
   if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0)
     return fail(WB200_ERR_INVALID_ARGUMENT, "TMA base address must be 16-byte aligned");
-  for (uint32_t i = 0; i + 1 < rank; ++i)
+  for (uint32_t i = 0; i + 1 < rank; ++i) {
     if (strides[i] % 16 != 0)
       return fail(WB200_ERR_INVALID_ARGUMENT, "TMA strides must be multiples of 16 bytes");
+    if (strides[i] < dims[i] * (i > 0 ? strides[i - 1] : 2))
+      return fail(WB200_ERR_INVALID_ARGUMENT, "TMA dimensions are given innermost first, each stride spanning the dimension before it");
+  }
   const cuuint32_t element_strides[4] = {1, 1, 1, 1};
   CUresult result =
       fn(map, format == WB200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
@@ -66,12 +69,15 @@ wb200_status encode_tmap_3d(CUtensorMap *map, const void *base, int format, uint
   return encode(map, base, format, 3, dims, strides, box);
 }
 
-wb200_status encode_tmap_4d(CUtensorMap *map, const void *base, int format, uint64_t inner, uint64_t extent1, uint64_t extent2,
-                            uint64_t extent3, uint64_t pitch1_bytes, uint64_t pitch2_bytes, uint64_t pitch3_bytes, uint32_t box_inner,
-                            uint32_t box_extent1) {
-  const cuuint64_t dims[4] = {inner, extent1, extent2, extent3};
-  const cuuint64_t strides[3] = {pitch1_bytes, pitch2_bytes, pitch3_bytes};
-  const cuuint32_t box[4] = {box_inner, box_extent1, 1, 1};
+wb200_status encode_tmap_4d_dense(CUtensorMap *map, const void *base, int format, const uint64_t (&extents)[4], const uint32_t (&box_extents)[4]) {
+  cuuint64_t dims[4], strides[3], pitch = 2;
+  cuuint32_t box[4];
+  for (int i = 0; i < 4; ++i) {
+    dims[i] = extents[i];
+    box[i] = box_extents[i];
+    pitch *= extents[i];
+    if (i < 3) strides[i] = pitch;
+  }
   return encode(map, base, format, 4, dims, strides, box);
 }
 

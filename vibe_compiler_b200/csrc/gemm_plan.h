@@ -50,9 +50,9 @@ inline TilePlan make_tile(int tile_cols, int tile_rows, const GemmUmmaArgs &a, i
 
 // Estimated clocks of a launch of either kernel; the cheaper one runs. Measured at 1.9 GHz with cold caches (both sides in
 // us, the launch on an idle stream included): a block of 64 of K costs a CTA about 300 clocks however few rows or columns it
-// covers (measured with a slower loader and two blocks to a stage; about 190 now with four, which moves no line between the
-// kernels that was measured), or its products, or its operand bytes at about 52 per clock, whichever is more; a pair of CTAs needs about 650 clocks for the same block of a
-// 256 x 256 tile. Rows x columns x K: 16 x 6144 x 4096 pair 31 / tile 19, 128 x 4096 x 4096 30 / 20, 512 x 4096 x 4096 32 / 28,
+// covers (two blocks to a stage; about 190 with four, but none of 19861 shapes drawn from 8 to 8192 rows, 256 to 28672 columns and
+// 256 to 14336 of K is cut differently with that), or its products, or its operand bytes at about 52 per clock, whichever is
+// more; a pair of CTAs needs about 650 clocks for the same block of a 256 x 256 tile. Rows x columns x K: 16 x 6144 x 4096 pair 31 / tile 19, 128 x 4096 x 4096 30 / 20, 512 x 4096 x 4096 32 / 28,
 // 1024 x 1024 x 8192 49 / 34, 8192 x 256 x 2048 24 / 22; the pairs win once their tiles fill the SMs: 1000 x 6144 x 4096
 // 54 / 68, 512 x 28672 x 4096 101 / 165.
 inline double tile_cost(const TilePlan &plan, const GemmUmmaArgs &a, int sm_count) {

@@ -635,7 +635,7 @@ def main():
                                  "value": c1_flops / (c1_ms * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": c1_ms,
                                  "max_rel_err_vs_f64": float((o1.double() - ref1).abs().max() / ref1.abs().max()),
                                  "roofline": {"bound": "latency", "achieved": c1_flops / (c1_ms * 1e-3) / 1e12, "peak": None, "unit": "TFLOP/s", "frac": None,
-                                              "traffic": None, "note": "0.5 GFLOP on 1024 warps: launch and dependency latency, not a pipe, bound it"}}
+                                              "traffic": None, "note": "0.5 GFLOP on 128 blocks of 16 warps: neither a pipe nor HBM bounds it"}}
         del flush1
     if not args.skip_extras:
         ga = gb = gout = fk = fv = None

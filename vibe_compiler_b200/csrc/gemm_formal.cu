@@ -139,8 +139,9 @@ bool small_gemm(const GemmFormalArgs &a, SmallGemm *g) {
 constexpr int64_t kFewTiles = 16;
 
 // Register-tiled variant for commands with at least 32 x 32 outputs: one gemm_formal_tile (gemm_formal.cuh) per block.
-// kTiles: blockIdx.z is the Tile (one matrix each), not the matrix of a batch. Forms of their own, because commands of one Tile
-// lose 3 to 4 % (NCx 1024 x 1024 x 1024 bf16 868 -> 903 us a call) to the registers that the shift takes.
+// kTiles: blockIdx.z is the Tile (one matrix each), not the matrix of a batch. The Tile's shift goes down as an argument, zero for
+// commands of one Tile: a shifted copy of the argument struct made three of the four forms spill (NCx 1024 x 1024 x 1024 bf16
+// 868 -> 903 us a call).
 template <bool kResolved, bool kSeparable, bool kWide, bool kTiles>
 __global__ void __launch_bounds__(256, 4) gemm_formal_tiled_kernel(const __grid_constant__ FormalParams p) {
   // rows padded by four floats: the k-fastest staging stores of an untransposed lhs (transposed rhs) spread over the

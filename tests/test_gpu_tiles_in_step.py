@@ -9,7 +9,7 @@ from vibe_compiler_b200.tile_program import TileProgram
 pytestmark = pytest.mark.gpu
 
 
-def _module(tile, tiles, count, scale, gap):
+def _module(tile, tiles, count, scale, gap, tail=()):
     """`count` f32 values of the Tile (4 * gap bytes between the Tiles' blocks): a constant vector, a product, exp, a repeated
     unit, a reduction over [1, 1, count / 64, 64], a 64 x 64 x 64 product when there are enough values, a transposing copy, an
     elementwise command by itself when there are more values than a launch for several Tiles takes."""
@@ -33,6 +33,7 @@ def _module(tile, tiles, count, scale, gap):
         body += [f"{call}elementwise_max(i64 {moved}, i64 {moved}, i64 {moved}, {vector}, {same})", f"{call}ncc_join(i32 1)"]
     body += [f"{call}reduce_sum(i64 {moved}, i64 {folded}, i32 1, i32 1, i32 1, i32 {count // 64}, i32 64, i32 5, i32 1)",
              f"{call}wdma(i64 {moved}, i64 %out, i32 {4 * count}, i32 {4 * count}, {flat})", f"{call}wdma(i64 {folded}, i64 %sums, i32 256, i32 256, {flat})"]
+    body += tail
     total = tiles * (count + gap)
     rows = [f'!{{i64 0, !"external-input", i64 0, !"", !"f32", !"tensor", i64 {4 * total}, i64 {total}, !"read-only", i64 {total}, i64 0}}',
             f'!{{i64 1, !"external-output", i64 0, !"", !"f32", !"tensor", i64 {4 * total}, i64 {total}, !"write-only", i64 {total}, i64 0}}',
@@ -74,6 +75,24 @@ def test_tiles_in_step_match_the_tiles_alone(backend, tiles, count, gap, differ)
         for _, one in singles:
             flags |= one["numeric_flags"]
         assert stats["numeric_flags"] == flags
+
+
+_CONVERT = "  call void @wafer_tx81_convert_fp32_bf16(i64 0, i64 65536, i32 64, i32 0, i32 0, i32 1)"
+
+
+@pytest.mark.parametrize("tail,in_step", [([], True), ([_CONVERT], False),
+                                          (["  %never = icmp eq i64 %0, 0", "  br i1 %never, label %dead, label %live", "dead:", _CONVERT,
+                                            "  br label %live", "live:"], True)])
+def test_what_is_issued_decides(backend, tail, in_step):
+    # a convert has no form for several Tiles; one that a branch never reaches does not count
+    program = TileProgram([_module(t, 4, 64, 0x3f000000, 0, tail) for t in range(4)], backend, spm_bytes=1 << 20)
+    one = TileProgram([_module(0, 1, 64, 0x3f000000, 0, tail)], backend, spm_bytes=1 << 20)
+    values = np.random.default_rng(2).standard_normal(4 * 64).astype(np.float32)
+    for _ in range(2):
+        ((out, _), _), launched = _launched(backend, lambda: program.run([values]))
+        ((first, _), _), alone = _launched(backend, lambda: one.run([values[:64]]))
+        assert launched == (alone if in_step else 4 * alone)
+        assert np.array_equal(out.reshape(-1)[:64], first.reshape(-1))
 
 
 def test_fusing_off_issues_every_command_of_every_tile(backend, monkeypatch):

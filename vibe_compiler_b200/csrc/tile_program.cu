@@ -1579,24 +1579,27 @@ bool serves_several_tiles(int command) {
 // Tiles, and DDR addresses that differ by one step from Tile to Tile) can be replayed in step: one launch per command for
 // all Tiles. With a branch of the graph per Tile every node costs its start, about a third of a microsecond: 16 Tiles x 107
 // launches of an attention program took 569 us a run that way and 419 in step, where one Tile alone takes 340.
-// Interprets all Tiles without executing; *stats are the invocation's (but for the launches). Modules that name a command
-// without a form for several Tiles are not interpreted: their capture does that once more.
+// Interprets all Tiles without executing; *stats are the invocation's (but for the launches). Tile 0 by itself goes first: where
+// it waits for another Tile, or issues a command without a form for several, the others are not interpreted for nothing.
 bool plan_in_step(wb200_tile_program *program, wb200_program_stats *stats) {
   const size_t tiles = program->tiles.size();
   if (tiles < 2 || tiles > 65535 || !program->fuse_chains || program->fuse_runs) return false;
-  for (const Module &module : program->tiles)
-    for (const Block &block : module.blocks)
-      for (const Inst &inst : block.insts)
-        if (inst.op == Op::Call && !serves_several_tiles(inst.command)) return false;
   std::vector<wb200_program_command> trace;
-  program->execute = false;
-  program->trace = &trace;
-  const wb200_status st = run_all_tiles(program);
-  program->trace = nullptr;
-  program->execute = true;
-  if (st != WB200_OK || trace.size() % tiles != 0) return false;
+  auto interpret = [&](size_t count) {
+    trace.clear();
+    program->execute = false;
+    program->trace = &trace;
+    const wb200_status st = run_tiles(program, count);
+    program->trace = nullptr;
+    program->execute = true;
+    return st == WB200_OK;
+  };
+  if (!interpret(1)) return false;
+  for (const wb200_program_command &command : trace)
+    if (!serves_several_tiles(static_cast<int>(command.kind))) return false;
+  const size_t length = trace.size();
+  if (!interpret(tiles) || trace.size() != length * tiles) return false;
   *stats = program->stats;
-  const size_t length = trace.size() / tiles;
   // without transfers no Tile waits, so the Tiles' records follow one another
   program->ddr_steps.clear();
   for (size_t i = 0; i < length; ++i) {
